@@ -1,0 +1,40 @@
+"""The radix sort's passes at the edges of their digit widths and tiles (4096 keys), heavily skewed ids, and the
+permutation kernel's record widths; bit-exact against numpy."""
+import numpy as np
+import pytest
+import torch
+
+from flexspmv_b200.python_wrapper.dynamic_replace_submodule import permute_edges, sort_edges_by_row
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [2, 3, 128, 129, 255, 256, 257, 65535, 65536, 65537, (1 << 24) + 1])
+@pytest.mark.parametrize("n", [1, 31, 33, 4095, 4096, 4097, 3 * 4096 + 5])
+def test_digit_widths_and_tiles(rows, n):
+    rng = np.random.default_rng(rows + n)
+    draws = {"uniform": rng.integers(0, rows, n), "last": np.full(n, rows - 1), "two": rng.choice([0, rows - 1], n),
+             "descending": np.sort(rng.integers(0, rows, n))[::-1]}
+    for what, ids in draws.items():
+        for dtype in (np.int32, np.int64):
+            perm, crow = sort_edges_by_row(torch.from_numpy(ids.astype(dtype)).cuda(), rows)
+            assert np.array_equal(perm.cpu().numpy(), np.argsort(ids, kind="stable").astype(np.int32)), what
+            want = np.searchsorted(np.sort(ids), np.arange(rows + 1)) if rows < 1 << 20 else None
+            if want is not None:
+                assert np.array_equal(crow.cpu().numpy(), want), what
+            else:
+                got = crow.cpu().numpy()
+                assert got[0] == 0 and got[-1] == n and np.array_equal(np.diff(got).nonzero()[0], np.unique(ids)), what
+
+
+@pytest.mark.parametrize("words", [1, 2, 3, 4, 6])
+@pytest.mark.parametrize("n", [1, 1023, 1025, 70001])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_permute_record_widths(words, n, offset):
+    """``offset``: the source begins one word into an allocation, so wide records are not aligned to their width."""
+    g = np.random.default_rng(n + words)
+    base = torch.from_numpy(g.integers(-2 ** 31, 2 ** 31, n * words + 1).astype(np.int32)).cuda()
+    src = base[offset:offset + n * words].view(n, words)
+    perm = torch.from_numpy(g.permutation(n).astype(np.int32)).cuda()
+    got = permute_edges(src, perm)
+    assert torch.equal(got, src[perm.long()])
