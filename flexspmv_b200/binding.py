@@ -385,6 +385,19 @@ class GraphExtension:
                   "device_status")
         return int(out.item())
 
+    def planned_whole_rows(self) -> bool:
+        """Whether the plan made last found a matrix of short rows, every tile of which holds whole rows only
+        (include/flexspmv.h, flexspmv_workspace_whole_rows).  Synchronises."""
+        if not self._plans:
+            return False
+        ws = next(reversed(self._plans.values())).ws
+        out = torch.zeros(1, dtype=torch.int32, device=ws.device)
+        with torch.cuda.device(ws.device):
+            self.lib.flexspmv_workspace_whole_rows.restype = ctypes.c_int
+            check(self.lib, self.lib.flexspmv_workspace_whole_rows(ctypes.c_void_p(ws.data_ptr()), ctypes.c_void_p(out.data_ptr()),
+                                                                   _stream_ptr()), "workspace_whole_rows")
+        return int(out.item()) == 1
+
     def check(self) -> None:
         """Waits for the work enqueued so far on every device this object planned for, then raises
         FlexSpmvError if a kernel gave up on any of its cached workspaces (a bounded wait ran out, or a

@@ -96,8 +96,8 @@ def smem_bytes(ir: GraphIR, dtype: str, block: int, ipt: int, stages: int) -> in
     per_edge, ns = _stream_bytes_per_edge(ir, vb)
     acc = max(1, sum(dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer"))
     tile = block * ipt
-    stage = 0 if direct_loads(ir, dtype) else -(-(tile * max(8, per_edge) + 32 * (ns + 1) + 16) // 128) * 128
-    fixed = 8 * stages + (32 + 4 * max(ns, 1) + 16) * stages + 4 * (block + 1) + 4 * (block // 32) \
+    stage = 0 if direct_loads(ir, dtype) else -(-(tile * max(8, per_edge) + 32 * per_edge + 32 * (ns + 1) + 16) // 128) * 128
+    fixed = 16 * 4 + (32 + 4 * max(ns, 1) + 16) * 4 + 4 * (block + 1) + 4 * (block // 32) \
         + vb * acc * (block // 32) + vb * acc * 2 + 16 + 8 * 16 + 128
     needs_row = any(s_.get("selector") == 1 and s_.get("row_identity") for s_ in ir.selector_register)
     buffers = 1   # 2 only when the kernel is built with tile pipelining (TileCfg::kPipeline)
@@ -131,7 +131,8 @@ TUNED_CONFIGS = {
     "spmv_f32": (256, 5, 2, 4),
     "spmv_i64": (256, 5, 2, 4),
     # warm / L2-flushed % of the HBM peak:
-    "spring_mass_f32": (256, 8, 2, 4, 0, 2),   # 35.5 / 31.2: 2048-item tiles hold ~228 rows of 8 edges, one per thread (batch 4: 34.9 / 31.2, batch 1 x 5 CTAs: 36.1 / 29.2, batch 8: 25)
+    # (seventh field: edges per batch in the loop over whole rows: spring_mass_f32 1 / 2 / 4: 38.9 / 40.5 / 44.3 us)
+    "spring_mass_f32": (256, 8, 2, 4, 0, 2, 1),   # 35.5 / 31.2: 2048-item tiles hold ~228 rows of 8 edges, one per thread (batch 4: 34.9 / 31.2, batch 1 x 5 CTAs: 36.1 / 29.2, batch 8: 25)
     "rusanov_f64": (256, 4, 2, 3, 0, 1),       # 33.1 / 30.9: 1024-item tiles hold 256 rows of 3 edges (batch 2: 29.4 / 27.6, batch 3: 27.3 / 25.9, batch 1 x 4 CTAs: 30.3 / 28.7)
     "swe_delta_f64": (256, 3, 2, 3, 0, 1),     # 52.7 / 45.3 with staged edge tensors ((256,4,2,3) batch 1: 48.7 / 39.8, direct: 35.3 / 32.2; heuristic (256,3,2,4) batch 2: 33.8 / 31.5)
 }
@@ -376,6 +377,14 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w("    load_edge_vals(p, t, le, e, r);")
     w("  }")
     w("  template <class Tile, class IdxT>")
+    w("  __device__ __forceinline__ static void load_edge_idx(const Tile& t, IdxT le, EReg& r) {")
+    for n_ in idx_names:
+        w(f"    r.idx_{n_} = *t.template stream<{stream_of['idx:' + n_]}, int>(le);")
+    w("    (void)t; (void)le; (void)r;")
+    w("  }")
+    w(f"  static constexpr bool kValuesStaged = {'true' if staged_values else 'false'};")
+    w(f"  static constexpr bool kStoresPerEdge = {'true' if (map_outs or inplace_targets) else 'false'};")
+    w("  template <class Tile, class IdxT>")
     w("  __device__ __forceinline__ static void load_edge_vals(const Params& p, const Tile& t, IdxT le, long long e, EReg& r) {")
     seen_e = set()
     for s_ in edge_regs_list:
@@ -601,7 +610,15 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
                           if s_.get("selector") == 1 and not s_.get("row_identity")})
     batch = next((b_ for b_ in (8, 4, 3, 2) if b_ * max(per_edge_regs, 1) <= 28), 2)
     batch = batch_override or batch
-    w(f"using Cfg = flex::TileCfg<{block}, {ipt}, {stages}, {min_ctas}, {batch}, {'true' if pipeline else 'false'}>;")
+    # the loop over whole rows reads staged values after the gathers have landed, so an edge in flight holds its gathered
+    # data and an index (batches of 8 / 6 / 4 / 3 / 2 edges on the 7-point fp64 SpMV, 512^3, at 4 CTAs per SM: 3305 / 2797 /
+    # 2602 / 2749 / 2620 us); graphs with values of their own in registers use the batch above
+    gather_words = sum(dim_of(s_["shape"]) * words for s_ in ir.selector_register
+                       if s_.get("selector") == 1 and not s_.get("row_identity"))
+    row_batch = batch if needs_row else next((b_ for b_ in (4, 2) if b_ * (gather_words + 1) <= 14), 1)
+    if len(cfg) > 6:
+        row_batch = cfg[6]       # seventh field
+    w(f"using Cfg = flex::TileCfg<{block}, {ipt}, {stages}, {min_ctas}, {batch}, {'true' if pipeline else 'false'}, {row_batch}>;")
     wb_, wi_, ws_, wm_ = tuple(_override(symbol + "_win") or TUNED_WIN_CONFIGS.get(symbol) or (block, ipt, stages, min_ctas))[:4]
     if windows:
         w(f"using CfgWin = flex::TileCfg<{wb_}, {wi_}, {ws_}, {wm_}, {batch}, false>;   // the gather-window variant of the kernel")

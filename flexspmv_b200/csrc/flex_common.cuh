@@ -46,10 +46,27 @@ struct WorkspaceHeader {
                                // ends (no row spans two CTAs of such a launch: no carries to hand over)
   uint64_t status_mirror;      // device alias of a pinned host int32 that receives a copy of `status` when a
                                // kernel raises an error (0: none); lets the host notice without a sync or a copy
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8];
+  uint64_t row_slots;          // what whole_rows_kernel counted: 32 x the longest row, over groups of 32 rows
+  int32_t whole_rows;          // 1: EVERY tile boundary sits on a row end and no row is longer than kWholeRowMax: the
+                               // tile kernel runs its loop without barriers, for any grid (-1: looked at and refused)
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 4];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
+
+#ifndef FLEX_WHOLE_ROW_MAX
+#define FLEX_WHOLE_ROW_MAX 32
+#endif
+constexpr int kWholeRowMax = FLEX_WHOLE_ROW_MAX;   // longest row of a matrix whose tiles hold whole rows only
+
+// What one tile of the tile kernel can take when a planning step moves its boundaries (in whole numbers of edges and
+// rows): its arrays hold max_edges edges, its stage stage_bytes bytes of per-edge records and row ends.
+struct TileRoom {
+  int max_edges, stage_bytes, edge_bytes, offset_bytes;
+  __host__ __device__ bool fits(long long edges, long long rows) const {
+    return edges <= max_edges && edges * edge_bytes + rows * offset_bytes <= stage_bytes;
+  }
+};
 
 // Raises `err` in the workspace header (first error wins, sticky until the workspace is planned again) and
 // copies it to the host-visible mirror when one is registered.

@@ -2,6 +2,7 @@
 // validation, status strings.  Integer-only kernels; results are bit-identical to the reference's
 // search (include/merged_spmv_kernels.cuh:19-99).
 #include <cuda_runtime.h>
+#include <stddef.h>
 
 #include "flex_common.cuh"
 
@@ -38,9 +39,10 @@ __global__ void partition_kernel(const OffsetT* __restrict__ row_offsets, long l
 // between CTAs (fence, ticket, fix-up by the last CTA).  When the part of the cut row in front of the boundary fits
 // into the tile behind it -- which has room for as many extra edges as it holds row ends -- the boundary is moved
 // back to the row's first edge instead.  All boundaries or none: the header records the grid size it was done for.
+// A tile takes at most max_edges edges and its stage room.stage_bytes bytes of records and row ends.
 template <typename OffsetT>
 __global__ void snap_cta_boundaries_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_tiles,
-                                           int grid, OffsetT* __restrict__ coords, WorkspaceHeader* h) {
+                                           int grid, const TileRoom room, OffsetT* __restrict__ coords, WorkspaceHeader* h) {
   __shared__ int s_ok;
   if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
@@ -52,7 +54,8 @@ __global__ void snap_cta_boundaries_kernel(const OffsetT* __restrict__ row_offse
     const long long begin = (long long)row_offsets[x];              // first edge of the row the boundary cuts
     const long long rows_behind = (long long)coords[2 * t + 2] - x; // row ends in the tile behind the boundary
     const long long y_before = (long long)coords[2 * t - 1];        // where the tile in front of it starts
-    if (y - begin > rows_behind || begin < y_before) s_ok = 0;
+    const long long edges_behind = (long long)coords[2 * t + 3] - begin;
+    if (y - begin > rows_behind || begin < y_before || !room.fits(edges_behind, rows_behind)) s_ok = 0;
   }
   __syncthreads();
   if (!s_ok) return;
@@ -65,16 +68,84 @@ __global__ void snap_cta_boundaries_kernel(const OffsetT* __restrict__ row_offse
 }
 
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
-                               void* d_coords, void* ws, cudaStream_t stream) {
+                               const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream) {
   if (grid < 2 || num_tiles < grid) return 0;
   if (offset_bits == 32)
-    snap_cta_boundaries_kernel<int><<<1, 256, 0, stream>>>(static_cast<const int*>(d_row_offsets), num_rows, num_tiles, grid,
+    snap_cta_boundaries_kernel<int><<<1, 256, 0, stream>>>(static_cast<const int*>(d_row_offsets), num_rows, num_tiles, grid, room,
                                                            static_cast<int*>(d_coords), static_cast<WorkspaceHeader*>(ws));
   else
     snap_cta_boundaries_kernel<long long><<<1, 256, 0, stream>>>(static_cast<const long long*>(d_row_offsets), num_rows,
-                                                                 num_tiles, grid, static_cast<long long*>(d_coords),
+                                                                 num_tiles, grid, room, static_cast<long long*>(d_coords),
                                                                  static_cast<WorkspaceHeader*>(ws));
   return (int)cudaGetLastError();
+}
+
+// One warp per tile: would every row stay whole with all tile boundaries moved back to row starts -- rows of at most
+// kWholeRowMax edges, tiles that still fit -- and how many thread-steps would one thread per row take?  Leaves
+// whole_rows = -1 when a row or a tile is too large.
+template <typename OffsetT>
+__global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
+                                                         long long num_tiles, const TileRoom room, const OffsetT* __restrict__ coords,
+                                                         WorkspaceHeader* h) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  unsigned long long slots = 0;
+  bool bad = false;
+  for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < num_tiles && !bad; t += warps) {
+    const long long x0 = (long long)coords[2 * t], x1 = (long long)coords[2 * t + 2];
+    const long long y0 = (long long)row_offsets[x0];                        // x0 == num_rows: num_edges
+    const long long y1 = (t + 1 < num_tiles) ? (long long)row_offsets[x1] : num_edges;
+    bad = !room.fits(y1 - y0, x1 - x0);
+    for (long long r0 = x0; r0 < x1; r0 += 32) {
+      const long long r = r0 + lane;
+      long long len = 0;
+      if (r < x1) len = (long long)row_offsets[r + 1] - (long long)row_offsets[r];
+      const int longest = __reduce_max_sync(0xffffffffu, (int)(len > kWholeRowMax ? kWholeRowMax + 1 : len));
+      bad |= longest > kWholeRowMax;
+      slots += 32u * (unsigned)longest;
+    }
+  }
+  if (lane == 0) {
+    if (bad) h->whole_rows = -1;
+    else if (slots) atomicAdd(reinterpret_cast<unsigned long long*>(&h->row_slots), slots);
+  }
+}
+// Moves the boundaries when the kernel above found nothing against it and at least two fifths of the thread-steps have
+// an edge to work on: rows of very different lengths are better off with the two-phase loop, whose lanes take
+// consecutive edges.  1 M rows, fp64 SpMV, this loop / the two-phase loop: lengths 0 - 8 evenly (share 0.50) 16.4 / 21.0 us,
+// 0 - 16 evenly (0.51) 29.0 / 35.6 us, exponential of mean 4 (0.22) 24.4 / 24.3 us, 32 in 3 % of the rows and 2 elsewhere
+// (0.14) 30.9 / 20.1 us.
+template <typename OffsetT>
+__global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
+                                                               long long num_tiles, OffsetT* __restrict__ coords, WorkspaceHeader* h) {
+  if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1) return;
+  if (2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) return;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t > 0 && t < num_tiles) {
+    const long long x = (long long)coords[2 * t];
+    if (x < num_rows) coords[2 * t + 1] = row_offsets[x];
+  }
+  if (t == 0) *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;     // read by this kernel only as "-1 or not"
+}
+
+template <typename OffsetT>
+static int whole_rows_launch_as(const void* d_row_offsets, long long num_rows, long long num_edges, long long num_tiles,
+                                const TileRoom& room, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
+  const OffsetT* ro = static_cast<const OffsetT*>(d_row_offsets);
+  OffsetT* coords = static_cast<OffsetT*>(d_coords);
+  long long grid = (num_tiles + 7) / 8;
+  const long long cap = (long long)device_sm_count() * 8;
+  if (grid > cap) grid = cap;
+  whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, coords, h);
+  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, coords, h);
+  return (int)cudaGetLastError();
+}
+int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
+                      const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream) {
+  if (num_tiles < 1 || num_rows < 1) return 0;
+  WorkspaceHeader* h = static_cast<WorkspaceHeader*>(ws);
+  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, d_coords, h, stream);
+  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, d_coords, h, stream);
 }
 
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,
@@ -480,6 +551,13 @@ int flexspmv_workspace_status_mirror(void* d_workspace, int32_t* pinned_host_sta
   }
   flex::status_mirror_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<flex::WorkspaceHeader*>(d_workspace), alias);
   return (int)cudaGetLastError();
+}
+
+int flexspmv_workspace_whole_rows(const void* d_workspace, int32_t* d_out, void* stream) {
+  if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;
+  if (!d_out) return FLEXSPMV_ERR_BAD_ARG;
+  const char* src = static_cast<const char*>(d_workspace) + offsetof(flex::WorkspaceHeader, whole_rows);
+  return (int)cudaMemcpyAsync(d_out, src, sizeof(int32_t), cudaMemcpyDefault, static_cast<cudaStream_t>(stream));
 }
 
 int flexspmv_halo_plan(const int64_t* first_row, const int64_t* min_col, const int64_t* max_col, int32_t world,

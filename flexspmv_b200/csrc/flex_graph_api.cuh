@@ -22,7 +22,9 @@ int partition_launch(const void* d_row_offsets, int offset_bits, long long num_r
 int device_sm_count();
 int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream);
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
-                               void* d_coords, void* ws, cudaStream_t stream);
+                               const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
+int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
+                      const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
 int window_plan_launch(const void* d_coords, int offset_bits, long long num_tiles, const int* d_idx, int rec_bytes,
                        int win_bytes, void* d_table, void* d_local_idx, cudaStream_t st);
 int window_ready_launch(void* ws, cudaStream_t st);
@@ -139,7 +141,20 @@ struct GraphApi {
     return 0;
   }
 
-  static int plan(const flexspmv_desc* d, const void* row_offsets, void* ws, size_t ws_bytes, cudaStream_t st) {
+  // What a tile of the kernel compiled with configuration C can take (the layout of its stage).
+  template <class C>
+  static TileRoom tile_room(const flexspmv_desc* d) {
+    TileRoom room;
+    room.max_edges = C::kTile;
+    room.edge_bytes = G::kStreamBytesPerEdge;
+    room.offset_bytes = d->offset_bits / 8;
+    room.stage_bytes = d->offset_bits == 64 ? TileSmemLayout<G, long long, C>::kRecordBytes : TileSmemLayout<G, int, C>::kRecordBytes;
+    if (G::kDirectLoads) room.stage_bytes = 0x7fffffff;
+    return room;
+  }
+
+  // `whole_rows`: also look for a matrix of short rows whose tiles can all hold whole rows (two more kernels).
+  static int plan(const flexspmv_desc* d, const void* row_offsets, void* ws, size_t ws_bytes, cudaStream_t st, bool whole_rows = true) {
     if (int e = check_desc(d)) return e;
     if (!ws) return FLEXSPMV_ERR_WORKSPACE;
     WorkspaceHeader h{};
@@ -155,6 +170,12 @@ struct GraphApi {
       if (!aligned16(row_offsets)) return FLEXSPMV_ERR_ALIGN;
       if (int e = partition_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, tile_items(d),
                                    static_cast<char*>(ws) + h.coords_offset, st)) return e;
+      if constexpr (WholeRows<G, Cfg, false>::value) {
+        // rows longer than kWholeRowMax on average: no need to look
+        if (whole_rows && !use_lean(d) && !use_win(d) && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
+          if (int e = whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d),
+                                        static_cast<char*>(ws) + h.coords_offset, ws, st)) return e;
+      }
       // the tile kernel: boundaries between the CTAs of its grid moved onto row ends where the tiles have room
       if (!use_lean(d) && h.num_tiles > 1) {
         int resident = 0;
@@ -168,7 +189,9 @@ struct GraphApi {
         if (e) return e;
         long long grid = max_ctas(d, resident);
         if (grid > h.num_tiles) grid = h.num_tiles;
-        return snap_cta_boundaries_launch(row_offsets, d->offset_bits, d->num_rows, h.num_tiles, (int)grid,
+        TileRoom room = tile_room<Cfg>(d);
+        if constexpr (G::kWindowGather && kWindowsBuilt) { if (win) room = tile_room<CfgWin>(d); }
+        return snap_cta_boundaries_launch(row_offsets, d->offset_bits, d->num_rows, h.num_tiles, (int)grid, room,
                                           static_cast<char*>(ws) + h.coords_offset, ws, st);
       }
       return 0;
@@ -432,7 +455,7 @@ struct GraphApi {
     cudaStream_t stream = static_cast<cudaStream_t>(st);                                                        \
     /* the array keeps the previous call's contents: planning rewrites the header (ticket, status) and */      \
     /* every tile coordinate this problem reads; the carry slots are written before they are read      */      \
-    if (int e = Api::plan(d, ro, ws, (size_t)(BYTES), stream)) return e;                                        \
+    if (int e = Api::plan(d, ro, ws, (size_t)(BYTES), stream, false)) return e;                                      \
     return Api::launch(d, v, ix, ro, o, ws, (size_t)(BYTES), stream);                                           \
   }                                                                                                             \
   extern "C" int flexspmv_##SYM##_static_device_status(int32_t* d_out, void* st) {                              \

@@ -10,6 +10,9 @@
 //   thread per row loads the row's own record once, gathers and maps its edges in register batches and
 //   stores the row; in tiles with a long row whole warps take the rows one at a time (lanes 32 edges
 //   apart, shuffle tree).  Nothing of a row-mode graph passes through a shared-memory product buffer.
+//   Whole rows (either kind of graph, when the plan found a matrix of short rows whose tiles can all hold whole rows):
+//   no carries at all, so no barriers either -- every warp takes 32 rows of a staged tile, one per lane, and keeps
+//   everything in registers.
 // The carry of a row that spans tiles travels inside the CTA in shared memory; the only cross-CTA state
 // is one carry per CTA, folded in by the last CTA to finish (ticket counter), in CTA order.  No atomics
 // on the output, no pre-zeroed output, run-to-run deterministic.
@@ -24,7 +27,7 @@
 
 namespace flex {
 
-template <int BLOCK_, int IPT_, int STAGES_, int MIN_CTAS_, int BATCH_ = 8, bool PIPELINE_ = false>
+template <int BLOCK_, int IPT_, int STAGES_, int MIN_CTAS_, int BATCH_ = 8, bool PIPELINE_ = false, int ROW_BATCH_ = BATCH_>
 struct TileCfg {
   // software pipelining across tiles (gathers of tile k in flight while tile k-1 is reduced); measured
   // slower than the plain loop on B200 (58% against 68% of the HBM peak on the 7-point fp64 SpMV: one
@@ -45,6 +48,14 @@ struct TileCfg {
   static constexpr int kTile = BLOCK_ * IPT_;
   static constexpr int kWarps = BLOCK_ / 32;
   static constexpr int kBatch = BATCH_;   // edges of one row whose gathers are in flight together (short-row tiles)
+  static constexpr int kRowBatch = ROW_BATCH_;   // the same in the loop over whole rows
+};
+
+// Whether the kernel has the loop over whole rows: staged graphs that write nothing per edge (a thread that walks a row
+// would store its edges' outputs a row length apart).
+template <class G, class Cfg, bool WIN>
+struct WholeRows {
+  static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
 };
 
 constexpr int kMaxCtas = 2048;            // capacity of the per-CTA carry arrays in the workspace
@@ -88,9 +99,12 @@ struct TileSmemLayout {
   static constexpr int kAcc = G::kAccDim;
   static constexpr int kBytesPerEdge = G::kStreamBytesPerEdge;
   static constexpr int kPerItem = (int(sizeof(OffsetT)) > kBytesPerEdge) ? int(sizeof(OffsetT)) : kBytesPerEdge;
+  // a tile's records: kTile merge items, and the edges in front of its first row end when the plan moves the tile's
+  // front boundary back to the start of that row
+  static constexpr int kRecordBytes = Cfg::kTile * kPerItem + kWholeRowMax * kBytesPerEdge;
   // each staged window may grow by < 32 bytes from aligning both ends to 16
   static constexpr int kStreamBytes =
-      G::kDirectLoads ? 0 : int(align_up(uint64_t(Cfg::kTile) * kPerItem + 32u * (G::kNumStreams + 1) + 16, 128));
+      G::kDirectLoads ? 0 : int(align_up(uint64_t(kRecordBytes) + 32u * (G::kNumStreams + 1) + 16, 128));
   // gather windows (WIN): the segments of the gathered vector follow the streams in every stage
   static constexpr int kWinBytes = int(align_up(uint64_t(WinBytesOf<G, WIN>::value), 128));
   static constexpr int kStageBytes = kStreamBytes + kWinBytes;
@@ -101,9 +115,10 @@ struct TileSmemLayout {
     uint32_t roff_off;
     uint32_t stream_off[G::kNumStreams > 0 ? G::kNumStreams : 1];
   };
+  static constexpr int kMaxStages = 4;
   static constexpr int kOffBars = 0;
-  static constexpr int kOffCtl = int(align_up(kOffBars + 16 * Cfg::kStages, 16));
-  static constexpr int kOffXs = int(align_up(kOffCtl + sizeof(Ctl) * Cfg::kStages, 16));
+  static constexpr int kOffCtl = int(align_up(kOffBars + 16 * kMaxStages, 16));
+  static constexpr int kOffXs = int(align_up(kOffCtl + sizeof(Ctl) * kMaxStages, 16));
   static constexpr int kOffWKey = int(align_up(kOffXs + 4 * (Cfg::kBlock + 1), 16));
   static constexpr int kOffWVal = int(align_up(kOffWKey + 4 * Cfg::kWarps, 16));
   static constexpr int kOffCarry = int(align_up(kOffWVal + sizeof(V) * kAcc * Cfg::kWarps, 16));
@@ -119,7 +134,16 @@ struct TileSmemLayout {
   // second at 228 / 196 / 164 / 132 / <= 32 KB of shared memory per SM).
   static constexpr int kOffProd = int(align_up(kOffRel + 4 * (Cfg::kTile + 1) * kBuffers, 16));
   static constexpr int kOffStages = int(align_up(kOffProd + (G::kGatherNeedsRow ? 0 : sizeof(V) * kAcc * Cfg::kTile * kBuffers), 128));
-  static constexpr int kTotal = kOffStages + kStageBytes * Cfg::kStages;
+  static constexpr int kTwoPhase = kOffStages + kStageBytes * Cfg::kStages;
+  // The loop over whole rows needs neither row ends nor products in shared memory: its stages begin where those would,
+  // and as many fit as the other loop's total allows, one more where that costs at most 2 KB.
+  static constexpr bool kWhole = WholeRows<G, Cfg, WIN>::value;
+  static constexpr int kOffRowStages = int(align_up(kOffLong, 128));
+  static constexpr int kFit = kWhole ? (kTwoPhase + 2048 - kOffRowStages) / kStageBytes : 0;
+  static constexpr int kRowStages = kFit > kMaxStages ? kMaxStages : kFit;
+  static constexpr int kRowLoop = kOffRowStages + kStageBytes * kRowStages;
+  static constexpr int kTotal = (kWhole && kRowLoop > kTwoPhase) ? kRowLoop : kTwoPhase;
+  static_assert(Cfg::kStages <= kMaxStages && (!kWhole || kRowStages >= Cfg::kStages), "stages of the two loops");
 };
 
 struct TileKernelArgs {
@@ -181,7 +205,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
 
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBars);    // "full": a stage's copies have landed
-  uint64_t* empty = bars + S;                                          // "empty": the consumers released a stage
+  uint64_t* empty = bars + L::kMaxStages;                              // "empty": the consumers released a stage
   Ctl* ctls = reinterpret_cast<Ctl*>(smem + L::kOffCtl);
   int* s_wkey = reinterpret_cast<int*>(smem + L::kOffWKey);
   V* s_wval = reinterpret_cast<V*>(smem + L::kOffWVal);
@@ -192,6 +216,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   int* s_rel = reinterpret_cast<int*>(smem + L::kOffRel);
   V* s_prod = reinterpret_cast<V*>(smem + L::kOffProd);
   unsigned char* s_stage = smem + L::kOffStages;
+  constexpr bool WHOLE = L::kWhole;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const OffsetT* row_offsets = static_cast<const OffsetT*>(a.row_offsets);
@@ -225,6 +250,11 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     return;
   }
 
+  // every tile holds whole rows only (any grid): stages of the loop over whole rows, in its places
+  const bool whole = WHOLE && a.header->whole_rows == 1;
+  const int nstages = WHOLE ? (whole ? L::kRowStages : S) : S;
+  unsigned char* const stage_base = (WHOLE && whole) ? smem + L::kOffRowStages : s_stage;
+
   const bool win_ready = WIN && a.header->win_ready == 1;   // until the window plan has run every tile gathers globally
   (void)win_ready;
 
@@ -249,7 +279,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   // lane 1+I: stream I, lane 16+j: gather-window segment j), a shuffle prefix sum places the windows in the
   // stage, lane 0 posts the byte count, then every lane issues its own bulk copy.
   auto issue = [&](long long row0, long long nz0, long long row1, long long nz1, int s, const WinEnt& we) {
-    unsigned char* dst = s_stage + (size_t)s * L::kStageBytes;
+    unsigned char* dst = stage_base + (size_t)s * L::kStageBytes;
     Window w;
     w.src = nullptr; w.bulk_bytes = 0; w.lead = 0; w.span = 0; w.tail_src = nullptr; w.tail_bytes = 0;
     const int nseg = we.nseg;
@@ -320,7 +350,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   if constexpr (!DIRECT) {
     if (tid == 0) {
 #pragma unroll
-      for (int s = 0; s < S; ++s) { mbar_init(&bars[s], 1); mbar_init(&empty[s], Cfg::kWarps); }   // empty: one arrive per consumer warp
+      for (int s = 0; s < L::kMaxStages; ++s) { mbar_init(&bars[s], 1); mbar_init(&empty[s], Cfg::kWarps); }   // empty: one arrive per consumer warp
       mbar_fence_init();
     }
   }
@@ -341,27 +371,29 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // testing aid (flexspmv_debug_withhold_stage): the stage of tile `withhold - 1` and of every later tile is
       // never filled, so that the consumers' bounded wait runs out and the error path can be exercised
       const unsigned long long withhold = a.header->debug[7];
+      int s = 0;                  // stage of tile k; round: how often the stages have been filled before
+      uint32_t round = 0;
       for (int k = 0; k < count; ++k) {
         if (withhold && (unsigned long long)(t_begin + k) + 1ull >= withhold) break;
-        const int s = k % S;
         long long nn_row = 0, nn_nz = 0;
         if (k + 1 < count) { nn_row = (long long)coords[2 * (t_begin + k + 2)]; nn_nz = (long long)coords[2 * (t_begin + k + 2) + 1]; }
         const WinEnt n_we = (k + 1 < count) ? load_win_entry(t_begin + k + 1) : WinEnt{0, 0, 0};
-        if (k >= S) {
-          const bool ok = mbar_wait_bounded(&empty[s], (uint32_t)(k / S - 1) & 1u, kWaitPolls);
+        if (round > 0) {
+          const bool ok = mbar_wait_bounded(&empty[s], (round - 1) & 1u, kWaitPolls);
           if (!__all_sync(0xffffffffu, ok)) { pfail = true; break; }
         }
         issue(c_row, c_nz, n_row, n_nz, s, c_we);
         c_row = n_row; c_nz = n_nz; n_row = nn_row; n_nz = nn_nz; c_we = n_we;
         issued = k + 1;
+        if (++s == nstages) { s = 0; ++round; }
         if (k >= 1) prefetch_gathers(k - 1);   // tile k-1 has (almost certainly) landed: warm L1 for its gathers
       }
       if (!pfail && count >= 1) prefetch_gathers(count - 1);
       if (pfail && lane == 0) {   // the consumers never released a stage: flag it, let copies in flight land, leave
         raise_status(a.header, FLEXSPMV_ERR_TIMEOUT);
         a.header->debug[4] = (uint32_t)issued; a.header->debug[5] = blockIdx.x;
-        for (int j = issued > S ? issued - S : 0; j < issued; ++j)
-          mbar_wait_bounded(&bars[j % S], (uint32_t)(j / S) & 1u, kWaitPolls);
+        for (int j = issued > nstages ? issued - nstages : 0; j < issued; ++j)
+          mbar_wait_bounded(&bars[j % nstages], (uint32_t)(j / nstages) & 1u, kWaitPolls);
       }
     }
     return;
@@ -463,6 +495,95 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       for (int j = 0; j < d; ++j) dst[j] = v[o + j];
     });
   };
+
+  if constexpr (WHOLE) {
+    if (whole) {
+      // ---- tiles of whole, short rows: warps work alone, no barrier, no carry, no products in shared memory ----------
+      // A warp takes 32 rows of a tile, one per lane: it reads the rows' column indices from the stage, has the gathers
+      // of kRowBatch edges per row in flight together -- lane r and lane r + 1 gather neighbours on a stencil, so a warp
+      // gather touches 2-3 cache lines instead of the 8-9 of 32 consecutive edges -- and reads the values only when the
+      // gathers are back.  Groups of rows go round the warps across tiles (`turn`), so a tile need not hold a multiple of
+      // the CTA's rows.  Sums run left to right over the row, as in the two-phase loop.
+      // What the two-phase loop is bound by on short rows is the shared-memory / L1 data pipe (75 - 80 % busy at 55 % of
+      // DRAM) and two CTA barriers a tile; this one moves no product through shared memory, a third of the gather lines,
+      // and is bound by the latency of the gathers at the registers of 4 CTAs per SM.  7-point fp64 SpMV 512^3: 3205 ->
+      // 2602 us (5.56 TB/s); 145^3 fp32: 54.1 -> 43.0 us; 2-D 512^2 fp64: 9.05 -> 7.3 us; 27 columns a row fp64, 300 007
+      // rows: 26.2 -> 24.2 us; spring-mass 1024^2: 44.5 -> 38.9 us; Rusanov 1024^2: 92 -> 82 us.
+      constexpr int RB = Cfg::kRowBatch;
+      int s = 0, turn = 0;
+      uint32_t parity = 0;
+      for (int k = 0; k < count; ++k) {
+        const bool ok = mbar_wait_bounded(&bars[s], parity, kWaitPolls);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0) {
+            raise_status(a.header, FLEXSPMV_ERR_TIMEOUT);
+            a.header->debug[0] = (uint32_t)(t_begin + k); a.header->debug[1] = (uint32_t)s; a.header->debug[2] = blockIdx.x;
+          }
+          return;
+        }
+        Ctl c;
+        {
+          const int4* src = reinterpret_cast<const int4*>(&ctls[s]);
+          int4* dst16 = reinterpret_cast<int4*>(&c);
+#pragma unroll
+          for (int i = 0; i < int(sizeof(Ctl) / 16); ++i) dst16[i] = src[i];
+        }
+        const unsigned char* stage = smem + L::kOffRowStages + (size_t)s * L::kStageBytes;
+        const OffsetT* rend = reinterpret_cast<const OffsetT*>(stage + c.roff_off);
+        SmemTile<G> tile;
+        static_for<NS>([&](auto I) { tile.base[I.value] = reinterpret_cast<const char*>(stage + c.stream_off[I.value]); });
+        const int groups = (c.nrows + 31) >> 5;
+        int g = warp - turn;
+        if (g < 0) g += Cfg::kWarps;
+        for (; g < groups; g += Cfg::kWarps) {
+          const int r = (g << 5) + lane;
+          int lo = 0, hi = 0;
+          if (r < c.nrows) {
+            hi = (int)rend[r] - (int)c.nz0;
+            if (r) lo = (int)rend[r - 1] - (int)c.nz0;
+          }
+          V sum[kAcc];
+#pragma unroll
+          for (int j = 0; j < kAcc; ++j) sum[j] = V(0);
+          typename G::GRow grow;
+          if constexpr (G::kGatherNeedsRow) { if (lo < hi) G::gather_row(p, c.row0 + r, grow); }
+          for (int e0 = lo; e0 < hi; e0 += RB) {
+            typename G::EReg er[RB];
+            typename G::GEdge ge[RB];
+#pragma unroll
+            for (int b = 0; b < RB; ++b)
+              if (e0 + b < hi) G::load_edge_idx(tile, e0 + b, er[b]);
+#pragma unroll
+            for (int b = 0; b < RB; ++b)
+              if (e0 + b < hi) {
+                if constexpr (!G::kValuesStaged) G::load_edge_vals(p, tile, e0 + b, c.nz0 + e0 + b, er[b]);
+                G::gather_edge(p, er[b], ge[b]);
+              }
+#pragma unroll
+            for (int b = 0; b < RB; ++b)
+              if (e0 + b < hi) {
+                if constexpr (G::kValuesStaged) G::load_edge_vals(p, tile, e0 + b, c.nz0 + e0 + b, er[b]);
+                G::map(p, er[b], c.nz0 + e0 + b, grow, ge[b], sum);
+              }
+          }
+          if (r < c.nrows) {
+            static_for<G::kNumReducers>([&](auto Rd) {
+              constexpr int d = G::template red_dim<Rd.value>();
+              constexpr int o = G::template red_off<Rd.value>();
+              V* dst = G::template red_out<Rd.value>(p) + (size_t)(c.row0 + r) * d;
+#pragma unroll
+              for (int j = 0; j < d; ++j) dst[j] = sum[o + j];
+            });
+          }
+        }
+        turn = (turn + groups) % Cfg::kWarps;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+        if (++s == L::kRowStages) { s = 0; parity ^= 1u; }
+      }
+      return;
+    }
+  }
 
   // ---- phase 1 pieces: lanes on consecutive edges ------------------------------------------------------
   auto map_load = [&](const TileRef& t, const TileT& tile, typename G::EReg (&er)[IPT]) {

@@ -218,6 +218,11 @@ int flexspmv_swe_rk_stage(int32_t value_bytes, const void *const *d_r, const voi
                           void *const *d_stage, double c, double w, int64_t n, int32_t first,
                           int32_t last, void *stream);
 
+/* Copies to *d_out (int32 in device or page-locked host memory), without synchronising, 1 when the plan in the workspace
+ * found a matrix of short rows (at most 32 edges) whose tiles all hold whole rows: the launches then run a loop without
+ * carries or barriers. */
+int flexspmv_workspace_whole_rows(const void *d_workspace, int32_t *d_out, void *stream);
+
 /* ---- per fused graph ---------------------------------------------------------------------------
  * One set of five symbols per (graph, value type); the per-edge map is compiled into the kernel, so
  * a graph is identified by its symbol prefix.  For graph G and value type T (f32 | f64 | i64):

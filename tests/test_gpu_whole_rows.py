@@ -1,0 +1,115 @@
+"""The tile kernel's loop over whole rows: which matrices the plan sends there (short rows that every tile can hold
+whole), and its results against the CPU oracle at the edges -- rows of 0, 1, a batch, a batch more, 32 and 33 edges,
+tiles smaller than a row, one row, both offset widths -- and against the loop with carries."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from flexspmv_b200 import graphs, problems
+from flexspmv_b200.binding import Desc, GraphExtension, load_library
+from oracle import ir_eval
+from parity import assert_outputs_match
+from test_gpu_parity import run_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def with_lengths(ir, lengths, seed, dtype):
+    """A random problem of the given row lengths."""
+    lengths = np.asarray(lengths)
+    rows, nnz = lengths.size, int(lengths.sum())
+    prob = problems.random_problem(ir, rows, rows, nnz, seed=seed, dtype=dtype)
+    prob.row_offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    for s in ir.selector_register:
+        if s.get("row_identity"):
+            prob.indices[s["selector_name"]] = np.repeat(np.arange(rows, dtype=np.int32), lengths)
+    return prob
+
+
+LENGTHS = {
+    "empty_and_full": ([0, 32, 0, 31, 1, 32, 32] * 300 + [0] * 5, None),   # at the limit: depends on the rows a tile holds
+    "all_5": ([5] * 4001, 1),
+    "all_8": ([8] * 3000, 1),
+    "batch_and_one_more": ([4, 5] * 1500 + [9] * 7, 1),
+    "all_32": ([32] * 777, 1),
+    "a_row_of_33": ([8] * 1000 + [33] + [8] * 1000, -1),
+    "one_row": ([7], 0),                                                  # one lane of a warp
+    "uneven": ([1] * 310 + [32] * 10 + [1] * 3000, 1),
+    "mostly_empty": (([0] * 31 + [32]) * 100, 0),                         # one lane in 32 would work
+    "leading_and_trailing_empty": ([0] * 100 + [6] * 500 + [0] * 100, 1),
+}
+
+
+@pytest.mark.parametrize("gname,dt", [("spmv", "float64"), ("spmv", "float32"), ("spmv", "int64"), ("spring_mass", "float32"),
+                                      ("rusanov", "float64"), ("swe_delta", "float32"), ("ops_zoo", "float64")])
+@pytest.mark.parametrize("case", sorted(LENGTHS))
+def test_whole_rows_match_the_oracle(gname, dt, case):
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    lengths, planned = LENGTHS[case]
+    prob = with_lengths(ir, lengths, 7, dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    for kw, offsets in (({}, np.int32), ({}, np.int64), ({"tile_items": 5, "max_ctas": 3}, np.int32),
+                        ({"tile_items": 40, "max_ctas": 7}, np.int64), ({"max_ctas": 1}, np.int32)):
+        ext = GraphExtension(ir, random_gather=False, **kw)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=offsets)
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname}/{dt}/{case}/{kw}")
+        ext.check()
+        # tiles of a few rows leave most lanes of a warp idle: refused; the small tiles of other graphs have no room for
+        # the front of a 32-edge row
+        if planned is not None and "tile_items" not in kw and (case != "all_32" or gname == "spmv"):
+            assert ext.planned_whole_rows() == (planned == 1), (case, kw)
+
+
+def test_whole_rows_equal_the_two_phase_loop_bit_for_bit():
+    """The same matrix with one row of 33 edges behind it goes through the loop with carries; all other rows are the
+    same sums, left to right."""
+    ir = graphs.spmv_graph()
+    rng = np.random.default_rng(3)
+    lengths = rng.integers(0, 17, 5000)
+    a = with_lengths(ir, lengths, 11, np.float64)
+    b = with_lengths(ir, np.concatenate([lengths, [33]]), 11, np.float64)
+    n, nnz = a.num_rows, a.nnz
+    b.values["vals"][:nnz] = a.values["vals"]
+    b.values["x"][:n] = a.values["x"]
+    b.indices["selector"][:nnz] = a.indices["selector"]
+    whole, carry = GraphExtension(ir, max_ctas=1), GraphExtension(ir, max_ctas=1)
+    got_a, _ = run_gpu(whole, ir, a, np.float64)
+    got_b, _ = run_gpu(carry, ir, b, np.float64)
+    assert whole.planned_whole_rows() and not carry.planned_whole_rows()
+    assert np.array_equal(got_a[0], got_b[0][:n])
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_a_moved_boundary_never_overfills_a_stage(bits):
+    """Many rows of one edge behind a long row that a boundary between two CTAs cuts: with the cut part moved behind
+    the boundary the tile's records and row ends would take more bytes than its stage holds, so the plan must leave
+    the boundaries alone (header, int32 at byte 132)."""
+    ir, dtype = graphs.spmv_graph(), np.float64
+    tile = 1280
+    lengths = np.ones(40 * tile, dtype=np.int64)
+    # rows in front of the second tile's boundary: the cut row has 600 edges in front of it and ends in the second tile
+    lengths[(tile - 600) // 2] = 601
+    prob = with_lengths(ir, lengths, 13, dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    lib = load_library()
+    desc = Desc(prob.num_rows, prob.nnz, prob.num_cols, bits, 0, 0, 0)
+    nbytes = ctypes.c_size_t()
+    for name in ("workspace_bytes", "plan", "launch"):
+        getattr(lib, f"flexspmv_spmv_f64_{name}").restype = ctypes.c_int
+    assert lib.flexspmv_spmv_f64_workspace_bytes(ctypes.byref(desc), ctypes.byref(nbytes)) == 0
+    ws = torch.zeros(nbytes.value, dtype=torch.uint8, device="cuda")
+    ro = torch.from_numpy(prob.row_offsets.astype(np.int32 if bits == 32 else np.int64)).cuda()
+    assert lib.flexspmv_spmv_f64_plan(ctypes.byref(desc), ctypes.c_void_p(ro.data_ptr()), ctypes.c_void_p(ws.data_ptr()),
+                                      ctypes.c_size_t(nbytes.value), None) == 0
+    torch.cuda.synchronize()
+    raw = ws[:256].cpu().numpy().view(np.int32)
+    coords = ws[256:256 + 48].cpu().numpy().view(np.int32 if bits == 32 else np.int64)
+    rows_behind, begin = int(coords[4] - coords[2]), int(prob.row_offsets[coords[2]])
+    extra = int(coords[3]) - begin
+    assert 0 < extra <= rows_behind                                  # the row count alone would have allowed it ...
+    assert (int(coords[5]) - begin) * 12 + rows_behind * bits // 8 > tile * 12 + 32 * 12     # ... the bytes do not
+    assert raw[33] == 0
+    got, _ = run_gpu(GraphExtension(ir), ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+    assert_outputs_match(ir, got, ref, sums, np.dtype(dtype), what="cut row in front of short ones")
