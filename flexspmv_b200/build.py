@@ -63,6 +63,9 @@ def generated_units():
             # the fp64 SpMV also gets the entry point that keeps its scratch in a static device array
             static_bytes = (2 << 20) if sym == "spmv_f64" else 0
             units.append((sym, emit_graph(ir, dt, sym, static_scratch_bytes=static_bytes)))
+            if name == "swe_delta":      # the same sums with the model's stage update behind them (shallow_water.py)
+                rk = f"swe_delta_rk_{CTYPE[dt][1]}"
+                units.append((rk, emit_graph(ir, dt, rk, windows=False, swe_rk=True)))
     return units
 
 

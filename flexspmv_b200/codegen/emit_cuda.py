@@ -194,15 +194,25 @@ def _with_node_names(ir: GraphIR) -> GraphIR:
     return ir
 
 
+# Extra pointers of the swe_delta graph with the model's stage update as its epilogue (csrc/flex_swe_rk.cuh), behind the
+# graph's own values: (field, C type, expression of a void pointer `q` that sets it)
+SWE_RK_FIELDS = [(n, "const V*", "static_cast<const V*>(q)") for n in ("area", "bsx", "bsy")] + \
+                [(n, "const int*", "static_cast<const int*>(q)") for n in ("wall_start", "wall_cell")] + \
+                [(f"{a}_{n}", "V*", "static_cast<V*>(const_cast<void*>(q))") for a in ("x", "acc") for n in ("h", "uh", "vh")] + \
+                [("coef", "flex::SweRkCoef<V>", "flex::SweRkCoef<V>::read(q)")]
+
+
 def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, static_scratch_bytes: int = 0,
-               windows: bool = True) -> str:
+               windows: bool = True, swe_rk: bool = False) -> str:
     """One translation unit for ``ir`` compiled for ``dtype``.  ``windows=False`` leaves out the gather-window
-    variant of the tile kernel (half the kernel instantiations: the form the torch-extension shim is built in)."""
+    variant of the tile kernel (half the kernel instantiations: the form the torch-extension shim is built in).
+    ``swe_rk`` (the swe_delta graph): a row's sums go through the model's stage update instead of to the outputs, which
+    are the next state; such a unit holds the loop over whole rows only."""
     ir = _with_node_names(ir)
     cty, sfx = CTYPE[dtype]
     symbol = symbol or f"{ir.name}_{sfx}"
     # measured configurations are keyed by graph and value type, whatever symbol prefix the unit is emitted under
-    cfg = tuple(config or _override(symbol) or TUNED_CONFIGS.get(f"{ir.name}_{sfx}") or choose_config(ir, dtype))
+    cfg = tuple(config or _override(symbol) or TUNED_CONFIGS.get(symbol) or TUNED_CONFIGS.get(f"{ir.name}_{sfx}") or choose_config(ir, dtype))
     block, ipt, stages, min_ctas = cfg[:4]
     pipeline = len(cfg) > 4 and bool(cfg[4])     # fifth field: software-pipelined tiles (TileCfg::kPipeline)
     batch_override = cfg[5] if len(cfg) > 5 else 0   # sixth field: edges per register batch in the fused row mode
@@ -253,11 +263,14 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w = L.append
     w(f"// GENERATED by flexspmv_b200.codegen.emit_cuda -- graph '{ir.name}' ({dtype}), digest {ir.digest()}")
     w('#include "flex_graph_api.cuh"')
+    if swe_rk:
+        w('#include "flex_swe_rk.cuh"')
+    extra = SWE_RK_FIELDS if swe_rk else []
     w("namespace {")
     w(f"namespace gen_{symbol} {{      // several generated units may share one translation unit")
     w("struct Graph {")
     w(f"  using V = {cty};")
-    w(f"  static constexpr int kNumValues = {len(value_names)}, kNumIndices = {len(index_names)}, kNumOutputs = {len(ir.outputs)};")
+    w(f"  static constexpr int kNumValues = {len(value_names) + len(extra)}, kNumIndices = {len(index_names)}, kNumOutputs = {len(ir.outputs)};")
     w(f"  static constexpr bool kHasReducer = {'true' if has_reducer else 'false'};")
     w(f"  static constexpr int kNumReducers = {len(reducers)}, kAccDim = {max(acc_off, 1)}, kAggDim = {agg_off};")
     w(f"  static constexpr int kNumStreams = {len(streams)};")
@@ -272,11 +285,15 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         w(f"    const int* {n}_idx;")
     for o in ir.outputs:
         w(f"    V* out_{o['name']};")
+    for n, ty, _ in extra:
+        w(f"    {ty} {n};")
     w("  };")
     w("  static Params make_params(const void* const* values, const void* const* indices, void* const* outputs) {")
     w("    Params p{};")
     for i, n in enumerate(value_names):
         w(f"    p.{n} = static_cast<V*>(const_cast<void*>(values[{i}]));")
+    for i, (n, _, get) in enumerate(extra):
+        w(f"    {{ const void* q = values[{len(value_names) + i}]; p.{n} = {get}; }}")
     for i, n in enumerate(index_names):
         w(f"    p.{n}_idx = static_cast<const int*>(indices[{i}]);")
     for i, o in enumerate(ir.outputs):
@@ -323,6 +340,24 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     for i, (n, _, _, _) in enumerate(reducers):
         w(f"    if constexpr (R == {i}) return p.out_{n};")
     w("    (void)p; return nullptr;")
+    w("  }")
+    # a row's finished sums: to the reducers' outputs, or through the epilogue
+    w(f"  static constexpr bool kEpilogue = {'true' if swe_rk else 'false'};")
+    w("  __device__ __forceinline__ static void finish_row(const Params& p, long long row, const V* v) {")
+    if swe_rk:
+        w("    flex::swe_rk_row<V>(p, row, v);")
+    else:
+        for n, d, off, _ in reducers:
+            for j in range(d):
+                w(f"    p.out_{n}[row * {d} + {j}] = v[{off + j}];")
+        w("    (void)p; (void)row; (void)v;")
+    w("  }")
+    w("  __device__ __forceinline__ static void prefetch_rows(const Params& p, long long row0, long long row1, int lane) {")
+    if swe_rk:      # one array per lane: the cell's own records and what the epilogue reads (the running sums from stage 2 on)
+        for i, n in enumerate(("area", "x_h", "x_uh", "x_vh", "h", "uh", "vh", "acc_h", "acc_uh", "acc_vh")):
+            when = f"lane == {i}" + (" && !p.coef.first" if n.startswith("acc") else "")
+            w(f"    if ({when}) flex::bulk_prefetch_l2(p.{n} + row0, (uint64_t)(row1 - row0) * sizeof(V));")
+    w("    (void)p; (void)row0; (void)row1; (void)lane;")
     w("  }")
     w("  __device__ __forceinline__ static void store_aggregate(const Params& p, int i, V s) {")
     for n, d, off, _ in aggs:

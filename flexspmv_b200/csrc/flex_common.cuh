@@ -204,6 +204,12 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
                "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
                : "memory");
 }
+// Asks for [p, p + bytes) in L2, in whole 16-byte chunks (a ragged end is left out).
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint64_t bytes) {
+  const uintptr_t from = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)15;
+  const uintptr_t to = (reinterpret_cast<uintptr_t>(p) + bytes) & ~(uintptr_t)15;
+  if (to > from) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"((uint32_t)(to - from)) : "memory");
+}
 // Programmatic dependent launch: a kernel launched with the programmatic-stream-serialization attribute may
 // start while the kernel before it on the stream is still running; everything it does before pdl_wait() must
 // touch no global memory.  pdl_wait() returns once that kernel has completed and its writes are visible (at

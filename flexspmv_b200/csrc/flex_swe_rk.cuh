@@ -1,0 +1,69 @@
+// What the shallow-water model does with a cell's three flux sums, as the epilogue of the kernel that forms them: the
+// wall terms of boundary cells, d = -(r [+ wall]) / area and the Runge-Kutta update of the stage
+// (shallow_water_equation/swe_main.py:86-146).  Every operation is the one, in the order, of the separate launches it
+// stands for (the swe_boundary graph's pow / mul / sum and flexspmv_swe_rk_stage), so the states are bit-identical to
+// theirs.  In the flux kernel the sums never leave their registers and the wall terms cost nothing on cells without a
+// wall: per cell 16 bytes of memory traffic a sum, 32 a wall sum and two launches a stage less.
+// Bound by the latency of the gathers and of the cell's own records (26 warps per SM at 72 registers); the producer warp
+// therefore asks for those records in L2 when it stages a tile (prefetch_rows: 510 -> 454 us a step).  A step of the
+// model on 2 097 152 cells, fp64: 606 us as 12 launches, 454 us as 4 (1024 x 1024 squares); on 20 402 cells 57.5 -> 32.8 us.
+// Batches of 1 / 2 edges per thread at 3 CTAs per SM, 3 at 2, 1 at 4 (before the prefetch): 510 / 546 / 625 / 555 us.
+#pragma once
+#include "flex_tensor.cuh"
+
+namespace flex {
+
+// The records j0 .. j1-1 that belong to `cell`, added in order.  Out of line: few cells have a wall.
+template <typename V>
+struct WallTerms { V uh, vh; };
+template <typename V>
+__device__ __noinline__ WallTerms<V> swe_wall_terms(V h, const int* wall_cell, const V* bsx, const V* bsy, int j0, int j1, int cell) {
+  WallTerms<V> t{V(0), V(0)};
+  const V half_sq = fx::vmul(V(0.5), fx::vpow(h, V(2)));
+  for (int j = j0; j < j1; ++j) {
+    if (__ldg(wall_cell + j) != cell) continue;
+    t.uh = fx::vadd(t.uh, fx::vmul(half_sq, __ldg(bsx + j)));
+    t.vh = fx::vadd(t.vh, fx::vmul(half_sq, __ldg(bsy + j)));
+  }
+  return t;
+}
+
+// P: Params of a generated graph with the fields named below.  `coef` points to host memory that is read when the
+// launch is made: c, w, first, last.  Records of the walls: wall_cell ascending, wall_start[i] = first record of a cell
+// >= 32 i (cells / 32 rounded up, plus one, entries).
+template <typename V, class P>
+__device__ __forceinline__ void swe_rk_row(const P& p, long long row, const V* r) {
+  const V area = __ldg(p.area + row);
+  WallTerms<V> wall{V(0), V(0)};
+  const int j0 = __ldg(p.wall_start + (row >> 5)), j1 = __ldg(p.wall_start + (row >> 5) + 1);
+  if (j0 < j1) wall = swe_wall_terms<V>(__ldg(p.h + row), p.wall_cell, p.bsx, p.bsy, j0, j1, (int)row);
+  V* const x[3] = {p.x_h, p.x_uh, p.x_vh};
+  V* const acc[3] = {p.acc_h, p.acc_uh, p.acc_vh};
+  V* const next[3] = {p.out_r_h, p.out_r_uh, p.out_r_vh};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    V sum = r[k];
+    if (k > 0) sum = fx::vadd(sum, k == 1 ? wall.uh : wall.vh);
+    const V d = fx::vdiv(-sum, area);
+    const V a = p.coef.first ? d : fx::vadd(acc[k][row], d);
+    const V at = x[k][row];
+    if (p.coef.last) {
+      x[k][row] = fx::vadd(at, fx::vmul(p.coef.w, a));
+    } else {
+      acc[k][row] = a;
+      next[k][row] = fx::vadd(at, fx::vmul(p.coef.c, d));
+    }
+  }
+}
+
+template <typename V>
+struct SweRkCoef {
+  V c, w;
+  bool first, last;
+  static SweRkCoef read(const void* host) {
+    const V* v = static_cast<const V*>(host);
+    return SweRkCoef{v[0], v[1], v[2] != V(0), v[3] != V(0)};
+  }
+};
+
+}  // namespace flex

@@ -326,6 +326,8 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     if (lane == 0) mbar_expect_tx(&bars[s], total);
     __syncwarp();
     if (w.bulk_bytes) bulk_g2s(dst + off, w.src, w.bulk_bytes, &bars[s]);
+    // what an epilogue reads per row comes from L2 then, not from DRAM, when the tile's rows get there
+    if constexpr (G::kEpilogue) G::prefetch_rows(p, row0, row1, lane);
 #ifdef FLEX_PREFETCH_DIRECT
     if constexpr (G::kHasDirectEdgeTensors) G::prefetch_direct(p, nz0, nz1, lane);
 #endif
@@ -535,6 +537,10 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
         const int groups = (c.nrows + 31) >> 5;
         int g = warp - turn;
         if (g < 0) g += Cfg::kWarps;
+        if (g >= groups) {                                         // no rows for this warp
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[s]);
+        }
         for (; g < groups; g += Cfg::kWarps) {
           const int r = (g << 5) + lane;
           int lo = 0, hi = 0;
@@ -566,23 +572,24 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
                 G::map(p, er[b], c.nz0 + e0 + b, grow, ge[b], sum);
               }
           }
-          if (r < c.nrows) {
-            static_for<G::kNumReducers>([&](auto Rd) {
-              constexpr int d = G::template red_dim<Rd.value>();
-              constexpr int o = G::template red_off<Rd.value>();
-              V* dst = G::template red_out<Rd.value>(p) + (size_t)(c.row0 + r) * d;
-#pragma unroll
-              for (int j = 0; j < d; ++j) dst[j] = sum[o + j];
-            });
+          // the warp's last rows of this tile: nothing more is read from the stage
+          if (g + Cfg::kWarps >= groups) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
           }
+          if (r < c.nrows) G::finish_row(p, c.row0 + r, sum);
         }
         turn = (turn + groups) % Cfg::kWarps;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
         if (++s == L::kRowStages) { s = 0; parity ^= 1u; }
       }
       return;
     }
+  }
+
+  // an epilogue needs a row's whole sum: a matrix that was not planned with whole rows is refused
+  if constexpr (G::kEpilogue) {
+    if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
+    return;
   }
 
   // ---- phase 1 pieces: lanes on consecutive edges ------------------------------------------------------

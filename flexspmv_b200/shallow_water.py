@@ -4,12 +4,13 @@ The reference model (shallow_water_equation/swe_main.py:12-146) is an ``easier``
 is a classical Runge-Kutta step; each of its four ``delta`` evaluations gathers h, uh, vh over the edges
 (``gather_src`` / ``gather_dst``), blends them to face values, and scatters three flux sums per cell
 (``scatter``) plus two wall terms on the boundary cells (``scatter_b``).  The reference replaces those
-fused regions by generated operators and leaves the per-cell arithmetic to torch.  ``ShallowWaterStep``
-runs the step on this package's kernels: per ``delta`` one launch of the ``swe_delta`` graph and one of
-the ``swe_boundary`` graph (both bound once with ``GraphExtension.prepare``: no per-call marshalling, no
-allocation), then one launch of ``flexspmv_swe_rk_stage`` for ``-(...)/area`` and the Runge-Kutta update
-of that stage (about 60 torch element-wise kernels per step in the reference).  ``capture()`` records the
-whole step (12 launches) into one CUDA graph.
+fused regions by generated operators and leaves the per-cell arithmetic to torch (about 60 element-wise
+kernels per step).  ``ShallowWaterStep`` runs a stage as ONE launch: the ``swe_delta`` graph's kernel with the
+stage's per-cell arithmetic -- wall terms, ``-(...)/area``, the Runge-Kutta update -- as what it does with a
+cell's finished flux sums (csrc/flex_swe_rk.cuh), bound once with ``GraphExtension.prepare``.  Meshes whose
+cells are too irregular for that kernel (a cell with more than 32 edges), and steps with operator objects of the
+caller's, run a stage as three launches with the same results, bit for bit: ``swe_delta``, ``swe_boundary``,
+``flexspmv_swe_rk_stage``.  ``capture()`` records the whole step (4 launches, or 12) into one CUDA graph.
 
 Edges must be sorted by destination cell and ``bcells`` ascending: both Reducers then see sorted indices,
 which is what the merge-path kernels need (python_wrapper/dynamic_replace_submodule.py:20-41 makes the
@@ -24,6 +25,7 @@ import ctypes
 import torch
 
 from .binding import GraphExtension, check, load_builtin
+from .graphs import swe_delta_graph
 from .python_wrapper.dynamic_replace_submodule import coo_rows_to_csr_ptr
 
 
@@ -39,23 +41,54 @@ class ShallowWaterStep:
         self.nc = int(m["h"].numel())
         self.ne = int(m["src"].numel())
         self.nbc = int(m["bcells"].numel())
+        own = delta_ext is not None or boundary_ext is not None
         self.delta_ext = delta_ext or load_builtin("swe_delta")
         self.boundary_ext = boundary_ext or load_builtin("swe_boundary")
         self.ro = coo_rows_to_csr_ptr(m["dst"], self.nc)
+        if self.ne < 2 ** 31 - self.nc:
+            self.ro = self.ro.to(torch.int32)             # half the bytes to stream per stage
         self.ro_b = coo_rows_to_csr_ptr(m["bcells"], self.nc)
         dt_ = m["h"].dtype
-        # stage inputs (the state the current delta is evaluated at) and the reducers' outputs
-        self.stage = [torch.empty(self.nc, dtype=dt_, device=dev) for _ in range(3)]
-        self.red = [torch.empty(self.nc, dtype=dt_, device=dev) for _ in range(3)]
-        self.red_b = [torch.empty(self.nc, dtype=dt_, device=dev) for _ in range(2)]
+        new = lambda k: [torch.empty(self.nc, dtype=dt_, device=dev) for _ in range(k)]
+        self.stage = new(3)                               # the state the next delta is evaluated at
+        self.acc = new(3)                                 # running sum of the increments
+        self._graph: Optional[torch.cuda.CUDAGraph] = None
+        self._fused = None if own else self._bind_fused(new)
+        if self._fused is not None:
+            return
+        self.red, self.red_b = new(3), new(2)             # the reducers' outputs
         self._on_state = self._bind(m["h"], m["uh"], m["vh"])
         self._on_stage = self._bind(*self.stage)
-        self.acc = [torch.empty(self.nc, dtype=dt_, device=dev) for _ in range(3)]
         ptrs = lambda ts: (ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
         self._p_red, self._p_red_b, self._p_acc, self._p_stage = ptrs(self.red), ptrs(self.red_b), ptrs(self.acc), ptrs(self.stage)
         self._p_x = ptrs([m["h"], m["uh"], m["vh"]])
         self.delta_ext.lib.flexspmv_swe_rk_stage.restype = ctypes.c_int
-        self._graph: Optional[torch.cuda.CUDAGraph] = None
+
+    def _coefficients(self):
+        """(c, first, last) of the four stages: the next state is x + c d, the last one adds dt / 6 of the sum."""
+        return ((0.5 * self.dt, 1, 0), (0.5 * self.dt, 0, 0), (self.dt, 0, 0), (0.0, 0, 1))
+
+    def _bind_fused(self, new):
+        """The four launches of a step, or None when the mesh was not planned with whole rows.  A stage reads one
+        state and writes the next, and neighbours read what a cell wrote, so the states alternate between two sets
+        of arrays."""
+        m, dt_ = self.m, self.m["h"].dtype
+        ext = GraphExtension(swe_delta_graph(), symbol_prefix="swe_delta_rk")
+        cells = m["bcells"].to(torch.int32).contiguous()
+        starts = torch.arange(0, self.nc + 32, 32, device=cells.device, dtype=torch.int32)
+        self._wall_start = torch.searchsorted(cells, starts, right=False).to(torch.int32)
+        other = new(3)
+        state = [m["h"], m["uh"], m["vh"]]
+        launches = []
+        for k, (c, first, last) in enumerate(self._coefficients()):
+            src = state if k == 0 else (self.stage if k % 2 else other)
+            dst = other if k % 2 else self.stage          # the last stage writes the state itself
+            coef = torch.tensor([c, self.dt / 6, first, last], dtype=dt_)      # host memory, read at every launch
+            values = [m["alpha"], m["sx"], m["sy"]] + src + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [coef]
+            launches.append(ext.prepare(values, [m["src"], m["dst"]], self.ro, dst, self.nc, self.ne, self.nc))
+            if k == 0 and not ext.planned_whole_rows():
+                return None
+        return launches
 
     def _bind(self, h, uh, vh):
         m = self.m
@@ -76,12 +109,15 @@ class ShallowWaterStep:
 
     def forward(self) -> None:
         """swe_main.py:121-146: four delta evaluations (:86-119), each followed by its stage update."""
-        dt = self.dt
-        for k, c in enumerate((0.5 * dt, 0.5 * dt, dt, 0.0)):
+        if self._fused is not None:
+            for launch in self._fused:
+                launch.launch()
+            return
+        for k, (c, first, last) in enumerate(self._coefficients()):
             bound = self._on_state if k == 0 else self._on_stage
             bound[0].launch()
             bound[1].launch()
-            self._stage(c, first=(k == 0), last=(k == 3))
+            self._stage(c, first=bool(first), last=bool(last))
 
     __call__ = forward
 

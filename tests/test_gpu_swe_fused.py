@@ -1,0 +1,58 @@
+"""The shallow-water step with the stage arithmetic behind the flux sums (one launch a stage) against the same step as
+three launches a stage: the same operations in the same order, so the same bits."""
+import numpy as np
+import pytest
+import torch
+
+from flexspmv_b200 import problems
+from flexspmv_b200.binding import load_builtin
+from flexspmv_b200.shallow_water import ShallowWaterStep
+
+pytestmark = pytest.mark.gpu
+
+
+def mesh_of(n, dtype, split_walls):
+    m = {k: v for k, v in problems.swe_model_inputs(n).items() if k != "row_offsets"}
+    if split_walls:      # a wall record per face: cells with several come several times, ascending
+        keep = np.repeat(np.arange(m["bcells"].size), np.where(np.arange(m["bcells"].size) % 3 == 0, 3, 1))
+        m["bcells"] = m["bcells"][keep]
+        m["bsx"], m["bsy"] = 0.3 * m["bsx"][keep], 0.7 * m["bsy"][keep]
+    cast = lambda v: v.astype(dtype) if v.dtype.kind == "f" else v
+    return {k: torch.from_numpy(np.ascontiguousarray(cast(v))).cuda() for k, v in m.items()}
+
+
+@pytest.mark.parametrize("n", [1, 3, 16, 33, 97])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("split_walls", [False, True])
+def test_fused_stage_equals_three_launches(n, dtype, split_walls):
+    dt = 0.05 / n
+    a, b = mesh_of(n, dtype, split_walls), mesh_of(n, dtype, split_walls)
+    fused = ShallowWaterStep(a, dt=dt)
+    apart = ShallowWaterStep(b, dt=dt, delta_ext=load_builtin("swe_delta"), boundary_ext=load_builtin("swe_boundary"))
+    assert apart._fused is None
+    if n >= 16:
+        assert fused._fused is not None      # a tile of a few cells leaves most of a warp idle: either way then
+        fused.capture()
+    for k in range(3):
+        fused.replay() if n >= 16 else fused.forward()
+        apart.forward()
+    torch.cuda.synchronize()
+    for name in ("h", "uh", "vh"):
+        assert torch.isfinite(a[name]).all()
+        assert torch.equal(a[name], b[name]), name
+
+
+def test_a_cell_with_many_edges_takes_three_launches():
+    m = mesh_of(24, np.float64, False)
+    src, dst = m["src"], m["dst"]
+    many = torch.full((40,), 5, dtype=torch.int32, device="cuda")          # 40 more edges into cell 7
+    order = torch.argsort(torch.cat([dst, many + 2]).long(), stable=True)
+    for k, extra in (("src", many), ("dst", many + 2)):
+        m[k] = torch.cat([m[k], extra])[order].contiguous()
+    for k in ("alpha", "sx", "sy"):
+        m[k] = torch.cat([m[k], torch.full((40,), 0.25, dtype=torch.float64, device="cuda") * (0.0 if k != "alpha" else 1.0)])[order].contiguous()
+    step = ShallowWaterStep(m, dt=1e-3)
+    assert step._fused is None
+    step.forward()
+    torch.cuda.synchronize()
+    assert torch.isfinite(m["h"]).all()
