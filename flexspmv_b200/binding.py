@@ -87,10 +87,11 @@ _CHECK_EVERY_CALL = os.environ.get("FLEXSPMV_CHECK_STATUS", "0") == "1"
 class _Plan:
     """One planned workspace: the scratch tensor, its size, the tensors whose addresses it depends on, and
     the page-locked int the kernels copy their error status to."""
-    __slots__ = ("ws", "nbytes", "keep", "flag", "_flag_view")
+    __slots__ = ("ws", "nbytes", "keep", "flag", "_flag_view", "desc", "ws_ptr")
 
-    def __init__(self, ws, nbytes, keep):
+    def __init__(self, ws, nbytes, keep, desc):
         self.ws, self.nbytes, self.keep = ws, nbytes, keep
+        self.desc, self.ws_ptr = desc, ws.data_ptr()
         self.flag = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._flag_view = self.flag.numpy()
 
@@ -109,6 +110,22 @@ def _stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+# The call path asks for the current device and stream on every launch; these are the plain integers behind
+# torch.cuda.current_device() and torch.cuda.current_stream(index).cuda_stream, without the Stream object that the
+# latter builds each time (CUDA is initialised by then: the arguments are CUDA tensors).
+_current_device = torch._C._cuda_getDevice
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+# flexspmv_<graph>_launch(desc, values, indices, row_offsets, outputs, workspace, workspace_bytes, stream): with the
+# argument types declared ctypes converts plain integers itself, without a wrapper object per pointer
+_LAUNCH = ctypes.CFUNCTYPE(ctypes.c_int, *([ctypes.c_void_p] * 6), ctypes.c_size_t, ctypes.c_void_p)
+
+
+def _pointers(tensors):
+    """C array of the tensors' addresses (at least one slot)."""
+    return (ctypes.c_void_p * (len(tensors) or 1))(*[t.data_ptr() for t in tensors])
+
+
 class _Symbols:
     def __init__(self, lib, sym: str):
         def fn(name):
@@ -120,7 +137,8 @@ class _Symbols:
             return f
         self.info, self.workspace_bytes, self.plan = fn("info"), fn("workspace_bytes"), fn("plan")
         self.plan_windows = fn("plan_windows")
-        self.launch, self.device_status = fn("launch"), fn("device_status")
+        fn("launch")
+        self.launch, self.device_status = _LAUNCH((f"flexspmv_{sym}_launch", lib)), fn("device_status")
         gi = GraphInfo()
         check(lib, self.info(ctypes.byref(gi)), f"{sym}_info")
         self.graph_info = gi
@@ -167,7 +185,12 @@ class GraphExtension:
         self.value_names = self.non_gather + self.gathers
         self.arg_names = self.value_names + [n + "_idx" for n in self.index_names] + \
             ["row_end_offsets", "num_rows", "num_cols"]
+        self._tensor_names = self.arg_names[:-2]
+        self._out_kinds = [("row" if str(o["target"]) == "reducer" else "one" if "sum" in str(o["target"]) else "edge",
+                            dim_of(o["shape"])) for o in ir.outputs]
+        self._has_reducer = ir.has_reducer
         self._syms: Dict[str, _Symbols] = {}
+        self._by_dtype: Dict[torch.dtype, _Symbols] = {}
         self._plans: "OrderedDict[tuple, tuple]" = OrderedDict()
         self.launches = 0    # kernels this object enqueued (plan kernels included)
 
@@ -214,6 +237,9 @@ class GraphExtension:
             self._locality[key] = hit
         return hit
 
+    def _by_type(self, dtype: torch.dtype) -> _Symbols:
+        return self._by_dtype.get(dtype) or self._by_dtype.setdefault(dtype, self.symbols(dtype))
+
     def _flags(self, syms: _Symbols, values=(), indices=()) -> int:
         flags = 1 if (self.gather_windows and (syms.graph_info.reserved & 1)) else 0
         if (syms.graph_info.reserved & 2) and self.random_gather is not False and len(indices):
@@ -221,28 +247,32 @@ class GraphExtension:
                 flags = 2
         return flags
 
-    def _desc(self, syms: _Symbols, values, row_end_offsets, num_rows: int, num_edges: int, num_cols: int,
-              indices=()) -> Desc:
-        has_red = self.ir.has_reducer
+    def _plan_for(self, syms: _Symbols, values, indices, ro: Optional[torch.Tensor], num_rows: int, num_edges: int,
+                  num_cols: int, device) -> Tuple["_Plan", Desc]:
+        """The planned workspace of a problem on the current stream (``device`` is current) and its descriptor."""
         flags = self._flags(syms, values, indices)
         if flags & 1:      # the windows are bounded by the gathered array's length: take it from the tensor itself
             num_cols = int(values[len(self.non_gather)].shape[0])
-        return Desc(num_rows if has_red else 0, num_edges, num_cols,
-                    64 if (has_red and row_end_offsets.dtype == torch.int64) else 32,
-                    self.tile_items, self.max_ctas, flags)
-
-    def _workspace(self, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device,
-                   indices: Sequence[torch.Tensor] = ()) -> "_Plan":
+        if self._has_reducer:
+            bits = 64 if ro.dtype == torch.int64 else 32
+            of = (ro.data_ptr(), ro._version)
+        else:
+            num_rows, bits, of, ro = 0, 32, None, None
         # a workspace holds per-launch state (ticket, carries): launches that may overlap on the GPU must not
         # share one, so the plan is cached per stream as well as per matrix
-        key = (id(syms), desc.num_rows, desc.num_edges, desc.offset_bits, desc.tile_items, desc.max_ctas, desc.reserved,
-               (ro.data_ptr(), ro._version) if ro is not None else None, device.index,
-               torch.cuda.current_stream(device).cuda_stream,
-               tuple((t.data_ptr(), t._version) for t in indices) if (desc.reserved & 1) else None)
-        hit = self._plans.get(key)
-        if hit is not None:
+        key = (id(syms), num_rows, num_edges, bits, self.tile_items, self.max_ctas, flags, of, device.index,
+               _raw_stream(device.index), tuple((t.data_ptr(), t._version) for t in indices) if (flags & 1) else None)
+        plan = self._plans.get(key)
+        if plan is not None:
             self._plans.move_to_end(key)
-            return hit
+            if plan.desc.num_vertices == num_cols:
+                return plan, plan.desc
+            return plan, Desc(num_rows, num_edges, num_cols, bits, self.tile_items, self.max_ctas, flags)
+        desc = Desc(num_rows, num_edges, num_cols, bits, self.tile_items, self.max_ctas, flags)
+        return self._make_plan(key, syms, desc, ro, device, indices), desc
+
+    def _make_plan(self, key, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device,
+                   indices: Sequence[torch.Tensor] = ()) -> "_Plan":
         nbytes = ctypes.c_size_t()
         check(self.lib, syms.workspace_bytes(ctypes.byref(desc), ctypes.byref(nbytes)), "workspace_bytes")
         ws = torch.empty(nbytes.value, dtype=torch.uint8, device=device)
@@ -256,7 +286,7 @@ class GraphExtension:
             self.launches += 2
         self.launches += 2 if ro is not None else 1
         # keep the row-offset tensor alive so its address cannot be recycled under a cached plan
-        plan = _Plan(ws, nbytes.value, (ro, tuple(indices) if (desc.reserved & 1) else None))
+        plan = _Plan(ws, nbytes.value, (ro, tuple(indices) if (desc.reserved & 1) else None), desc)
         check(self.lib, self.lib.flexspmv_workspace_status_mirror(ctypes.c_void_p(ws.data_ptr()),
                                                                   ctypes.c_void_p(plan.flag.data_ptr()), _stream_ptr()),
               "workspace_status_mirror")
@@ -268,12 +298,12 @@ class GraphExtension:
 
     # -- the operator --------------------------------------------------------------------------------
     def merged_spmv_launch(self, *args, **kwargs):
-        a = self._bind(args, kwargs)
-        nv, ni = len(self.value_names), len(self.index_names)
-        values: List[torch.Tensor] = a[:nv]
-        indices: List[torch.Tensor] = a[nv:nv + ni]
-        row_end_offsets, num_rows, num_cols = a[nv + ni], int(a[nv + ni + 1]), int(a[nv + ni + 2])
-        for n, t in zip(self.arg_names, values + indices + [row_end_offsets]):
+        a = args if (not kwargs and len(args) == len(self.arg_names)) else self._bind(args, kwargs)
+        nv = len(self.value_names)
+        ni = nv + len(self.index_names)
+        values, indices = a[:nv], a[nv:ni]
+        row_end_offsets, num_rows, num_cols = a[ni], int(a[ni + 1]), int(a[ni + 2])
+        for n, t in zip(self._tensor_names, a):
             if not isinstance(t, torch.Tensor):
                 raise TypeError(f"{n} must be a torch.Tensor")
             if not t.is_cuda:
@@ -282,7 +312,7 @@ class GraphExtension:
                 raise FlexSpmvError(f"{n} must be contiguous")
         dispatch = values[0]
         dt = dispatch.dtype
-        syms = self.symbols(dt)
+        syms = self._by_type(dt)
         for n, t in zip(self.value_names, values):
             if t.dtype != dt:
                 raise FlexSpmvError(f"{n} dtype mismatch")
@@ -292,41 +322,39 @@ class GraphExtension:
         ne = int(indices[0].numel()) if indices else num_cols
         if ne <= 0:
             raise FlexSpmvError("selector index must be non-empty")
-        has_red = self.ir.has_reducer
-        if has_red:
+        if self._has_reducer:
             if row_end_offsets.dtype not in (torch.int32, torch.int64):
                 raise FlexSpmvError("row_end_offsets dtype mismatch")
             if row_end_offsets.numel() != num_rows + 1:
                 raise FlexSpmvError("row_end_offsets must have length num_rows + 1")
         device = dispatch.device
-        desc = self._desc(syms, values, row_end_offsets, num_rows, ne, num_cols, indices)
         outputs: List[torch.Tensor] = []
-        for o in self.ir.outputs:
-            d = dim_of(o["shape"])
-            tgt = str(o["target"])
-            if tgt == "reducer":
-                shape = (num_rows,) if d == 1 else (num_rows, d)
-            elif "sum" in tgt:
+        for kind, d in self._out_kinds:
+            if kind == "one":
                 shape = (d,)
             else:
-                shape = (ne,) if d == 1 else (ne, d)
+                n = num_rows if kind == "row" else ne
+                shape = (n,) if d == 1 else (n, d)
             outputs.append(torch.empty(shape, dtype=dt, device=device))
-        with torch.cuda.device(device):
-            plan = self._workspace(syms, desc, row_end_offsets if has_red else None, device, indices)
-            _raise_if_failed(self.lib, plan, "merged_spmv_launch")
-            vp = (ctypes.c_void_p * max(nv, 1))(*[t.data_ptr() for t in values])
-            ip = (ctypes.c_void_p * max(ni, 1))(*[t.data_ptr() for t in indices])
-            op = (ctypes.c_void_p * max(len(outputs), 1))(*[t.data_ptr() for t in outputs])
-            st = syms.launch(ctypes.byref(desc), vp, ip,
-                             ctypes.c_void_p(row_end_offsets.data_ptr() if has_red else 0), op,
-                             ctypes.c_void_p(plan.ws.data_ptr()), ctypes.c_size_t(plan.nbytes), _stream_ptr())
-        check(self.lib, st, "merged_spmv_launch")
-        self.launches += 1
-        if _CHECK_EVERY_CALL:
-            self.check()
+        self._launch(syms, values, indices, row_end_offsets, outputs, num_rows, ne, num_cols, device, "merged_spmv_launch")
         if not outputs:
             return None
         return tuple(outputs)
+
+    def _launch(self, syms: _Symbols, values, indices, ro, outputs, num_rows: int, num_edges: int, num_cols: int, device,
+                what: str) -> None:
+        if _current_device() != device.index:
+            with torch.cuda.device(device):
+                return self._launch(syms, values, indices, ro, outputs, num_rows, num_edges, num_cols, device, what)
+        plan, desc = self._plan_for(syms, values, indices, ro, num_rows, num_edges, num_cols, device)
+        _raise_if_failed(self.lib, plan, what)
+        st = syms.launch(ctypes.byref(desc), _pointers(values), _pointers(indices), ro.data_ptr() if self._has_reducer else 0,
+                         _pointers(outputs), plan.ws_ptr, plan.nbytes, _raw_stream(device.index))
+        if st != 0:
+            check(self.lib, st, what)
+        self.launches += 1
+        if _CHECK_EVERY_CALL:
+            self.check()
 
     __call__ = merged_spmv_launch
 
@@ -336,24 +364,8 @@ class GraphExtension:
         """Same fused pass as ``merged_spmv_launch`` but into caller-provided output tensors (any
         tensor or slice whose storage is large enough; e.g. the owned part of the next iteration's
         vector).  No allocation, no checks beyond the C ABI's own; one kernel launch."""
-        dt = values[0].dtype
-        syms = self.symbols(dt)
-        has_red = self.ir.has_reducer
-        device = values[0].device
-        desc = self._desc(syms, values, row_end_offsets, num_rows, num_edges, num_cols, indices)
-        with torch.cuda.device(device):
-            plan = self._workspace(syms, desc, row_end_offsets if has_red else None, device, indices)
-            _raise_if_failed(self.lib, plan, "launch_into")
-            vp = (ctypes.c_void_p * max(len(values), 1))(*[t.data_ptr() for t in values])
-            ip = (ctypes.c_void_p * max(len(indices), 1))(*[t.data_ptr() for t in indices])
-            op = (ctypes.c_void_p * max(len(outputs), 1))(*[t.data_ptr() for t in outputs])
-            st = syms.launch(ctypes.byref(desc), vp, ip,
-                             ctypes.c_void_p(row_end_offsets.data_ptr() if has_red else 0), op,
-                             ctypes.c_void_p(plan.ws.data_ptr()), ctypes.c_size_t(plan.nbytes), _stream_ptr())
-        check(self.lib, st, "launch_into")
-        self.launches += 1
-        if _CHECK_EVERY_CALL:
-            self.check()
+        self._launch(self._by_type(values[0].dtype), values, indices, row_end_offsets, outputs, num_rows, num_edges, num_cols,
+                     values[0].device, "launch_into")
 
     def prepare(self, values: Sequence[torch.Tensor], indices: Sequence[torch.Tensor],
                 row_end_offsets: Optional[torch.Tensor], outputs: Sequence[torch.Tensor],
@@ -363,14 +375,11 @@ class GraphExtension:
         the reference wrapper re-marshals every argument on every call
         (python_wrapper/dynamic_replace_submodule.py:147-199).  The row offsets must not change while the
         object is in use; the value / index / output tensors may be rewritten in place."""
-        dt = values[0].dtype
-        syms = self.symbols(dt)
-        has_red = self.ir.has_reducer
+        syms = self._by_type(values[0].dtype)
         device = values[0].device
-        desc = self._desc(syms, values, row_end_offsets, num_rows, num_edges, num_cols, indices)
         with torch.cuda.device(device):
-            plan = self._workspace(syms, desc, row_end_offsets if has_red else None, device, indices)
-        return PreparedLaunch(self, syms, desc, list(values), list(indices), row_end_offsets if has_red else None,
+            plan, desc = self._plan_for(syms, values, indices, row_end_offsets, num_rows, num_edges, num_cols, device)
+        return PreparedLaunch(self, syms, desc, list(values), list(indices), row_end_offsets if self._has_reducer else None,
                               list(outputs), plan)
 
     def device_status(self, dtype: torch.dtype, row_end_offsets: Optional[torch.Tensor] = None) -> int:
@@ -422,31 +431,28 @@ class PreparedLaunch:
         self._planned = torch.cuda.Event()                    # the plan kernels were enqueued on this stream
         self._planned.record(torch.cuda.current_stream(ws.device))
         self._ordered = {torch.cuda.current_stream(ws.device).cuda_stream}
-        vp = (ctypes.c_void_p * max(len(values), 1))(*[t.data_ptr() for t in values])
-        ip = (ctypes.c_void_p * max(len(indices), 1))(*[t.data_ptr() for t in indices])
-        op = (ctypes.c_void_p * max(len(outputs), 1))(*[t.data_ptr() for t in outputs])
-        self._args = (ctypes.byref(desc), vp, ip, ctypes.c_void_p(ro.data_ptr() if ro is not None else 0), op,
-                      ctypes.c_void_p(ws.data_ptr()), ctypes.c_size_t(ws_bytes))
+        self._args = (ctypes.byref(desc), _pointers(values), _pointers(indices), ro.data_ptr() if ro is not None else 0,
+                      _pointers(outputs), ws.data_ptr(), ws_bytes)
         self._fn = syms.launch
 
     def launch(self) -> None:
         """Enqueues the fused pass on the current stream of the tensors' device.  The workspace carries
         per-launch state, so launches of one prepared object must be stream-ordered with one another:
         launching from a second stream needs a second prepared object."""
-        if torch.cuda.current_device() != self._device:
+        if _current_device() != self._device:
             with torch.cuda.device(self._device):
                 return self.launch()
         if self._plan._flag_view[0]:
             _raise_if_failed(self.ext.lib, self._plan, "launch")
-        stream = torch.cuda.current_stream()
-        if stream.cuda_stream not in self._ordered:           # first use on another stream: after the plan
+        stream = _raw_stream(self._device)
+        if stream not in self._ordered:                       # first use on another stream: after the plan
             if torch.cuda.is_current_stream_capturing():
                 # an event recorded outside a capture cannot be waited on inside it
                 raise FlexSpmvError("first launch of a prepared object on a stream that is being captured: launch it "
                                     "once on that stream before the capture begins")
-            stream.wait_event(self._planned)
-            self._ordered.add(stream.cuda_stream)
-        st = self._fn(*self._args, ctypes.c_void_p(stream.cuda_stream))
+            torch.cuda.current_stream().wait_event(self._planned)
+            self._ordered.add(stream)
+        st = self._fn(*self._args, stream)
         if st != 0:
             check(self.ext.lib, st, "launch")
         self.ext.launches += 1
