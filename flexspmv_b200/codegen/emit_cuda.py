@@ -127,10 +127,13 @@ def choose_config(ir: GraphIR, dtype: str) -> Tuple[int, int, int, int]:
 # heuristic of choose_config.  In the fused row mode one more resident CTA beats a wider register batch: the
 # other warps hide the gather latency better than more loads in flight per thread do.
 TUNED_CONFIGS = {
-    "spmv_f64": (256, 5, 2, 4),          # 7-point fp64 SpMV: 70 % of the HBM peak; 3 stages / bigger CTAs / 3 or 5 CTAs all lower
+    # 7-point fp64 SpMV: 70 % of the HBM peak in the loop with carries, 85 % in the loop over whole rows (512^3, us: 2602; 3 / 5
+    # CTAs per SM 2818 / 3006, 384 threads x 3 2560, 512 x 2 2533, 192 x 5 2750, 2048-item tiles x 3 3264)
+    "spmv_f64": (256, 5, 2, 4),
     "spmv_f32": (256, 5, 2, 4),
     "spmv_i64": (256, 5, 2, 4),
-    # warm / L2-flushed % of the HBM peak:
+    # warm / L2-flushed % of the HBM peak, in the loop with carries (matrices of short rows now take the loop over whole
+    # rows: 47.5 % on the lattice, 52 % on the Rusanov mesh):
     # (seventh field: edges per batch in the loop over whole rows: spring_mass_f32 1 / 2 / 4: 38.9 / 40.5 / 44.3 us)
     "spring_mass_f32": (256, 8, 2, 4, 0, 2, 1),   # 35.5 / 31.2: 2048-item tiles hold ~228 rows of 8 edges, one per thread (batch 4: 34.9 / 31.2, batch 1 x 5 CTAs: 36.1 / 29.2, batch 8: 25)
     "rusanov_f64": (256, 4, 2, 3, 0, 1),       # 33.1 / 30.9: 1024-item tiles hold 256 rows of 3 edges (batch 2: 29.4 / 27.6, batch 3: 27.3 / 25.9, batch 1 x 4 CTAs: 30.3 / 28.7)
