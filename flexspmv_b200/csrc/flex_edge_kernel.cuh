@@ -37,6 +37,8 @@ __global__ void __launch_bounds__(BLOCK) flex_edge_kernel(const typename G::Para
   __shared__ V s_part[kWarps * kAgg];
   __shared__ int s_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();                  // launched while the kernel before it on the stream drains (see flex_tile_kernel.cuh)
+  pdl_launch_dependents();
   // a workspace that was not planned for this problem holds an arbitrary ticket: every CTA sees the same
   // header, so all of them leave here and nothing is written
   if (a.header->magic != kMagic || a.header->num_edges != a.num_edges || a.header->num_tiles != 0) {

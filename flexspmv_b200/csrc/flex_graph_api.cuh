@@ -37,6 +37,20 @@ inline bool pdl_enabled() {
   return on;
 }
 
+// Launches with the programmatic-dependent-launch attribute: the CTAs may be placed while the kernel before this one on
+// the stream drains; the kernels touch no global memory before their griddepcontrol.wait.  Back-to-back launches of
+// small problems (a time-stepping loop) then overlap one launch's set-up with the tail of the one before.
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3((unsigned)block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 struct NoWindows {   // in place of CfgWin: the gather-window variant of the kernel is not built and the flag is ignored
   static constexpr int kTile = 0;
 };
@@ -252,16 +266,7 @@ struct GraphApi {
       a.win_table = reinterpret_cast<const int*>(static_cast<char*>(ws) + h.win_table_offset);
       a.win_index = reinterpret_cast<const unsigned short*>(static_cast<char*>(ws) + h.win_index_offset);
     }
-    // Programmatic dependent launch: the CTAs may be placed while the kernel before this one on the stream drains; the
-    // kernel touches no global memory before its griddepcontrol.wait.  Back-to-back launches of small problems
-    // (a time-stepping loop) then overlap one launch's set-up with the tail of the one before.
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = L::kTotal; cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, p, a);
+    return launch_pdl(kernel, (unsigned)grid, kThreads, L::kTotal, st, p, a);
   }
 
   template <typename OffsetT>
@@ -304,8 +309,7 @@ struct GraphApi {
       a.carry_row = reinterpret_cast<long long*>(static_cast<char*>(ws) + h.carry_row_offset);
       a.carry_val = static_cast<char*>(ws) + h.carry_val_offset;
       a.num_rows = d->num_rows; a.num_edges = d->num_edges; a.num_chunks = chunks;
-      kernel<<<(unsigned)grid, CfgLean::kBlock, kSmem, st>>>(p, a);
-      return (int)cudaGetLastError();
+      return launch_pdl(kernel, (unsigned)grid, CfgLean::kBlock, kSmem, st, p, a);
     } else {
       (void)d; (void)p; (void)row_offsets; (void)ws; (void)h; (void)st;
       return FLEXSPMV_ERR_BAD_ARG;
@@ -373,8 +377,7 @@ struct GraphApi {
     a.header = static_cast<WorkspaceHeader*>(ws);
     a.partials = static_cast<char*>(ws) + h.carry_val_offset;
     a.num_edges = d->num_edges;
-    flex_edge_kernel<G, kEdgeBlock, kEdgeIpt><<<(unsigned)grid, kEdgeBlock, 0, st>>>(p, a);
-    return (int)cudaGetLastError();
+    return launch_pdl(flex_edge_kernel<G, kEdgeBlock, kEdgeIpt>, (unsigned)grid, kEdgeBlock, 0, st, p, a);
     }
   }
 

@@ -105,6 +105,10 @@ flex_warp_kernel(const typename G::Params p, const WarpKernelArgs a) {
   const OffsetT* ro = static_cast<const OffsetT*>(a.row_offsets);
   const OffsetT* coords = static_cast<const OffsetT*>(a.coords);
 
+  // launched while the kernel before it on the stream drains (see flex_tile_kernel.cuh): 200 003 power-law rows fp64,
+  // back to back, 32.6 -> 30.7 us
+  pdl_wait();
+  pdl_launch_dependents();
   if (a.header->magic != kMagic || a.header->num_tiles != a.num_chunks || a.header->num_rows != a.num_rows ||
       a.header->num_edges != a.num_edges || a.header->offset_bits != (int)(8 * sizeof(OffsetT))) {
     if (tid == 0 && blockIdx.x == 0) raise_not_planned(a.header);
