@@ -250,8 +250,16 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     return;
   }
 
+  // An epilogue needs a row's whole sum: a matrix that was not planned with whole rows is refused here, where every CTA
+  // leaves before its producer warp has issued a copy (one still in flight would write into shared memory that a later CTA owns).
+  if constexpr (G::kEpilogue) {
+    if (a.header->whole_rows != 1) {
+      if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
+      return;
+    }
+  }
   // every tile holds whole rows only (any grid): stages of the loop over whole rows, in its places
-  const bool whole = WHOLE && a.header->whole_rows == 1;
+  const bool whole = WHOLE && (G::kEpilogue || a.header->whole_rows == 1);
   const int nstages = WHOLE ? (whole ? L::kRowStages : S) : S;
   unsigned char* const stage_base = (WHOLE && whole) ? smem + L::kOffRowStages : s_stage;
 
@@ -586,11 +594,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     }
   }
 
-  // an epilogue needs a row's whole sum: a matrix that was not planned with whole rows is refused
-  if constexpr (G::kEpilogue) {
-    if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
-    return;
-  }
+  if constexpr (G::kEpilogue) return;     // has the loop above only
 
   // ---- phase 1 pieces: lanes on consecutive edges ------------------------------------------------------
   auto map_load = [&](const TileRef& t, const TileT& tile, typename G::EReg (&er)[IPT]) {

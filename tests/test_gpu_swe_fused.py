@@ -4,8 +4,8 @@ import numpy as np
 import pytest
 import torch
 
-from flexspmv_b200 import problems
-from flexspmv_b200.binding import load_builtin
+from flexspmv_b200 import graphs, problems
+from flexspmv_b200.binding import FlexSpmvError, GraphExtension, load_builtin
 from flexspmv_b200.shallow_water import ShallowWaterStep
 
 pytestmark = pytest.mark.gpu
@@ -42,8 +42,8 @@ def test_fused_stage_equals_three_launches(n, dtype, split_walls):
         assert torch.equal(a[name], b[name]), name
 
 
-def test_a_cell_with_many_edges_takes_three_launches():
-    m = mesh_of(24, np.float64, False)
+def mesh_with_a_long_row(n):
+    m = mesh_of(n, np.float64, False)
     src, dst = m["src"], m["dst"]
     many = torch.full((40,), 5, dtype=torch.int32, device="cuda")          # 40 more edges into cell 7
     order = torch.argsort(torch.cat([dst, many + 2]).long(), stable=True)
@@ -51,8 +51,35 @@ def test_a_cell_with_many_edges_takes_three_launches():
         m[k] = torch.cat([m[k], extra])[order].contiguous()
     for k in ("alpha", "sx", "sy"):
         m[k] = torch.cat([m[k], torch.full((40,), 0.25, dtype=torch.float64, device="cuda") * (0.0 if k != "alpha" else 1.0)])[order].contiguous()
+    return m
+
+
+def test_a_cell_with_many_edges_takes_three_launches():
+    m = mesh_with_a_long_row(24)
     step = ShallowWaterStep(m, dt=1e-3)
     assert step._fused is None
     step.forward()
     torch.cuda.synchronize()
     assert torch.isfinite(m["h"]).all()
+
+
+@pytest.mark.parametrize("max_ctas", [0, 1])      # one tile a CTA, and more tiles than a CTA has stages
+def test_the_epilogue_refuses_a_plan_without_whole_rows(max_ctas):
+    """The launch leaves at the header, before any copy: the status is "not planned" (no wait ran out), nothing is written."""
+    m = mesh_with_a_long_row(48)
+    nc, ne = m["h"].numel(), m["src"].numel()
+    ext = GraphExtension(graphs.swe_delta_graph(), symbol_prefix="swe_delta_rk", max_ctas=max_ctas)
+    ro = torch.searchsorted(m["dst"], torch.arange(nc + 1, dtype=torch.int32, device="cuda")).to(torch.int32)
+    walls = torch.searchsorted(m["bcells"], torch.arange(0, nc + 32, 32, dtype=torch.int32, device="cuda")).to(torch.int32)
+    state = [m[k] for k in ("h", "uh", "vh")]
+    before = [t.clone() for t in state]
+    acc, out = ([torch.full((nc,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(3)] for _ in range(2))
+    coef = torch.tensor([1e-3, 1e-3, 0.0, 1.0], dtype=torch.float64)
+    values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], walls, m["bcells"]] + state + acc + [coef]
+    launch = ext.prepare(values, [m["src"], m["dst"]], ro, out, nc, ne, nc)
+    assert not ext.planned_whole_rows()
+    launch.launch()
+    with pytest.raises(FlexSpmvError, match="status -7"):
+        ext.check()
+    assert all(torch.equal(a, b) for a, b in zip(state, before))
+    assert all(torch.isnan(t).all() for t in acc + out)
