@@ -55,7 +55,8 @@ __global__ void snap_cta_boundaries_kernel(const OffsetT* __restrict__ row_offse
     const long long rows_behind = (long long)coords[2 * t + 2] - x; // row ends in the tile behind the boundary
     const long long y_before = (long long)coords[2 * t - 1];        // where the tile in front of it starts
     const long long edges_behind = (long long)coords[2 * t + 3] - begin;
-    if (y - begin > rows_behind || begin < y_before || !room.fits(edges_behind, rows_behind)) s_ok = 0;
+    // begin > y: offsets that do not start at 0 or do not ascend; the boundary would move forward
+    if (begin > y || y - begin > rows_behind || begin < y_before || !room.fits(edges_behind, rows_behind)) s_ok = 0;
   }
   __syncthreads();
   if (!s_ok) return;
@@ -80,9 +81,21 @@ int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long 
   return (int)cudaGetLastError();
 }
 
+// First edge of tile t once its front boundary has moved to a row start.  Edge 0 belongs to the first tile whatever
+// row_offsets[0] says, and boundaries behind the last row end stay where the merge path put them.
+template <typename OffsetT>
+__device__ __forceinline__ long long moved_edge(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
+                                                long long num_tiles, const OffsetT* __restrict__ coords, long long t) {
+  if (t <= 0) return 0;
+  if (t >= num_tiles) return num_edges;
+  const long long x = (long long)coords[2 * t];
+  return x < num_rows ? (long long)row_offsets[x] : (long long)coords[2 * t + 1];
+}
 // One warp per tile: would every row stay whole with all tile boundaries moved back to row starts -- rows of at most
 // kWholeRowMax edges, tiles that still fit -- and how many thread-steps would one thread per row take?  Leaves
-// whole_rows = -1 when a row or a tile is too large.
+// whole_rows = -1 when a row or a tile is too large.  Unlike the merge path, which stays inside [0, num_edges] for any
+// offsets, moved boundaries are offsets themselves: ones that descend, end behind the edges or leave a gap in front of the
+// first row (all of which the loop with carries takes without reading out of range) are refused here.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
                                                          long long num_tiles, const TileRoom room, const OffsetT* __restrict__ coords,
@@ -93,13 +106,17 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
   bool bad = false;
   for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < num_tiles && !bad; t += warps) {
     const long long x0 = (long long)coords[2 * t], x1 = (long long)coords[2 * t + 2];
-    const long long y0 = (long long)row_offsets[x0];                        // x0 == num_rows: num_edges
-    const long long y1 = (t + 1 < num_tiles) ? (long long)row_offsets[x1] : num_edges;
-    bad = !room.fits(y1 - y0, x1 - x0);
+    const long long y0 = moved_edge(row_offsets, num_rows, num_edges, num_tiles, coords, t);
+    const long long y1 = moved_edge(row_offsets, num_rows, num_edges, num_tiles, coords, t + 1);
+    bad = y0 < 0 || y1 < y0 || y1 > num_edges || !room.fits(y1 - y0, x1 - x0);
     for (long long r0 = x0; r0 < x1; r0 += 32) {
       const long long r = r0 + lane;
       long long len = 0;
-      if (r < x1) len = (long long)row_offsets[r + 1] - (long long)row_offsets[r];
+      if (r < x1) {
+        const long long end = (long long)row_offsets[r + 1];
+        len = end - (r == x0 ? y0 : (long long)row_offsets[r]);
+        if (len < 0 || end > y1) len = kWholeRowMax + 1;
+      }
       const int longest = __reduce_max_sync(0xffffffffu, (int)(len > kWholeRowMax ? kWholeRowMax + 1 : len));
       bad |= longest > kWholeRowMax;
       slots += 32u * (unsigned)longest;

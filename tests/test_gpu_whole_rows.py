@@ -113,3 +113,36 @@ def test_a_moved_boundary_never_overfills_a_stage(bits):
     assert raw[33] == 0
     got, _ = run_gpu(GraphExtension(ir), ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
     assert_outputs_match(ir, got, ref, sums, np.dtype(dtype), what="cut row in front of short ones")
+
+
+@pytest.mark.parametrize("gname,dt", [("spmv", "float64"), ("rusanov", "float32")])
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("first_len,first_offset,unused,whole", [(5, 3, 0, True),      # the first row is [0, ends[0]) whatever
+                                                                 (5000, 5000, 0, False), (5000, 4999, 0, False),
+                                                                 (7, 0, 9, True), (7, 0, 9000, True)])    # edges of no row
+def test_offsets_that_do_not_span_the_edges_keep_every_tile_in_bounds(gname, dt, bits, first_len, first_offset, unused, whole):
+    """Offsets are taken as row ends: the leading one counts as 0 and edges behind the last row belong to none.  A boundary
+    moved to such a row start must not leave a tile with more edges than its stage holds (coordinates in the workspace),
+    and the rows are those of the same matrix with a leading 0 and without the unused edges."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [first_len] + [4, 6] * 1500, 17, dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    prob.row_offsets[0] = first_offset
+    edge_arrays = {s["target"] for s in ir.selector_register if s.get("selector") != 1}
+    for name in edge_arrays:
+        v = prob.values[name]
+        prob.values[name] = np.concatenate([v, v[:1].repeat(unused, axis=0)])
+    for k, v in prob.indices.items():
+        prob.indices[k] = np.concatenate([v, np.zeros(unused, v.dtype)])
+    for kw in ({}, {"max_ctas": 3}):
+        ext = GraphExtension(ir, random_gather=False, **kw)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+        ext.check()
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} {first_len} {first_offset} {unused} {kw}")
+        assert ext.planned_whole_rows() == whole
+        info = ext.symbols(torch.float64 if dt == "float64" else torch.float32).graph_info
+        tiles = -(-(prob.num_rows + prob.indices[ext.index_names[0]].size) // info.default_tile_items)
+        raw = next(reversed(ext._plans.values())).ws[256:256 + (tiles + 1) * bits // 4].cpu().numpy()
+        coords = raw.view(np.int32 if bits == 32 else np.int64).reshape(-1, 2)
+        steps = np.diff(coords[:, 1])
+        assert steps.min() >= 0 and steps.max() <= info.block_threads * info.items_per_thread
