@@ -553,8 +553,9 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
           const int r = (g << 5) + lane;
           int lo = 0, hi = 0;
           if (r < c.nrows) {
-            hi = (int)rend[r] - (int)c.nz0;
-            if (r) lo = (int)rend[r - 1] - (int)c.nz0;
+            // unsigned: the ends may lie on either side of edge 2^31, and the difference is right modulo 2^32
+            hi = (int)((unsigned)rend[r] - (unsigned)c.nz0);
+            if (r) lo = (int)((unsigned)rend[r - 1] - (unsigned)c.nz0);
           }
           V sum[kAcc];
 #pragma unroll

@@ -146,3 +146,37 @@ def test_offsets_that_do_not_span_the_edges_keep_every_tile_in_bounds(gname, dt,
         coords = raw.view(np.int32 if bits == 32 else np.int64).reshape(-1, 2)
         steps = np.diff(coords[:, 1])
         assert steps.min() >= 0 and steps.max() <= info.block_threads * info.items_per_thread
+
+
+def test_row_mode_rows_on_both_sides_of_edge_two_to_the_31():
+    """Rows of 16 edges with 64-bit offsets up to 2^31 + 160 000: in the tile around edge 2^31 the positions of a row's ends
+    differ in sign as 32-bit numbers.  The rows there, the first and the last ones against the map in torch."""
+    if torch.cuda.get_device_properties(0).total_memory < 120 * 2 ** 30:
+        pytest.skip("needs a 180 GB device")
+    rows = 2 ** 27 + 10_000
+    ne = 16 * rows
+    assert ne > 2 ** 31
+    rng = torch.Generator(device="cuda")
+    rng.manual_seed(23)
+    rest, stiff = (torch.rand(ne, generator=rng, device="cuda", dtype=torch.float32) for _ in range(2))
+    pos = torch.rand(rows, 2, generator=rng, device="cuda", dtype=torch.float32)
+    src = torch.arange(rows, device="cuda", dtype=torch.int32).repeat_interleave(16)
+    dst = src + torch.randint(1, 1000, (ne,), generator=rng, device="cuda", dtype=torch.int32)
+    dst[dst >= rows] -= rows
+    ro = torch.arange(rows + 1, device="cuda", dtype=torch.int64) * 16
+    ext = GraphExtension(graphs.spring_mass_graph())
+    (got,) = ext.merged_spmv_launch(rest, stiff, pos, src, dst, ro, rows, rows)
+    ext.check()
+    assert ext.planned_whole_rows()
+    for first in (0, 2 ** 27 - 5000, rows - 5000):
+        e = slice(16 * first, 16 * (first + 5000))
+        k, rest_len = stiff[e, None].double(), rest[e, None].double()
+        d = (pos[dst[e].long()] - pos[src[e].long()]).double()       # one rounding, the same as the map's
+        n = d.norm(dim=1, keepdim=True)
+        f = (k * (n - rest_len) * d / n).view(5000, 16, 2)
+        # in units of 2^-24: the norm is off by 3 n, which k d / n turns into 3 k |d|; five more roundings of the term and
+        # fifteen additions of at most the sum of the magnitudes
+        bound = (3 * (k * d.abs()).view(5000, 16, 2) + 20 * f.abs()).sum(dim=1) * 2.0 ** -24
+        assert ((got[first:first + 5000].double() - f.sum(dim=1)).abs() <= bound).all()
+    del rest, stiff, pos, src, dst, ro, got
+    torch.cuda.empty_cache()
