@@ -65,7 +65,8 @@ class ShallowWaterStep:
         self.delta_ext.lib.flexspmv_swe_rk_stage.restype = ctypes.c_int
 
     def _coefficients(self):
-        """(c, first, last) of the four stages: the next state is x + c d, the last one adds dt / 6 of the sum."""
+        """(c, first, last) of the four stages at the present ``dt``: the next state is x + c d, the last one adds dt / 6
+        of the sum."""
         return ((0.5 * self.dt, 1, 0), (0.5 * self.dt, 0, 0), (self.dt, 0, 0), (0.0, 0, 1))
 
     def _bind_fused(self, new):
@@ -80,10 +81,13 @@ class ShallowWaterStep:
         other = new(3)
         state = [m["h"], m["uh"], m["vh"]]
         launches = []
+        self._coef, self._coef_dt = [], float(self.dt)
         for k, (c, first, last) in enumerate(self._coefficients()):
             src = state if k == 0 else (self.stage if k % 2 else other)
             dst = other if k % 2 else self.stage          # the last stage writes the state itself
-            coef = torch.tensor([c, self.dt / 6, first, last], dtype=dt_)      # host memory, read at every launch
+            # host memory, read when a launch is made
+            coef = torch.tensor([c, self.dt / 6, first, last], dtype=dt_, device="cpu")
+            self._coef.append(coef)
             values = [m["alpha"], m["sx"], m["sy"]] + src + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [coef]
             launches.append(ext.prepare(values, [m["src"], m["dst"]], self.ro, dst, self.nc, self.ne, self.nc))
             if k == 0 and not ext.planned_whole_rows():
@@ -108,8 +112,14 @@ class ShallowWaterStep:
         check(self.delta_ext.lib, st, "swe_rk_stage")
 
     def forward(self) -> None:
-        """swe_main.py:121-146: four delta evaluations (:86-119), each followed by its stage update."""
+        """swe_main.py:121-146: four delta evaluations (:86-119), each followed by its stage update.  ``dt`` may be set
+        between calls (a step captured by ``capture`` keeps the one it was captured with)."""
         if self._fused is not None:
+            dt = float(self.dt)
+            if dt != self._coef_dt:
+                for coef, (c, first, last) in zip(self._coef, self._coefficients()):
+                    coef.copy_(torch.tensor([c, dt / 6, first, last], dtype=coef.dtype, device="cpu"))
+                self._coef_dt = dt
             for launch in self._fused:
                 launch.launch()
             return

@@ -42,6 +42,30 @@ def test_fused_stage_equals_three_launches(n, dtype, split_walls):
         assert torch.equal(a[name], b[name]), name
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_the_time_step_may_change_between_eager_steps(dtype):
+    """A program that sets ``dt`` from its state: every step takes the present one, in either form."""
+    a, b = mesh_of(33, dtype, False), mesh_of(33, dtype, False)
+    fused = ShallowWaterStep(a, dt=1e-3)
+    apart = ShallowWaterStep(b, dt=1e-3, delta_ext=load_builtin("swe_delta"), boundary_ext=load_builtin("swe_boundary"))
+    assert fused._fused is not None and apart._fused is None
+    for dt in (None, 2e-3, 0.5e-3, 0.5e-3, 1e-3):
+        start = a["h"].clone()
+        for step in (fused, apart):
+            if dt is not None:
+                step.dt = dt
+            step.forward()
+        assert not torch.equal(a["h"], start)
+        for name in ("h", "uh", "vh"):
+            assert torch.isfinite(a[name]).all() and torch.equal(a[name], b[name]), (dt, name)
+    fused.capture()                      # the captured step keeps the time step it was captured with
+    fused.dt = 5e-3
+    fused.replay()
+    apart.forward()
+    for name in ("h", "uh", "vh"):
+        assert torch.equal(a[name], b[name]), name
+
+
 def mesh_with_a_long_row(n):
     m = mesh_of(n, np.float64, False)
     src, dst = m["src"], m["dst"]
