@@ -280,6 +280,9 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w(f"  static constexpr bool kDirectLoads = {'true' if direct_loads(ir, dtype) else 'false'};")
     needs_row = any(s.get("selector") == 1 and s.get("row_identity") for s in ir.selector_register)
     w(f"  static constexpr bool kGatherNeedsRow = {'true' if needs_row else 'false'};")
+    # nothing in the map that takes tens of instructions an edge (flex_tile_kernel.cuh, WholeRows)
+    light = not any(op_["op"] in ("truediv", "pow", "exp", "norm") for op_ in ir.map_operations)
+    w(f"  static constexpr bool kLightMap = {'true' if light else 'false'};")
     w("  static constexpr int kStreamBytesPerEdge = 0" + "".join(f" + {b}" for _, _, b in streams) + ";")
     w("  struct Params {")
     for n in value_names:

@@ -47,9 +47,10 @@ struct WorkspaceHeader {
   uint64_t status_mirror;      // device alias of a pinned host int32 that receives a copy of `status` when a
                                // kernel raises an error (0: none); lets the host notice without a sync or a copy
   uint64_t row_slots;          // what whole_rows_kernel counted: 32 x the longest row, over groups of 32 rows
-  int32_t whole_rows;          // 1: EVERY tile boundary sits on a row end and no row is longer than kWholeRowMax: the
-                               // tile kernel runs its loop without barriers, for any grid (-1: looked at and refused)
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 4];
+  int32_t whole_rows;          // 1: EVERY tile boundary sits on a row end and no row is longer than kWholeRowMax: no launch
+                               // on this workspace hands carries over, whatever its grid (-1: looked at and refused)
+  int32_t row_loop;            // 1: and the tile kernel runs its loop over whole rows
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 2 * 4];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"

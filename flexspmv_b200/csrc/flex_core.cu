@@ -131,10 +131,11 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
 // an edge to work on: rows of very different lengths are better off with the two-phase loop, whose lanes take
 // consecutive edges.  1 M rows, fp64 SpMV, this loop / the two-phase loop: lengths 0 - 8 evenly (share 0.50) 16.4 / 21.0 us,
 // 0 - 16 evenly (0.51) 29.0 / 35.6 us, exponential of mean 4 (0.22) 24.4 / 24.3 us, 32 in 3 % of the rows and 2 elsewhere
-// (0.14) 30.9 / 20.1 us.
+// (0.14) 30.9 / 20.1 us.  `row_loop`: the kernel has the loop over whole rows.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                                               long long num_tiles, OffsetT* __restrict__ coords, WorkspaceHeader* h) {
+                                                               long long num_tiles, int row_loop, OffsetT* __restrict__ coords,
+                                                               WorkspaceHeader* h) {
   if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1) return;
   if (2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -142,27 +143,30 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __
     const long long x = (long long)coords[2 * t];
     if (x < num_rows) coords[2 * t + 1] = row_offsets[x];
   }
-  if (t == 0) *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;     // read by this kernel only as "-1 or not"
+  if (t == 0) {
+    *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;     // read by this kernel only as "-1 or not"
+    h->row_loop = row_loop;
+  }
 }
 
 template <typename OffsetT>
 static int whole_rows_launch_as(const void* d_row_offsets, long long num_rows, long long num_edges, long long num_tiles,
-                                const TileRoom& room, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
+                                const TileRoom& room, bool row_loop, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
   const OffsetT* ro = static_cast<const OffsetT*>(d_row_offsets);
   OffsetT* coords = static_cast<OffsetT*>(d_coords);
   long long grid = (num_tiles + 7) / 8;
   const long long cap = (long long)device_sm_count() * 8;
   if (grid > cap) grid = cap;
   whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, coords, h);
-  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, coords, h);
+  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, row_loop ? 1 : 0, coords, h);
   return (int)cudaGetLastError();
 }
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream) {
+                      const TileRoom& room, bool row_loop, void* d_coords, void* ws, cudaStream_t stream) {
   if (num_tiles < 1 || num_rows < 1) return 0;
   WorkspaceHeader* h = static_cast<WorkspaceHeader*>(ws);
-  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, d_coords, h, stream);
-  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, d_coords, h, stream);
+  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, row_loop, d_coords, h, stream);
+  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, row_loop, d_coords, h, stream);
 }
 
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,

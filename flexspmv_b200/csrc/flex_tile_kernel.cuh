@@ -10,9 +10,9 @@
 //   thread per row loads the row's own record once, gathers and maps its edges in register batches and
 //   stores the row; in tiles with a long row whole warps take the rows one at a time (lanes 32 edges
 //   apart, shuffle tree).  Nothing of a row-mode graph passes through a shared-memory product buffer.
-//   Whole rows (either kind of graph, when the plan found a matrix of short rows whose tiles can all hold whole rows):
-//   no carries at all, so no barriers either -- every warp takes 32 rows of a staged tile, one per lane, and keeps
-//   everything in registers.
+//   Whole rows (row-mode graphs and graphs of light maps, when the plan found a matrix of short rows whose tiles can all
+//   hold whole rows): no carries at all, so no barriers either -- every warp takes 32 rows of a staged tile, one per lane,
+//   and keeps everything in registers.  The other two loops run on such tiles too, without carries between CTAs.
 // The carry of a row that spans tiles travels inside the CTA in shared memory; the only cross-CTA state
 // is one carry per CTA, folded in by the last CTA to finish (ticket counter), in CTA order.  No atomics
 // on the output, no pre-zeroed output, run-to-run deterministic.
@@ -51,11 +51,20 @@ struct TileCfg {
   static constexpr int kRowBatch = ROW_BATCH_;   // the same in the loop over whole rows
 };
 
-// Whether the kernel has the loop over whole rows: staged graphs that write nothing per edge (a thread that walks a row
-// would store its edges' outputs a row length apart).
+// Whether the plan may move all tile boundaries of the graph to row starts: staged graphs that write nothing per edge.
+template <class G, class Cfg, bool WIN>
+struct WholeTiles {
+  static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
+};
+// Whether the kernel has the loop over whole rows, one row per lane: graphs with per-row data, whose other loop has a thread
+// per row as well, and graphs whose map is a few adds and multiplies.  A map that divides or calls pow or exp is worth more
+// than the gathers it waits for, and there lanes on consecutive edges do nothing in vain: in the loop over rows a lane idles
+// while another one's row goes on.  us, this loop / the two-phase loop, 6 M edges fp64, 3 / 8 / 20 / 31 edges a row and 0 - 8:
+//   4 divisions an edge  39 / 50,  40 / 45,  41 / 43,  55 / 43,  66 / 48;   1 pow  65 / 74,  70 / 70,  72 / 68,  99 / 69,  120 / 73;
+//   0.2 M edges, 31 a row:  1 / 2 divisions  8.7 / 7.1,  10.4 / 6.9,  1 pow  20 / 8.7.
 template <class G, class Cfg, bool WIN>
 struct WholeRows {
-  static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
+  static constexpr bool value = WholeTiles<G, Cfg, WIN>::value && (G::kGatherNeedsRow || G::kLightMap);
 };
 
 constexpr int kMaxCtas = 2048;            // capacity of the per-CTA carry arrays in the workspace
@@ -258,8 +267,8 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       return;
     }
   }
-  // every tile holds whole rows only (any grid): stages of the loop over whole rows, in its places
-  const bool whole = WHOLE && (G::kEpilogue || a.header->whole_rows == 1);
+  // the loop over whole rows has its own stages, in its own places
+  const bool whole = WHOLE && (G::kEpilogue || a.header->row_loop == 1);
   const int nstages = WHOLE ? (whole ? L::kRowStages : S) : S;
   unsigned char* const stage_base = (WHOLE && whole) ? smem + L::kOffRowStages : s_stage;
 
@@ -366,7 +375,8 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   }
   if (tid < 2 * kAcc) s_carry[tid] = V(0);
   if (tid < 4) s_nlong[tid] = 0;
-  if (tid == 0) s_flag[1] = (a.header->snapped_grid == (int)gridDim.x) ? 1 : 0;   // no row spans two CTAs of this launch
+  // no row spans two CTAs of this launch
+  if (tid == 0) s_flag[1] = (a.header->whole_rows == 1 || a.header->snapped_grid == (int)gridDim.x) ? 1 : 0;
   __syncthreads();   // the only barrier that includes the producer warp
 
   // ---- producer warp: runs up to S tiles ahead of the consumers, off their critical path -----------

@@ -219,9 +219,10 @@ int flexspmv_swe_rk_stage(int32_t value_bytes, const void *const *d_r, const voi
                           int32_t last, void *stream);
 
 /* Copies to *d_out (int32 in device or page-locked host memory), without synchronising, 1 when the plan in the workspace
- * found a matrix of short rows (at most 32 edges) whose tiles all hold whole rows: the launches then run a loop without
- * carries or barriers, and a graph with an epilogue (swe_delta_rk_*: swe_delta with the stage of flexspmv_swe_rk_stage
- * behind its sums, csrc/flex_swe_rk.cuh) accepts the workspace. */
+ * found a matrix of short rows (at most 32 edges) whose tiles all hold whole rows.  Launches on it hand no carries over,
+ * whatever their grid; row-mode graphs and graphs of light maps run a loop without barriers on it, and a graph with an
+ * epilogue (swe_delta_rk_*: swe_delta with the stage of flexspmv_swe_rk_stage behind its sums, csrc/flex_swe_rk.cuh)
+ * accepts the workspace. */
 int flexspmv_workspace_whole_rows(const void *d_workspace, int32_t *d_out, void *stream);
 
 /* ---- per fused graph ---------------------------------------------------------------------------

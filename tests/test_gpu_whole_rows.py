@@ -62,6 +62,31 @@ def test_whole_rows_match_the_oracle(gname, dt, case):
             assert ext.planned_whole_rows() == (planned == 1), (case, kw)
 
 
+def row_loop_planned(ext):
+    """Whether the last plan chose the loop over whole rows (workspace header, int32 at byte 156)."""
+    return int(next(reversed(ext._plans.values())).ws[:256].cpu().numpy().view(np.int32)[39])
+
+
+@pytest.mark.parametrize("gname,dt,expected", [("spmv", "float64", 1), ("rusanov", "float64", 1), ("swe_boundary", "float32", 1),
+                                               ("ops_zoo", "float64", 0), ("ops_zoo", "float32", 0)])
+def test_maps_that_divide_keep_the_two_phase_loop(gname, dt, expected):
+    """A two-phase graph whose map takes tens of instructions an edge: its tiles hold whole rows, so no grid hands carries
+    over, but lanes stay on consecutive edges.  Rows longer than a tile's share of threads, every grid."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [3, 8, 5] * 2000 + [32] * 50, 29, dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    results = []
+    for max_ctas in (0, 1, 7, 50):
+        ext = GraphExtension(ir, random_gather=False, max_ctas=max_ctas)
+        got, _ = run_gpu(ext, ir, prob, dtype)
+        ext.check()
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} {max_ctas}")
+        assert ext.planned_whole_rows() and row_loop_planned(ext) == expected
+        results.append(got)
+    for got in results[1:]:                    # no carries: the grid changes no bit
+        assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(got, results[0]))
+
+
 def test_whole_rows_equal_the_two_phase_loop_bit_for_bit():
     """The same matrix with one row of 33 edges behind it goes through the loop with carries; all other rows are the
     same sums, left to right."""
