@@ -89,6 +89,17 @@ def direct_loads(ir: GraphIR, dtype: str) -> bool:
     return True
 
 
+def light_map(ir: GraphIR) -> bool:
+    """Nothing in the map that takes tens of instructions an edge (WholeRows in csrc/flex_tile_kernel.cuh)."""
+    return not any(op_["op"] in ("truediv", "pow", "exp", "norm") for op_ in ir.map_operations)
+
+
+def stores_per_edge(ir: GraphIR) -> bool:
+    """The map writes per-edge outputs, allocated or in place."""
+    return any(str(o["target"]) != "reducer" and "sum" not in str(o["target"]) for o in ir.outputs) or \
+        any(op_["op"] in ("add_", "copy_", "setitem") for op_ in ir.map_operations)
+
+
 def smem_bytes(ir: GraphIR, dtype: str, block: int, ipt: int, stages: int) -> int:
     """Upper bound of the tile kernel's dynamic shared memory (mirrors TileSmemLayout in
     csrc/flex_tile_kernel.cuh for 64-bit row offsets, the larger of the two instantiations)."""
@@ -96,10 +107,15 @@ def smem_bytes(ir: GraphIR, dtype: str, block: int, ipt: int, stages: int) -> in
     per_edge, ns = _stream_bytes_per_edge(ir, vb)
     acc = max(1, sum(dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer"))
     tile = block * ipt
-    stage = 0 if direct_loads(ir, dtype) else -(-(tile * max(8, per_edge) + 32 * per_edge + 32 * (ns + 1) + 16) // 128) * 128
-    fixed = 16 * 4 + (32 + 4 * max(ns, 1) + 16) * 4 + 4 * (block + 1) + 4 * (block // 32) \
-        + vb * acc * (block // 32) + vb * acc * 2 + 16 + 8 * 16 + 128
     needs_row = any(s_.get("selector") == 1 and s_.get("row_identity") for s_ in ir.selector_register)
+    # tiles whose boundaries the plan may move hold up to 32 edges more; the loop over whole rows has up to four stages
+    moves = not (stores_per_edge(ir) or direct_loads(ir, dtype))
+    row_loop = moves and (needs_row or light_map(ir))
+    ctl = 4 if row_loop else stages
+    stage = 0 if direct_loads(ir, dtype) else \
+        -(-(tile * max(8, per_edge) + (32 * per_edge if moves else 0) + 32 * (ns + 1) + 16) // 128) * 128
+    fixed = 16 * ctl + (32 + 4 * max(ns, 1) + 16) * ctl + 4 * (block + 1) + 4 * (block // 32) \
+        + vb * acc * (block // 32) + vb * acc * 2 + 16 + 8 * 16 + 128
     buffers = 1   # 2 only when the kernel is built with tile pipelining (TileCfg::kPipeline)
     # row-mode graphs reduce in registers: no product buffer
     return fixed + 4 * (tile + 1) * buffers + (0 if needs_row else vb * acc * tile * buffers) + stages * stage
@@ -280,9 +296,7 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w(f"  static constexpr bool kDirectLoads = {'true' if direct_loads(ir, dtype) else 'false'};")
     needs_row = any(s.get("selector") == 1 and s.get("row_identity") for s in ir.selector_register)
     w(f"  static constexpr bool kGatherNeedsRow = {'true' if needs_row else 'false'};")
-    # nothing in the map that takes tens of instructions an edge (flex_tile_kernel.cuh, WholeRows)
-    light = not any(op_["op"] in ("truediv", "pow", "exp", "norm") for op_ in ir.map_operations)
-    w(f"  static constexpr bool kLightMap = {'true' if light else 'false'};")
+    w(f"  static constexpr bool kLightMap = {'true' if light_map(ir) else 'false'};")
     w("  static constexpr int kStreamBytesPerEdge = 0" + "".join(f" + {b}" for _, _, b in streams) + ";")
     w("  struct Params {")
     for n in value_names:
@@ -424,7 +438,7 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w("    (void)t; (void)le; (void)r;")
     w("  }")
     w(f"  static constexpr bool kValuesStaged = {'true' if staged_values else 'false'};")
-    w(f"  static constexpr bool kStoresPerEdge = {'true' if (map_outs or inplace_targets) else 'false'};")
+    w(f"  static constexpr bool kStoresPerEdge = {'true' if stores_per_edge(ir) else 'false'};")
     w("  template <class Tile, class IdxT>")
     w("  __device__ __forceinline__ static void load_edge_vals(const Params& p, const Tile& t, IdxT le, long long e, EReg& r) {")
     seen_e = set()

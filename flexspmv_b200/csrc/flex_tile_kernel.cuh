@@ -109,8 +109,9 @@ struct TileSmemLayout {
   static constexpr int kBytesPerEdge = G::kStreamBytesPerEdge;
   static constexpr int kPerItem = (int(sizeof(OffsetT)) > kBytesPerEdge) ? int(sizeof(OffsetT)) : kBytesPerEdge;
   // a tile's records: kTile merge items, and the edges in front of its first row end when the plan moves the tile's
-  // front boundary back to the start of that row
-  static constexpr int kRecordBytes = Cfg::kTile * kPerItem + kWholeRowMax * kBytesPerEdge;
+  // front boundary back to the start of that row (the gather-window variant may meet such a plan too)
+  static constexpr bool kTilesMove = WholeTiles<G, Cfg, false>::value;
+  static constexpr int kRecordBytes = Cfg::kTile * kPerItem + (kTilesMove ? kWholeRowMax * kBytesPerEdge : 0);
   // each staged window may grow by < 32 bytes from aligning both ends to 16
   static constexpr int kStreamBytes =
       G::kDirectLoads ? 0 : int(align_up(uint64_t(kRecordBytes) + 32u * (G::kNumStreams + 1) + 16, 128));
@@ -124,35 +125,47 @@ struct TileSmemLayout {
     uint32_t roff_off;
     uint32_t stream_off[G::kNumStreams > 0 ? G::kNumStreams : 1];
   };
-  static constexpr int kMaxStages = 4;
-  static constexpr int kOffBars = 0;
-  static constexpr int kOffCtl = int(align_up(kOffBars + 16 * kMaxStages, 16));
-  static constexpr int kOffXs = int(align_up(kOffCtl + sizeof(Ctl) * kMaxStages, 16));
-  static constexpr int kOffWKey = int(align_up(kOffXs + 4 * (Cfg::kBlock + 1), 16));
-  static constexpr int kOffWVal = int(align_up(kOffWKey + 4 * Cfg::kWarps, 16));
-  static constexpr int kOffCarry = int(align_up(kOffWVal + sizeof(V) * kAcc * Cfg::kWarps, 16));
-  static constexpr int kOffFlag = int(align_up(kOffCarry + sizeof(V) * kAcc * 2, 16));
+  // Offsets with `stages` barriers and control blocks.  The shared memory a kernel does not claim stays L1 cache, and the
+  // number of gather misses an SM can have in flight grows with that cache (measured on B200: 63 / 130 / 183 / 225 / 265 G
+  // random 4-byte gathers per second at 228 / 196 / 164 / 132 / <= 32 KB of shared memory per SM).  The steps are coarse: with
+  // 4 CTAs an SM, 128 bytes more than 49152 take the next one (ops_zoo in fp64: 208 -> 214 us), so nothing is reserved here
+  // that the graph's loops do not use.
+  static constexpr int off_ctl(int stages) { return int(align_up(16 * stages, 16)); }
+  static constexpr int off_xs(int stages) { return int(align_up(off_ctl(stages) + sizeof(Ctl) * stages, 16)); }
+  static constexpr int off_wkey(int stages) { return int(align_up(off_xs(stages) + 4 * (Cfg::kBlock + 1), 16)); }
+  static constexpr int off_wval(int stages) { return int(align_up(off_wkey(stages) + 4 * Cfg::kWarps, 16)); }
+  static constexpr int off_carry(int stages) { return int(align_up(off_wval(stages) + sizeof(V) * kAcc * Cfg::kWarps, 16)); }
+  static constexpr int off_flag(int stages) { return int(align_up(off_carry(stages) + sizeof(V) * kAcc * 2, 16)); }
   // rows longer than kShortRowMax inside the current tile: [0..1] counters by tile parity, [2..] local rows
   static constexpr int kMaxLong = Cfg::kTile / (kShortRowMax + 1) + 2;
-  static constexpr int kOffLong = int(align_up(kOffFlag + 16, 16));
+  static constexpr int off_long(int stages) { return int(align_up(off_flag(stages) + 16, 16)); }
   static constexpr int kBuffers = (!G::kGatherNeedsRow && Cfg::kPipeline) ? 2 : 1;   // s_rel / s_prod / long-row list double-buffered when tiles are pipelined
-  static constexpr int kOffRel = int(align_up(kOffLong + 4 * (4 + kMaxLong * kBuffers), 16));
-  // Row-mode graphs (a selector equals the row id) reduce in registers in every tile: no product buffer.  The
-  // shared memory a kernel does not claim stays L1 cache, and the number of gather misses an SM can have in
-  // flight grows with that cache (measured on B200: 63 / 130 / 183 / 225 / 265 G random 4-byte gathers per
-  // second at 228 / 196 / 164 / 132 / <= 32 KB of shared memory per SM).
-  static constexpr int kOffProd = int(align_up(kOffRel + 4 * (Cfg::kTile + 1) * kBuffers, 16));
-  static constexpr int kOffStages = int(align_up(kOffProd + (G::kGatherNeedsRow ? 0 : sizeof(V) * kAcc * Cfg::kTile * kBuffers), 128));
-  static constexpr int kTwoPhase = kOffStages + kStageBytes * Cfg::kStages;
+  static constexpr int off_rel(int stages) { return int(align_up(off_long(stages) + 4 * (4 + kMaxLong * kBuffers), 16)); }
+  // Row-mode graphs (a selector equals the row id) reduce in registers in every tile: no product buffer.
+  static constexpr int off_prod(int stages) { return int(align_up(off_rel(stages) + 4 * (Cfg::kTile + 1) * kBuffers, 16)); }
+  static constexpr int off_stages(int stages) {
+    return int(align_up(off_prod(stages) + (G::kGatherNeedsRow ? 0 : sizeof(V) * kAcc * Cfg::kTile * kBuffers), 128));
+  }
+  static constexpr int two_phase(int stages) { return off_stages(stages) + kStageBytes * Cfg::kStages; }
   // The loop over whole rows needs neither row ends nor products in shared memory: its stages begin where those would,
   // and as many fit as the other loop's total allows, one more where that costs at most 2 KB.
   static constexpr bool kWhole = WholeRows<G, Cfg, WIN>::value;
-  static constexpr int kOffRowStages = int(align_up(kOffLong, 128));
-  static constexpr int kFit = kWhole ? (kTwoPhase + 2048 - kOffRowStages) / kStageBytes : 0;
-  static constexpr int kRowStages = kFit > kMaxStages ? kMaxStages : kFit;
+  static constexpr int off_row_stages(int stages) { return int(align_up(off_long(stages), 128)); }
+  static constexpr int row_stages() {
+    int n = kWhole ? Cfg::kStages : 0;
+    while (kWhole && n < 4 && off_row_stages(n + 1) + kStageBytes * (n + 1) <= two_phase(n + 1) + 2048) ++n;
+    return n;
+  }
+  static constexpr int kRowStages = row_stages();
+  static constexpr int kMaxStages = kRowStages > Cfg::kStages ? kRowStages : Cfg::kStages;
+  static constexpr int kOffBars = 0;
+  static constexpr int kOffCtl = off_ctl(kMaxStages), kOffXs = off_xs(kMaxStages), kOffWKey = off_wkey(kMaxStages);
+  static constexpr int kOffWVal = off_wval(kMaxStages), kOffCarry = off_carry(kMaxStages), kOffFlag = off_flag(kMaxStages);
+  static constexpr int kOffLong = off_long(kMaxStages), kOffRel = off_rel(kMaxStages), kOffProd = off_prod(kMaxStages);
+  static constexpr int kOffStages = off_stages(kMaxStages), kOffRowStages = off_row_stages(kMaxStages);
+  static constexpr int kTwoPhase = two_phase(kMaxStages);
   static constexpr int kRowLoop = kOffRowStages + kStageBytes * kRowStages;
   static constexpr int kTotal = (kWhole && kRowLoop > kTwoPhase) ? kRowLoop : kTwoPhase;
-  static_assert(Cfg::kStages <= kMaxStages && (!kWhole || kRowStages >= Cfg::kStages), "stages of the two loops");
 };
 
 struct TileKernelArgs {
@@ -259,6 +272,13 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     return;
   }
 
+  // stages without room for moved boundaries: a plan of another graph's (this one's never moves them all)
+  if constexpr (!L::kTilesMove && !DIRECT) {
+    if (a.header->whole_rows == 1) {
+      if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
+      return;
+    }
+  }
   // An epilogue needs a row's whole sum: a matrix that was not planned with whole rows is refused here, where every CTA
   // leaves before its producer warp has issued a copy (one still in flight would write into shared memory that a later CTA owns).
   if constexpr (G::kEpilogue) {

@@ -119,3 +119,26 @@ def test_warp_kernel_configuration_follows_the_value_width():
     assert "using CfgLean = flex::WarpCfg<1024, 5, 1>;" in emit_graph(ir, "float32", "spmv_f32")
     for dt, sym in (("float64", "spmv_f64"), ("int64", "spmv_i64")):
         assert "using CfgLean = flex::WarpCfg<768, 5, 1>;" in emit_graph(ir, dt, sym)
+
+
+def test_shared_memory_holds_nothing_a_graphs_loops_do_not_use():
+    """What a CTA claims is taken from the L1 cache in coarse steps: four CTAs of an SM stay below the 196 KB one, and a
+    graph whose tiles are never moved to row starts (per-edge outputs) has no room for moved boundaries."""
+    import ctypes
+    from flexspmv_b200.binding import GraphInfo, load_library
+    lib = load_library()
+
+    def claimed(name, dtype):
+        gi = GraphInfo()
+        assert getattr(lib, f"flexspmv_{name}_{emit_cuda.CTYPE[dtype][1]}_info")(ctypes.byref(gi)) == 0
+        return gi.smem_bytes
+
+    for name, dtype in (("spmv", "float64"), ("spmv", "int64"), ("rusanov", "float32"), ("swe_delta", "float32"), ("swe_delta_rk", "float32"),
+                        ("ops_zoo", "float32"), ("ops_zoo", "float64")):
+        assert 4 * (claimed(name, dtype) + 1024) <= 196 * 1024, name      # the system takes 1 KB a CTA
+    for dtype, tile in (("float32", 768), ("float64", 256), ("int64", 256)):
+        ir = graphs.mixed_dims_graph()
+        per_edge, streams = emit_cuda._stream_bytes_per_edge(ir, emit_cuda.VBYTES[dtype])
+        acc = 8                                                           # two reducers, 2 and 6 wide
+        per_tile = tile * (2 * per_edge + acc * emit_cuda.VBYTES[dtype] + 4)
+        assert claimed("mixed_dims", dtype) <= per_tile + 2 * (32 * (streams + 1) + 16 + 128) + 2048
