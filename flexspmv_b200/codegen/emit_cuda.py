@@ -154,6 +154,9 @@ TUNED_CONFIGS = {
     "spring_mass_f32": (256, 8, 2, 4, 0, 2, 1),   # 35.5 / 31.2: 2048-item tiles hold ~228 rows of 8 edges, one per thread (batch 4: 34.9 / 31.2, batch 1 x 5 CTAs: 36.1 / 29.2, batch 8: 25)
     "rusanov_f64": (256, 4, 2, 3, 0, 1),       # 33.1 / 30.9: 1024-item tiles hold 256 rows of 3 edges (batch 2: 29.4 / 27.6, batch 3: 27.3 / 25.9, batch 1 x 4 CTAs: 30.3 / 28.7)
     "swe_delta_f64": (256, 3, 2, 3, 0, 1),     # 52.7 / 45.3 with staged edge tensors ((256,4,2,3) batch 1: 48.7 / 39.8, direct: 35.3 / 32.2; heuristic (256,3,2,4) batch 2: 33.8 / 31.5)
+    # rows of 8 / 27 / 0 - 32 edges, 6 M of them, in the loop over whole rows with batches of 1 / 2 / 4 / 8: 35 / 36 / 38 / 52 us,
+    # 34 / 38 / 44 / 56, 41 / 44 / 48 / 64; in the loop with carries 4: rows of 40 in 84 us
+    "swe_boundary_f64": (256, 5, 2, 4, 0, 4, 1),
 }
 
 
@@ -656,20 +659,20 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w("    (void)p; (void)r; (void)e; (void)gr; (void)ge; (void)acc;")
     w("  }")
     w("};")
-    # registers one edge keeps live in the fused thread-per-row loop: its staged record (indices + edge
-    # tensors) and its gathered vertex data; the batch is the largest of 8/4/3/2 edges that stays under ~28
+    # Edges of a row whose gathers are in flight together where a thread has a row.  Row-mode graphs: one.  A second edge's
+    # record costs registers that four CTAs an SM do not have (56 a thread): one at a time spills least, leaves the warps to
+    # hide the latency, and was the fastest in both loops wherever it was measured (batch 3 - 4 / 1, us, 6 M edges: the loop
+    # over whole rows, rows of 3: spring-mass fp64 79 / 58, Rusanov fp32 47 / 43, swe_delta fp32 42 / 39; the loop with
+    # carries, rows of 40: 274 / 236, 127 / 117, 118 / 92; graphs tuned one by one are in TUNED_CONFIGS).  Row-mode graphs
+    # that gather nothing but the row's own record hold only an edge's tensors: the largest of 8 / 4 / 3 / 2 that stays
+    # under 28 registers.  Graphs without per-row data: the largest of 4 / 2 whose gathered data and index fit, since the
+    # loop over whole rows reads staged values after the gathers have landed (batches of 8 / 6 / 4 / 3 / 2 edges on the
+    # 7-point fp64 SpMV, 512^3, at 4 CTAs per SM: 3305 / 2797 / 2602 / 2749 / 2620 us).
     words = VBYTES[dtype] // 4
-    per_edge_regs = sum(dim_of(s_["shape"]) * words for s_ in ir.selector_register
-                        if not (s_.get("selector") == 1 and s_.get("row_identity")))
-    per_edge_regs += len({s_["selector_name"] for s_ in ir.selector_register
-                          if s_.get("selector") == 1 and not s_.get("row_identity")})
-    batch = next((b_ for b_ in (8, 4, 3, 2) if b_ * max(per_edge_regs, 1) <= 28), 2)
-    batch = batch_override or batch
-    # the loop over whole rows reads staged values after the gathers have landed, so an edge in flight holds its gathered
-    # data and an index (batches of 8 / 6 / 4 / 3 / 2 edges on the 7-point fp64 SpMV, 512^3, at 4 CTAs per SM: 3305 / 2797 /
-    # 2602 / 2749 / 2620 us); graphs with values of their own in registers use the batch above
     gather_words = sum(dim_of(s_["shape"]) * words for s_ in ir.selector_register
                        if s_.get("selector") == 1 and not s_.get("row_identity"))
+    edge_words = sum(dim_of(s_["shape"]) * words for s_ in ir.selector_register if s_.get("selector") != 1)
+    batch = batch_override or (1 if gather_words else next((b_ for b_ in (8, 4, 3, 2) if b_ * max(edge_words, 1) <= 28), 2))
     row_batch = batch if needs_row else next((b_ for b_ in (4, 2) if b_ * (gather_words + 1) <= 14), 1)
     if len(cfg) > 6:
         row_batch = cfg[6]       # seventh field

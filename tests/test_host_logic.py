@@ -142,3 +142,15 @@ def test_shared_memory_holds_nothing_a_graphs_loops_do_not_use():
         acc = 8                                                           # two reducers, 2 and 6 wide
         per_tile = tile * (2 * per_edge + acc * emit_cuda.VBYTES[dtype] + 4)
         assert claimed("mixed_dims", dtype) <= per_tile + 2 * (32 * (streams + 1) + 16 + 128) + 2048
+
+
+@pytest.mark.parametrize("make,dtype,batches", [(graphs.spring_mass_graph, "float64", (1, 1)), (graphs.rusanov_graph, "float32", (1, 1)),
+                                                (graphs.swe_delta_graph, "float32", (1, 1)), (graphs.spring_mass_graph, "float32", (2, 1)),
+                                                (graphs.swe_boundary_graph, "float32", (8, 8)), (graphs.swe_boundary_graph, "float64", (4, 1)),
+                                                (graphs.spmv_graph, "float64", (1, 4))])
+def test_edges_in_flight_per_row(make, dtype, batches):
+    """(loop with carries, loop over whole rows): a row-mode graph with gathers takes one edge at a time unless it was
+    tuned; more were spilled to local memory."""
+    import re
+    fields = re.search(r"using Cfg = flex::TileCfg<([^>]*)>", emit_cuda.emit_graph(make(), dtype)).group(1).split(", ")
+    assert (int(fields[4]), int(fields[6])) == batches
