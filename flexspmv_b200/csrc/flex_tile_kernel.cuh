@@ -264,31 +264,26 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     }
   }
 
+  // All that the header says, requested before the first branch: one round trip.
+  const uint32_t h_magic = a.header->magic;
+  const int h_bits = a.header->offset_bits;
+  const long long h_rows = a.header->num_rows, h_edges = a.header->num_edges, h_tiles = a.header->num_tiles;
+  const int h_snapped = a.header->snapped_grid, h_whole = a.header->whole_rows, h_row_loop = a.header->row_loop;
   // a workspace that was never planned for this problem holds no usable coordinates: every CTA
   // sees the same header, so all of them leave here and the ticket stays untouched
-  if (a.header->magic != kMagic || a.header->num_tiles != a.num_tiles || a.header->num_rows != a.num_rows ||
-      a.header->num_edges != a.num_edges || a.header->offset_bits != (int)(8 * sizeof(OffsetT))) {
+  if (h_magic != kMagic || h_tiles != a.num_tiles || h_rows != a.num_rows || h_edges != a.num_edges || h_bits != (int)(8 * sizeof(OffsetT))) {
     if (tid == 0 && blockIdx.x == 0) raise_not_planned(a.header);
     return;
   }
-
-  // stages without room for moved boundaries: a plan of another graph's (this one's never moves them all)
-  if constexpr (!L::kTilesMove && !DIRECT) {
-    if (a.header->whole_rows == 1) {
-      if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
-      return;
-    }
-  }
   // An epilogue needs a row's whole sum: a matrix that was not planned with whole rows is refused here, where every CTA
-  // leaves before its producer warp has issued a copy (one still in flight would write into shared memory that a later CTA owns).
-  if constexpr (G::kEpilogue) {
-    if (a.header->whole_rows != 1) {
-      if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
-      return;
-    }
+  // leaves before its producer warp has issued a copy (one still in flight would write into shared memory that a later CTA
+  // owns).  So is a plan with moved boundaries (another graph's) where the stages have no room for them.
+  if ((G::kEpilogue && h_whole != 1) || (!L::kTilesMove && !DIRECT && h_whole == 1)) {
+    if (tid == 0 && blockIdx.x == 0) raise_status(a.header, FLEXSPMV_ERR_NOT_PLANNED);
+    return;
   }
   // the loop over whole rows has its own stages, in its own places
-  const bool whole = WHOLE && (G::kEpilogue || a.header->row_loop == 1);
+  const bool whole = WHOLE && (G::kEpilogue || h_row_loop == 1);
   const int nstages = WHOLE ? (whole ? L::kRowStages : S) : S;
   unsigned char* const stage_base = (WHOLE && whole) ? smem + L::kOffRowStages : s_stage;
 
@@ -396,7 +391,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   if (tid < 2 * kAcc) s_carry[tid] = V(0);
   if (tid < 4) s_nlong[tid] = 0;
   // no row spans two CTAs of this launch
-  if (tid == 0) s_flag[1] = (a.header->whole_rows == 1 || a.header->snapped_grid == (int)gridDim.x) ? 1 : 0;
+  if (tid == 0) s_flag[1] = (h_whole == 1 || h_snapped == (int)gridDim.x) ? 1 : 0;
   __syncthreads();   // the only barrier that includes the producer warp
 
   // ---- producer warp: runs up to S tiles ahead of the consumers, off their critical path -----------
