@@ -50,7 +50,9 @@ struct WorkspaceHeader {
   int32_t whole_rows;          // 1: EVERY tile boundary sits on a row end and no row is longer than kWholeRowMax: no launch
                                // on this workspace hands carries over, whatever its grid (-1: looked at and refused)
   int32_t row_loop;            // 1: and the tile kernel runs its loop over whole rows
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 2 * 4];
+  uint32_t bank_groups;        // sampled groups of 32 rows, and over them the largest number of rows of a group whose
+  uint32_t bank_degree;        // first edges lie a multiple of 32 apart
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 4 * 4];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
@@ -59,6 +61,13 @@ constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
 #define FLEX_WHOLE_ROW_MAX 32
 #endif
 constexpr int kWholeRowMax = FLEX_WHOLE_ROW_MAX;   // longest row of a matrix whose tiles hold whole rows only
+
+// Which loop a graph's kernel runs on tiles of whole rows.
+enum class RowLoop : int {
+  kNone,           // it has no loop over whole rows
+  kAlways,         // its other loop has a thread per row as well
+  kUnlessSameBank  // its other loop has lanes on consecutive edges
+};
 
 // What one tile of the tile kernel can take when a planning step moves its boundaries (in whole numbers of edges and
 // rows): its arrays hold max_edges edges, its stage stage_bytes bytes of per-edge records and row ends.

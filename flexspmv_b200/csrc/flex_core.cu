@@ -103,38 +103,70 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   unsigned long long slots = 0;
+  unsigned groups = 0, degree = 0;
+  constexpr int kAhead = 4;
+  const long long step = num_tiles / 1024 + 1;                              // tiles whose first 32 rows are looked at for banks
   bool bad = false;
   for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < num_tiles && !bad; t += warps) {
     const long long x0 = (long long)coords[2 * t], x1 = (long long)coords[2 * t + 2];
     const long long y0 = moved_edge(row_offsets, num_rows, num_edges, num_tiles, coords, t);
     const long long y1 = moved_edge(row_offsets, num_rows, num_edges, num_tiles, coords, t + 1);
     bad = y0 < 0 || y1 < y0 || y1 > num_edges || !room.fits(y1 - y0, x1 - x0);
-    for (long long r0 = x0; r0 < x1; r0 += 32) {
-      const long long r = r0 + lane;
-      long long len = 0;
-      if (r < x1) {
-        const long long end = (long long)row_offsets[r + 1];
-        len = end - (r == x0 ? y0 : (long long)row_offsets[r]);
-        if (len < 0 || end > y1) len = kWholeRowMax + 1;
+    for (long long r0 = x0; r0 < x1; r0 += 32 * kAhead) {
+      long long begin[kAhead], end[kAhead];                                 // all loads before the first vote
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        const long long r = r0 + 32 * j + lane;
+        begin[j] = end[j] = y1;
+        if (r < x1) {
+          begin[j] = r == x0 ? y0 : (long long)row_offsets[r];
+          end[j] = (long long)row_offsets[r + 1];
+        }
       }
-      const int longest = __reduce_max_sync(0xffffffffu, (int)(len > kWholeRowMax ? kWholeRowMax + 1 : len));
-      bad |= longest > kWholeRowMax;
-      slots += 32u * (unsigned)longest;
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        if (r0 + 32 * j >= x1) break;                                       // the same for the whole warp
+        const long long len = end[j] - begin[j];
+        const bool fits = len >= 0 && len <= kWholeRowMax && end[j] <= y1;
+        const int longest = __reduce_max_sync(0xffffffffu, fits ? (int)len : kWholeRowMax + 1);
+        bad |= longest > kWholeRowMax;
+        slots += 32u * (unsigned)longest;
+        if (j == 0 && r0 == x0 && t % step == 0) {
+          const int bank = (int)(begin[0] & 31);
+          unsigned same = __ballot_sync(0xffffffffu, len > 0);
+          groups += same != 0;
+#pragma unroll
+          for (int b = 0; b < 5; ++b) {
+            const unsigned set = __ballot_sync(0xffffffffu, (bank >> b) & 1);
+            same &= (bank >> b) & 1 ? set : ~set;
+          }
+          degree += __reduce_max_sync(0xffffffffu, len > 0 ? (unsigned)__popc(same) : 0u);
+        }
+      }
     }
   }
   if (lane == 0) {
     if (bad) h->whole_rows = -1;
     else if (slots) atomicAdd(reinterpret_cast<unsigned long long*>(&h->row_slots), slots);
+    if (!bad && groups) {
+      atomicAdd(&h->bank_groups, groups);
+      atomicAdd(&h->bank_degree, degree);
+    }
   }
 }
 // Moves the boundaries when the kernel above found nothing against it and at least two fifths of the thread-steps have
 // an edge to work on: rows of very different lengths are better off with the two-phase loop, whose lanes take
 // consecutive edges.  1 M rows, fp64 SpMV, this loop / the two-phase loop: lengths 0 - 8 evenly (share 0.50) 16.4 / 21.0 us,
 // 0 - 16 evenly (0.51) 29.0 / 35.6 us, exponential of mean 4 (0.22) 24.4 / 24.3 us, 32 in 3 % of the rows and 2 elsewhere
-// (0.14) 30.9 / 20.1 us.  `row_loop`: the kernel has the loop over whole rows.
+// (0.14) 30.9 / 20.1 us.
+// Whether the kernel then takes its loop over whole rows is row_loop's to say.  Lanes there read the indices and values of
+// rows a row length apart: rows of 16 or 32 edges all begin in two banks or one, and every read of the stage is 16 or 32 in a
+// row.  Graphs whose other loop has lanes on consecutive edges (its sums meet the same banks, once an edge, not twice) take
+// that one when more than 10 of 32 rows begin in one bank on average.  fp64 SpMV, 12 M edges, this loop / the other: rows of 8
+// (degree 8) 50 / 52 us, 16 (16) 81 / 73, 24 (8) 51 / 52, 32 (32) 104 / 73; 0.4 M edges, 16: 8.7 / 7.9, 32: 10.2 / 7.7.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                                               long long num_tiles, int row_loop, OffsetT* __restrict__ coords,
+                                                               long long num_tiles, RowLoop row_loop, OffsetT* __restrict__ coords,
                                                                WorkspaceHeader* h) {
   if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1) return;
   if (2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) return;
@@ -145,24 +177,25 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __
   }
   if (t == 0) {
     *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;     // read by this kernel only as "-1 or not"
-    h->row_loop = row_loop;
+    const bool same_bank = h->bank_degree > 10 * h->bank_groups;
+    h->row_loop = row_loop == RowLoop::kAlways || (row_loop == RowLoop::kUnlessSameBank && !same_bank);
   }
 }
 
 template <typename OffsetT>
 static int whole_rows_launch_as(const void* d_row_offsets, long long num_rows, long long num_edges, long long num_tiles,
-                                const TileRoom& room, bool row_loop, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
+                                const TileRoom& room, RowLoop row_loop, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
   const OffsetT* ro = static_cast<const OffsetT*>(d_row_offsets);
   OffsetT* coords = static_cast<OffsetT*>(d_coords);
   long long grid = (num_tiles + 7) / 8;
   const long long cap = (long long)device_sm_count() * 8;
   if (grid > cap) grid = cap;
   whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, coords, h);
-  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, row_loop ? 1 : 0, coords, h);
+  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, row_loop, coords, h);
   return (int)cudaGetLastError();
 }
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, bool row_loop, void* d_coords, void* ws, cudaStream_t stream) {
+                      const TileRoom& room, RowLoop row_loop, void* d_coords, void* ws, cudaStream_t stream) {
   if (num_tiles < 1 || num_rows < 1) return 0;
   WorkspaceHeader* h = static_cast<WorkspaceHeader*>(ws);
   if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, row_loop, d_coords, h, stream);

@@ -24,7 +24,7 @@ int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream);
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, bool row_loop, void* d_coords, void* ws, cudaStream_t stream);
+                      const TileRoom& room, RowLoop row_loop, void* d_coords, void* ws, cudaStream_t stream);
 int window_plan_launch(const void* d_coords, int offset_bits, long long num_tiles, const int* d_idx, int rec_bytes,
                        int win_bytes, void* d_table, void* d_local_idx, cudaStream_t st);
 int window_ready_launch(void* ws, cudaStream_t st);
@@ -185,10 +185,12 @@ struct GraphApi {
       if (int e = partition_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, tile_items(d),
                                    static_cast<char*>(ws) + h.coords_offset, st)) return e;
       if constexpr (WholeTiles<G, Cfg, false>::value) {
+        constexpr RowLoop row_loop = !WholeRows<G, Cfg, false>::value ? RowLoop::kNone
+                                     : G::kGatherNeedsRow ? RowLoop::kAlways : RowLoop::kUnlessSameBank;
         // rows longer than kWholeRowMax on average: no need to look
         if (whole_rows && !use_lean(d) && !use_win(d) && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
           if (int e = whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d),
-                                        WholeRows<G, Cfg, false>::value, static_cast<char*>(ws) + h.coords_offset, ws, st)) return e;
+                                        row_loop, static_cast<char*>(ws) + h.coords_offset, ws, st)) return e;
       }
       // the tile kernel: boundaries between the CTAs of its grid moved onto row ends where the tiles have room
       if (!use_lean(d) && h.num_tiles > 1) {

@@ -87,6 +87,24 @@ def test_maps_that_divide_keep_the_two_phase_loop(gname, dt, expected):
         assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(got, results[0]))
 
 
+@pytest.mark.parametrize("gname,dt", [("spmv", "float64"), ("spmv", "float32"), ("spmv", "int64"), ("spring_mass", "float32")])
+@pytest.mark.parametrize("lengths,same_bank", [([8] * 3000, 0), ([16] * 3000, 1), ([24] * 2000, 0), ([32] * 1500, 1), ([31] * 1500, 0),
+                                               ([16, 0] * 2500, 0), ([0] * 31 + [32] * 997 + [0] * 400, 1), ([7, 9] * 2000, 0), ([15, 16] * 1000, 0)])
+def test_rows_that_begin_in_one_bank_keep_lanes_on_consecutive_edges(gname, dt, lengths, same_bank):
+    """Rows of 16 or 32 edges all begin in two shared-memory banks or in one: graphs whose other loop walks consecutive edges
+    take that one on the tiles of whole rows; graphs with per-row data have a thread per row in both."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, lengths, 31, dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    for kw, offsets in (({}, np.int32), ({"max_ctas": 2}, np.int64)):
+        ext = GraphExtension(ir, random_gather=False, **kw)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=offsets)
+        ext.check()
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} {dt} {lengths[:3]} {kw}")
+        assert ext.planned_whole_rows()
+        assert row_loop_planned(ext) == (1 if gname == "spring_mass" else 1 - same_bank)
+
+
 def test_whole_rows_equal_the_two_phase_loop_bit_for_bit():
     """The same matrix with one row of 33 edges behind it goes through the loop with carries; all other rows are the
     same sums, left to right."""
