@@ -135,7 +135,7 @@ class _Symbols:
                 raise FlexSpmvError(f"library has no graph '{sym}' (symbol flexspmv_{sym}_{name})") from e
             f.restype = ctypes.c_int
             return f
-        self.info, self.workspace_bytes, self.plan = fn("info"), fn("workspace_bytes"), fn("plan")
+        self.info, self.workspace_bytes, self.plan = fn("info"), fn("workspace_bytes"), fn("plan_indexed")
         self.plan_windows = fn("plan_windows")
         fn("launch")
         self.launch, self.device_status = _LAUNCH((f"flexspmv_{sym}_launch", lib)), fn("device_status")
@@ -276,11 +276,11 @@ class GraphExtension:
         nbytes = ctypes.c_size_t()
         check(self.lib, syms.workspace_bytes(ctypes.byref(desc), ctypes.byref(nbytes)), "workspace_bytes")
         ws = torch.empty(nbytes.value, dtype=torch.uint8, device=device)
-        check(self.lib, syms.plan(ctypes.byref(desc), ctypes.c_void_p(ro.data_ptr() if ro is not None else 0),
+        ip = _pointers(indices)
+        check(self.lib, syms.plan(ctypes.byref(desc), ip, ctypes.c_void_p(ro.data_ptr() if ro is not None else 0),
                                   ctypes.c_void_p(ws.data_ptr()), ctypes.c_size_t(nbytes.value), _stream_ptr()),
               "plan")
         if desc.reserved & 1:      # gather windows: the second planning step reads the index array
-            ip = (ctypes.c_void_p * max(len(indices), 1))(*[t.data_ptr() for t in indices])
             check(self.lib, syms.plan_windows(ctypes.byref(desc), ip, ctypes.c_void_p(ws.data_ptr()),
                                               ctypes.c_size_t(nbytes.value), _stream_ptr()), "plan_windows")
             self.launches += 2

@@ -471,6 +471,15 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w("  }")
     w(f"  static constexpr bool kHasDirectEdgeTensors = {'true' if (edge_regs_list and not staged_values) else 'false'};")
     # L1 prefetch of what gather_edge will read, issued by the producer warp one tile ahead
+    # the gathers that depend on the edge, for the plan: index array and record width of up to `most` of them
+    w("  static int gathers(const void* const* indices, const int** index, int* record_bytes, int most) {")
+    w("    int n = 0;")
+    for s_ in edge_sel:
+        w(f"    if (n < most) {{ index[n] = static_cast<const int*>(indices[{index_names.index(s_['selector_name'])}]); "
+          f"record_bytes[n++] = {VBYTES[dtype] * dim_of(s_['shape'])}; }}")
+    w("    (void)indices; (void)index; (void)record_bytes; (void)most;")
+    w("    return n;")
+    w("  }")
     w("  __device__ __forceinline__ static void gather_edge(const Params& p, const EReg& r, GEdge& g) {")
     for s_ in edge_sel:
         d = dim_of(s_["shape"])

@@ -86,18 +86,18 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w("")
     w("struct Entry {   // the C entry points of one value type")
     w("  int (*workspace_bytes)(const flexspmv_desc*, size_t*);")
-    w("  int (*plan)(const flexspmv_desc*, const void*, void*, size_t, void*);")
+    w("  int (*plan)(const flexspmv_desc*, const void* const*, const void*, void*, size_t, void*);")
     w("  int (*launch)(const flexspmv_desc*, const void* const*, const void* const*, const void*, void* const*, void*, size_t, void*);")
     w("  int (*device_status)(const void*, int32_t*, void*);")
     w("  int type_tag;")
     w("};")
     for i, dt in enumerate(dtypes):
         s = f"{symbol}_{CTYPE[dt][1]}"
-        w(f"const Entry kEntry_{CTYPE[dt][1]} = {{flexspmv_{s}_workspace_bytes, flexspmv_{s}_plan, flexspmv_{s}_launch, "
+        w(f"const Entry kEntry_{CTYPE[dt][1]} = {{flexspmv_{s}_workspace_bytes, flexspmv_{s}_plan_indexed, flexspmv_{s}_launch, "
           f"flexspmv_{s}_device_status, {i}}};")
     w("")
-    w("torch::Tensor planned_workspace(const Entry& e, const flexspmv_desc& d, const torch::Tensor& ro, bool has_rows,")
-    w("                                const torch::Tensor& like, cudaStream_t stream) {")
+    w("torch::Tensor planned_workspace(const Entry& e, const flexspmv_desc& d, const void* const* indices, const torch::Tensor& ro,")
+    w("                                bool has_rows, const torch::Tensor& like, cudaStream_t stream) {")
     w("  const void* ro_ptr = has_rows ? ro.data_ptr() : nullptr;")
     w("  const uint32_t ver = has_rows ? ro._version() : 0u;")
     w("  const int device = like.get_device();")
@@ -113,7 +113,7 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w("  int st = e.workspace_bytes(&d, &bytes);")
     w('  TORCH_CHECK(st == 0, "merged_spmv_launch (workspace size) failed: ", flexspmv_error_string(st));')
     w("  torch::Tensor ws = torch::empty({(int64_t)bytes}, torch::TensorOptions().dtype(torch::kUInt8).device(like.device()));")
-    w("  st = e.plan(&d, ro_ptr, ws.data_ptr(), bytes, stream);")
+    w("  st = e.plan(&d, indices, ro_ptr, ws.data_ptr(), bytes, stream);")
     w('  TORCH_CHECK(st == 0, "merged_spmv_launch (plan) failed: ", flexspmv_error_string(st));')
     w("  g_plans.push_front(PlanEntry{ro_ptr, ver, d.num_rows, d.num_edges, d.offset_bits, device, stream, e.type_tag, ws,")
     w("                               has_rows ? ro : torch::Tensor()});")
@@ -156,9 +156,9 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w(f"  d.offset_bits = {'row_end_offsets.scalar_type() == torch::kLong ? 64 : 32' if has_red else '32'};")
     w("  d.tile_items = 0; d.max_ctas = 0; d.reserved = 0;")
     w("  cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();")
-    w(f"  torch::Tensor ws = planned_workspace(e, d, row_end_offsets, {'true' if has_red else 'false'}, {dispatch}, stream);")
     w("  const void* values[] = {" + ", ".join(f"{n}.data_ptr()" for n in values) + ("" if values else "nullptr") + "};")
     w("  const void* indices[] = {" + ", ".join(f"{n}.data_ptr()" for n in idx_args) + ("" if idx_args else "nullptr") + "};")
+    w(f"  torch::Tensor ws = planned_workspace(e, d, indices, row_end_offsets, {'true' if has_red else 'false'}, {dispatch}, stream);")
     w("  void* outputs[] = {" + ", ".join(f"{v}.data_ptr()" for v in out_vars) + ("" if out_vars else "nullptr") + "};")
     w(f"  const int st = e.launch(&d, values, indices, {'row_end_offsets.data_ptr()' if has_red else 'nullptr'}, outputs, ws.data_ptr(),")
     w("                          (size_t)ws.numel(), stream);")

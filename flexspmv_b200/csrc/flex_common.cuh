@@ -52,7 +52,9 @@ struct WorkspaceHeader {
   int32_t row_loop;            // 1: and the tile kernel runs its loop over whole rows
   uint32_t bank_groups;        // sampled groups of 32 rows, and over them the largest number of rows of a group whose
   uint32_t bank_degree;        // first edges lie a multiple of 32 apart
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 4 * 4];
+  uint32_t line_rows, line_row_lines;       // over the same groups, when the plan saw the columns: rows with an edge and the
+  uint32_t line_edges, line_edge_lines;     // cache lines their middle edges gather from; consecutive edges and their lines
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
@@ -62,11 +64,15 @@ constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
 #endif
 constexpr int kWholeRowMax = FLEX_WHOLE_ROW_MAX;   // longest row of a matrix whose tiles hold whole rows only
 
-// Which loop a graph's kernel runs on tiles of whole rows.
-enum class RowLoop : int {
-  kNone,           // it has no loop over whole rows
-  kAlways,         // its other loop has a thread per row as well
-  kUnlessSameBank  // its other loop has lanes on consecutive edges
+// What the plan has to know to choose the loop that runs on tiles of whole rows.
+struct RowLoopRule {
+  static constexpr int kMaxGathers = 4;
+  bool built;                        // the kernel has the loop over whole rows
+  bool edge_lanes;                   // its other loop has lanes on consecutive edges (else a thread per row, as this one)
+  int accumulators;                  // width of a row's sum
+  int gathers;                       // gathers whose columns the plan sees (0: none)
+  const int* index[kMaxGathers];
+  int record_bytes[kMaxGathers];
 };
 
 // What one tile of the tile kernel can take when a planning step moves its boundaries (in whole numbers of edges and

@@ -91,6 +91,12 @@ __device__ __forceinline__ long long moved_edge(const OffsetT* __restrict__ row_
   const long long x = (long long)coords[2 * t];
   return x < num_rows ? (long long)row_offsets[x] : (long long)coords[2 * t + 1];
 }
+// Cache line of a gathered record, up to the array's offset in its first line; lines among the lanes with `in`.
+__device__ __forceinline__ unsigned line_of(int column, int record_bytes) { return (unsigned)(((long long)column * record_bytes) >> 7); }
+__device__ __forceinline__ unsigned distinct(unsigned line, bool in) {
+  const unsigned lane = threadIdx.x & 31u, same = __match_any_sync(0xffffffffu, line) & __ballot_sync(0xffffffffu, in);
+  return __popc(__ballot_sync(0xffffffffu, in && (same & ((1u << lane) - 1u)) == 0));
+}
 // One warp per tile: would every row stay whole with all tile boundaries moved back to row starts -- rows of at most
 // kWholeRowMax edges, tiles that still fit -- and how many thread-steps would one thread per row take?  Leaves
 // whole_rows = -1 when a row or a tile is too large.  Unlike the merge path, which stays inside [0, num_edges] for any
@@ -98,14 +104,14 @@ __device__ __forceinline__ long long moved_edge(const OffsetT* __restrict__ row_
 // first row (all of which the loop with carries takes without reading out of range) are refused here.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                                         long long num_tiles, const TileRoom room, const OffsetT* __restrict__ coords,
-                                                         WorkspaceHeader* h) {
+                                                         long long num_tiles, const TileRoom room, const RowLoopRule rule,
+                                                         const OffsetT* __restrict__ coords, WorkspaceHeader* h) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   unsigned long long slots = 0;
-  unsigned groups = 0, degree = 0;
+  unsigned groups = 0, degree = 0, rows = 0, row_lines = 0, edges = 0, edge_lines = 0;
   constexpr int kAhead = 4;
-  const long long step = num_tiles / 1024 + 1;                              // tiles whose first 32 rows are looked at for banks
+  const long long step = num_tiles / 1024 + 1;                              // tiles whose first 32 rows are looked at closely
   bool bad = false;
   for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < num_tiles && !bad; t += warps) {
     const long long x0 = (long long)coords[2 * t], x1 = (long long)coords[2 * t + 2];
@@ -127,7 +133,7 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
       for (int j = 0; j < kAhead; ++j) {
         if (r0 + 32 * j >= x1) break;                                       // the same for the whole warp
         const long long len = end[j] - begin[j];
-        const bool fits = len >= 0 && len <= kWholeRowMax && end[j] <= y1;
+        const bool fits = len >= 0 && len <= kWholeRowMax && begin[j] >= y0 && end[j] <= y1;
         const int longest = __reduce_max_sync(0xffffffffu, fits ? (int)len : kWholeRowMax + 1);
         bad |= longest > kWholeRowMax;
         slots += 32u * (unsigned)longest;
@@ -141,6 +147,18 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
             same &= (bank >> b) & 1 ? set : ~set;
           }
           degree += __reduce_max_sync(0xffffffffu, len > 0 ? (unsigned)__popc(same) : 0u);
+          // lines of the rows' middle edges and of consecutive edges, where the offsets lead into the arrays
+          const bool row = fits && len > 0, edge = lane < (int)(y1 - y0 < 32 ? y1 - y0 : 32);
+#pragma unroll
+          for (int i = 0; i < RowLoopRule::kMaxGathers; ++i) {
+            if (i >= rule.gathers || bad) break;                            // the same for the whole warp
+            const unsigned at_row = row ? line_of(rule.index[i][begin[0] + (len >> 1)], rule.record_bytes[i]) : 0u;
+            const unsigned at_edge = edge ? line_of(rule.index[i][y0 + lane], rule.record_bytes[i]) : 0u;
+            rows += __popc(__ballot_sync(0xffffffffu, row));
+            edges += __popc(__ballot_sync(0xffffffffu, edge));
+            row_lines += distinct(at_row, row);
+            edge_lines += distinct(at_edge, edge);
+          }
         }
       }
     }
@@ -151,6 +169,12 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
     if (!bad && groups) {
       atomicAdd(&h->bank_groups, groups);
       atomicAdd(&h->bank_degree, degree);
+      if (rule.gathers) {
+        atomicAdd(&h->line_rows, rows);
+        atomicAdd(&h->line_row_lines, row_lines);
+        atomicAdd(&h->line_edges, edges);
+        atomicAdd(&h->line_edge_lines, edge_lines);
+      }
     }
   }
 }
@@ -159,14 +183,21 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
 // consecutive edges.  1 M rows, fp64 SpMV, this loop / the two-phase loop: lengths 0 - 8 evenly (share 0.50) 16.4 / 21.0 us,
 // 0 - 16 evenly (0.51) 29.0 / 35.6 us, exponential of mean 4 (0.22) 24.4 / 24.3 us, 32 in 3 % of the rows and 2 elsewhere
 // (0.14) 30.9 / 20.1 us.
-// Whether the kernel then takes its loop over whole rows is row_loop's to say.  Lanes there read the indices and values of
+// Whether the kernel then takes its loop over whole rows is the rule's to say.  Lanes there read the indices and values of
 // rows a row length apart: rows of 16 or 32 edges all begin in two banks or one, and every read of the stage is 16 or 32 in a
 // row.  Graphs whose other loop has lanes on consecutive edges (its sums meet the same banks, once an edge, not twice) take
 // that one when more than 10 of 32 rows begin in one bank on average.  fp64 SpMV, 12 M edges, this loop / the other: rows of 8
 // (degree 8) 50 / 52 us, 16 (16) 81 / 73, 24 (8) 51 / 52, 32 (32) 104 / 73; 0.4 M edges, 16: 8.7 / 7.9, 32: 10.2 / 7.7.
+// Likewise where the columns of a row lie side by side and those of neighbouring rows do not (runs of columns at arbitrary
+// places): a gather costs the L1 cache a pass for every line it touches, and 32 rows with one edge each touch 32 lines, 32
+// consecutive edges a few.  The rest of the two-phase loop's work -- its products go through shared memory -- is worth about
+// 22 lines an accumulator.  fp64 / fp32 SpMV, 12 M edges in runs of columns, this loop / the other, us: runs of 4 (32 against 10
+// lines a gather) 55 / 57 and 41 / 44, 5 (32, 8) 46 / 43 and 36 / 35, 8 (32, 5) 67 / 52 and 49 / 37, 20 (32, 2) 54 / 41 and 36 / 32;
+// stencils (2 - 3 against 8 - 16 lines), banded and random columns: this loop, by 4 - 50 %.  A plan that has not been shown the
+// columns goes by the rows alone.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                                               long long num_tiles, RowLoop row_loop, OffsetT* __restrict__ coords,
+                                                               long long num_tiles, const RowLoopRule rule, OffsetT* __restrict__ coords,
                                                                WorkspaceHeader* h) {
   if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1) return;
   if (2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) return;
@@ -178,28 +209,30 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __
   if (t == 0) {
     *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;     // read by this kernel only as "-1 or not"
     const bool same_bank = h->bank_degree > 10 * h->bank_groups;
-    h->row_loop = row_loop == RowLoop::kAlways || (row_loop == RowLoop::kUnlessSameBank && !same_bank);
+    const long long lines_more = 32ll * h->line_row_lines * h->line_edges - 32ll * h->line_edge_lines * h->line_rows;   // x rows x edges
+    const bool edges_share_lines = lines_more * rule.gathers > 22ll * rule.accumulators * h->line_rows * h->line_edges;
+    h->row_loop = rule.built && !(rule.edge_lanes && (same_bank || edges_share_lines));
   }
 }
 
 template <typename OffsetT>
 static int whole_rows_launch_as(const void* d_row_offsets, long long num_rows, long long num_edges, long long num_tiles,
-                                const TileRoom& room, RowLoop row_loop, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
+                                const TileRoom& room, const RowLoopRule& rule, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
   const OffsetT* ro = static_cast<const OffsetT*>(d_row_offsets);
   OffsetT* coords = static_cast<OffsetT*>(d_coords);
   long long grid = (num_tiles + 7) / 8;
   const long long cap = (long long)device_sm_count() * 8;
   if (grid > cap) grid = cap;
-  whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, coords, h);
-  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, row_loop, coords, h);
+  whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, rule, coords, h);
+  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, rule, coords, h);
   return (int)cudaGetLastError();
 }
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, RowLoop row_loop, void* d_coords, void* ws, cudaStream_t stream) {
+                      const TileRoom& room, const RowLoopRule& rule, void* d_coords, void* ws, cudaStream_t stream) {
   if (num_tiles < 1 || num_rows < 1) return 0;
   WorkspaceHeader* h = static_cast<WorkspaceHeader*>(ws);
-  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, row_loop, d_coords, h, stream);
-  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, row_loop, d_coords, h, stream);
+  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, rule, d_coords, h, stream);
+  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, rule, d_coords, h, stream);
 }
 
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,

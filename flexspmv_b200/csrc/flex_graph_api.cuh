@@ -24,7 +24,7 @@ int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream);
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, RowLoop row_loop, void* d_coords, void* ws, cudaStream_t stream);
+                      const TileRoom& room, const RowLoopRule& rule, void* d_coords, void* ws, cudaStream_t stream);
 int window_plan_launch(const void* d_coords, int offset_bits, long long num_tiles, const int* d_idx, int rec_bytes,
                        int win_bytes, void* d_table, void* d_local_idx, cudaStream_t st);
 int window_ready_launch(void* ws, cudaStream_t st);
@@ -168,7 +168,9 @@ struct GraphApi {
   }
 
   // `whole_rows`: also look for a matrix of short rows whose tiles can all hold whole rows (two more kernels).
-  static int plan(const flexspmv_desc* d, const void* row_offsets, void* ws, size_t ws_bytes, cudaStream_t st, bool whole_rows = true) {
+  // `indices` (may be null): the launch's index arrays, which the choice of the loop on such tiles looks at.
+  static int plan(const flexspmv_desc* d, const void* const* indices, const void* row_offsets, void* ws, size_t ws_bytes, cudaStream_t st,
+                  bool whole_rows = true) {
     if (int e = check_desc(d)) return e;
     if (!ws) return FLEXSPMV_ERR_WORKSPACE;
     WorkspaceHeader h{};
@@ -185,12 +187,16 @@ struct GraphApi {
       if (int e = partition_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, tile_items(d),
                                    static_cast<char*>(ws) + h.coords_offset, st)) return e;
       if constexpr (WholeTiles<G, Cfg, false>::value) {
-        constexpr RowLoop row_loop = !WholeRows<G, Cfg, false>::value ? RowLoop::kNone
-                                     : G::kGatherNeedsRow ? RowLoop::kAlways : RowLoop::kUnlessSameBank;
+        RowLoopRule rule{};
+        rule.built = WholeRows<G, Cfg, false>::value;
+        rule.edge_lanes = !G::kGatherNeedsRow;
+        rule.accumulators = G::kAccDim;
+        if (rule.built && rule.edge_lanes && indices) rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
+        for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
         // rows longer than kWholeRowMax on average: no need to look
         if (whole_rows && !use_lean(d) && !use_win(d) && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
           if (int e = whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d),
-                                        row_loop, static_cast<char*>(ws) + h.coords_offset, ws, st)) return e;
+                                        rule, static_cast<char*>(ws) + h.coords_offset, ws, st)) return e;
       }
       // the tile kernel: boundaries between the CTAs of its grid moved onto row ends where the tiles have room
       if (!use_lean(d) && h.num_tiles > 1) {
@@ -399,7 +405,11 @@ struct GraphApi {
     return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::workspace_bytes(d, b);                                           \
   }                                                                                                             \
   int flexspmv_##SYM##_plan(const flexspmv_desc* d, const void* ro, void* ws, size_t wb, void* st) {            \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan(d, ro, ws, wb, static_cast<cudaStream_t>(st));              \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan(d, nullptr, ro, ws, wb, static_cast<cudaStream_t>(st));     \
+  }                                                                                                             \
+  int flexspmv_##SYM##_plan_indexed(const flexspmv_desc* d, const void* const* ix, const void* ro, void* ws, size_t wb, void* st) { \
+    if (!ix) return FLEXSPMV_ERR_BAD_ARG;                                                                       \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan(d, ix, ro, ws, wb, static_cast<cudaStream_t>(st));          \
   }                                                                                                             \
   int flexspmv_##SYM##_plan_windows(const flexspmv_desc* d, const void* const* ix, void* ws, size_t wb, void* st) { \
     return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan_windows(d, ix, ws, wb, static_cast<cudaStream_t>(st));      \
@@ -460,7 +470,7 @@ struct GraphApi {
     cudaStream_t stream = static_cast<cudaStream_t>(st);                                                        \
     /* the array keeps the previous call's contents: planning rewrites the header (ticket, status) and */      \
     /* every tile coordinate this problem reads; the carry slots are written before they are read      */      \
-    if (int e = Api::plan(d, ro, ws, (size_t)(BYTES), stream, false)) return e;                                      \
+    if (int e = Api::plan(d, nullptr, ro, ws, (size_t)(BYTES), stream, false)) return e;                             \
     return Api::launch(d, v, ix, ro, o, ws, (size_t)(BYTES), stream);                                           \
   }                                                                                                             \
   extern "C" int flexspmv_##SYM##_static_device_status(int32_t* d_out, void* st) {                              \

@@ -226,7 +226,7 @@ int flexspmv_swe_rk_stage(int32_t value_bytes, const void *const *d_r, const voi
 int flexspmv_workspace_whole_rows(const void *d_workspace, int32_t *d_out, void *stream);
 
 /* ---- per fused graph ---------------------------------------------------------------------------
- * One set of five symbols per (graph, value type); the per-edge map is compiled into the kernel, so
+ * One set of symbols per (graph, value type); the per-edge map is compiled into the kernel, so
  * a graph is identified by its symbol prefix.  For graph G and value type T (f32 | f64 | i64):
  *
  *   flexspmv_G_T_info            sizes of the three pointer arrays and of the compiled defaults
@@ -235,6 +235,11 @@ int flexspmv_workspace_whole_rows(const void *d_workspace, int32_t *d_out, void 
  *   flexspmv_G_T_plan            partitions the problem into the workspace (cacheable while the row
  *                                offsets do not change; replaces the per-call search kernel,
  *                                include/merged_spmv.cuh:98-119)
+ *   flexspmv_G_T_plan_indexed    the same plan by a caller who has the index arrays of launch at hand (the other
+ *                                arguments as in plan): on matrices of short rows the choice between two loops
+ *                                then also looks at a sample of the columns.  plan goes by the rows alone, which
+ *                                is the better choice unless rows hold runs of consecutive columns at
+ *                                unrelated places (graphs without per-row data only).
  *   flexspmv_G_T_plan_windows    second planning step of descriptors with FLEXSPMV_FLAG_GATHER_WINDOWS,
  *                                after plan on the same workspace; takes the index arrays of launch.
  *                                A no-op (returns 0) for other descriptors and graphs.
@@ -272,6 +277,9 @@ typedef struct flexspmv_graph_info {
   int flexspmv_##G##_workspace_bytes(const flexspmv_desc *desc, size_t *bytes);                     \
   int flexspmv_##G##_plan(const flexspmv_desc *desc, const void *d_row_offsets, void *d_workspace,  \
                           size_t workspace_bytes, void *stream);                                    \
+  int flexspmv_##G##_plan_indexed(const flexspmv_desc *desc, const void *const *indices,            \
+                                  const void *d_row_offsets, void *d_workspace,                     \
+                                  size_t workspace_bytes, void *stream);                            \
   int flexspmv_##G##_plan_windows(const flexspmv_desc *desc, const void *const *indices,            \
                                   void *d_workspace, size_t workspace_bytes, void *stream);         \
   int flexspmv_##G##_launch(const flexspmv_desc *desc, const void *const *values,                   \

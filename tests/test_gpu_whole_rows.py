@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from flexspmv_b200 import graphs, problems
-from flexspmv_b200.binding import Desc, GraphExtension, load_library
+from flexspmv_b200.binding import Desc, FlexSpmvError, GraphExtension, load_library
 from oracle import ir_eval
 from parity import assert_outputs_match
 from test_gpu_parity import run_gpu
@@ -103,6 +103,118 @@ def test_rows_that_begin_in_one_bank_keep_lanes_on_consecutive_edges(gname, dt, 
         assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} {dt} {lengths[:3]} {kw}")
         assert ext.planned_whole_rows()
         assert row_loop_planned(ext) == (1 if gname == "spring_mass" else 1 - same_bank)
+
+
+def with_columns(ir, prob, kind, seed):
+    """Columns of a matrix: consecutive ones from an arbitrary start per row ("runs"), consecutive rows side by side
+    ("stencil"), the first half of the rows one way and the second half the other ("both"), anywhere ("random")."""
+    rng = np.random.default_rng(seed)
+    lengths = np.diff(prob.row_offsets)
+    n, own = lengths.size, np.repeat(np.arange(lengths.size), lengths)
+    place = np.arange(own.size) - prob.row_offsets[own]
+    runs = rng.integers(0, n, n)[own] + place
+    stencil = own + 50 * place
+    cols = {"runs": runs, "stencil": stencil, "both": np.where(own < n // 2, stencil, runs), "random": rng.integers(0, n, own.size)}[kind]
+    for k in prob.indices:
+        prob.indices[k] = (cols % n).astype(np.int32)
+    return prob
+
+
+@pytest.mark.parametrize("dt", ["float64", "float32", "int64"])
+@pytest.mark.parametrize("kind,row_loop", [("runs", 0), ("stencil", 1), ("both", None), ("random", 1)])
+@pytest.mark.parametrize("lengths", [[20] * 2500, [9] * 9000, [0, 9, 3, 12] * 1500, [3] * 40, [7] * 9])
+def test_either_loop_on_whole_rows_gives_the_same_bits(dt, kind, row_loop, lengths):
+    """The plan looks at a sample of the columns and leaves rows that are runs of columns on the two-phase loop, whose lanes
+    walk consecutive edges.  Whichever loop runs, on whatever grid, a row is its products from left to right: the bits of the
+    loop with carries on one CTA (the same matrix with a row of 33 edges behind it)."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    n = len(lengths)
+    prob = with_columns(ir, with_lengths(ir, lengths, 37, dtype), kind, 41)
+    carry = with_lengths(ir, lengths + [33], 37, dtype)
+    carry.values["vals"][:prob.nnz], carry.values["x"][:n] = prob.values["vals"], prob.values["x"]
+    carry.indices["selector"][:prob.nnz] = prob.indices["selector"]
+    ext = GraphExtension(ir, random_gather=False, max_ctas=1)
+    want, _ = run_gpu(ext, ir, carry, dtype)
+    assert not ext.planned_whole_rows()
+    for kw, offsets in (({}, np.int32), ({}, np.int64), ({"max_ctas": 1}, np.int32), ({"max_ctas": 2}, np.int64), ({"max_ctas": 7}, np.int32),
+                        ({"tile_items": 200, "max_ctas": 3}, np.int32)):
+        ext = GraphExtension(ir, random_gather=False, **kw)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=offsets)
+        ext.check()
+        assert ext.planned_whole_rows() or "tile_items" in kw or n < 32
+        if not kw and n > 1000 and row_loop is not None:
+            assert row_loop_planned(ext) == row_loop
+        assert np.array_equal(got[0], want[0][:n]), (kw, offsets)
+
+
+def test_a_plan_that_has_not_seen_the_columns_goes_by_the_rows():
+    """flexspmv_G_plan and flexspmv_G_plan_indexed differ in the loop they choose for runs of columns and in nothing else; the
+    sample reads no column of matrices whose offsets lead outside of the arrays."""
+    lib = load_library()
+    ir, dtype = graphs.spmv_graph(), np.float64
+    prob = with_columns(ir, with_lengths(ir, [12] * 4000, 53, dtype), "runs", 59)
+    cols, ro = (torch.from_numpy(a).cuda() for a in (prob.indices["selector"], prob.row_offsets.astype(np.int64)))
+    for name in ("workspace_bytes", "plan", "plan_indexed"):
+        getattr(lib, f"flexspmv_spmv_f64_{name}").restype = ctypes.c_int
+    desc = Desc(prob.num_rows, prob.nnz, prob.num_cols, 64, 0, 0, 0)
+    nbytes = ctypes.c_size_t()
+    assert lib.flexspmv_spmv_f64_workspace_bytes(ctypes.byref(desc), ctypes.byref(nbytes)) == 0
+    ix = (ctypes.c_void_p * 1)(cols.data_ptr())
+    none = (ctypes.c_void_p * 1)(None)
+
+    def planned(indexed, offsets):
+        ws = torch.zeros(nbytes.value, dtype=torch.uint8, device="cuda")
+        args = [ctypes.c_void_p(offsets.data_ptr()), ctypes.c_void_p(ws.data_ptr()), nbytes, None]
+        if indexed:
+            assert lib.flexspmv_spmv_f64_plan_indexed(ctypes.byref(desc), ix, *args) == 0
+        else:
+            assert lib.flexspmv_spmv_f64_plan(ctypes.byref(desc), *args) == 0
+        torch.cuda.synchronize()
+        header = ws[:256].cpu().numpy().view(np.int32)
+        tiles = -(-(prob.num_rows + prob.nnz) // 1280)
+        return header[38:40].tolist(), ws[256:256 + 16 * (tiles + 1)].cpu()
+
+    (by_rows, coords), (by_columns, same) = planned(False, ro), planned(True, ro)
+    assert by_rows == [1, 1] and by_columns == [1, 0] and torch.equal(coords, same)
+    for wrong in (ro - 40, ro + 10 ** 9, ro.flip(0).contiguous(), ro * 1000):
+        assert planned(True, wrong)[0] == [-1, 0]
+    # no index arrays
+    ws = torch.zeros(nbytes.value, dtype=torch.uint8, device="cuda")
+    args = [ctypes.c_void_p(ro.data_ptr()), ctypes.c_void_p(ws.data_ptr()), nbytes, None]
+    assert lib.flexspmv_spmv_f64_plan_indexed(ctypes.byref(desc), None, *args) == -1
+    assert lib.flexspmv_spmv_f64_plan_indexed(ctypes.byref(desc), none, *args) == -1
+
+
+@pytest.mark.parametrize("gname,dt,kind", [("spmv", "float64", "runs"), ("spmv", "float64", "stencil"), ("spring_mass", "float32", None),
+                                           ("ops_zoo", "float64", None)])
+def test_bounded_wait_runs_out_on_tiles_of_whole_rows(gname, dt, kind):
+    """A stage that is never filled, on matrices of short rows: the consumers of either loop give up after their bounded wait,
+    the status says so, and a fresh plan gives the full result."""
+    lib = load_library()
+    lib.flexspmv_debug_withhold_stage.restype = ctypes.c_int
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [9] * 3000, 43, dtype)
+    if kind:
+        prob = with_columns(ir, prob, kind, 47)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    for withhold in (1, 2, 6):
+        ext = GraphExtension(ir, random_gather=False, max_ctas=2)
+        non_gather, gathers, index_names = graphs.operator_signature(ir)
+        v = [torch.from_numpy(np.ascontiguousarray(prob.values[n])).cuda() for n in non_gather + gathers]
+        ix = [torch.from_numpy(prob.indices[n]).cuda() for n in index_names]
+        ro = torch.from_numpy(prob.row_offsets).cuda()
+        outs = [torch.full(o.shape, float("nan"), dtype=v[0].dtype, device="cuda") for o in map(torch.from_numpy, ref)]
+        ext.prepare(v, ix, ro, outs, prob.num_rows, prob.nnz, prob.num_cols)
+        assert ext.planned_whole_rows()
+        ws = next(reversed(ext._plans.values())).ws
+        assert lib.flexspmv_debug_withhold_stage(ctypes.c_void_p(ws.data_ptr()), ctypes.c_uint32(withhold), None) == 0
+        ext.launch_into(v, ix, ro, outs, prob.num_rows, prob.nnz, prob.num_cols)
+        with pytest.raises(FlexSpmvError, match="bounded device-side wait"):
+            ext.check()
+        again = GraphExtension(ir, random_gather=False, max_ctas=2)
+        got, _ = run_gpu(again, ir, prob, dtype)
+        again.check()
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} after a wait ran out")
 
 
 def test_whole_rows_equal_the_two_phase_loop_bit_for_bit():
