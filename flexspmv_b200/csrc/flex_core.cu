@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <type_traits>
+
 #include "flex_common.cuh"
 
 namespace flex {
@@ -20,11 +22,14 @@ int device_sm_count() {
   return cached[dev];
 }
 
-// One thread per tile boundary: coordinate of diagonal t * tile_items (clamped to rows + edges).
+// One thread per tile boundary: coordinate of diagonal t * tile_items (clamped to rows + edges).  A plan's header goes along
+// (null: coordinates alone): a launch less in the first call on a matrix.
 template <typename OffsetT>
 __global__ void partition_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                 long long tile_items, long long num_tiles, OffsetT* __restrict__ coords) {
+                                 long long tile_items, long long num_tiles, OffsetT* __restrict__ coords,
+                                 WorkspaceHeader* header, const WorkspaceHeader contents) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0 && header) *header = contents;
   if (t > num_tiles) return;
   long long d = t * tile_items;
   if (d > num_rows + num_edges) d = num_rows + num_edges;
@@ -41,9 +46,10 @@ __global__ void partition_kernel(const OffsetT* __restrict__ row_offsets, long l
 // back to the row's first edge instead.  All boundaries or none: the header records the grid size it was done for.
 // A tile takes at most max_edges edges and its stage room.stage_bytes bytes of records and row ends.
 template <typename OffsetT>
-__global__ void snap_cta_boundaries_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_tiles,
-                                           int grid, const TileRoom room, OffsetT* __restrict__ coords, WorkspaceHeader* h) {
+__device__ void snap_cta_boundaries(const OffsetT* row_offsets, long long num_rows, long long num_tiles, int grid, const TileRoom& room,
+                                    OffsetT* coords, WorkspaceHeader* h) {
   __shared__ int s_ok;
+  if (grid < 2 || num_tiles < grid) return;
   if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
   const long long q = num_tiles / grid, r = num_tiles % grid;
@@ -68,6 +74,12 @@ __global__ void snap_cta_boundaries_kernel(const OffsetT* __restrict__ row_offse
   if (threadIdx.x == 0) h->snapped_grid = grid;
 }
 
+template <typename OffsetT>
+__global__ void snap_cta_boundaries_kernel(const OffsetT* row_offsets, long long num_rows, long long num_tiles, int grid,
+                                           const TileRoom room, OffsetT* coords, WorkspaceHeader* h) {
+  snap_cta_boundaries(row_offsets, num_rows, num_tiles, grid, room, coords, h);
+}
+
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream) {
   if (grid < 2 || num_tiles < grid) return 0;
@@ -81,16 +93,6 @@ int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long 
   return (int)cudaGetLastError();
 }
 
-// First edge of tile t once its front boundary has moved to a row start.  Edge 0 belongs to the first tile whatever
-// row_offsets[0] says, and boundaries behind the last row end stay where the merge path put them.
-template <typename OffsetT>
-__device__ __forceinline__ long long moved_edge(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                                long long num_tiles, const OffsetT* __restrict__ coords, long long t) {
-  if (t <= 0) return 0;
-  if (t >= num_tiles) return num_edges;
-  const long long x = (long long)coords[2 * t];
-  return x < num_rows ? (long long)row_offsets[x] : (long long)coords[2 * t + 1];
-}
 // Cache line of a gathered record, up to the array's offset in its first line; lines among the lanes with `in`.
 __device__ __forceinline__ unsigned line_of(int column, int record_bytes) { return (unsigned)(((long long)column * record_bytes) >> 7); }
 __device__ __forceinline__ unsigned distinct(unsigned line, bool in) {
@@ -102,62 +104,93 @@ __device__ __forceinline__ unsigned distinct(unsigned line, bool in) {
 // whole_rows = -1 when a row or a tile is too large.  Unlike the merge path, which stays inside [0, num_edges] for any
 // offsets, moved boundaries are offsets themselves: ones that descend, end behind the edges or leave a gap in front of the
 // first row (all of which the loop with carries takes without reading out of range) are refused here.
+// Part of the first call on every new matrix.  Bound by the latency of a tile's loads: coordinates are requested a tile ahead,
+// four groups of rows at once, positions in a tile are 32-bit.  Plan of 17 M rows of 7 edges 63 us with 32-bit offsets, 80 with
+// 64-bit ones (coordinates and rows one after the other, and five launches instead of three: 66 and 81; 4000 rows 24 -> 16);
+// eight groups of rows at once 59 and 87, 48 / 40 registers 61 / 75 and 88 / 93.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
                                                          long long num_tiles, const TileRoom room, const RowLoopRule rule,
                                                          const OffsetT* __restrict__ coords, WorkspaceHeader* h) {
+  constexpr int kAhead = 4;                 // loads in flight
+  __shared__ unsigned long long s_slots;
+  __shared__ unsigned s_seen[6];            // the header's bank_groups .. line_edge_lines
+  if (threadIdx.x == 0) s_slots = 0;
+  if (threadIdx.x < 6) s_seen[threadIdx.x] = 0;
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  unsigned long long slots = 0;
-  unsigned groups = 0, degree = 0, rows = 0, row_lines = 0, edges = 0, edge_lines = 0;
-  constexpr int kAhead = 4;
   const long long step = num_tiles / 1024 + 1;                              // tiles whose first 32 rows are looked at closely
+  unsigned long long slots = 0;
+  unsigned seen[6] = {0, 0, 0, 0, 0, 0};
   bool bad = false;
-  for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < num_tiles && !bad; t += warps) {
-    const long long x0 = (long long)coords[2 * t], x1 = (long long)coords[2 * t + 2];
-    const long long y0 = moved_edge(row_offsets, num_rows, num_edges, num_tiles, coords, t);
-    const long long y1 = moved_edge(row_offsets, num_rows, num_edges, num_tiles, coords, t + 1);
+  long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  OffsetT next[4] = {0, 0, 0, 0};           // coordinates are requested a tile ahead
+  int turn = 0;
+  if (t < num_tiles) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) next[i] = coords[2 * t + i];
+  }
+  for (; t < num_tiles && !bad; t += warps) {
+    const long long x0 = (long long)next[0], x1 = (long long)next[2];
+    // first edge of the tile and of the one behind it, once their boundaries have moved to row starts: edge 0 belongs to the
+    // first tile whatever row_offsets[0] says, and boundaries behind the last row end stay where the merge path put them
+    const OffsetT at0 = x0 < num_rows ? row_offsets[x0] : next[1], at1 = x1 < num_rows ? row_offsets[x1] : next[3];
+    // refused by another warp?  Not at every tile: one word that every warp reads is served at a few warps a clock
+    const int refused = (++turn & 7) == 0 ? __ldcg(&h->whole_rows) : 0;
+    if (t + warps < num_tiles) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) next[i] = coords[2 * (t + warps) + i];
+    }
+    const long long y0 = t == 0 ? 0 : (long long)at0, y1 = t + 1 == num_tiles ? num_edges : (long long)at1;
     bad = y0 < 0 || y1 < y0 || y1 > num_edges || !room.fits(y1 - y0, x1 - x0);
-    for (long long r0 = x0; r0 < x1; r0 += 32 * kAhead) {
-      long long begin[kAhead], end[kAhead];                                 // all loads before the first vote
+    if (bad || refused == -1) break;
+    // from here on positions in the tile, which is at most a tile's edges long: 32 bits
+    const int rows = (int)(x1 - x0), edges = (int)(y1 - y0);
+    const OffsetT* ends = row_offsets + x0 + 1 + lane;
+    int before = 0;                                                         // where lane 0's next row begins
+    for (int r0 = 0; r0 < rows; r0 += 32 * kAhead) {
+      OffsetT end[kAhead];
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) end[j] = r0 + 32 * j + lane < rows ? ends[r0 + 32 * j] : OffsetT(0);
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
-        const long long r = r0 + 32 * j + lane;
-        begin[j] = end[j] = y1;
-        if (r < x1) {
-          begin[j] = r == x0 ? y0 : (long long)row_offsets[r];
-          end[j] = (long long)row_offsets[r + 1];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j) {
-        if (r0 + 32 * j >= x1) break;                                       // the same for the whole warp
-        const long long len = end[j] - begin[j];
-        const bool fits = len >= 0 && len <= kWholeRowMax && begin[j] >= y0 && end[j] <= y1;
-        const int longest = __reduce_max_sync(0xffffffffu, fits ? (int)len : kWholeRowMax + 1);
+        if (r0 + 32 * j >= rows) break;                                     // the same for the whole warp
+        const bool in = r0 + 32 * j + lane < rows;
+        const auto ahead = static_cast<std::make_unsigned_t<OffsetT>>(end[j] - (OffsetT)y0);     // huge where the end lies in front
+        const bool inside = ahead <= static_cast<std::make_unsigned_t<OffsetT>>(edges);
+        const int to = (int)ahead, rotated = __shfl_sync(0xffffffffu, to, (lane + 31) & 31);
+        const int from = lane ? rotated : before, len = to - from;
+        before = rotated;                                                   // lane 0: the end of lane 31's row
+        const int counted = !in ? 0 : (inside && (unsigned)len <= (unsigned)kWholeRowMax ? len : kWholeRowMax + 1);
+        const int longest = __reduce_max_sync(0xffffffffu, counted);
         bad |= longest > kWholeRowMax;
         slots += 32u * (unsigned)longest;
-        if (j == 0 && r0 == x0 && t % step == 0) {
-          const int bank = (int)(begin[0] & 31);
-          unsigned same = __ballot_sync(0xffffffffu, len > 0);
-          groups += same != 0;
+        if (j == 0 && r0 == 0 && t % step == 0 && !bad) {
+          const int bank = (int)(y0 + from) & 31;
+          const bool row = counted > 0, edge = lane < edges;
+          unsigned same = __ballot_sync(0xffffffffu, row);
+          seen[0] += same != 0;
 #pragma unroll
           for (int b = 0; b < 5; ++b) {
             const unsigned set = __ballot_sync(0xffffffffu, (bank >> b) & 1);
             same &= (bank >> b) & 1 ? set : ~set;
           }
-          degree += __reduce_max_sync(0xffffffffu, len > 0 ? (unsigned)__popc(same) : 0u);
-          // lines of the rows' middle edges and of consecutive edges, where the offsets lead into the arrays
-          const bool row = fits && len > 0, edge = lane < (int)(y1 - y0 < 32 ? y1 - y0 : 32);
+          seen[1] += __reduce_max_sync(0xffffffffu, row ? (unsigned)__popc(same) : 0u);
+          // lines of the rows' middle edges and of consecutive edges: these offsets lead into the arrays
+#pragma unroll 1
+          for (int i = 0; i < rule.gathers; ++i) {
+            const int* index = rule.index[0];
+            int record_bytes = rule.record_bytes[0];
 #pragma unroll
-          for (int i = 0; i < RowLoopRule::kMaxGathers; ++i) {
-            if (i >= rule.gathers || bad) break;                            // the same for the whole warp
-            const unsigned at_row = row ? line_of(rule.index[i][begin[0] + (len >> 1)], rule.record_bytes[i]) : 0u;
-            const unsigned at_edge = edge ? line_of(rule.index[i][y0 + lane], rule.record_bytes[i]) : 0u;
-            rows += __popc(__ballot_sync(0xffffffffu, row));
-            edges += __popc(__ballot_sync(0xffffffffu, edge));
-            row_lines += distinct(at_row, row);
-            edge_lines += distinct(at_edge, edge);
+            for (int g = 1; g < RowLoopRule::kMaxGathers; ++g)
+              if (i == g) { index = rule.index[g]; record_bytes = rule.record_bytes[g]; }
+            const unsigned at_row = row ? line_of(index[y0 + from + (len >> 1)], record_bytes) : 0u;
+            const unsigned at_edge = edge ? line_of(index[y0 + lane], record_bytes) : 0u;
+            seen[2] += __popc(__ballot_sync(0xffffffffu, row));
+            seen[3] += distinct(at_row, row);
+            seen[4] += __popc(__ballot_sync(0xffffffffu, edge));
+            seen[5] += distinct(at_edge, edge);
           }
         }
       }
@@ -165,18 +198,15 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
   }
   if (lane == 0) {
     if (bad) h->whole_rows = -1;
-    else if (slots) atomicAdd(reinterpret_cast<unsigned long long*>(&h->row_slots), slots);
-    if (!bad && groups) {
-      atomicAdd(&h->bank_groups, groups);
-      atomicAdd(&h->bank_degree, degree);
-      if (rule.gathers) {
-        atomicAdd(&h->line_rows, rows);
-        atomicAdd(&h->line_row_lines, row_lines);
-        atomicAdd(&h->line_edges, edges);
-        atomicAdd(&h->line_edge_lines, edge_lines);
-      }
+    if (!bad && slots) atomicAdd(&s_slots, slots);
+    if (!bad && seen[0]) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) atomicAdd(&s_seen[i], seen[i]);
     }
   }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_slots) atomicAdd(reinterpret_cast<unsigned long long*>(&h->row_slots), s_slots);
+  if (threadIdx.x < 6 && s_seen[threadIdx.x]) atomicAdd(&h->bank_groups + threadIdx.x, s_seen[threadIdx.x]);
 }
 // Moves the boundaries when the kernel above found nothing against it and at least two fifths of the thread-steps have
 // an edge to work on: rows of very different lengths are better off with the two-phase loop, whose lanes take
@@ -195,19 +225,24 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
 // lines a gather) 55 / 57 and 41 / 44, 5 (32, 8) 46 / 43 and 36 / 35, 8 (32, 5) 67 / 52 and 49 / 37, 20 (32, 2) 54 / 41 and 36 / 32;
 // stencils (2 - 3 against 8 - 16 lines), banded and random columns: this loop, by 4 - 50 %.  A plan that has not been shown the
 // columns goes by the rows alone.
+// Where it does not move them all, its first CTA looks after the boundaries between the CTAs of the plan's grid.
 template <typename OffsetT>
-__global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __restrict__ row_offsets, long long num_rows, long long num_edges,
-                                                               long long num_tiles, const RowLoopRule rule, OffsetT* __restrict__ coords,
-                                                               WorkspaceHeader* h) {
-  if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1) return;
-  if (2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) return;
+__global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* row_offsets, long long num_rows, long long num_edges,
+                                                               long long num_tiles, const RowLoopRule rule, int grid, const TileRoom room,
+                                                               OffsetT* coords, WorkspaceHeader* h) {
+  // whole_rows is read by this kernel only as "-1 or not"
+  if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1 || 2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) {
+    if (blockIdx.x == 0) snap_cta_boundaries(row_offsets, num_rows, num_tiles, grid, room, coords, h);
+    return;
+  }
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t > 0 && t < num_tiles) {
     const long long x = (long long)coords[2 * t];
     if (x < num_rows) coords[2 * t + 1] = row_offsets[x];
   }
   if (t == 0) {
-    *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;     // read by this kernel only as "-1 or not"
+    *reinterpret_cast<volatile int32_t*>(&h->whole_rows) = 1;
+    if (grid >= 2 && num_tiles >= grid) h->snapped_grid = grid;
     const bool same_bank = h->bank_degree > 10 * h->bank_groups;
     const long long lines_more = 32ll * h->line_row_lines * h->line_edges - 32ll * h->line_edge_lines * h->line_rows;   // x rows x edges
     const bool edges_share_lines = lines_more * rule.gathers > 22ll * rule.accumulators * h->line_rows * h->line_edges;
@@ -217,40 +252,44 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* __
 
 template <typename OffsetT>
 static int whole_rows_launch_as(const void* d_row_offsets, long long num_rows, long long num_edges, long long num_tiles,
-                                const TileRoom& room, const RowLoopRule& rule, void* d_coords, WorkspaceHeader* h, cudaStream_t stream) {
+                                const TileRoom& room, const RowLoopRule& rule, int cta_grid, void* d_coords, WorkspaceHeader* h,
+                                cudaStream_t stream) {
   const OffsetT* ro = static_cast<const OffsetT*>(d_row_offsets);
   OffsetT* coords = static_cast<OffsetT*>(d_coords);
   long long grid = (num_tiles + 7) / 8;
   const long long cap = (long long)device_sm_count() * 8;
   if (grid > cap) grid = cap;
   whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, rule, coords, h);
-  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, rule, coords, h);
+  whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, rule, cta_grid,
+                                                                                           room, coords, h);
   return (int)cudaGetLastError();
 }
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, const RowLoopRule& rule, void* d_coords, void* ws, cudaStream_t stream) {
+                      const TileRoom& room, const RowLoopRule& rule, int grid, void* d_coords, void* ws, cudaStream_t stream) {
   if (num_tiles < 1 || num_rows < 1) return 0;
   WorkspaceHeader* h = static_cast<WorkspaceHeader*>(ws);
-  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, rule, d_coords, h, stream);
-  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, rule, d_coords, h, stream);
+  if (offset_bits == 32) return whole_rows_launch_as<int>(d_row_offsets, num_rows, num_edges, num_tiles, room, rule, grid, d_coords, h, stream);
+  return whole_rows_launch_as<long long>(d_row_offsets, num_rows, num_edges, num_tiles, room, rule, grid, d_coords, h, stream);
 }
 
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,
-                     int tile_items, void* d_coords, cudaStream_t stream) {
+                     int tile_items, void* d_coords, cudaStream_t stream, void* ws, const WorkspaceHeader* h) {
   if (!d_row_offsets || !d_coords || tile_items <= 0 || num_rows < 0 || num_edges < 0) return FLEXSPMV_ERR_BAD_ARG;
   if (offset_bits != 32 && offset_bits != 64) return FLEXSPMV_ERR_BAD_ARG;
   if (offset_bits == 32 && num_rows + num_edges >= (1ll << 31)) return FLEXSPMV_ERR_TOO_LARGE;
   const long long tiles = (num_rows + num_edges + tile_items - 1) / tile_items;
   const int block = 128;
+  WorkspaceHeader* header = static_cast<WorkspaceHeader*>(ws);
+  const WorkspaceHeader contents = h ? *h : WorkspaceHeader{};
   const long long grid = (tiles + 1 + block - 1) / block;
   if (grid > 0x7fffffffLL) return FLEXSPMV_ERR_TOO_LARGE;
   if (offset_bits == 32)
     partition_kernel<int><<<(unsigned)grid, block, 0, stream>>>(static_cast<const int*>(d_row_offsets), num_rows, num_edges,
-                                                                tile_items, tiles, static_cast<int*>(d_coords));
+                                                                tile_items, tiles, static_cast<int*>(d_coords), header, contents);
   else
     partition_kernel<long long><<<(unsigned)grid, block, 0, stream>>>(static_cast<const long long*>(d_row_offsets), num_rows,
                                                                       num_edges, tile_items, tiles,
-                                                                      static_cast<long long*>(d_coords));
+                                                                      static_cast<long long*>(d_coords), header, contents);
   return (int)cudaGetLastError();
 }
 
@@ -601,7 +640,7 @@ int flexspmv_partition_bytes(int64_t num_rows, int64_t num_edges, int32_t offset
 int flexspmv_partition(const void* d_row_offsets, int32_t offset_bits, int64_t num_rows, int64_t num_edges,
                        int32_t tile_items, void* d_coords, void* stream) {
   return flex::partition_launch(d_row_offsets, offset_bits, num_rows, num_edges, tile_items, d_coords,
-                                static_cast<cudaStream_t>(stream));
+                                static_cast<cudaStream_t>(stream), nullptr, nullptr);
 }
 
 int flexspmv_row_blocks(const void* d_row_offsets, int32_t offset_bits, int64_t num_rows, int32_t parts, int64_t snap,

@@ -18,13 +18,13 @@ namespace flex {
 
 // implemented in flex_core.cu
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,
-                     int tile_items, void* d_coords, cudaStream_t stream);
+                     int tile_items, void* d_coords, cudaStream_t stream, void* ws, const WorkspaceHeader* h);
 int device_sm_count();
 int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream);
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
 int whole_rows_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges, long long num_tiles,
-                      const TileRoom& room, const RowLoopRule& rule, void* d_coords, void* ws, cudaStream_t stream);
+                      const TileRoom& room, const RowLoopRule& rule, int grid, void* d_coords, void* ws, cudaStream_t stream);
 int window_plan_launch(const void* d_coords, int offset_bits, long long num_tiles, const int* d_idx, int rec_bytes,
                        int win_bytes, void* d_table, void* d_local_idx, cudaStream_t st);
 int window_ready_launch(void* ws, cudaStream_t st);
@@ -167,7 +167,7 @@ struct GraphApi {
     return room;
   }
 
-  // `whole_rows`: also look for a matrix of short rows whose tiles can all hold whole rows (two more kernels).
+  // `whole_rows`: also look for a matrix of short rows whose tiles can all hold whole rows.
   // `indices` (may be null): the launch's index arrays, which the choice of the loop on such tiles looks at.
   static int plan(const flexspmv_desc* d, const void* const* indices, const void* row_offsets, void* ws, size_t ws_bytes, cudaStream_t st,
                   bool whole_rows = true) {
@@ -180,12 +180,26 @@ struct GraphApi {
     h.magic = kMagic; h.ticket = 0; h.status = 0; h.offset_bits = d->offset_bits;
     h.num_rows = d->num_rows; h.num_edges = d->num_edges; h.num_tiles = num_tiles(d);
     h.tile_items = tile_items(d); h.max_ctas = d->max_ctas;
-    if (int e = header_init_launch(ws, h, st)) return e;   // a one-thread kernel: stream-ordered, no host sync
-    if (G::kHasReducer) {
+    if constexpr (G::kHasReducer) {
       if (!row_offsets) return FLEXSPMV_ERR_BAD_ARG;
       if (!aligned16(row_offsets)) return FLEXSPMV_ERR_ALIGN;
-      if (int e = partition_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, tile_items(d),
-                                   static_cast<char*>(ws) + h.coords_offset, st)) return e;
+      char* const coords = static_cast<char*>(ws) + h.coords_offset;
+      if (int e = partition_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, tile_items(d), coords, st, ws, &h)) return e;
+      if (use_lean(d)) return 0;
+      // the tile kernel: the grid it will have
+      int grid = 0;
+      bool win = false;
+      if constexpr (G::kWindowGather && kWindowsBuilt) win = use_win(d);
+      if (h.num_tiles > 1) {
+        int resident = 0, e = 0;
+        if constexpr (G::kWindowGather && kWindowsBuilt) {
+          if (win) e = d->offset_bits == 64 ? resident_ctas<long long, CfgWin, true>(&resident) : resident_ctas<int, CfgWin, true>(&resident);
+        }
+        if (!win) e = d->offset_bits == 64 ? resident_ctas<long long>(&resident) : resident_ctas<int>(&resident);
+        if (e) return e;
+        const long long most = max_ctas(d, resident);
+        grid = (int)(most < h.num_tiles ? most : h.num_tiles);
+      }
       if constexpr (WholeTiles<G, Cfg, false>::value) {
         RowLoopRule rule{};
         rule.built = WholeRows<G, Cfg, false>::value;
@@ -194,31 +208,17 @@ struct GraphApi {
         if (rule.built && rule.edge_lanes && indices) rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
         for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
         // rows longer than kWholeRowMax on average: no need to look
-        if (whole_rows && !use_lean(d) && !use_win(d) && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
-          if (int e = whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d),
-                                        rule, static_cast<char*>(ws) + h.coords_offset, ws, st)) return e;
+        if (whole_rows && !use_win(d) && d->num_rows > 0 && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
+          return whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d), rule, grid, coords, ws, st);
       }
-      // the tile kernel: boundaries between the CTAs of its grid moved onto row ends where the tiles have room
-      if (!use_lean(d) && h.num_tiles > 1) {
-        int resident = 0;
-        int e = 0;
-        bool win = false;
-        if constexpr (G::kWindowGather && kWindowsBuilt) win = use_win(d);
-        if constexpr (G::kWindowGather && kWindowsBuilt) {
-          if (win) e = d->offset_bits == 64 ? resident_ctas<long long, CfgWin, true>(&resident) : resident_ctas<int, CfgWin, true>(&resident);
-        }
-        if (!win) e = d->offset_bits == 64 ? resident_ctas<long long>(&resident) : resident_ctas<int>(&resident);
-        if (e) return e;
-        long long grid = max_ctas(d, resident);
-        if (grid > h.num_tiles) grid = h.num_tiles;
-        TileRoom room = tile_room<Cfg>(d);
-        if constexpr (G::kWindowGather && kWindowsBuilt) { if (win) room = tile_room<CfgWin>(d); }
-        return snap_cta_boundaries_launch(row_offsets, d->offset_bits, d->num_rows, h.num_tiles, (int)grid, room,
-                                          static_cast<char*>(ws) + h.coords_offset, ws, st);
-      }
-      return 0;
+      // boundaries between the CTAs of that grid moved onto row ends where the tiles have room
+      TileRoom room = tile_room<Cfg>(d);
+      if constexpr (G::kWindowGather && kWindowsBuilt) { if (win) room = tile_room<CfgWin>(d); }
+      return snap_cta_boundaries_launch(row_offsets, d->offset_bits, d->num_rows, h.num_tiles, grid, room, coords, ws, st);
+    } else {
+      (void)indices; (void)row_offsets; (void)whole_rows;
+      return header_init_launch(ws, h, st);   // a one-thread kernel: stream-ordered, no host sync
     }
-    return 0;
   }
 
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
