@@ -72,6 +72,7 @@ def load_library(path: Optional[str] = None) -> ctypes.CDLL:
         lib = ctypes.CDLL(path)
         lib.flexspmv_error_string.restype = ctypes.c_char_p
         lib.flexspmv_error_string.argtypes = [ctypes.c_int]
+        lib.flexspmv_plan_launches.restype = ctypes.c_int64
         _libs[path] = lib
     return _libs[path]
 
@@ -277,20 +278,19 @@ class GraphExtension:
         check(self.lib, syms.workspace_bytes(ctypes.byref(desc), ctypes.byref(nbytes)), "workspace_bytes")
         ws = torch.empty(nbytes.value, dtype=torch.uint8, device=device)
         ip = _pointers(indices)
+        before = self.lib.flexspmv_plan_launches()
         check(self.lib, syms.plan(ctypes.byref(desc), ip, ctypes.c_void_p(ro.data_ptr() if ro is not None else 0),
                                   ctypes.c_void_p(ws.data_ptr()), ctypes.c_size_t(nbytes.value), _stream_ptr()),
               "plan")
         if desc.reserved & 1:      # gather windows: the second planning step reads the index array
             check(self.lib, syms.plan_windows(ctypes.byref(desc), ip, ctypes.c_void_p(ws.data_ptr()),
                                               ctypes.c_size_t(nbytes.value), _stream_ptr()), "plan_windows")
-            self.launches += 2
-        self.launches += 2 if ro is not None else 1
         # keep the row-offset tensor alive so its address cannot be recycled under a cached plan
         plan = _Plan(ws, nbytes.value, (ro, tuple(indices) if (desc.reserved & 1) else None), desc)
         check(self.lib, self.lib.flexspmv_workspace_status_mirror(ctypes.c_void_p(ws.data_ptr()),
                                                                   ctypes.c_void_p(plan.flag.data_ptr()), _stream_ptr()),
               "workspace_status_mirror")
-        self.launches += 1
+        self.launches += self.lib.flexspmv_plan_launches() - before
         self._plans[key] = plan
         while len(self._plans) > self.PLAN_CACHE_ENTRIES:
             self._plans.popitem(last=False)

@@ -22,6 +22,9 @@ int device_sm_count() {
   return cached[dev];
 }
 
+// Kernels that planning has enqueued from this thread (flexspmv_plan_launches).
+static thread_local long long plan_launches = 0;
+
 // One thread per tile boundary: coordinate of diagonal t * tile_items (clamped to rows + edges).  A plan's header goes along
 // (null: coordinates alone): a launch less in the first call on a matrix.
 template <typename OffsetT>
@@ -83,6 +86,7 @@ __global__ void snap_cta_boundaries_kernel(const OffsetT* row_offsets, long long
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream) {
   if (grid < 2 || num_tiles < grid) return 0;
+  plan_launches += 1;
   if (offset_bits == 32)
     snap_cta_boundaries_kernel<int><<<1, 256, 0, stream>>>(static_cast<const int*>(d_row_offsets), num_rows, num_tiles, grid, room,
                                                            static_cast<int*>(d_coords), static_cast<WorkspaceHeader*>(ws));
@@ -259,6 +263,7 @@ static int whole_rows_launch_as(const void* d_row_offsets, long long num_rows, l
   long long grid = (num_tiles + 7) / 8;
   const long long cap = (long long)device_sm_count() * 8;
   if (grid > cap) grid = cap;
+  plan_launches += 2;
   whole_rows_kernel<OffsetT><<<(unsigned)grid, 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, room, rule, coords, h);
   whole_rows_apply_kernel<OffsetT><<<(unsigned)((num_tiles + 255) / 256), 256, 0, stream>>>(ro, num_rows, num_edges, num_tiles, rule, cta_grid,
                                                                                            room, coords, h);
@@ -283,6 +288,7 @@ int partition_launch(const void* d_row_offsets, int offset_bits, long long num_r
   const WorkspaceHeader contents = h ? *h : WorkspaceHeader{};
   const long long grid = (tiles + 1 + block - 1) / block;
   if (grid > 0x7fffffffLL) return FLEXSPMV_ERR_TOO_LARGE;
+  plan_launches += 1;
   if (offset_bits == 32)
     partition_kernel<int><<<(unsigned)grid, block, 0, stream>>>(static_cast<const int*>(d_row_offsets), num_rows, num_edges,
                                                                 tile_items, tiles, static_cast<int*>(d_coords), header, contents);
@@ -309,10 +315,12 @@ __global__ void status_mirror_kernel(WorkspaceHeader* h, int32_t* mirror) {
   }
 }
 int window_ready_launch(void* ws, cudaStream_t st) {
+  plan_launches += 1;
   window_ready_kernel<<<1, 32, 0, st>>>(static_cast<WorkspaceHeader*>(ws));
   return (int)cudaGetLastError();
 }
 int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream) {
+  plan_launches += 1;
   header_init_kernel<<<1, 32, 0, stream>>>(static_cast<WorkspaceHeader*>(ws), h);
   return (int)cudaGetLastError();
 }
@@ -470,6 +478,7 @@ int window_plan_launch(const void* d_coords, int offset_bits, long long num_tile
   long long grid = num_tiles;
   const long long cap = (long long)device_sm_count() * 8;
   if (grid > cap) grid = cap;
+  plan_launches += 1;
   if (offset_bits == 64)
     window_plan_kernel<long long><<<(unsigned)grid, 256, 0, st>>>(static_cast<const long long*>(d_coords), num_tiles, d_idx,
                                                                   rec_bytes, win_bytes, static_cast<int*>(d_table),
@@ -675,9 +684,12 @@ int flexspmv_workspace_status_mirror(void* d_workspace, int32_t* pinned_host_sta
     if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
     alias = static_cast<int32_t*>(dptr);
   }
+  ++flex::plan_launches;
   flex::status_mirror_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<flex::WorkspaceHeader*>(d_workspace), alias);
   return (int)cudaGetLastError();
 }
+
+int64_t flexspmv_plan_launches(void) { return flex::plan_launches; }
 
 int flexspmv_workspace_whole_rows(const void* d_workspace, int32_t* d_out, void* stream) {
   if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;

@@ -218,6 +218,10 @@ int flexspmv_swe_rk_stage(int32_t value_bytes, const void *const *d_r, const voi
                           void *const *d_stage, double c, double w, int64_t n, int32_t first,
                           int32_t last, void *stream);
 
+/* Kernels that plan, plan_indexed, plan_windows and flexspmv_workspace_status_mirror have enqueued from the calling thread
+ * since it started; the difference over a call is that call's. */
+int64_t flexspmv_plan_launches(void);
+
 /* Copies to *d_out (int32 in device or page-locked host memory), without synchronising, 1 when the plan in the workspace
  * found a matrix of short rows (at most 32 edges) whose tiles all hold whole rows.  Launches on it hand no carries over,
  * whatever their grid; row-mode graphs and graphs of light maps run a loop without barriers on it, and a graph with an

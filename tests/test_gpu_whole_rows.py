@@ -335,3 +335,19 @@ def test_row_mode_rows_on_both_sides_of_edge_two_to_the_31():
         assert ((got[first:first + 5000].double() - f.sum(dim=1)).abs() <= bound).all()
     del rest, stiff, pos, src, dst, ro, got
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("gname,dt,lengths,kw,planned", [
+    ("spmv", "float64", [5] * 3000, {}, 4),                                 # partition, look, move; status mirror
+    ("spmv", "float64", [40] * 3000, {}, 3),                                # partition, boundaries between CTAs; mirror
+    ("spmv", "float64", [40] * 20, {}, 2),                                  # one tile: partition; mirror
+    ("spmv", "float64", [40] * 3000, {"random_gather": True}, 2),           # partition into chunks; mirror
+    ("spmv", "float64", [5] * 3000, {"gather_windows": True}, 5),           # partition, boundaries, windows, their flag; mirror
+    ("mixed_dims", "float32", [5] * 3000, {}, 3),
+    ("edge_sum", "float32", [5] * 3000, {}, 2)])                            # header; mirror
+def test_the_launch_count_holds_the_plans_kernels(gname, dt, lengths, kw, planned):
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    ext = GraphExtension(ir, **{"random_gather": False, "gather_windows": False, **kw})
+    prob = with_lengths(ir, lengths, 61, dtype)
+    run_gpu(ext, ir, prob, dtype)
+    assert ext.launches == planned + 1
