@@ -113,9 +113,10 @@ def _stream_ptr() -> ctypes.c_void_p:
 
 # The call path asks for the current device and stream on every launch; these are the plain integers behind
 # torch.cuda.current_device() and torch.cuda.current_stream(index).cuda_stream, without the Stream object that the
-# latter builds each time (CUDA is initialised by then: the arguments are CUDA tensors).
-_current_device = torch._C._cuda_getDevice
-_raw_stream = torch._C._cuda_getCurrentRawStream
+# latter builds each time (CUDA is initialised by then: the arguments are CUDA tensors).  They are torch's own internals,
+# which a torch without CUDA or a later one may not have: then the public functions serve.
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 # flexspmv_<graph>_launch(desc, values, indices, row_offsets, outputs, workspace, workspace_bytes, stream): with the
 # argument types declared ctypes converts plain integers itself, without a wrapper object per pointer

@@ -154,3 +154,20 @@ def test_edges_in_flight_per_row(make, dtype, batches):
     import re
     fields = re.search(r"using Cfg = flex::TileCfg<([^>]*)>", emit_cuda.emit_graph(make(), dtype)).group(1).split(", ")
     assert (int(fields[4]), int(fields[6])) == batches
+
+
+def test_the_package_imports_without_torchs_cuda_internals():
+    """A torch without CUDA has no torch._C._cuda_getDevice: the import must get as far as load_library's own message."""
+    import os
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for n in ('_cuda_getDevice', '_cuda_getCurrentRawStream'):\n"
+            "    if hasattr(torch._C, n): delattr(torch._C, n)\n"
+            "from flexspmv_b200 import binding\n"
+            "assert binding._current_device is torch.cuda.current_device\n"
+            "try: binding.load_library('/nowhere.so')\n"
+            "except binding.FlexSpmvError as e: print(e)\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert r.returncode == 0 and "not found" in r.stdout, r.stderr
