@@ -13,7 +13,12 @@ pytestmark = pytest.mark.gpu
 
 def mesh_of(n, dtype, split_walls):
     m = {k: v for k, v in problems.swe_model_inputs(n).items() if k != "row_offsets"}
-    if split_walls:      # a wall record per face: cells with several come several times, ascending
+    if split_walls == "everywhere":      # 1 to 3 records on most cells, none on some, up to 96 in a group of 32 cells
+        cells = m["h"].size
+        counts = np.random.default_rng(5).choice([0, 1, 2, 3], cells, p=[0.1, 0.2, 0.2, 0.5])
+        m["bcells"] = np.repeat(np.arange(cells), counts).astype(m["bcells"].dtype)
+        m["bsx"], m["bsy"] = np.random.default_rng(7).uniform(-1e-3, 1e-3, (2, m["bcells"].size))
+    elif split_walls:      # a wall record per face: cells with several come several times, ascending
         keep = np.repeat(np.arange(m["bcells"].size), np.where(np.arange(m["bcells"].size) % 3 == 0, 3, 1))
         m["bcells"] = m["bcells"][keep]
         m["bsx"], m["bsy"] = 0.3 * m["bsx"][keep], 0.7 * m["bsy"][keep]
@@ -23,7 +28,7 @@ def mesh_of(n, dtype, split_walls):
 
 @pytest.mark.parametrize("n", [1, 3, 16, 33, 97])
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-@pytest.mark.parametrize("split_walls", [False, True])
+@pytest.mark.parametrize("split_walls", [False, True, "everywhere"])
 def test_fused_stage_equals_three_launches(n, dtype, split_walls):
     dt = 0.05 / n
     a, b = mesh_of(n, dtype, split_walls), mesh_of(n, dtype, split_walls)
