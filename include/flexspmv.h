@@ -321,6 +321,28 @@ FLEXSPMV_DECLARE_GRAPH(edge_copy_f64)
 FLEXSPMV_DECLARE_GRAPH(edge_copy_i64)
 
 /*
+ * swe_delta_rk_T: the swe_delta graph with one stage of the model's Runge-Kutta step behind its sums (the arithmetic of
+ * flexspmv_swe_rk_stage, and the swe_boundary graph's wall terms, with c, w, first and last as there), so that a stage is one
+ * launch.  No reference counterpart.  The same entry points as every graph's; launch's arrays, all of num_rows (= cells) or
+ * num_edges records of T in device memory unless said otherwise:
+ *   values[0..2]    alpha, sx, sy (per edge)
+ *   values[3..5]    h, uh, vh: the state that the fluxes are evaluated at (gathered; must not be an output)
+ *   values[6..8]    area (per cell), bsx, bsy (per wall record)
+ *   values[9]       int32, ceil(cells / 32) + 1 entries: entry i is the first wall record of a cell >= 32 i
+ *   values[10]      int32, the cell of every wall record, ascending
+ *   values[11..13]  h, uh, vh: the state at the beginning of the step; read, and advanced in place by the last stage
+ *   values[14..16]  running sums of the increments: written by the first stage, read and written by the others
+ *   values[17]      a HOST pointer to four T: c, w, first, last (0 or 1); read before launch returns
+ *   indices[0..1]   src, dst (edges sorted by dst, as row_offsets say)
+ *   outputs[0..2]   the state that the next stage's fluxes are evaluated at (not written by the last stage)
+ * The workspace's plan must hold whole rows (flexspmv_workspace_whole_rows): otherwise launch raises
+ * FLEXSPMV_ERR_NOT_PLANNED in the workspace status and writes nothing.  flexspmv_b200/shallow_water.py binds a step.
+ */
+#define FLEXSPMV_DECLARE_EPILOGUE_GRAPH(G) FLEXSPMV_DECLARE_GRAPH(G)
+FLEXSPMV_DECLARE_EPILOGUE_GRAPH(swe_delta_rk_f64)
+FLEXSPMV_DECLARE_EPILOGUE_GRAPH(swe_delta_rk_f32)
+
+/*
  * flexspmv_spmv_f64_launch_static -- the fused fp64 SpMV for callers that must not allocate.
  *
  * No counterpart in the reference: its operator allocates temporary storage with cudaMalloc on every

@@ -99,3 +99,17 @@ def test_header_is_plain_c_and_links(tmp_path):
                     "-L", lib_dir, "-lflexspmv_b200", f"-Wl,-rpath,{lib_dir}"], check=True, capture_output=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert int(out[0]) >= 1 and int(out[1]) > 0
+
+
+def test_header_is_c_and_declares_the_epilogue_graphs(lib, tmp_path):
+    """Every entry point that the macros declare, plan_indexed among them, compiled as C and found in the library."""
+    import subprocess
+    graphs = re.findall(r"^FLEXSPMV_DECLARE_(?:EPILOGUE_)?GRAPH\((\w+)\)", open(HEADER).read(), flags=re.M)
+    assert "swe_delta_rk_f64" in graphs and "swe_delta_rk_f32" in graphs
+    names = [f"flexspmv_{g}_{fn}" for g in graphs for fn in ("info", "workspace_bytes", "plan", "plan_indexed", "plan_windows", "launch", "device_status")]
+    src = tmp_path / "uses.c"
+    src.write_text('#include "flexspmv.h"\nvoid *all[] = {' + ", ".join(f"(void *){n}" for n in names) + "};\n")
+    subprocess.run(["gcc", "-std=c99", "-Wall", "-Wextra", "-Werror", "-c", str(src), "-I", os.path.dirname(HEADER), "-o", str(tmp_path / "uses.o")],
+                   check=True)
+    missing = [n for n in names if not hasattr(lib, n)]
+    assert not missing, missing
