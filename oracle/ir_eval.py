@@ -23,7 +23,7 @@ from __future__ import annotations
 import ctypes
 import os
 import subprocess
-from typing import Dict, List, Optional, Tuple
+from typing import Dict, List, NamedTuple, Optional, Sequence, Tuple
 
 import numpy as np
 
@@ -95,12 +95,24 @@ def tile_coordinates(row_offsets: np.ndarray, tile_items: int) -> np.ndarray:
     return out
 
 
-def snap_cta_boundaries(coords: np.ndarray, row_offsets: np.ndarray, grid: int):
+class TileRoom(NamedTuple):
+    """What a tile of the tile kernel takes: edges, and bytes of per-edge records and row ends in its stage."""
+    max_edges: int
+    stage_bytes: int
+    edge_bytes: int
+    offset_bytes: int
+
+    def fits(self, edges, rows):
+        return (edges <= self.max_edges) & (edges * self.edge_bytes + rows * self.offset_bytes <= self.stage_bytes)
+
+
+def snap_cta_boundaries(coords: np.ndarray, row_offsets: np.ndarray, grid: int, room: Optional[TileRoom] = None):
     """Restatement of the plan step that moves the tile boundaries in front of the CTAs of a ``grid``-CTA launch
     onto row ends (this package's own step, no reference counterpart).  CTA c starts at tile
     ``c q + min(c, r)`` (q, r = divmod(tiles, grid)); a boundary (x, y) that cuts row x moves back to
     ``(x, row_offsets[x])`` when the cut-off part fits the tile behind it (at most as many edges as that tile
-    holds row ends) and the row starts inside the tile in front.  All boundaries or none.
+    holds row ends), the tile's records and row ends still fit its stage (``room``) and the row starts inside the tile in
+    front.  All boundaries or none.
     Returns (coords', snapped)."""
     tiles = coords.shape[0] - 1
     n = row_offsets.shape[0] - 1
@@ -114,10 +126,67 @@ def snap_cta_boundaries(coords: np.ndarray, row_offsets: np.ndarray, grid: int):
         if x >= n:
             continue
         begin = int(row_offsets[x])
-        if y - begin > int(coords[t + 1, 0]) - x or begin < int(coords[t - 1, 1]):
+        rows_behind = int(coords[t + 1, 0]) - x
+        if begin > y or y - begin > rows_behind or begin < int(coords[t - 1, 1]):
+            return coords, False
+        if room is not None and not room.fits(int(coords[t + 1, 1]) - begin, rows_behind):
             return coords, False
         out[t, 1] = begin
     return out, True
+
+
+WHOLE_ROW_MAX = 32
+
+
+def whole_rows_plan(coords: np.ndarray, row_offsets: np.ndarray, num_edges: int, room: TileRoom, row_loop_built: bool = True,
+                    edge_lanes: bool = False, accumulators: int = 1, gathers: Sequence = ()):
+    """Restatement of the plan step for matrices of short rows (this package's own step, no reference counterpart): every
+    tile boundary moves back to the start of the row it cuts when no row has more than ``WHOLE_ROW_MAX`` edges, every tile
+    then still fits its ``room``, and at least two fifths of the steps that one lane per row would take have an edge to work
+    on.  ``gathers``: (index array, record bytes) of the gathers whose columns the plan sees.  Returns (coords', whole_rows,
+    row_loop) as the workspace holds them: whole_rows 1, 0 (too few lanes busy) or -1 (a row or a tile too large); row_loop 1
+    when the kernel's loop over whole rows is to run.  Where its other loop has lanes on consecutive edges (``edge_lanes``) that
+    one is kept when more than 10 of 32 rows begin in one of 32 banks on average, or when 32 consecutive edges gather from more
+    than 22 lines an accumulator fewer than 32 rows do."""
+    tiles, n = coords.shape[0] - 1, row_offsets.shape[0] - 1
+    ro = row_offsets.astype(np.int64)
+    x, y = coords[:, 0].astype(np.int64), coords[:, 1].astype(np.int64).copy()
+    y[0], y[tiles] = 0, num_edges
+    inner = np.arange(tiles + 1)
+    moves = (inner > 0) & (inner < tiles) & (x < n)
+    y[moves] = ro[x[moves]]
+    if (y[1:] < y[:-1]).any() or y.min() < 0 or y.max() > num_edges or not room.fits(np.diff(y), np.diff(x)).all():
+        return coords, -1, 0
+    slots, groups, degree = 0, 0, 0
+    seen = np.zeros(4, np.int64)                 # rows with an edge, lines of their middle edges, consecutive edges, their lines
+    step = tiles // 1024 + 1
+    for t in range(tiles):
+        begin, end = ro[x[t]:x[t + 1]].copy(), ro[x[t] + 1:x[t + 1] + 1]
+        if begin.size == 0:
+            continue
+        begin[0] = y[t]
+        length = end - begin
+        if (length < 0).any() or (length > WHOLE_ROW_MAX).any() or (begin < y[t]).any() or (end > y[t + 1]).any():
+            return coords, -1, 0
+        slots += 32 * sum(int(length[r:r + 32].max()) for r in range(0, length.size, 32))
+        if t % step == 0:
+            some = length[:32] > 0
+            first, of = begin[:32][some], length[:32][some]
+            if some.any():
+                groups += 1
+                degree += int(np.bincount(first % 32).max())
+            consecutive = np.arange(y[t], min(y[t] + 32, y[t + 1]))
+            for index, record_bytes in gathers:
+                for k, edges in ((0, first + of // 2), (2, consecutive)):
+                    seen[k] += edges.size
+                    seen[k + 1] += np.unique(index[edges].astype(np.int64) * record_bytes >> 7).size
+    if 2 * slots > 5 * num_edges:
+        return coords, 0, 0
+    out = coords.copy()
+    out[moves, 1] = y[moves]
+    rows, row_lines, edges, edge_lines = (int(v) for v in seen)
+    share_lines = 32 * (row_lines * edges - edge_lines * rows) * len(gathers) > 22 * accumulators * rows * edges
+    return out, 1, int(row_loop_built and not (edge_lanes and (degree > 10 * groups or share_lines)))
 
 
 def gather_window_plan(coords: np.ndarray, idx: np.ndarray, rec_bytes: int, win_bytes: int,

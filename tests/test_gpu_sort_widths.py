@@ -38,3 +38,17 @@ def test_permute_record_widths(words, n, offset):
     perm = torch.from_numpy(g.permutation(n).astype(np.int32)).cuda()
     got = permute_edges(src, perm)
     assert torch.equal(got, src[perm.long()])
+
+
+def test_counts_of_more_than_a_thousand_tiles_and_records_beyond_one_sweep():
+    """4.3 M ids are 1050 tiles of counts (the scan over a digit's counts takes a second round from 1024 on), and 8-byte
+    records beyond 2.4 M are the second sweep of the permutation's grid."""
+    n, rows = 4_300_003, 70_001
+    ids = np.random.default_rng(83).integers(0, rows, n)
+    perm, ro = sort_edges_by_row(torch.from_numpy(ids).cuda(), rows)
+    want = np.argsort(ids, kind="stable")
+    assert np.array_equal(perm.cpu().numpy(), want)
+    assert np.array_equal(ro.cpu().numpy(), np.searchsorted(ids[want], np.arange(rows + 1)))
+    for dtype in (np.float64, np.float32):
+        src = np.random.default_rng(89).random(n).astype(dtype)
+        assert np.array_equal(permute_edges(torch.from_numpy(src).cuda(), perm).cpu().numpy(), src[want])

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from flexspmv_b200 import graphs, problems
+from flexspmv_b200.codegen import emit_cuda
 from flexspmv_b200.binding import Desc, FlexSpmvError, GraphExtension, load_library
 from oracle import ir_eval
 from parity import assert_outputs_match
@@ -351,3 +352,90 @@ def test_the_launch_count_holds_the_plans_kernels(gname, dt, lengths, kw, planne
     prob = with_lengths(ir, lengths, 61, dtype)
     run_gpu(ext, ir, prob, dtype)
     assert ext.launches == planned + 1
+
+
+def planned_state(ext, ir, dt, bits, num_rows, num_edges):
+    """(coordinates, whole_rows, row_loop, snapped grid) of the last plan's workspace, and the room of its tiles."""
+    ws = next(reversed(ext._plans.values())).ws
+    header = ws[:256].cpu().numpy().view(np.int32)
+    tile_items = int(header[10])
+    tiles = -(-(num_rows + num_edges) // tile_items)
+    coords = ws[256:256 + (tiles + 1) * bits // 4].cpu().numpy().view(np.int32 if bits == 32 else np.int64).reshape(-1, 2)
+    info = ext.symbols(torch.from_numpy(np.zeros(1, dt)).dtype).graph_info
+    per_edge, _ = emit_cuda._stream_bytes_per_edge(ir, np.dtype(dt).itemsize)
+    tile = info.block_threads * info.items_per_thread
+    moves = not emit_cuda.stores_per_edge(ir)
+    room = ir_eval.TileRoom(tile, tile * max(bits // 8, per_edge) + (32 * per_edge if moves else 0), per_edge, bits // 8)
+    return coords, int(header[38]), int(header[39]), int(header[33]), tile_items, room
+
+
+PLANS = {
+    "all_5": [5] * 6001, "all_16": [16] * 2000, "all_32": [32] * 700, "long_row_late": [8] * 4000 + [33] + [8] * 10,
+    "uneven": [1] * 310 + [32] * 10 + [1] * 3000, "mostly_empty": ([0] * 31 + [32]) * 100, "empty_ends": [0] * 700 + [6] * 900 + [0] * 700,
+    "cut_long_rows": [300, 1, 1, 1] * 60, "many_short_behind_a_long": [1] * 340 + [601] + [1] * 9000, "one_row": [7],
+    "any": np.random.default_rng(67).integers(0, 33, 5000).tolist(), "any_short": np.random.default_rng(71).integers(0, 4, 60000).tolist(),
+}
+
+
+@pytest.mark.parametrize("gname,dt", [("spmv", "float64"), ("spmv", "float32"), ("spring_mass", "float32"), ("swe_delta", "float64"),
+                                      ("ops_zoo", "float64"), ("mixed_dims", "float32")])
+@pytest.mark.parametrize("case", sorted(PLANS))
+def test_plan_coordinates_equal_their_restatement(gname, dt, case):
+    """Every coordinate, and what the header says about them, against the steps restated with numpy: partition, boundaries
+    of whole rows, or boundaries between the CTAs of the plan's grid."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, PLANS[case], 73, dtype)
+    needs_row = any(s.get("row_identity") for s in ir.selector_register)
+    light = emit_cuda.light_map(ir)
+    gathers = [(prob.indices[s["selector_name"]], dtype.itemsize * graphs.dim_of(s["shape"])) for s in ir.selector_register
+               if s.get("selector") == 1 and not s.get("row_identity")] if light and not needs_row else []
+    acc = sum(graphs.dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer")
+    for bits, kw in ((32, {"max_ctas": 5}), (64, {"max_ctas": 40}), (32, {"max_ctas": 3, "tile_items": 100}), (64, {"max_ctas": 1})):
+        ext = GraphExtension(ir, random_gather=False, gather_windows=False, **kw)
+        run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+        got, whole, loop, snapped, tile_items, room = planned_state(ext, ir, dt, bits, prob.num_rows, prob.nnz)
+        ro = prob.row_offsets.astype(np.int32 if bits == 32 else np.int64)
+        want = ir_eval.tile_coordinates(ro, tile_items)
+        want_whole = want_loop = 0
+        if not emit_cuda.stores_per_edge(ir) and prob.nnz <= 32 * prob.num_rows:
+            want, want_whole, want_loop = ir_eval.whole_rows_plan(want, ro, prob.nnz, room, row_loop_built=needs_row or light,
+                                                                  edge_lanes=not needs_row, accumulators=acc, gathers=gathers)
+        tiles = want.shape[0] - 1
+        grid = min(kw["max_ctas"], tiles)
+        ok = want_whole == 1 and grid >= 2
+        if want_whole != 1:
+            want, ok = ir_eval.snap_cta_boundaries(want, ro, grid, room)
+        assert (whole, loop, snapped) == (want_whole, want_loop, grid if ok else 0), (bits, kw)
+        assert np.array_equal(got, want), (bits, kw)
+
+
+def test_boundaries_aligned_for_one_grid_and_cut_for_another_hand_carries_over():
+    """Rows of few edges that stay on the loop with carries (one lane in ten would have an edge to work on): the plan puts the
+    boundaries between the CTAs of its grid on row ends; other grids find boundaries that cut rows and hand carries over."""
+    lib = load_library()
+    ir = graphs.spmv_graph()
+    lengths = ([32] + [1] * 40) * 400
+    prob = with_lengths(ir, lengths, 79, np.float64)
+    ref, _, sums = ir_eval.run_graph(ir, prob, np.float64, num_threads=4, want_abs_sums=True)
+    ext = GraphExtension(ir, random_gather=False, max_ctas=7)
+    run_gpu(ext, ir, prob, np.float64)
+    coords, whole, _, snapped, tile_items, room = planned_state(ext, ir, "float64", 32, prob.num_rows, prob.nnz)
+    assert not ext.planned_whole_rows() and whole == 0 and snapped == 7
+    tiles, ro = coords.shape[0] - 1, prob.row_offsets
+    cut = {t for t in range(1, tiles) if coords[t, 0] < prob.num_rows and coords[t, 1] != ro[coords[t, 0]]}
+    plan = next(reversed(ext._plans.values()))
+    v, x = (torch.from_numpy(prob.values[k]).cuda() for k in ("vals", "x"))
+    cols, ro_t = torch.from_numpy(prob.indices["selector"]).cuda(), plan.keep[0]
+    y = torch.empty(prob.num_rows, dtype=torch.float64, device="cuda")
+    vp, ip, op = (ctypes.c_void_p * 2)(v.data_ptr(), x.data_ptr()), (ctypes.c_void_p * 1)(cols.data_ptr()), (ctypes.c_void_p * 1)(y.data_ptr())
+    lib.flexspmv_spmv_f64_launch.restype = ctypes.c_int
+    for grid in (7, 1, 5, 11, 29, tiles):
+        starts = {c * (tiles // grid) + min(c, tiles % grid) for c in range(1, grid)}
+        assert bool(starts & cut) == (grid not in (1, 7))               # carries between the CTAs of the other grids
+        desc = Desc(prob.num_rows, prob.nnz, prob.num_cols, 32, 0, grid, 0)
+        y.fill_(float("nan"))
+        assert lib.flexspmv_spmv_f64_launch(ctypes.byref(desc), vp, ip, ctypes.c_void_p(ro_t.data_ptr()), op, ctypes.c_void_p(plan.ws.data_ptr()),
+                                            ctypes.c_size_t(plan.nbytes), None) == 0
+        torch.cuda.synchronize()
+        assert_outputs_match(ir, [y.cpu().numpy()], ref, sums, np.dtype(np.float64), what=f"grid {grid}")
+    ext.check()

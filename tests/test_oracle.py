@@ -182,3 +182,51 @@ def test_snapped_cta_boundaries_keep_every_tile_within_its_capacity():
     c2 = ir_eval.tile_coordinates(long_rows, tile)
     same, ok = ir_eval.snap_cta_boundaries(c2, long_rows, 4)
     assert not ok and same is c2
+
+
+def test_whole_rows_plan_restatement():
+    """Coordinates by hand: tiles of 10 items over rows of 3 edges cut every third row or so; moved back, every tile begins
+    at a row's first edge.  Rows of 33, tiles without room, few busy lanes and single banks are told apart."""
+    from oracle import ir_eval
+    room = ir_eval.TileRoom(10, 10 ** 6, 12, 4)
+    ro = np.arange(0, 34, 3, dtype=np.int32)                            # 11 rows of 3 edges
+    coords = ir_eval.tile_coordinates(ro, 10)
+    assert coords.tolist() == [[0, 0], [2, 8], [5, 15], [7, 23], [10, 30], [11, 33]]
+    wide = ir_eval.TileRoom(16, 10 ** 6, 12, 4)
+    got, whole, loop = ir_eval.whole_rows_plan(coords, ro, 33, wide)
+    assert (whole, loop) == (0, 0)                                       # 2 - 3 rows a tile: a lane in twelve
+    ro = np.concatenate([[0], np.cumsum([3] * 400)]).astype(np.int32)
+    coords = ir_eval.tile_coordinates(ro, 160)
+    got, whole, loop = ir_eval.whole_rows_plan(coords, ro, 1200, ir_eval.TileRoom(160, 10 ** 6, 12, 4))
+    assert (whole, loop) == (1, 1) and all(y == ro[x] for x, y in got.tolist()) and np.array_equal(got[:, 0], coords[:, 0])
+    assert ir_eval.whole_rows_plan(coords, ro, 1200, ir_eval.TileRoom(119, 10 ** 6, 12, 4))[1] == -1        # 40 rows of 3 a tile
+    assert ir_eval.whole_rows_plan(coords, ro, 1200, ir_eval.TileRoom(160, 120 * 12, 12, 4))[1] == -1
+    late = ro.copy()
+    late[200:] += 30                                                     # a row of 33
+    assert ir_eval.whole_rows_plan(ir_eval.tile_coordinates(late, 160), late, 1230, ir_eval.TileRoom(160, 10 ** 6, 12, 4))[1] == -1
+    # the leading offset counts as 0; a larger one would leave a first tile that holds everything in front of it
+    shifted = ro + 200
+    assert ir_eval.whole_rows_plan(coords, shifted, 1400, ir_eval.TileRoom(160, 10 ** 6, 12, 4))[1] == -1
+    rows16 = np.arange(0, 16 * 401, 16, dtype=np.int32)
+    plan16 = lambda **kw: ir_eval.whole_rows_plan(ir_eval.tile_coordinates(rows16, 1280), rows16, 6400, ir_eval.TileRoom(1280, 10 ** 6, 12, 4), **kw)[1:]
+    assert plan16() == (1, 1) and plan16(edge_lanes=True) == (1, 0) and plan16(row_loop_built=False) == (1, 0)
+    # runs of columns at arbitrary places: 32 rows touch 32 lines, 32 edges touch a few; worth two accumulators' products and not more
+    rows9 = np.arange(0, 9 * 401, 9, dtype=np.int32)
+    starts = np.random.default_rng(1).integers(0, 10 ** 6, 400)
+    runs = (starts[:, None] + np.arange(9)).ravel()
+    plan9 = lambda index, acc=1: ir_eval.whole_rows_plan(ir_eval.tile_coordinates(rows9, 1280), rows9, 3600, ir_eval.TileRoom(1280, 10 ** 6, 12, 4),
+                                                         edge_lanes=True, accumulators=acc, gathers=[(index, 8)])[2]
+    assert plan9(runs) == 0 and plan9(runs, acc=2) == 1 and plan9(np.arange(3600) // 9) == 1
+
+
+def test_boundaries_between_ctas_need_room_in_the_stage():
+    """A row of 601 edges cut by a boundary, rows of one edge behind it: by the count of row ends it could move, by the bytes not."""
+    from oracle import ir_eval
+    lengths = np.ones(40 * 1280, dtype=np.int64)
+    lengths[340] = 601
+    ro = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    coords = ir_eval.tile_coordinates(ro, 1280)
+    grid = coords.shape[0] - 1
+    assert ir_eval.snap_cta_boundaries(coords, ro, grid)[1]
+    assert not ir_eval.snap_cta_boundaries(coords, ro, grid, ir_eval.TileRoom(1280, 1280 * 12 + 32 * 12, 12, 4))[1]
+    assert ir_eval.snap_cta_boundaries(coords, ro, grid, ir_eval.TileRoom(1280, 1280 * 24, 12, 4))[1]
