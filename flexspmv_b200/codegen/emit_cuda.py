@@ -143,7 +143,7 @@ def choose_config(ir: GraphIR, dtype: str) -> Tuple[int, int, int, int]:
 # heuristic of choose_config.  In the fused row mode one more resident CTA beats a wider register batch: the
 # other warps hide the gather latency better than more loads in flight per thread do.
 TUNED_CONFIGS = {
-    # 7-point fp64 SpMV: 70 % of the HBM peak in the loop with carries, 85 % in the loop over whole rows (512^3, us: 2602; 3 / 5
+    # 7-point fp64 SpMV: 70 % of the HBM peak in the loop with carries, 86 % in the loop over whole rows (512^3, us: 2602; 3 / 5
     # CTAs per SM 2818 / 3006, 384 threads x 3 2560, 512 x 2 2533, 192 x 5 2750, 2048-item tiles x 3 3264)
     "spmv_f64": (256, 5, 2, 4),
     "spmv_f32": (256, 5, 2, 4),

@@ -514,10 +514,11 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // gathers are back.  Groups of rows go round the warps across tiles (`turn`), so a tile need not hold a multiple of
       // the CTA's rows.  Sums run left to right over the row, as in the two-phase loop.
       // What the two-phase loop is bound by on short rows is the shared-memory / L1 data pipe (75 - 80 % busy at 55 % of
-      // DRAM) and two CTA barriers a tile; this one moves no product through shared memory, a third of the gather lines,
-      // and is bound by the latency of the gathers at the registers of 4 CTAs per SM.  7-point fp64 SpMV 512^3: 3205 ->
-      // 2602 us (5.56 TB/s); 145^3 fp32: 54.1 -> 43.0 us; 2-D 512^2 fp64: 9.05 -> 7.3 us; 27 columns a row fp64, 300 007
-      // rows: 26.2 -> 24.2 us; spring-mass 1024^2: 44.5 -> 38.9 us; Rusanov 1024^2: 92 -> 82 us.
+      // DRAM) and two CTA barriers a tile; this one moves no product through shared memory and a third of the gather lines
+      // (41 % of the pipe at 70 % of DRAM), and is bound by the latency of the gathers at the registers of 4 CTAs per SM: 10 of
+      // 16 stall cycles per issue are long_scoreboard.  us a launch, two-phase / this loop: 7-point fp64 SpMV 512^3 3205 / 2564
+      // (5.65 TB/s); 145^3 fp32 54.1 / 42.6; 5-point 512^2 fp64 9.1 / 7.1; 27 columns a row fp64, 300 007 rows 26.2 / 23.9;
+      // spring-mass 1024^2 fp32 44.5 / 38.4; Rusanov 1024^2 fp64 92 / 83.5.
       constexpr int RB = Cfg::kRowBatch;
       int s = 0, turn = 0;
       uint32_t parity = 0;
