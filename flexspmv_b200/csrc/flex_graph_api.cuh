@@ -205,7 +205,8 @@ struct GraphApi {
         rule.built = WholeRows<G, Cfg, false>::value;
         rule.edge_lanes = !G::kGatherNeedsRow;
         rule.accumulators = G::kAccDim;
-        if (rule.built && rule.edge_lanes && indices) rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
+        if (rule.built && rule.edge_lanes && indices && d->num_edges > 0)
+          rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
         for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
         // rows longer than kWholeRowMax on average: no need to look
         if (whole_rows && !use_win(d) && d->num_rows > 0 && d->num_edges <= (long long)kWholeRowMax * d->num_rows)

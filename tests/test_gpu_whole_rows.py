@@ -439,3 +439,13 @@ def test_boundaries_aligned_for_one_grid_and_cut_for_another_hand_carries_over()
         torch.cuda.synchronize()
         assert_outputs_match(ir, [y.cpu().numpy()], ref, sums, np.dtype(np.float64), what=f"grid {grid}")
     ext.check()
+
+
+@pytest.mark.parametrize("offset_dtype", [torch.int32, torch.int64])
+def test_a_matrix_without_edges_can_be_planned(offset_dtype):
+    """Empty index tensors have no address: binding and planning such a block (a rank's empty share) is no error."""
+    ext = GraphExtension(graphs.spmv_graph(), random_gather=False)
+    vals, x = torch.empty(0, dtype=torch.float64, device="cuda"), torch.ones(50, dtype=torch.float64, device="cuda")
+    cols, ro = torch.empty(0, dtype=torch.int32, device="cuda"), torch.zeros(51, dtype=offset_dtype, device="cuda")
+    ext.prepare([vals, x], [cols], ro, [torch.empty(50, dtype=torch.float64, device="cuda")], 50, 0, 50)
+    ext.check()
