@@ -90,7 +90,7 @@ def direct_loads(ir: GraphIR, dtype: str) -> bool:
 
 
 def light_map(ir: GraphIR) -> bool:
-    """Nothing in the map that takes tens of instructions an edge (WholeRows in csrc/flex_tile_kernel.cuh)."""
+    """Nothing in the map that takes tens of instructions an edge (RowLoopRule in csrc/flex_common.cuh)."""
     return not any(op_["op"] in ("truediv", "pow", "exp", "norm") for op_ in ir.map_operations)
 
 
@@ -108,7 +108,8 @@ def smem_bytes(ir: GraphIR, dtype: str, block: int, ipt: int, stages: int) -> in
     acc = max(1, sum(dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer"))
     tile = block * ipt
     needs_row = any(s_.get("selector") == 1 and s_.get("row_identity") for s_ in ir.selector_register)
-    # tiles whose boundaries the plan may move hold up to 32 edges more; the loop over whole rows has up to four stages
+    # tiles whose boundaries the plan may move hold up to 32 edges more; the loop over whole rows has up to four stages where
+    # it is the usual one
     moves = not (stores_per_edge(ir) or direct_loads(ir, dtype))
     row_loop = moves and (needs_row or light_map(ir))
     ctl = 4 if row_loop else stages
@@ -674,6 +675,10 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     edge_words = sum(dim_of(s_["shape"]) * words for s_ in ir.selector_register if s_.get("selector") != 1)
     batch = batch_override or (1 if gather_words else next((b_ for b_ in (8, 4, 3, 2) if b_ * max(edge_words, 1) <= 28), 2))
     row_batch = batch if needs_row else next((b_ for b_ in (4, 2) if b_ * (gather_words + 1) <= 14), 1)
+    # a division's call in the loop over whole rows: 56 bytes spilled in fp64 without that loop, 116 / 64 / 64 - 72 with batches of
+    # 4 / 2 / 1, which the two-phase loop of the same kernel pays for (two divisions, rows of 20: 36.6, 37.4 / 36.4 / 38.5 us)
+    if not needs_row and not light_map(ir):
+        row_batch = min(row_batch, 2)
     if len(cfg) > 6:
         row_batch = cfg[6]       # seventh field
     w(f"using Cfg = flex::TileCfg<{block}, {ipt}, {stages}, {min_ctas}, {batch}, {'true' if pipeline else 'false'}, {row_batch}>;")

@@ -67,8 +67,8 @@ constexpr int kWholeRowMax = FLEX_WHOLE_ROW_MAX;   // longest row of a matrix wh
 // What the plan has to know to choose the loop that runs on tiles of whole rows.
 struct RowLoopRule {
   static constexpr int kMaxGathers = 4;
-  bool built;                        // the kernel has the loop over whole rows
-  bool edge_lanes;                   // its other loop has lanes on consecutive edges (else a thread per row, as this one)
+  bool edge_lanes;                   // the other loop has lanes on consecutive edges (else a thread per row, as this one)
+  bool heavy;                        // the map takes tens of instructions an edge: it divides or calls pow or exp
   int accumulators;                  // width of a row's sum
   int gathers;                       // gathers whose columns the plan sees (0: none)
   const int* index[kMaxGathers];

@@ -229,6 +229,13 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
 // lines a gather) 55 / 57 and 41 / 44, 5 (32, 8) 46 / 43 and 36 / 35, 8 (32, 5) 67 / 52 and 49 / 37, 20 (32, 2) 54 / 41 and 36 / 32;
 // stencils (2 - 3 against 8 - 16 lines), banded and random columns: this loop, by 4 - 50 %.  A plan that has not been shown the
 // columns goes by the rows alone.
+// And a map that divides or calls pow or exp is worth more than the gathers it waits for: lanes on consecutive edges do
+// nothing in vain, a lane with a row of its own idles while another one's row goes on.  It takes this loop on rows of up to
+// seven edges, nine lane-steps in ten with an edge.  us, this loop / the other, 12 M values, 1 / 3 / 5 / 7 edges a row fp64:
+// 4 divisions an edge 53 / 80, 37 / 50, 37 / 44, 37 / 43;  1 pow 67 / 101, 62 / 75, 63 / 70, 63 / 69;  ops_zoo 205 / 260, 190 / 220,
+// 189 / 209, 204 / 208.  8 / 20 / 31 edges a row and 0 - 8:  4 divisions 40 / 45, 41 / 43, 55 / 43, 66 / 48;  1 pow 70 / 70,
+// 72 / 68, 99 / 69, 120 / 73;  ops_zoo 214 / 217, 339 / 209, 337 / 209, 386 / 225.  A thirtieth of the values, 7 and 31 edges
+// a row: 1 pow 8.2 / 8.2, 20.3 / 8.7;  4 pow 18.0 / 16.3 (7).
 // Where it does not move them all, its first CTA looks after the boundaries between the CTAs of the plan's grid.
 template <typename OffsetT>
 __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* row_offsets, long long num_rows, long long num_edges,
@@ -250,7 +257,8 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* ro
     const bool same_bank = h->bank_degree > 10 * h->bank_groups;
     const long long lines_more = 32ll * h->line_row_lines * h->line_edges - 32ll * h->line_edge_lines * h->line_rows;   // x rows x edges
     const bool edges_share_lines = lines_more * rule.gathers > 22ll * rule.accumulators * h->line_rows * h->line_edges;
-    h->row_loop = rule.built && !(rule.edge_lanes && (same_bank || edges_share_lines));
+    const bool lanes_idle = num_edges > 7 * num_rows || 9 * (long long)h->row_slots > 10 * num_edges;
+    h->row_loop = !(rule.edge_lanes && (same_bank || edges_share_lines || (rule.heavy && lanes_idle)));
   }
 }
 

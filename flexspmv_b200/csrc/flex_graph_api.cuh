@@ -200,12 +200,12 @@ struct GraphApi {
         const long long most = max_ctas(d, resident);
         grid = (int)(most < h.num_tiles ? most : h.num_tiles);
       }
-      if constexpr (WholeTiles<G, Cfg, false>::value) {
+      if constexpr (WholeRows<G, Cfg, false>::value) {
         RowLoopRule rule{};
-        rule.built = WholeRows<G, Cfg, false>::value;
         rule.edge_lanes = !G::kGatherNeedsRow;
+        rule.heavy = !G::kLightMap;
         rule.accumulators = G::kAccDim;
-        if (rule.built && rule.edge_lanes && indices && d->num_edges > 0)
+        if (rule.edge_lanes && indices && d->num_edges > 0)
           rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
         for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
         // rows longer than kWholeRowMax on average: no need to look

@@ -10,8 +10,8 @@
 //   thread per row loads the row's own record once, gathers and maps its edges in register batches and
 //   stores the row; in tiles with a long row whole warps take the rows one at a time (lanes 32 edges
 //   apart, shuffle tree).  Nothing of a row-mode graph passes through a shared-memory product buffer.
-//   Whole rows (row-mode graphs and graphs of light maps, when the plan found a matrix of short rows whose tiles can all
-//   hold whole rows): no carries at all, so no barriers either -- every warp takes 32 rows of a staged tile, one per lane,
+//   Whole rows (either kind of graph, when the plan found a matrix of short rows whose tiles can all hold whole rows, and
+//   that one lane per row suits): no carries at all, so no barriers either -- every warp takes 32 rows of a staged tile, one per lane,
 //   and keeps everything in registers.  The other two loops run on such tiles too, without carries between CTAs.
 // The carry of a row that spans tiles travels inside the CTA in shared memory; the only cross-CTA state
 // is one carry per CTA, folded in by the last CTA to finish (ticket counter), in CTA order.  No atomics
@@ -43,20 +43,12 @@ struct TileCfg {
   static constexpr int kRowBatch = ROW_BATCH_;   // the same in the loop over whole rows
 };
 
-// Whether the plan may move all tile boundaries of the graph to row starts: staged graphs that write nothing per edge.
-template <class G, class Cfg, bool WIN>
-struct WholeTiles {
-  static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
-};
-// Whether the kernel has the loop over whole rows, one row per lane: graphs with per-row data, whose other loop has a thread
-// per row as well, and graphs whose map is a few adds and multiplies.  A map that divides or calls pow or exp is worth more
-// than the gathers it waits for, and there lanes on consecutive edges do nothing in vain: in the loop over rows a lane idles
-// while another one's row goes on.  us, this loop / the two-phase loop, 6 M edges fp64, 3 / 8 / 20 / 31 edges a row and 0 - 8:
-//   4 divisions an edge  39 / 50,  40 / 45,  41 / 43,  55 / 43,  66 / 48;   1 pow  65 / 74,  70 / 70,  72 / 68,  99 / 69,  120 / 73;
-//   0.2 M edges, 31 a row:  1 / 2 divisions  8.7 / 7.1,  10.4 / 6.9,  1 pow  20 / 8.7.
+// Whether the plan may move all tile boundaries of the graph to row starts, and the kernel has the loop over whole rows, one
+// row per lane: staged graphs that write nothing per edge (a thread that walks a row would store its edges' outputs a row
+// length apart).
 template <class G, class Cfg, bool WIN>
 struct WholeRows {
-  static constexpr bool value = WholeTiles<G, Cfg, WIN>::value && (G::kGatherNeedsRow || G::kLightMap);
+  static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
 };
 
 constexpr int kMaxCtas = 2048;            // capacity of the per-CTA carry arrays in the workspace
@@ -102,7 +94,7 @@ struct TileSmemLayout {
   static constexpr int kPerItem = (int(sizeof(OffsetT)) > kBytesPerEdge) ? int(sizeof(OffsetT)) : kBytesPerEdge;
   // a tile's records: kTile merge items, and the edges in front of its first row end when the plan moves the tile's
   // front boundary back to the start of that row (the gather-window variant may meet such a plan too)
-  static constexpr bool kTilesMove = WholeTiles<G, Cfg, false>::value;
+  static constexpr bool kTilesMove = WholeRows<G, Cfg, false>::value;
   static constexpr int kRecordBytes = Cfg::kTile * kPerItem + (kTilesMove ? kWholeRowMax * kBytesPerEdge : 0);
   // each staged window may grow by < 32 bytes from aligning both ends to 16
   static constexpr int kStreamBytes =
@@ -143,9 +135,10 @@ struct TileSmemLayout {
   // and as many fit as the other loop's total allows, one more where that costs at most 2 KB.
   static constexpr bool kWhole = WholeRows<G, Cfg, WIN>::value;
   static constexpr int off_row_stages(int stages) { return int(align_up(off_long(stages), 128)); }
+  static constexpr bool kMore = G::kGatherNeedsRow || G::kLightMap;      // (maps that divide run this loop on the shortest rows only)
   static constexpr int row_stages() {
     int n = kWhole ? Cfg::kStages : 0;
-    while (kWhole && n < 4 && off_row_stages(n + 1) + kStageBytes * (n + 1) <= two_phase(n + 1) + 2048) ++n;
+    while (kWhole && kMore && n < 4 && off_row_stages(n + 1) + kStageBytes * (n + 1) <= two_phase(n + 1) + 2048) ++n;
     return n;
   }
   static constexpr int kRowStages = row_stages();

@@ -138,8 +138,8 @@ def snap_cta_boundaries(coords: np.ndarray, row_offsets: np.ndarray, grid: int, 
 WHOLE_ROW_MAX = 32
 
 
-def whole_rows_plan(coords: np.ndarray, row_offsets: np.ndarray, num_edges: int, room: TileRoom, row_loop_built: bool = True,
-                    edge_lanes: bool = False, accumulators: int = 1, gathers: Sequence = ()):
+def whole_rows_plan(coords: np.ndarray, row_offsets: np.ndarray, num_edges: int, room: TileRoom, edge_lanes: bool = False,
+                    heavy: bool = False, accumulators: int = 1, gathers: Sequence = ()):
     """Restatement of the plan step for matrices of short rows (this package's own step, no reference counterpart): every
     tile boundary moves back to the start of the row it cuts when no row has more than ``WHOLE_ROW_MAX`` edges, every tile
     then still fits its ``room``, and at least two fifths of the steps that one lane per row would take have an edge to work
@@ -147,7 +147,8 @@ def whole_rows_plan(coords: np.ndarray, row_offsets: np.ndarray, num_edges: int,
     row_loop) as the workspace holds them: whole_rows 1, 0 (too few lanes busy) or -1 (a row or a tile too large); row_loop 1
     when the kernel's loop over whole rows is to run.  Where its other loop has lanes on consecutive edges (``edge_lanes``) that
     one is kept when more than 10 of 32 rows begin in one of 32 banks on average, or when 32 consecutive edges gather from more
-    than 22 lines an accumulator fewer than 32 rows do."""
+    than 22 lines an accumulator fewer than 32 rows do, or when the map is ``heavy`` (it divides or calls pow or exp) and rows
+    have more than five edges on average or more than one lane-step in ten has none."""
     tiles, n = coords.shape[0] - 1, row_offsets.shape[0] - 1
     ro = row_offsets.astype(np.int64)
     x, y = coords[:, 0].astype(np.int64), coords[:, 1].astype(np.int64).copy()
@@ -186,7 +187,8 @@ def whole_rows_plan(coords: np.ndarray, row_offsets: np.ndarray, num_edges: int,
     out[moves, 1] = y[moves]
     rows, row_lines, edges, edge_lines = (int(v) for v in seen)
     share_lines = 32 * (row_lines * edges - edge_lines * rows) * len(gathers) > 22 * accumulators * rows * edges
-    return out, 1, int(row_loop_built and not (edge_lanes and (degree > 10 * groups or share_lines)))
+    idle = num_edges > 7 * n or 9 * slots > 10 * num_edges
+    return out, 1, int(not (edge_lanes and (degree > 10 * groups or share_lines or (heavy and idle))))
 
 
 def gather_window_plan(coords: np.ndarray, idx: np.ndarray, rec_bytes: int, win_bytes: int,

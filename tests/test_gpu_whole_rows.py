@@ -68,13 +68,16 @@ def row_loop_planned(ext):
     return int(next(reversed(ext._plans.values())).ws[:256].cpu().numpy().view(np.int32)[39])
 
 
-@pytest.mark.parametrize("gname,dt,expected", [("spmv", "float64", 1), ("rusanov", "float64", 1), ("swe_boundary", "float32", 1),
-                                               ("ops_zoo", "float64", 0), ("ops_zoo", "float32", 0)])
-def test_maps_that_divide_keep_the_two_phase_loop(gname, dt, expected):
+@pytest.mark.parametrize("gname,dt,lengths,expected", [
+    ("spmv", "float64", [3, 8, 5] * 2000 + [32] * 50, 1), ("rusanov", "float64", [3, 8, 5] * 2000 + [32] * 50, 1),
+    ("swe_boundary", "float32", [3, 8, 5] * 2000 + [32] * 50, 1), ("ops_zoo", "float64", [3, 8, 5] * 2000 + [32] * 50, 0),
+    ("ops_zoo", "float32", [3, 8, 5] * 2000 + [32] * 50, 0), ("ops_zoo", "float64", [4, 6] * 4000, 0), ("ops_zoo", "float32", [0, 8] * 4000, 0),
+    ("ops_zoo", "float64", [7] * 9000, 1), ("ops_zoo", "float32", [3] * 9000, 1)])
+def test_maps_that_divide_keep_the_two_phase_loop(gname, dt, lengths, expected):
     """A two-phase graph whose map takes tens of instructions an edge: its tiles hold whole rows, so no grid hands carries
-    over, but lanes stay on consecutive edges.  Rows longer than a tile's share of threads, every grid."""
+    over, but lanes stay on consecutive edges unless every lane has a row of about the same few edges."""
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
-    prob = with_lengths(ir, [3, 8, 5] * 2000 + [32] * 50, 29, dtype)
+    prob = with_lengths(ir, lengths, 29, dtype)
     ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
     results = []
     for max_ctas in (0, 1, 7, 50):
@@ -388,7 +391,7 @@ def test_plan_coordinates_equal_their_restatement(gname, dt, case):
     needs_row = any(s.get("row_identity") for s in ir.selector_register)
     light = emit_cuda.light_map(ir)
     gathers = [(prob.indices[s["selector_name"]], dtype.itemsize * graphs.dim_of(s["shape"])) for s in ir.selector_register
-               if s.get("selector") == 1 and not s.get("row_identity")] if light and not needs_row else []
+               if s.get("selector") == 1 and not s.get("row_identity")] if not needs_row else []
     acc = sum(graphs.dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer")
     for bits, kw in ((32, {"max_ctas": 5}), (64, {"max_ctas": 40}), (32, {"max_ctas": 3, "tile_items": 100}), (64, {"max_ctas": 1})):
         ext = GraphExtension(ir, random_gather=False, gather_windows=False, **kw)
@@ -398,8 +401,8 @@ def test_plan_coordinates_equal_their_restatement(gname, dt, case):
         want = ir_eval.tile_coordinates(ro, tile_items)
         want_whole = want_loop = 0
         if not emit_cuda.stores_per_edge(ir) and prob.nnz <= 32 * prob.num_rows:
-            want, want_whole, want_loop = ir_eval.whole_rows_plan(want, ro, prob.nnz, room, row_loop_built=needs_row or light,
-                                                                  edge_lanes=not needs_row, accumulators=acc, gathers=gathers)
+            want, want_whole, want_loop = ir_eval.whole_rows_plan(want, ro, prob.nnz, room, edge_lanes=not needs_row, heavy=not light,
+                                                                  accumulators=acc, gathers=gathers)
         tiles = want.shape[0] - 1
         grid = min(kw["max_ctas"], tiles)
         ok = want_whole == 1 and grid >= 2

@@ -147,10 +147,10 @@ def test_shared_memory_holds_nothing_a_graphs_loops_do_not_use():
 @pytest.mark.parametrize("make,dtype,batches", [(graphs.spring_mass_graph, "float64", (1, 1)), (graphs.rusanov_graph, "float32", (1, 1)),
                                                 (graphs.swe_delta_graph, "float32", (1, 1)), (graphs.spring_mass_graph, "float32", (2, 1)),
                                                 (graphs.swe_boundary_graph, "float32", (8, 8)), (graphs.swe_boundary_graph, "float64", (4, 1)),
-                                                (graphs.spmv_graph, "float64", (1, 4))])
+                                                (graphs.spmv_graph, "float64", (1, 4)), (graphs.ops_zoo_graph, "float64", (1, 2))])
 def test_edges_in_flight_per_row(make, dtype, batches):
     """(loop with carries, loop over whole rows): a row-mode graph with gathers takes one edge at a time unless it was
-    tuned; more were spilled to local memory."""
+    tuned, and a map that divides at most two; more were spilled to local memory."""
     import re
     fields = re.search(r"using Cfg = flex::TileCfg<([^>]*)>", emit_cuda.emit_graph(make(), dtype)).group(1).split(", ")
     assert (int(fields[4]), int(fields[6])) == batches

@@ -209,7 +209,11 @@ def test_whole_rows_plan_restatement():
     assert ir_eval.whole_rows_plan(coords, shifted, 1400, ir_eval.TileRoom(160, 10 ** 6, 12, 4))[1] == -1
     rows16 = np.arange(0, 16 * 401, 16, dtype=np.int32)
     plan16 = lambda **kw: ir_eval.whole_rows_plan(ir_eval.tile_coordinates(rows16, 1280), rows16, 6400, ir_eval.TileRoom(1280, 10 ** 6, 12, 4), **kw)[1:]
-    assert plan16() == (1, 1) and plan16(edge_lanes=True) == (1, 0) and plan16(row_loop_built=False) == (1, 0)
+    assert plan16() == (1, 1) and plan16(edge_lanes=True) == (1, 0) and plan16(heavy=True) == (1, 1)
+    for length, want in ((7, 1), (9, 0)):
+        ro = np.arange(0, length * 513, length, dtype=np.int32)
+        assert ir_eval.whole_rows_plan(ir_eval.tile_coordinates(ro, 1280), ro, int(ro[-1]), ir_eval.TileRoom(1280, 10 ** 6, 12, 4), edge_lanes=True,
+                                       heavy=True)[1:] == (1, want)
     # runs of columns at arbitrary places: 32 rows touch 32 lines, 32 edges touch a few; worth two accumulators' products and not more
     rows9 = np.arange(0, 9 * 401, 9, dtype=np.int32)
     starts = np.random.default_rng(1).integers(0, 10 ** 6, 400)
