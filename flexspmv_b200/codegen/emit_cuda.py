@@ -441,6 +441,8 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         w(f"    r.idx_{n_} = *t.template stream<{stream_of['idx:' + n_]}, int>(le);")
     w("    (void)t; (void)le; (void)r;")
     w("  }")
+    sources = {s_["target"]: dim_of(s_["shape"]) for s_ in gsel}
+    w(f"  static constexpr int kGatherRecordBytes = {sum(sources.values())} * int(sizeof(V));      // of one vertex, in all gathered vectors")
     w(f"  static constexpr bool kValuesStaged = {'true' if staged_values else 'false'};")
     w(f"  static constexpr bool kStoresPerEdge = {'true' if stores_per_edge(ir) else 'false'};")
     w("  template <class Tile, class IdxT>")

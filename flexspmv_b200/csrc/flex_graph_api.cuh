@@ -222,6 +222,12 @@ struct GraphApi {
     }
   }
 
+  // Where the gathered vectors are larger than this, tiles of whole rows go round the CTAs (round_tile in flex_tile_kernel.cuh).
+  // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its
+  // neighbours in L1: 7-point fp32 145^3 (12 MB) 42.6 us in runs of its own, 45.0 in rounds; 27 columns a row fp64, 3 M rows
+  // (24 MB) 188 / 194; 5-point fp64 3000^2 (72 MB) 128 / 118.
+  static constexpr long long kKeepBytes = 48ll << 20;
+
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
   // once for each device of the process.
   template <typename OffsetT, class C = Cfg, bool WIN = false>
@@ -268,6 +274,11 @@ struct GraphApi {
     a.carry_row = reinterpret_cast<long long*>(static_cast<char*>(ws) + h.carry_row_offset);
     a.carry_val = static_cast<char*>(ws) + h.carry_val_offset;
     a.num_rows = d->num_rows; a.num_edges = d->num_edges; a.num_tiles = tiles;
+    a.rounds = 0;
+    if constexpr (L::kWhole) {
+      const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
+      if (vertices * G::kGatherRecordBytes > kKeepBytes) a.rounds = (int)(tiles / (grid * kTileRun));
+    }
     a.win_table = nullptr; a.win_index = nullptr; a.num_vertices = d->num_vertices;
     if constexpr (WIN) {
       if (d->num_vertices <= 0) return FLEXSPMV_ERR_BAD_ARG;

@@ -51,6 +51,7 @@ struct WholeRows {
   static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
 };
 
+constexpr int kTileRun = 4;               // consecutive tiles of a CTA where whole rows go round the CTAs (TileKernelArgs::rounds)
 constexpr int kMaxCtas = 2048;            // capacity of the per-CTA carry arrays in the workspace
 #ifndef FLEX_SHORT_ROW_MAX
 #define FLEX_SHORT_ROW_MAX 64
@@ -162,6 +163,7 @@ struct TileKernelArgs {
   long long num_rows;
   long long num_edges;
   long long num_tiles;
+  int rounds;               // > 0: on whole rows, how often every CTA takes kTileRun tiles in turn before the rest is split
   const int* win_table;                // gather windows (WIN kernels): per-tile segment table,
   const unsigned short* win_index;     // per-edge positions inside the window area,
   long long num_vertices;              // rows of the gathered array
@@ -239,13 +241,28 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   const long long t_begin = (long long)blockIdx.x * q + ((long long)blockIdx.x < rem ? blockIdx.x : rem);
   const int count = (int)(q + ((long long)blockIdx.x < rem ? 1 : 0));
 
+  // Tile k of the CTA where whole rows go round the CTAs: no carry ties a CTA to consecutive tiles, so in each round it takes
+  // kTileRun of them, and what is left behind the last full round is split like above (the same number of tiles a CTA).  The
+  // CTAs then walk the matrix as one front.  In a run of its own a CTA meets the columns a plane (or a line) away at a time
+  // of its own: on a 512^3 grid the three places where a vector record is gathered lie 2.3 GB of traffic apart, so it is read
+  // from DRAM three times (7-point fp64 SpMV, us, own runs / rounds of 4, 8, 16, 32, 64 tiles: 2529 / 2133, 2146, 2161, 2214,
+  // 2328; 300^3 480 / 422, 429, 434, 443, 464; 400^3 fp32 905 / 821, 827, 835, 839, 846; 5-point 3000^2 128 / 118, 122, 123, 125, 126).
+  auto round_tile = [&](int k) -> long long {
+    if (k < a.rounds * kTileRun) return ((long long)(k / kTileRun) * gridDim.x + blockIdx.x) * kTileRun + k % kTileRun;
+    return t_begin + (long long)a.rounds * kTileRun * (gridDim.x - 1 - blockIdx.x) + k;
+  };
+
   // The producer warp asks for its first coordinates together with the header (two round trips become one).  The
   // words lie inside the workspace whether it was planned or not; nothing is done with them before the check below.
-  OffsetT first_coords[4] = {0, 0, 0, 0};
+  OffsetT first_coords[4] = {0, 0, 0, 0}, first_of_round[4] = {0, 0, 0, 0};
   if constexpr (!DIRECT) {
     if (warp == Cfg::kWarps && count) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) first_coords[i] = coords[2 * t_begin + i];
+      if (L::kWhole && a.rounds) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) first_of_round[i] = coords[2ll * kTileRun * blockIdx.x + i];
+      }
     }
   }
 
@@ -371,6 +388,14 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // coordinates are read one tile ahead, so their load latency overlaps the wait for a free stage
       long long c_row = (long long)first_coords[0], c_nz = (long long)first_coords[1];
       long long n_row = (long long)first_coords[2], n_nz = (long long)first_coords[3];
+      long long t = t_begin;      // tile k
+      int run = 0x7fffffff;       // tiles until the CTA's next one is not the one behind
+      if (WHOLE && whole && a.rounds) {
+        c_row = (long long)first_of_round[0]; c_nz = (long long)first_of_round[1];
+        n_row = (long long)first_of_round[2]; n_nz = (long long)first_of_round[3];
+        t = (long long)kTileRun * blockIdx.x;
+        run = kTileRun;
+      }
       WinEnt c_we = count ? load_win_entry(t_begin) : WinEnt{0, 0, 0};
       // testing aid (flexspmv_debug_withhold_stage): the stage of tile `withhold - 1` and of every later tile is
       // never filled, so that the consumers' bounded wait runs out and the error path can be exercised
@@ -378,16 +403,24 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       int s = 0;                  // stage of tile k; round: how often the stages have been filled before
       uint32_t round = 0;
       for (int k = 0; k < count; ++k) {
-        if (withhold && (unsigned long long)(t_begin + k) + 1ull >= withhold) break;
-        long long nn_row = 0, nn_nz = 0;
-        if (k + 1 < count) { nn_row = (long long)coords[2 * (t_begin + k + 2)]; nn_nz = (long long)coords[2 * (t_begin + k + 2) + 1]; }
+        if (withhold && (unsigned long long)t + 1ull >= withhold) break;
+        ++t;
+        long long nf_row = n_row, nf_nz = n_nz, nn_row = 0, nn_nz = 0;       // front and end of the next tile
+        if (k + 1 < count) {
+          if (WHOLE && --run == 0) {
+            t = round_tile(k + 1);
+            run = k + 1 < a.rounds * kTileRun ? kTileRun : 0x7fffffff;
+            nf_row = (long long)coords[2 * t]; nf_nz = (long long)coords[2 * t + 1];
+          }
+          nn_row = (long long)coords[2 * t + 2]; nn_nz = (long long)coords[2 * t + 3];
+        }
         const WinEnt n_we = (k + 1 < count) ? load_win_entry(t_begin + k + 1) : WinEnt{0, 0, 0};
         if (round > 0) {
           const bool ok = mbar_wait_bounded(&empty[s], (round - 1) & 1u, kWaitPolls);
           if (!__all_sync(0xffffffffu, ok)) { pfail = true; break; }
         }
         issue(c_row, c_nz, n_row, n_nz, s, c_we);
-        c_row = n_row; c_nz = n_nz; n_row = nn_row; n_nz = nn_nz; c_we = n_we;
+        c_row = nf_row; c_nz = nf_nz; n_row = nn_row; n_nz = nn_nz; c_we = n_we;
         issued = k + 1;
         if (++s == nstages) { s = 0; ++round; }
       }
@@ -520,7 +553,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
         if (!__all_sync(0xffffffffu, ok)) {
           if (lane == 0) {
             raise_status(a.header, FLEXSPMV_ERR_TIMEOUT);
-            a.header->debug[0] = (uint32_t)(t_begin + k); a.header->debug[1] = (uint32_t)s; a.header->debug[2] = blockIdx.x;
+            a.header->debug[0] = (uint32_t)round_tile(k); a.header->debug[1] = (uint32_t)s; a.header->debug[2] = blockIdx.x;
           }
           return;
         }
