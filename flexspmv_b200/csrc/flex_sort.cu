@@ -4,60 +4,69 @@
 // (python_wrapper/dynamic_replace_submodule.py:20-41); here the permutation that sorts them is computed once,
 // the per-edge arrays are permuted with it, and the CSR offsets come from the sorted ids.
 //
-// Least-significant-digit radix sort on the row ids, which are dense: ceil(log2(num_rows)) bits in as few passes of at
-// most 8 bits as cover them, every pass the same width (20 bits: 3 x 7).  A pass is three launches: digit counts per
-// tile of 4096 keys, one CTA per digit that scans that digit's counts over the tiles, and the stable scatter.  No block
-// waits for another one.  The first pass reads the caller's ids and takes the positions as values, so there is no
-// separate initialisation; the passes alternate between two buffers so that the last one writes the caller's
-// permutation.  Equal digits keep their input order in every pass (see sort_scatter_kernel), so the permutation equals
-// a stable argsort (bit-exact against numpy.argsort(kind="stable")).
+// Least-significant-digit radix sort on the row ids, which are dense: ceil(log2(num_rows)) bits in as few passes as cover
+// them, every pass the same width (20 bits: 2 x 10).  A pass is three launches: digit counts per tile of keys, one CTA per
+// digit that scans that digit's counts over the tiles, and the stable scatter.  No block waits for another one.  Digits have
+// up to 8 bits, or up to 10 where that saves a pass (SortShape).  The first pass reads the caller's ids and takes the
+// positions as values, so there is no separate initialisation; the passes alternate between two buffers so that the last one
+// writes the caller's permutation.  Equal digits keep their input order in every pass (see sort_scatter_kernel), so the
+// permutation equals a stable argsort (bit-exact against numpy.argsort(kind="stable")).
 #include <cuda_runtime.h>
 
 #include "flex_common.cuh"
 
 namespace flex {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortKeysPerThread = 16;
-constexpr int kSortTile = kSortThreads * kSortKeysPerThread;
-constexpr int kMaxRadix = 256;                // bins of the widest digit
+// One width of digit: bins, threads of a CTA, and with 16 keys a thread the tile.  A pass with 1024 bins has tiles of 8192
+// keys, so that a digit's keys in a tile still leave in runs of 8 and more.
+template <int BITS_, int THREADS_>
+struct SortShape {
+  static constexpr int kBits = BITS_, kBins = 1 << BITS_, kThreads = THREADS_, kWarps = THREADS_ / 32;
+  static constexpr int kTile = THREADS_ * kSortKeysPerThread;
+  static constexpr int kWordsPerThread = kBins / 2 > THREADS_ ? kBins / 2 / THREADS_ : 1;    // two 16-bit counters a word
+  static constexpr int kCntPitch = kBins + 2;            // per warp; the bin behind the last takes the lanes behind the end
+  // shared memory of the scatter: tile in digit order, global place of every digit, counters by warp
+  static constexpr int kSmem = kTile * 8 + kBins * 4 + kWarps * kCntPitch * 2;
+};
+using SortNarrow = SortShape<8, 256>;
+using SortWide = SortShape<10, 512>;
 
 template <typename KeyT>
 __device__ __forceinline__ unsigned digit_of(KeyT key, int shift, unsigned mask) { return ((unsigned)key >> shift) & mask; }
 
 // Per tile: number of keys with each digit -> hist[digit * num_tiles + tile].  CHECK (first pass): flags ids outside
 // [0, num_rows).
-template <typename KeyT, bool CHECK>
-__global__ void __launch_bounds__(kSortThreads) sort_count_kernel(const KeyT* __restrict__ keys, long long n, long long num_rows,
-                                                                  int shift, unsigned mask, int num_tiles,
-                                                                  unsigned* __restrict__ hist, int* status) {
-  __shared__ unsigned s_cnt[kMaxRadix];
+template <typename KeyT, bool CHECK, class S>
+__global__ void __launch_bounds__(S::kThreads) sort_count_kernel(const KeyT* __restrict__ keys, long long n, long long num_rows,
+                                                                 int shift, unsigned mask, int num_tiles,
+                                                                 unsigned* __restrict__ hist, int* status) {
+  __shared__ unsigned s_cnt[S::kBins];
   const int tid = threadIdx.x;
-  s_cnt[tid] = 0;
-  static_assert(kMaxRadix == kSortThreads, "one bin per thread");
+  for (int d = tid; d < S::kBins; d += S::kThreads) s_cnt[d] = 0;
   __syncthreads();
-  const long long base = (long long)blockIdx.x * kSortTile + tid;
+  const long long base = (long long)blockIdx.x * S::kTile + tid;
   bool bad = false;
   KeyT k[kSortKeysPerThread];           // all loads before the first atomic
 #pragma unroll
   for (int i = 0; i < kSortKeysPerThread; ++i) {
-    const long long e = base + i * kSortThreads;
+    const long long e = base + i * S::kThreads;
     k[i] = e < n ? keys[e] : KeyT(0);
   }
 #pragma unroll
   for (int i = 0; i < kSortKeysPerThread; ++i) {
-    if (base + i * kSortThreads < n) {
+    if (base + i * S::kThreads < n) {
       if (CHECK) bad |= (long long)k[i] < 0 || (long long)k[i] >= num_rows;
       atomicAdd(&s_cnt[digit_of(k[i], shift, mask)], 1u);     // integer counts: order does not matter
     }
   }
   if (CHECK && bad) atomicCAS(status, 0, FLEXSPMV_ERR_BAD_ARG);
   __syncthreads();
-  if (tid <= (int)mask) hist[(size_t)tid * num_tiles + blockIdx.x] = s_cnt[tid];
+  for (int d = tid; d <= (int)mask; d += S::kThreads) hist[(size_t)d * num_tiles + blockIdx.x] = s_cnt[d];
 }
 
-// Exclusive scan over the CTA's kSortThreads threads; `total` is the sum of all.  s_warp: kSortWarps words.
+// Exclusive scan over the CTA's 32 * WARPS threads; `total` is the sum of all.  s_warp: WARPS words.
+template <int WARPS>
 __device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned* s_warp, unsigned& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned x = v;
@@ -70,7 +79,7 @@ __device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned* s_warp
   __syncthreads();
   unsigned before = 0, sum = 0;
 #pragma unroll
-  for (int w = 0; w < kSortWarps; ++w) {
+  for (int w = 0; w < WARPS; ++w) {
     const unsigned c = s_warp[w];
     if (w < warp) before += c;
     sum += c;
@@ -81,18 +90,19 @@ __device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned* s_warp
 }
 
 // One CTA per digit: exclusive scan of the digit's counts over the tiles, in place; the digit's total.
-__global__ void __launch_bounds__(kSortThreads) sort_scan_kernel(unsigned* __restrict__ hist, int num_tiles, unsigned* __restrict__ totals) {
-  __shared__ unsigned s_warp[kSortWarps];
+constexpr int kScanThreads = 256;
+__global__ void __launch_bounds__(kScanThreads) sort_scan_kernel(unsigned* __restrict__ hist, int num_tiles, unsigned* __restrict__ totals) {
+  __shared__ unsigned s_warp[kScanThreads / 32];
   unsigned* row = hist + (size_t)blockIdx.x * num_tiles;
   unsigned run = 0;
   constexpr int kPer = 4;
-  for (int base = 0; base < num_tiles; base += kSortThreads * kPer) {
+  for (int base = 0; base < num_tiles; base += kScanThreads * kPer) {
     unsigned v[kPer], sum = 0;
     const int i0 = base + threadIdx.x * kPer;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) { v[j] = i0 + j < num_tiles ? row[i0 + j] : 0u; sum += v[j]; }
     unsigned total;
-    unsigned at = run + block_exclusive(sum, s_warp, total);
+    unsigned at = run + block_exclusive<kScanThreads / 32>(sum, s_warp, total);
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       if (i0 + j < num_tiles) row[i0 + j] = at;
@@ -103,94 +113,121 @@ __global__ void __launch_bounds__(kSortThreads) sort_scan_kernel(unsigned* __res
   if (threadIdx.x == 0) totals[blockIdx.x] = run;
 }
 
-// Stable scatter of one pass.  Bound by memory traffic (8 bytes in and 8 out per key) once the stores leave in runs:
-// a warp ranks its 512 consecutive keys 32 at a time (lanes with the same digit find one another with one vote per bit
-// of the digit -- __match_any_sync took four times as long, 80 us a pass; the rank counts the lanes below), the tile is put in digit order in shared memory and leaves from there, so that a digit's
-// keys are stored side by side.  Storing straight from the ranks would touch a sector per key.  Order: warps own
-// consecutive runs of keys, a warp's rounds follow one another and lanes are ranked in order, so equal digits never
-// change places.  FIRST: the values are the positions.
-// Measured (8.4 M 64-bit ids, 1 M rows, B200): the whole sort with offsets and one permuted tensor 1106 us with 4-bit
-// digits, a one-CTA scan of all counts and stores straight from the ranks; 334 us like this (a pass 70 us).
-template <typename KeyT, bool FIRST>
-__global__ void __launch_bounds__(kSortThreads, 4) sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ vals_in,
-                                                                    long long n, int shift, unsigned mask, int num_tiles,
-                                                                    const unsigned* __restrict__ hist,
-                                                                    const unsigned* __restrict__ totals,
-                                                                    unsigned* __restrict__ keys_out, int* __restrict__ vals_out) {
-  __shared__ unsigned short s_cnt[kSortWarps][kMaxRadix + 1];    // the last bin takes the lanes behind the end
-  __shared__ unsigned s_out[kMaxRadix];                          // where the digit's run goes, less its place in the tile
-  __shared__ unsigned short s_first[kMaxRadix];                  // the digit's place in the tile
-  __shared__ unsigned s_warp[kSortWarps];
-  __shared__ unsigned s_key[kSortTile];
-  __shared__ int s_val[kSortTile];
+// Stable scatter of one pass.  A warp ranks its 512 consecutive keys 32 at a time (lanes with the same digit find one another
+// with one vote per bit of the digit -- __match_any_sync took four times as long, 80 us a pass; the rank counts the lanes
+// below), the tile is put in digit order in shared memory and leaves from there, so that a digit's keys are stored side by
+// side.  Storing straight from the ranks would touch a sector per key.  Order: warps own consecutive runs of keys, a warp's
+// rounds follow one another and lanes are ranked in order, so equal digits never change places.  FIRST: the values are the
+// positions.  Bound by the instructions of the ranking and the moves (135 for 32 keys a pass with 7-bit digits, half of the
+// issue slots) and by shared memory's wavefronts (52 %), so what helps is a pass less.
+template <typename KeyT, bool FIRST, class S>
+__global__ void __launch_bounds__(S::kThreads, 1024 / S::kThreads)
+sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ vals_in, long long n, int shift, unsigned mask,
+                    int num_tiles, const unsigned* __restrict__ hist, const unsigned* __restrict__ totals,
+                    unsigned* __restrict__ keys_out, int* __restrict__ vals_out) {
+  constexpr int KPT = kSortKeysPerThread, T = S::kThreads, W = S::kWarps, WPT = S::kWordsPerThread;
+  extern __shared__ __align__(16) unsigned char s_sort[];
+  uint2* const s_pair = reinterpret_cast<uint2*>(s_sort);                                  // [kTile] the tile in digit order
+  unsigned* const s_out = reinterpret_cast<unsigned*>(s_pair + S::kTile);                  // [kBins] where the digit's run goes, less its place in the tile
+  unsigned short* const s_cnt = reinterpret_cast<unsigned short*>(s_out + S::kBins);       // [W][kCntPitch]
+  __shared__ unsigned s_warp[W];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long long tile0 = (long long)blockIdx.x * kSortTile;
-  const int count = (int)(n - tile0 < kSortTile ? n - tile0 : kSortTile);
-  for (int i = tid; i < kSortWarps * (kMaxRadix + 1); i += kSortThreads) (&s_cnt[0][0])[i] = 0;
-  unsigned k[kSortKeysPerThread];
-  int v[kSortKeysPerThread];
-  const int mine = warp * (32 * kSortKeysPerThread) + lane;      // place of the lane's first key in the tile
+  const long long tile0 = (long long)blockIdx.x * S::kTile;
+  const int count = (int)(n - tile0 < S::kTile ? n - tile0 : S::kTile);
+  for (int i = tid; i < W * S::kCntPitch / 2; i += T) reinterpret_cast<unsigned*>(s_cnt)[i] = 0;
+  unsigned k[KPT];
+  const int mine = warp * (32 * KPT) + lane;      // place of the lane's first key in the tile
 #pragma unroll
-  for (int i = 0; i < kSortKeysPerThread; ++i) {
+  for (int i = 0; i < KPT; ++i) {
     const int at = mine + i * 32;
-    k[i] = 0; v[i] = 0;
-    if (at < count) {
-      k[i] = (unsigned)keys_in[tile0 + at];
-      v[i] = FIRST ? (int)(tile0 + at) : vals_in[tile0 + at];
-    }
+    k[i] = at < count ? (unsigned)keys_in[tile0 + at] : 0u;
   }
   __syncthreads();
-  unsigned rank[kSortKeysPerThread];
+  unsigned short* const cnt = s_cnt + warp * S::kCntPitch;
+  unsigned rank[KPT / 2];                          // two 16-bit ranks a register
 #pragma unroll
-  for (int i = 0; i < kSortKeysPerThread; ++i) {
+  for (int i = 0; i < KPT; ++i) {
     const bool in = mine + i * 32 < count;
-    const unsigned d = in ? digit_of(k[i], shift, mask) : (unsigned)kMaxRadix;
+    const unsigned d = in ? digit_of(k[i], shift, mask) : (unsigned)S::kBins;
     unsigned same = __ballot_sync(0xffffffffu, in);
     if (!in) same = ~same;
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
+    for (int b = 0; b < S::kBits; ++b) {
       if ((mask >> b) == 0) break;                              // the same for every lane
       const unsigned set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
       same &= (d >> b) & 1u ? set : ~set;
     }
     const unsigned below = __popc(same & ((1u << lane) - 1u));
-    const unsigned seen = s_cnt[warp][d];
+    const unsigned seen = cnt[d];
     __syncwarp();
-    if (below == 0) s_cnt[warp][d] = (unsigned short)(seen + __popc(same));
+    if (below == 0) cnt[d] = (unsigned short)(seen + __popc(same));
     __syncwarp();
-    rank[i] = seen + below;
+    rank[i / 2] = i & 1 ? rank[i / 2] | (seen + below) << 16 : seen + below;
   }
   __syncthreads();
+  // values: needed last, requested now
+  int v[KPT];
+#pragma unroll
+  for (int i = 0; i < KPT; ++i) {
+    const int at = mine + i * 32;
+    v[i] = FIRST ? (int)(tile0 + at) : (at < count ? vals_in[tile0 + at] : 0);
+  }
   {
-    // thread = digit: the warps' counts become places behind the warps before; the digits' places follow one another
-    unsigned mine_d = 0;
-    for (int w = 0; w < kSortWarps; ++w) {
-      const unsigned c = s_cnt[w][tid];
-      s_cnt[w][tid] = (unsigned short)mine_d;
-      mine_d += c;
+    // two digits a word: the warps' counts become places in the tile -- behind the digits before, behind the warps before
+    unsigned* const words = reinterpret_cast<unsigned*>(s_cnt);
+    constexpr int kPitch = S::kCntPitch / 2;
+    const int w0 = tid * WPT;
+    const bool has = w0 < S::kBins / 2;
+    unsigned sum[WPT], tot[2 * WPT], digits = 0, global = 0;
+#pragma unroll
+    for (int j = 0; j < WPT; ++j) {
+      sum[j] = 0;
+      tot[2 * j] = tot[2 * j + 1] = 0;
+      if (has) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) sum[j] += words[w * kPitch + w0 + j];
+        if (2 * (w0 + j) <= (int)mask) tot[2 * j] = totals[2 * (w0 + j)];
+        if (2 * (w0 + j) + 1 <= (int)mask) tot[2 * j + 1] = totals[2 * (w0 + j) + 1];
+      }
+      digits += (sum[j] & 0xffffu) + (sum[j] >> 16);
+      global += tot[2 * j] + tot[2 * j + 1];
     }
-    const bool real = tid <= (int)mask;
-    unsigned sum;
-    const unsigned place = block_exclusive(mine_d, s_warp, sum);
-    const unsigned global = block_exclusive(real ? totals[tid] : 0u, s_warp, sum);
-    s_first[tid] = (unsigned short)place;
-    if (real) s_out[tid] = global + hist[(size_t)tid * num_tiles + blockIdx.x] - place;
+    unsigned all;
+    unsigned place = block_exclusive<W>(digits, s_warp, all);
+    unsigned to = block_exclusive<W>(global, s_warp, all);
+    if (has) {
+#pragma unroll
+      for (int j = 0; j < WPT; ++j) {
+        const int d = 2 * (w0 + j);
+        const unsigned second = place + (sum[j] & 0xffffu);
+        if (d <= (int)mask) s_out[d] = to + hist[(size_t)d * num_tiles + blockIdx.x] - place;
+        if (d + 1 <= (int)mask) s_out[d + 1] = to + tot[2 * j] + hist[(size_t)(d + 1) * num_tiles + blockIdx.x] - second;
+        unsigned at = place | second << 16;        // places are at most a tile: no carry between the halves
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const unsigned c = words[w * kPitch + w0 + j];
+          words[w * kPitch + w0 + j] = at;
+          at += c;
+        }
+        place = second + (sum[j] >> 16);
+        to += tot[2 * j] + tot[2 * j + 1];
+      }
+    }
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kSortKeysPerThread; ++i)
+  for (int i = 0; i < KPT; ++i)
     if (mine + i * 32 < count) {
-      const unsigned d = digit_of(k[i], shift, mask);
-      const unsigned at = s_first[d] + s_cnt[warp][d] + rank[i];
-      s_key[at] = k[i];
-      s_val[at] = v[i];
+      const unsigned at = cnt[digit_of(k[i], shift, mask)] + (i & 1 ? rank[i / 2] >> 16 : rank[i / 2] & 0xffffu);
+      s_pair[at] = make_uint2(k[i], (unsigned)v[i]);
     }
   __syncthreads();
-  for (int j = tid; j < count; j += kSortThreads) {
-    const unsigned key = s_key[j];
-    const unsigned to = s_out[digit_of(key, shift, mask)] + (unsigned)j;
-    keys_out[to] = key;
-    vals_out[to] = s_val[j];
+#pragma unroll 4
+  for (int j = tid; j < count; j += T) {
+    const uint2 q = s_pair[j];
+    const unsigned to = s_out[digit_of(q.x, shift, mask)] + (unsigned)j;
+    keys_out[to] = q.x;
+    vals_out[to] = (int)q.y;
   }
 }
 
@@ -224,28 +261,71 @@ __device__ __forceinline__ long long warp_lower_bound(const unsigned* __restrict
   }
   return lo;
 }
-// CSR offsets of sorted ids: offsets[r] = number of ids < r.  A block owns 256 consecutive rows: two warps find the run
-// of ids of those rows (five rounds of 32 probes for 33 M ids), then every row bisects inside that run, which is a few
-// kilobytes on average and stays in L1 -- against a bisection over all ids per row (1 M rows, 8.4 M ids: 48 us).
+// CSR offsets of sorted ids: offsets[r] = number of ids < r.  A block owns kOffsetRows consecutive rows: two warps find the
+// run of ids of those rows (five rounds of 32 probes for 33 M ids).  Where the run is not much longer than the rows are many,
+// it is read once, side by side: a place whose id differs from the one before it is where that row begins, and a row without
+// ids begins where the next one does (a minimum from behind).  A longer run (few rows hold most edges) is bisected per row, as
+// every run was (1 M rows, 8.4 M ids: 28.6 us).
+constexpr int kOffsetRows = 1024, kOffsetThreads = 256;
 template <typename OffsetT>
-__global__ void __launch_bounds__(256) sorted_offsets_kernel(const unsigned* __restrict__ keys, long long n, long long num_rows,
-                                                             OffsetT* __restrict__ offsets) {
+__global__ void __launch_bounds__(kOffsetThreads) sorted_offsets_kernel(const unsigned* __restrict__ keys, long long n, long long num_rows,
+                                                                        OffsetT* __restrict__ offsets) {
+  constexpr int kPer = kOffsetRows / kOffsetThreads;
   __shared__ long long s_run[2];
-  const long long r0 = (long long)blockIdx.x * 256;
-  const int warp = threadIdx.x >> 5;
+  __shared__ unsigned s_begin[kOffsetRows];
+  __shared__ unsigned s_warp[kOffsetThreads / 32];
+  const long long r0 = (long long)blockIdx.x * kOffsetRows;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (warp < 2) {
-    const long long at = warp_lower_bound(keys, n, r0 + 256 * warp);
-    if ((threadIdx.x & 31) == 0) s_run[warp] = at;
+    const long long at = warp_lower_bound(keys, n, r0 + kOffsetRows * warp);
+    if (lane == 0) s_run[warp] = at;
+  }
+  for (int i = tid; i < kOffsetRows; i += kOffsetThreads) s_begin[i] = 0xffffffffu;
+  __syncthreads();
+  const long long lo = s_run[0], hi = s_run[1];
+  if (hi - lo > 64 * kOffsetRows) {
+    for (int i = tid; i < kOffsetRows; i += kOffsetThreads) {
+      const long long r = r0 + i;
+      if (r > num_rows) break;
+      long long from = lo, to = hi;
+      while (from < to) {
+        const long long mid = (from + to) >> 1;
+        if ((long long)keys[mid] < r) from = mid + 1; else to = mid;
+      }
+      offsets[r] = (OffsetT)from;
+    }
+    return;
+  }
+  for (long long e = lo + tid; e < hi; e += kOffsetThreads) {
+    const unsigned id = keys[e], row = id - (unsigned)r0;
+    if ((e == lo || keys[e - 1] != id) && row < (unsigned)kOffsetRows) s_begin[row] = (unsigned)e;    // (ids out of range are not in order)
   }
   __syncthreads();
-  const long long r = r0 + threadIdx.x;
-  if (r > num_rows) return;
-  long long lo = s_run[0], hi = s_run[1];
-  while (lo < hi) {
-    const long long mid = (lo + hi) >> 1;
-    if ((long long)keys[mid] < r) lo = mid + 1; else hi = mid;
+  // a row without ids: the smallest beginning behind it, or the run's end
+  unsigned b[kPer], least = 0xffffffffu;
+#pragma unroll
+  for (int j = kPer - 1; j >= 0; --j) {
+    b[j] = s_begin[tid * kPer + j];
+    least = min(least, b[j]);
   }
-  offsets[r] = (OffsetT)lo;
+  unsigned behind = least;                     // smallest of this thread's rows and of the lanes behind
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned t = __shfl_down_sync(0xffffffffu, behind, o);
+    if (lane + o < 32) behind = min(behind, t);
+  }
+  if (lane == 0) s_warp[warp] = behind;
+  __syncthreads();
+  unsigned next = __shfl_down_sync(0xffffffffu, behind, 1);
+  if (lane == 31) next = 0xffffffffu;
+  for (int w = warp + 1; w < kOffsetThreads / 32; ++w) next = min(next, s_warp[w]);
+  next = min(next, (unsigned)hi);
+#pragma unroll
+  for (int j = kPer - 1; j >= 0; --j) {
+    next = min(next, b[j]);
+    const long long r = r0 + tid * kPer + j;
+    if (r <= num_rows) offsets[r] = (OffsetT)next;
+  }
 }
 
 // dst[e] = src[perm[e]] for records of one machine word, read and written whole (T: the vector type of that width)
@@ -279,12 +359,48 @@ __global__ void permute_kernel(const unsigned* __restrict__ src, unsigned* __res
   }
 }
 
-template <typename IdT>
-static void sort_first_pass(const IdT* ids, long long n, long long num_rows, unsigned mask, int tiles, unsigned* hist, unsigned* totals,
-                            unsigned* keys_out, int* vals_out, int* status, cudaStream_t st) {
-  sort_count_kernel<IdT, true><<<tiles, kSortThreads, 0, st>>>(ids, n, num_rows, 0, mask, tiles, hist, status);
-  sort_scan_kernel<<<mask + 1, kSortThreads, 0, st>>>(hist, tiles, totals);
-  sort_scatter_kernel<IdT, true><<<tiles, kSortThreads, 0, st>>>(ids, nullptr, n, 0, mask, tiles, hist, totals, keys_out, vals_out);
+// One pass over `keys` (FIRST: the values are the positions, and the ids are checked).
+template <typename KeyT, bool FIRST, class S>
+static int sort_pass(const KeyT* keys, const int* vals, long long n, long long num_rows, int shift, unsigned mask, unsigned* hist,
+                     unsigned* totals, unsigned* keys_out, int* vals_out, int* status, cudaStream_t st) {
+  const int tiles = (int)((n + S::kTile - 1) / S::kTile);
+  auto scatter = sort_scatter_kernel<KeyT, FIRST, S>;
+  if (S::kSmem > 48 * 1024)
+    if (cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem); e != cudaSuccess) return (int)e;
+  sort_count_kernel<KeyT, FIRST, S><<<tiles, S::kThreads, 0, st>>>(keys, n, num_rows, shift, mask, tiles, hist, status);
+  sort_scan_kernel<<<mask + 1, kScanThreads, 0, st>>>(hist, tiles, totals);
+  scatter<<<tiles, S::kThreads, S::kSmem, st>>>(keys, vals, n, shift, mask, tiles, hist, totals, keys_out, vals_out);
+  return (int)cudaGetLastError();
+}
+
+// All passes; `cur` says which of the two key buffers holds the sorted ids.
+template <class S>
+static int sort_passes(const void* ids, int id_bits, long long n, long long num_rows, int bits, int* perm, unsigned* const keys[2],
+                       int* spare, unsigned* hist, unsigned* totals, int* status, cudaStream_t st, int& cur) {
+  const int passes = (bits + S::kBits - 1) / S::kBits, width = (bits + passes - 1) / passes;
+  const unsigned mask = (1u << width) - 1u;
+  // the last pass writes the caller's permutation; the ones before it alternate with the spare buffer
+  int* vals[2] = {(passes & 1) ? spare : perm, (passes & 1) ? perm : spare};
+  for (int p = 0; p < passes; ++p) {
+    const int to = cur ^ 1;
+    int e;
+    if (p > 0)
+      e = sort_pass<unsigned, false, S>(keys[cur], vals[cur], n, num_rows, p * width, mask, hist, totals, keys[to], vals[to], status, st);
+    else if (id_bits == 32)
+      e = sort_pass<int, true, S>(static_cast<const int*>(ids), nullptr, n, num_rows, 0, mask, hist, totals, keys[to], vals[to], status, st);
+    else
+      e = sort_pass<long long, true, S>(static_cast<const long long*>(ids), nullptr, n, num_rows, 0, mask, hist, totals, keys[to], vals[to],
+                                        status, st);
+    if (e) return e;
+    cur = to;
+  }
+  return 0;
+}
+
+// Bytes of the counts and totals of a pass.
+template <class S>
+static uint64_t sort_count_bytes(long long n) {
+  return align_up((uint64_t)((n + S::kTile - 1) / S::kTile) * S::kBins * 4u, 256) + S::kBins * 4u;
 }
 
 static int grid_for(long long work, int block) {
@@ -301,10 +417,9 @@ extern "C" {
 int flexspmv_sort_rows_bytes(int64_t num_edges, size_t* bytes) {
   if (!bytes || num_edges < 0) return FLEXSPMV_ERR_BAD_ARG;
   if (num_edges > 0x7fffffffLL) return FLEXSPMV_ERR_TOO_LARGE;
-  const uint64_t blocks = (uint64_t)(num_edges + flex::kSortTile - 1) / flex::kSortTile;
   // keys (2 buffers), values (1 extra buffer; the other is the caller's permutation array), digit x tile counts, digit totals
-  *bytes = (size_t)(flex::align_up((uint64_t)num_edges * 4u, 256) * 3 + flex::align_up(blocks * flex::kMaxRadix * 4u, 256) +
-                    flex::kMaxRadix * 4u);
+  const uint64_t wide = flex::sort_count_bytes<flex::SortWide>(num_edges), narrow = flex::sort_count_bytes<flex::SortNarrow>(num_edges);
+  *bytes = (size_t)(flex::align_up((uint64_t)num_edges * 4u, 256) * 3 + (wide > narrow ? wide : narrow));
   return 0;
 }
 
@@ -315,26 +430,27 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
     return FLEXSPMV_ERR_BAD_ARG;
   if ((id_bits != 32 && id_bits != 64) || (offset_bits != 32 && offset_bits != 64)) return FLEXSPMV_ERR_BAD_ARG;
   if (num_edges > 0x7fffffffLL || num_rows > 0x7fffffffLL) return FLEXSPMV_ERR_TOO_LARGE;
-  size_t need = 0;
-  if (int e = flexspmv_sort_rows_bytes(num_edges, &need)) return e;
-  if (!d_scratch || scratch_bytes < need) return FLEXSPMV_ERR_WORKSPACE;
+  const uint64_t seg = flex::align_up((uint64_t)num_edges * 4u, 256);
+  // scratch for 8-bit digits is enough; with less than flexspmv_sort_rows_bytes says the wider ones are not taken
+  const uint64_t narrow_bytes = 3 * seg + flex::sort_count_bytes<flex::SortNarrow>(num_edges);
+  const uint64_t wide_bytes = 3 * seg + flex::sort_count_bytes<flex::SortWide>(num_edges);
+  if (!d_scratch || scratch_bytes < narrow_bytes) return FLEXSPMV_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(d_scratch) & 15u) return FLEXSPMV_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaError_t e = cudaMemsetAsync(d_status, 0, sizeof(int32_t), st); e != cudaSuccess) return (int)e;
-  const uint64_t seg = flex::align_up((uint64_t)num_edges * 4u, 256);
   char* base = static_cast<char*>(d_scratch);
-  unsigned* keys[2] = {reinterpret_cast<unsigned*>(base), reinterpret_cast<unsigned*>(base + seg)};
+  unsigned* const keys[2] = {reinterpret_cast<unsigned*>(base), reinterpret_cast<unsigned*>(base + seg)};
   int* spare = reinterpret_cast<int*>(base + 2 * seg);
   unsigned* hist = reinterpret_cast<unsigned*>(base + 3 * seg);
-  const int tiles = (int)((num_edges + flex::kSortTile - 1) / flex::kSortTile);
-  char* behind = base + 3 * seg + flex::align_up((uint64_t)tiles * flex::kMaxRadix * 4u, 256);
-  unsigned* totals = reinterpret_cast<unsigned*>(behind);
   int cur = 0;
   if (num_edges > 0) {
     int bits = 0;
     while (bits < 31 && (1ll << bits) < num_rows) ++bits;
-    const int passes = (bits + 7) / 8;
-    if (passes == 0) {
+    // 10-bit digits where they save a pass
+    const bool wide = scratch_bytes >= wide_bytes && (bits + 9) / 10 < (bits + 7) / 8;
+    // the totals are the last words of the scratch that the shape takes
+    unsigned* totals = reinterpret_cast<unsigned*>(base + (wide ? wide_bytes : narrow_bytes)) - (wide ? flex::SortWide::kBins : flex::SortNarrow::kBins);
+    if (bits == 0) {
       const int g = flex::grid_for(num_edges, 256);
       if (id_bits == 32)
         flex::sort_identity_kernel<int><<<g, 256, 0, st>>>(static_cast<const int*>(d_row_ids), num_edges, num_rows, keys[0], d_perm, d_status);
@@ -342,33 +458,16 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
         flex::sort_identity_kernel<long long><<<g, 256, 0, st>>>(static_cast<const long long*>(d_row_ids), num_edges, num_rows, keys[0],
                                                                  d_perm, d_status);
     } else {
-      const int width = (bits + passes - 1) / passes;
-      const unsigned mask = (1u << width) - 1u;
-      // the last pass writes the caller's permutation; the ones before it alternate with the spare buffer
-      int* vals[2] = {(passes & 1) ? spare : d_perm, (passes & 1) ? d_perm : spare};
-      for (int p = 0; p < passes; ++p) {
-        const int shift = p * width, to = cur ^ 1;
-        if (p == 0 && id_bits == 32)
-          flex::sort_first_pass<int>(static_cast<const int*>(d_row_ids), num_edges, num_rows, mask, tiles, hist, totals, keys[to], vals[to], d_status, st);
-        else if (p == 0)
-          flex::sort_first_pass<long long>(static_cast<const long long*>(d_row_ids), num_edges, num_rows, mask, tiles, hist, totals, keys[to],
-                                           vals[to], d_status, st);
-        else {
-          flex::sort_count_kernel<unsigned, false><<<tiles, flex::kSortThreads, 0, st>>>(keys[cur], num_edges, num_rows, shift, mask, tiles, hist, d_status);
-          flex::sort_scan_kernel<<<mask + 1, flex::kSortThreads, 0, st>>>(hist, tiles, totals);
-          flex::sort_scatter_kernel<unsigned, false><<<tiles, flex::kSortThreads, 0, st>>>(keys[cur], vals[cur], num_edges, shift, mask, tiles,
-                                                                                           hist, totals, keys[to], vals[to]);
-        }
-        cur = to;
-      }
+      auto sort = wide ? flex::sort_passes<flex::SortWide> : flex::sort_passes<flex::SortNarrow>;
+      if (int e = sort(d_row_ids, id_bits, num_edges, num_rows, bits, d_perm, keys, spare, hist, totals, d_status, st, cur)) return e;
     }
   }
   if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return (int)e;
-  const unsigned g = (unsigned)((num_rows + 256) / 256);
+  const unsigned g = (unsigned)(num_rows / flex::kOffsetRows + 1);       // offsets[0 .. num_rows]
   if (offset_bits == 32)
-    flex::sorted_offsets_kernel<int><<<g, 256, 0, st>>>(keys[cur], num_edges, num_rows, static_cast<int*>(d_row_offsets));
+    flex::sorted_offsets_kernel<int><<<g, flex::kOffsetThreads, 0, st>>>(keys[cur], num_edges, num_rows, static_cast<int*>(d_row_offsets));
   else
-    flex::sorted_offsets_kernel<long long><<<g, 256, 0, st>>>(keys[cur], num_edges, num_rows, static_cast<long long*>(d_row_offsets));
+    flex::sorted_offsets_kernel<long long><<<g, flex::kOffsetThreads, 0, st>>>(keys[cur], num_edges, num_rows, static_cast<long long*>(d_row_offsets));
   return (int)cudaGetLastError();
 }
 
