@@ -133,6 +133,10 @@ def choose_config(ir: GraphIR, dtype: str) -> Tuple[int, int, int, int]:
         for ipt in (5, 3):
             if smem_bytes(ir, dtype, block, ipt, stages) <= limit:
                 return block, ipt, stages, ctas
+    # records too wide for that: small CTAs rather than one edge a thread (72 bytes staged and 8 doubles summed an edge, 2 M edges in
+    # rows of 0 - 16, us: 256 x 1 x 2 CTAs 70.5, 64 x 3 x 4 57.3, 64 x 3 x 5 64.0; 0.24 M edges 19.3, 19.1)
+    if smem_bytes(ir, dtype, 64, 3, stages) <= (227 * 1024) // 4 - 1024:
+        return 64, 3, stages, 4
     ipt = 1
     while block > 64 and smem_bytes(ir, dtype, block, ipt, stages) > 110 * 1024:
         block //= 2
