@@ -387,6 +387,14 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
             w(f"    if ({when}) flex::bulk_prefetch_l2(p.{n} + row0, (uint64_t)(row1 - row0) * sizeof(V));")
     w("    (void)p; (void)row0; (void)row1; (void)lane;")
     w("  }")
+    w("  __device__ __forceinline__ static void prefetch_row(const Params& p, long long row) {")
+    if swe_rk:      # what the epilogue will read, asked for when the row's edges are
+        for n in ("area", "x_h", "x_uh", "x_vh"):
+            w(f"    fx::prefetch_l1(p.{n} + row);")
+        w("    if (!p.coef.first) { fx::prefetch_l1(p.acc_h + row); fx::prefetch_l1(p.acc_uh + row); fx::prefetch_l1(p.acc_vh + row); }")
+        w("    fx::prefetch_l1(p.wall_start + (row >> 5));")
+    w("    (void)p; (void)row;")
+    w("  }")
     w("  __device__ __forceinline__ static void store_aggregate(const Params& p, int i, V s) {")
     for n, d, off, _ in aggs:
         w(f"    if (i >= {off} && i < {off + d}) p.out_{n}[i - {off}] = s;")

@@ -222,6 +222,12 @@ struct GraphApi {
     }
   }
 
+  // A launch of at most kSmallQuarters / 4 tiles a CTA is a few round trips long and takes the kernel without stages.  us, with
+  // stages / without: 5-point fp64, tiles a CTA 1.1 5.74 / 4.2, 2.1 7.13 / 5.63, 2.9 8.84 / 8.08, 3.9 10.14 / 10.46; 7-point 2.3 7.49 /
+  // 6.10, 5.4 11.98 / 14.2.  Row-mode graphs: spring-mass fp32 0.7 7.40 / 6.82, 1.9 11.4 / 11.4; Rusanov fp64 0.7 6.84 / 5.8, 1.6
+  // 11.2 / 9.9, 2.8 15.7 / 16.7; a shallow-water step (four launches) 0.2 30.7 / 24.6, 2.1 69.2 / 56.9, 5.9 124 / 129.
+  static constexpr long long kSmallQuarters = G::kGatherNeedsRow ? 9 : 12;
+
   // Where the gathered vectors are larger than this, tiles of whole rows go round the CTAs (round_tile in flex_tile_kernel.cuh).
   // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its
   // neighbours in L1: 7-point fp32 145^3 (12 MB) 42.6 us in runs of its own, 45.0 in rounds; 27 columns a row fp64, 3 M rows
@@ -230,11 +236,11 @@ struct GraphApi {
 
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
   // once for each device of the process.
-  template <typename OffsetT, class C = Cfg, bool WIN = false>
+  template <typename OffsetT, class C = Cfg, bool WIN = false, int MODE = kPlain>
   static int resident_ctas(int* out) {
     using L = TileSmemLayout<G, OffsetT, C, WIN>;
     static_assert(L::kTotal <= 227 * 1024, "tile kernel needs more shared memory than one sm_100a CTA can have");
-    auto kernel = flex_tile_kernel<G, OffsetT, C, WIN>;
+    auto kernel = flex_tile_kernel<G, OffsetT, C, WIN, MODE>;
     constexpr int kThreads = C::kBlock + (G::kDirectLoads ? 0 : 32);
     constexpr int kMaxDevices = 64;
     static std::mutex mu;
@@ -275,16 +281,23 @@ struct GraphApi {
     a.carry_val = static_cast<char*>(ws) + h.carry_val_offset;
     a.num_rows = d->num_rows; a.num_edges = d->num_edges; a.num_tiles = tiles;
     a.rounds = 0;
-    if constexpr (L::kWhole) {
-      const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
-      if (vertices * G::kGatherRecordBytes > kKeepBytes) a.rounds = (int)(tiles / (grid * kTileRun));
-    }
     a.win_table = nullptr; a.win_index = nullptr; a.num_vertices = d->num_vertices;
     if constexpr (WIN) {
       if (d->num_vertices <= 0) return FLEXSPMV_ERR_BAD_ARG;
       if (!aligned16(G::gather_base(p))) return FLEXSPMV_ERR_ALIGN;   // window sources are 16-byte aligned only then
       a.win_table = reinterpret_cast<const int*>(static_cast<char*>(ws) + h.win_table_offset);
       a.win_index = reinterpret_cast<const unsigned short*>(static_cast<char*>(ws) + h.win_index_offset);
+    }
+    if constexpr (L::kWhole) {
+      const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
+      if (4 * tiles <= kSmallQuarters * grid) {
+        kernel = flex_tile_kernel<G, OffsetT, C, WIN, kSmall>;
+        if (int e = resident_ctas<OffsetT, C, WIN, kSmall>(&resident)) return e;      // the grid stays the plan's
+      } else if (vertices * G::kGatherRecordBytes > kKeepBytes && tiles >= grid * kTileRun) {
+        a.rounds = (int)(tiles / (grid * kTileRun));
+        kernel = flex_tile_kernel<G, OffsetT, C, WIN, kRounds>;
+        if (int e = resident_ctas<OffsetT, C, WIN, kRounds>(&resident)) return e;
+      }
     }
     return launch_pdl(kernel, (unsigned)grid, kThreads, L::kTotal, st, p, a);
   }

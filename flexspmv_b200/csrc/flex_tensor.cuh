@@ -217,6 +217,8 @@ __device__ __forceinline__ Vec<V, D> ldg_vec(const V* p) {   // read-only global
   return r;
 }
 
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // L2 prefetch of the byte range [b, e) by one warp (one request per 128-byte line)
 __device__ __forceinline__ void prefetch_l2_range(const void* b, const void* e, int lane) {
   const char* q = reinterpret_cast<const char*>(reinterpret_cast<uintptr_t>(b) & ~(uintptr_t)127) + lane * 128;

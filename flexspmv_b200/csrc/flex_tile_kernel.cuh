@@ -84,6 +84,22 @@ struct DirectTile {
   }
 };
 
+// The per-edge arrays read straight from global memory through the read-only path; `e` counts from the array's front.
+template <typename T>
+struct LdgRef {
+  const T* ptr;
+  __device__ __forceinline__ T operator*() const { return __ldg(ptr); }
+  __device__ __forceinline__ T operator[](int i) const { return __ldg(ptr + i); }
+};
+template <class G>
+struct LdgTile {
+  const typename G::Params* p;
+  template <int I, class T>
+  __device__ __forceinline__ LdgRef<T> stream(long long e) const {
+    return LdgRef<T>{reinterpret_cast<const T*>(G::template stream_ptr<I>(*p) + (size_t)e * G::template stream_bytes<I>())};
+  }
+};
+
 template <class G, bool WIN> struct WinBytesOf { static constexpr int value = 0; };
 template <class G> struct WinBytesOf<G, true> { static constexpr int value = G::kWinBytes; };
 
@@ -163,7 +179,7 @@ struct TileKernelArgs {
   long long num_rows;
   long long num_edges;
   long long num_tiles;
-  int rounds;               // > 0: on whole rows, how often every CTA takes kTileRun tiles in turn before the rest is split
+  int rounds;               // kRounds: how often every CTA takes kTileRun tiles in turn before the rest is split
   const int* win_table;                // gather windows (WIN kernels): per-tile segment table,
   const unsigned short* win_index;     // per-edge positions inside the window area,
   long long num_vertices;              // rows of the gathered array
@@ -200,7 +216,14 @@ __device__ __forceinline__ Window make_window(const void* gbase, uint32_t eb, lo
   return w;
 }
 
-template <class G, typename OffsetT, class Cfg, bool WIN = false>
+// Instantiations of the kernel, picked by the size of a launch (GraphApi::launch_tiles).  They differ in what they do with a plan of
+// whole rows; other plans run the same loops in all of them.  One kernel for all three costs the plain one 2 % (145^3 fp32 42.3
+// -> 43.1 us, spring-mass 500^2 fp64 20.7 -> 21.1).
+constexpr int kPlain = 0;
+constexpr int kSmall = 1;       // few tiles a CTA: whole rows are read straight from global memory
+constexpr int kRounds = 2;      // tiles of whole rows go round the CTAs
+
+template <class G, typename OffsetT, class Cfg, bool WIN = false, int MODE = kPlain>
 __global__ void __launch_bounds__(Cfg::kBlock + (G::kDirectLoads ? 0 : 32), Cfg::kMinCtas)
 flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   using V = typename G::V;
@@ -259,11 +282,22 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
     if (warp == Cfg::kWarps && count) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) first_coords[i] = coords[2 * t_begin + i];
-      if (L::kWhole && a.rounds) {
+      if constexpr (MODE == kRounds) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) first_of_round[i] = coords[2ll * kTileRun * blockIdx.x + i];
       }
     }
+  }
+
+  // So do the threads of a small launch with the ends of their first rows.
+  OffsetT row_from = 0, row_to = 0;
+  long long small_row = 0, small_end = 0;
+  if constexpr (MODE == kSmall) {
+    const long long share = ((a.num_rows + gridDim.x - 1) / gridDim.x + 31) & ~31ll;
+    small_row = blockIdx.x * share + tid;
+    small_end = (blockIdx.x + 1) * share < a.num_rows ? (blockIdx.x + 1) * share : a.num_rows;
+    // (the first row begins at edge 0 whatever row_offsets[0] says)
+    if (small_row < small_end) { row_from = small_row ? row_offsets[small_row] : OffsetT(0); row_to = row_offsets[small_row + 1]; }
   }
 
   // All that the header says, requested before the first branch: one round trip.
@@ -271,6 +305,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   const int h_bits = a.header->offset_bits;
   const long long h_rows = a.header->num_rows, h_edges = a.header->num_edges, h_tiles = a.header->num_tiles;
   const int h_snapped = a.header->snapped_grid, h_whole = a.header->whole_rows, h_row_loop = a.header->row_loop;
+  const uint32_t h_withhold = MODE == kSmall ? a.header->debug[7] : 0u;      // (a test that withholds a stage means the loops with stages)
   // a workspace that was never planned for this problem holds no usable coordinates: every CTA
   // sees the same header, so all of them leave here and the ticket stays untouched
   if (h_magic != kMagic || h_tiles != a.num_tiles || h_rows != a.num_rows || h_edges != a.num_edges || h_bits != (int)(8 * sizeof(OffsetT))) {
@@ -286,6 +321,42 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   }
   // the loop over whole rows has its own stages, in its own places
   const bool whole = WHOLE && (G::kEpilogue || h_row_loop == 1);
+  if constexpr (MODE == kSmall) {
+    if (whole && h_withhold == 0) {
+      // ---- whole rows of a small launch: one row per thread, everything straight from global memory ----------------------
+      // Bound by round trips, of which there are three -- row ends (asked for with the header), the row's edges, its gathers --
+      // without barriers, bulk copies and the producer's coordinates in front of them.  Sums run left to right as in the loop
+      // below: the same bits.
+      LdgTile<G> tile{&p};
+      constexpr int RB = Cfg::kRowBatch;
+      for (; small_row < small_end; small_row += BLOCK + 32) {
+        const long long e_from = (long long)row_from;
+        const int n = (int)(row_to - row_from);
+        if constexpr (G::kEpilogue) G::prefetch_row(p, small_row);
+        V sum[kAcc];
+#pragma unroll
+        for (int j = 0; j < kAcc; ++j) sum[j] = V(0);
+        typename G::GRow grow;
+        if constexpr (G::kGatherNeedsRow) { if (n > 0) G::gather_row(p, small_row, grow); }
+        for (int e0 = 0; e0 < n; e0 += RB) {
+          typename G::EReg er[RB];
+          typename G::GEdge ge[RB];
+#pragma unroll
+          for (int b = 0; b < RB; ++b)
+            if (e0 + b < n) G::load_edge(p, tile, e_from + e0 + b, e_from + e0 + b, er[b]);
+#pragma unroll
+          for (int b = 0; b < RB; ++b)
+            if (e0 + b < n) G::gather_edge(p, er[b], ge[b]);
+#pragma unroll
+          for (int b = 0; b < RB; ++b)
+            if (e0 + b < n) G::map(p, er[b], e_from + e0 + b, grow, ge[b], sum);
+        }
+        if (small_row + BLOCK + 32 < small_end) { row_from = row_offsets[small_row + BLOCK + 32]; row_to = row_offsets[small_row + BLOCK + 33]; }
+        G::finish_row(p, small_row, sum);
+      }
+      return;
+    }
+  }
   const int nstages = WHOLE ? (whole ? L::kRowStages : S) : S;
   unsigned char* const stage_base = (WHOLE && whole) ? smem + L::kOffRowStages : s_stage;
 
@@ -390,7 +461,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       long long n_row = (long long)first_coords[2], n_nz = (long long)first_coords[3];
       long long t = t_begin;      // tile k
       int run = 0x7fffffff;       // tiles until the CTA's next one is not the one behind
-      if (WHOLE && whole && a.rounds) {
+      if (MODE == kRounds && whole) {
         c_row = (long long)first_of_round[0]; c_nz = (long long)first_of_round[1];
         n_row = (long long)first_of_round[2]; n_nz = (long long)first_of_round[3];
         t = (long long)kTileRun * blockIdx.x;
@@ -407,7 +478,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
         ++t;
         long long nf_row = n_row, nf_nz = n_nz, nn_row = 0, nn_nz = 0;       // front and end of the next tile
         if (k + 1 < count) {
-          if (WHOLE && --run == 0) {
+          if (MODE == kRounds && --run == 0) {
             t = round_tile(k + 1);
             run = k + 1 < a.rounds * kTileRun ? kTileRun : 0x7fffffff;
             nf_row = (long long)coords[2 * t]; nf_nz = (long long)coords[2 * t + 1];
@@ -553,7 +624,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
         if (!__all_sync(0xffffffffu, ok)) {
           if (lane == 0) {
             raise_status(a.header, FLEXSPMV_ERR_TIMEOUT);
-            a.header->debug[0] = (uint32_t)round_tile(k); a.header->debug[1] = (uint32_t)s; a.header->debug[2] = blockIdx.x;
+            a.header->debug[0] = (uint32_t)(MODE == kRounds ? round_tile(k) : t_begin + k); a.header->debug[1] = (uint32_t)s; a.header->debug[2] = blockIdx.x;
           }
           return;
         }

@@ -1,0 +1,112 @@
+"""Kernels picked by the size of a launch: the tile kernel without stages (few tiles a CTA) and with tiles going round the CTAs (large
+gathered vectors) against its plain form, bit for bit; the sort's 10-bit digits."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from flexspmv_b200 import graphs
+from flexspmv_b200.binding import GraphExtension, load_library
+from flexspmv_b200.python_wrapper.dynamic_replace_submodule import sort_edges_by_row
+from oracle import ir_eval
+from parity import assert_outputs_match
+from test_gpu_parity import run_gpu
+from test_gpu_whole_rows import with_lengths
+
+pytestmark = pytest.mark.gpu
+
+GRAPHS = [("spmv", "float64"), ("spmv", "float32"), ("spmv", "int64"), ("spring_mass", "float32"), ("rusanov", "float64"),
+          ("swe_delta", "float32"), ("swe_boundary", "float64"), ("ops_zoo", "float64")]
+
+
+def launch(ir, prob, dtype, num_cols, bits, **kw):
+    """Outputs (as bytes) of one launch; ``num_cols``: the number of vertices that the descriptor names."""
+    ext = GraphExtension(ir, random_gather=False, **kw)
+    non_gather, gathers, index_names = graphs.operator_signature(ir)
+    v = [torch.from_numpy(np.ascontiguousarray(prob.values[n].astype(dtype))).cuda() for n in non_gather + gathers]
+    ix = [torch.from_numpy(np.ascontiguousarray(prob.indices[n])).cuda() for n in index_names]
+    ro = torch.from_numpy(prob.row_offsets.astype(np.int32 if bits == 32 else np.int64)).cuda()
+    outs = [torch.full((prob.num_rows, d), -7, dtype=v[0].dtype, device="cuda") for _, d in ext._out_kinds]
+    ext.launch_into(v, ix, ro, outs, prob.num_rows, prob.nnz, num_cols)
+    ext.check()
+    return [o.cpu().numpy().tobytes() for o in outs], ext.planned_whole_rows()
+
+
+@pytest.mark.parametrize("gname,dt", GRAPHS)
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("lengths", [[5] * 4001, [0, 3, 7, 1] * 900 + [0] * 40, [32] * 333, [1] * 31, [6, 7] * 20_000],
+                         ids=["5", "uneven", "32", "31_rows", "several_rows_a_thread"])
+def test_small_launches_equal_staged_ones(gname, dt, bits, lengths):
+    """One CTA has all the tiles (more than three: stages) against the default grid (at most one a CTA: none)."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, lengths, 101, dtype)
+    small, whole = launch(ir, prob, dtype, prob.num_cols, bits)
+    staged, _ = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=1)
+    two, _ = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=29)       # two tiles a CTA where there are 58
+    assert small == staged == two
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    got, _ = run_gpu(GraphExtension(ir, random_gather=False), ir, prob, dtype)
+    assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} small")
+
+
+@pytest.mark.parametrize("gname,dt", GRAPHS)
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("ctas", [1, 3, 7])
+def test_rounds_equal_runs_of_consecutive_tiles(gname, dt, bits, ctas):
+    """A descriptor with many vertices takes tiles in rounds of four a CTA and splits the rest; the results are those of the plain
+    order.  40 001 rows of 6 and 7 edges are 200 tiles and more."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [6, 7] * 20_000 + [3], 103, dtype)
+    plain, whole = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=ctas)
+    rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, max_ctas=ctas)
+    assert whole and plain == rounds
+    long = with_lengths(ir, [6, 7] * 20_000 + [200], 103, dtype)             # not whole rows: the loop with carries in either
+    plain, whole = launch(ir, long, dtype, long.num_cols, bits, max_ctas=ctas)
+    rounds, _ = launch(ir, long, dtype, 1 << 27, bits, max_ctas=ctas)
+    assert not whole and plain == rounds
+
+
+@pytest.mark.parametrize("rows", [257, 512, 1023, 1024, 1025, (1 << 18) + 3, (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("n", [1, 8191, 8192, 8193, 5 * 8192 + 77])
+def test_ten_bit_digits(rows, n):
+    rng = np.random.default_rng(rows + n)
+    draws = {"uniform": rng.integers(0, rows, n), "last": np.full(n, rows - 1), "few": rng.choice([0, rows // 2, rows - 1], n)}
+    for what, ids in draws.items():
+        for dtype in (np.int32, np.int64):
+            perm, crow = sort_edges_by_row(torch.from_numpy(ids.astype(dtype)).cuda(), rows)
+            assert np.array_equal(perm.cpu().numpy(), np.argsort(ids, kind="stable").astype(np.int32)), what
+            assert np.array_equal(crow.cpu().numpy(), np.searchsorted(np.sort(ids), np.arange(rows + 1))), what
+
+
+def test_offsets_where_few_rows_hold_most_edges():
+    """More than 64 edges a row over 1024 rows: bisected; blocks beside them: read once."""
+    rows, n = 5000, 300_000
+    ids = np.random.default_rng(7).choice([3, 1023, 1024, 2500, 2501, 4999], n, p=[0.3, 0.1, 0.05, 0.25, 0.25, 0.05])
+    _, crow = sort_edges_by_row(torch.from_numpy(ids).cuda(), rows)
+    assert np.array_equal(crow.cpu().numpy(), np.searchsorted(np.sort(ids), np.arange(rows + 1)))
+
+
+def test_scratch_for_eight_bit_digits_is_enough():
+    """Three arrays of 4 bytes an edge and the counts of 256 digits a tile of 4096: what the sort asked for before it had wider
+    digits.  A byte less is refused."""
+    lib = load_library()
+    n, rows = 30_011, 1 << 20
+    ids = np.random.default_rng(9).integers(0, rows, n)
+    up = lambda b: -(-b // 256) * 256
+    need = 3 * up(4 * n) + up(-(-n // 4096) * 1024) + 1024
+    full = ctypes.c_size_t()
+    assert lib.flexspmv_sort_rows_bytes(ctypes.c_int64(n), ctypes.byref(full)) == 0 and full.value > need
+    d_ids = torch.from_numpy(ids).cuda()
+    for size in (need, full.value, need - 1):
+        perm = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+        crow = torch.empty(rows + 1, dtype=torch.int64, device="cuda")
+        scratch, status = torch.empty(full.value, dtype=torch.uint8, device="cuda"), torch.empty(1, dtype=torch.int32, device="cuda")
+        ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+        code = lib.flexspmv_sort_rows(ptr(d_ids), 64, ctypes.c_int64(n), ctypes.c_int64(rows), ptr(perm), ptr(crow), 64, ptr(scratch),
+                                      ctypes.c_size_t(size), ptr(status), None)
+        torch.cuda.synchronize()
+        if size < need:
+            assert code == -3
+        else:
+            assert code == 0 and np.array_equal(perm.cpu().numpy(), np.argsort(ids, kind="stable").astype(np.int32))
