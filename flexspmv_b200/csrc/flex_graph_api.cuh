@@ -231,8 +231,9 @@ struct GraphApi {
   // Where the gathered vectors are larger than this, tiles of whole rows go round the CTAs (round_tile in flex_tile_kernel.cuh).
   // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its
   // neighbours in L1: 7-point fp32 145^3 (12 MB) 42.6 us in runs of its own, 45.0 in rounds; 27 columns a row fp64, 3 M rows
-  // (24 MB) 188 / 194; 5-point fp64 3000^2 (72 MB) 128 / 118.
-  static constexpr long long kKeepBytes = 48ll << 20;
+  // (24 MB) 188 / 194; Rusanov fp64 1024^2 (50 MB) 80.7 / 76.7, a shallow-water step 1024^2 (50 MB) 450 / 384; 5-point fp64 3000^2
+  // (72 MB) 128 / 118.
+  static constexpr long long kKeepBytes = 40ll << 20;
 
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
   // once for each device of the process.

@@ -459,8 +459,9 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // coordinates are read one tile ahead, so their load latency overlaps the wait for a free stage
       long long c_row = (long long)first_coords[0], c_nz = (long long)first_coords[1];
       long long n_row = (long long)first_coords[2], n_nz = (long long)first_coords[3];
-      long long t = t_begin;      // tile k
-      int run = 0x7fffffff;       // tiles until the CTA's next one is not the one behind
+      long long t = 0;            // kRounds: tile k, and the tiles until the CTA's next one is not the one behind
+      int run = 0x7fffffff;
+      if constexpr (MODE == kRounds) t = t_begin;
       if (MODE == kRounds && whole) {
         c_row = (long long)first_of_round[0]; c_nz = (long long)first_of_round[1];
         n_row = (long long)first_of_round[2]; n_nz = (long long)first_of_round[3];
@@ -474,16 +475,22 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       int s = 0;                  // stage of tile k; round: how often the stages have been filled before
       uint32_t round = 0;
       for (int k = 0; k < count; ++k) {
-        if (withhold && (unsigned long long)t + 1ull >= withhold) break;
-        ++t;
-        long long nf_row = n_row, nf_nz = n_nz, nn_row = 0, nn_nz = 0;       // front and end of the next tile
-        if (k + 1 < count) {
-          if (MODE == kRounds && --run == 0) {
-            t = round_tile(k + 1);
-            run = k + 1 < a.rounds * kTileRun ? kTileRun : 0x7fffffff;
-            nf_row = (long long)coords[2 * t]; nf_nz = (long long)coords[2 * t + 1];
+        if (withhold && (unsigned long long)(MODE == kRounds ? t : t_begin + k) + 1ull >= withhold) break;
+        long long nn_row = 0, nn_nz = 0;
+        [[maybe_unused]] long long nf_row = 0, nf_nz = 0;      // kRounds: front of the next tile
+        if constexpr (MODE == kRounds) {
+          nf_row = n_row; nf_nz = n_nz;
+          ++t;
+          if (k + 1 < count) {
+            if (--run == 0) {
+              t = round_tile(k + 1);
+              run = k + 1 < a.rounds * kTileRun ? kTileRun : 0x7fffffff;
+              nf_row = (long long)coords[2 * t]; nf_nz = (long long)coords[2 * t + 1];
+            }
+            nn_row = (long long)coords[2 * t + 2]; nn_nz = (long long)coords[2 * t + 3];
           }
-          nn_row = (long long)coords[2 * t + 2]; nn_nz = (long long)coords[2 * t + 3];
+        } else {
+          if (k + 1 < count) { nn_row = (long long)coords[2 * (t_begin + k + 2)]; nn_nz = (long long)coords[2 * (t_begin + k + 2) + 1]; }
         }
         const WinEnt n_we = (k + 1 < count) ? load_win_entry(t_begin + k + 1) : WinEnt{0, 0, 0};
         if (round > 0) {
@@ -491,7 +498,9 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
           if (!__all_sync(0xffffffffu, ok)) { pfail = true; break; }
         }
         issue(c_row, c_nz, n_row, n_nz, s, c_we);
-        c_row = nf_row; c_nz = nf_nz; n_row = nn_row; n_nz = nn_nz; c_we = n_we;
+        if constexpr (MODE == kRounds) { c_row = nf_row; c_nz = nf_nz; }
+        else { c_row = n_row; c_nz = n_nz; }
+        n_row = nn_row; n_nz = nn_nz; c_we = n_we;
         issued = k + 1;
         if (++s == nstages) { s = 0; ++round; }
       }
