@@ -41,8 +41,8 @@ _PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 _ROOT = os.path.dirname(_PKG)
 _TORCH_TYPE = {"float32": "torch::kFloat", "float64": "torch::kDouble", "int64": "torch::kLong"}
 
-KERNEL_HEADERS = ("flex_common.cuh", "flex_tensor.cuh", "flex_tile_kernel.cuh", "flex_warp_kernel.cuh", "flex_edge_kernel.cuh",
-                  "flex_graph_api.cuh", "flex_core.cu")
+KERNEL_HEADERS = ("flex_common.cuh", "flex_tensor.cuh", "flex_tile_kernel.cuh", "flex_warp_kernel.cuh", "flex_warp_ahead.cuh",
+                  "flex_edge_kernel.cuh", "flex_graph_api.cuh", "flex_core.cu")
 
 
 def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:

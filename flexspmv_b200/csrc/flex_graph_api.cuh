@@ -12,6 +12,7 @@
 #include "flex_common.cuh"
 #include "flex_edge_kernel.cuh"
 #include "flex_tile_kernel.cuh"
+#include "flex_warp_ahead.cuh"
 #include "flex_warp_kernel.cuh"
 
 namespace flex {
@@ -303,13 +304,17 @@ struct GraphApi {
     return launch_pdl(kernel, (unsigned)grid, kThreads, L::kTotal, st, p, a);
   }
 
-  template <typename OffsetT>
+  template <typename OffsetT, class C = CfgLean, bool SMALL = false>
   static int launch_lean(const flexspmv_desc* d, const typename G::Params& p, const void* row_offsets, void* ws,
                          const WorkspaceHeader& h, cudaStream_t st) {
     if constexpr (G::kHasReducer && kLeanBuilt) {
-      auto kernel = flex_warp_kernel<G, OffsetT, CfgLean>;
+      // few chunks a warp (16: 500 000 power-law rows have 14 in fp32, 17 in fp64): the other kernel, on fewer warps
+      using Small = WarpCfg<C::kBlock * (sizeof(V) == 4 ? 9 : 10) / 12, C::kIpt, C::kMinCtas>;
+      auto kernel = flex_warp_kernel<G, OffsetT, C>;
+      if constexpr (SMALL) kernel = flex_warp_ahead_kernel<G, OffsetT, C>;
+      else if (h.num_tiles < 16ll * device_sm_count() * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
       // per warp: the product slots and marker words of one chunk (WarpSmem, the layout of flex_warp_kernel)
-      constexpr int kSmem = WarpSmem<G, CfgLean>::template cta_bytes<OffsetT>();
+      constexpr int kSmem = WarpSmem<G, C>::template cta_bytes<OffsetT>();
       constexpr int kMaxDevices = 64;
       static std::mutex mu;
       static int resident_of[kMaxDevices] = {};      // 0: not initialised yet
@@ -322,7 +327,7 @@ struct GraphApi {
         if (resident_of[dev] == 0) {
           cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
           int r = 0;
-          if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kernel, CfgLean::kBlock, kSmem);
+          if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kernel, C::kBlock, kSmem);
           if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
           resident_of[dev] = r < 1 ? -1 : r;
         }
@@ -332,9 +337,9 @@ struct GraphApi {
       const long long chunks = h.num_tiles;
       if (chunks == 0) return 0;
       long long grid = d->max_ctas > 0 ? d->max_ctas : (long long)device_sm_count() * resident;
-      const long long need = (chunks + CfgLean::kWarps - 1) / CfgLean::kWarps;
+      const long long need = (chunks + C::kWarps - 1) / C::kWarps;
       if (grid > need) grid = need;
-      if (grid > kMaxWarpCarries / CfgLean::kWarps) grid = kMaxWarpCarries / CfgLean::kWarps;
+      if (grid > kMaxWarpCarries / C::kWarps) grid = kMaxWarpCarries / C::kWarps;
       if (grid < 1) grid = 1;
       WarpKernelArgs a;
       a.row_offsets = row_offsets;
@@ -343,7 +348,7 @@ struct GraphApi {
       a.carry_row = reinterpret_cast<long long*>(static_cast<char*>(ws) + h.carry_row_offset);
       a.carry_val = static_cast<char*>(ws) + h.carry_val_offset;
       a.num_rows = d->num_rows; a.num_edges = d->num_edges; a.num_chunks = chunks;
-      return launch_pdl(kernel, (unsigned)grid, CfgLean::kBlock, kSmem, st, p, a);
+      return launch_pdl(kernel, (unsigned)grid, C::kBlock, kSmem, st, p, a);
     } else {
       (void)d; (void)p; (void)row_offsets; (void)ws; (void)h; (void)st;
       return FLEXSPMV_ERR_BAD_ARG;

@@ -33,6 +33,7 @@ namespace flex {
 
 template <int BLOCK_, int IPT_, int MIN_CTAS_>
 struct WarpCfg {
+  static_assert(BLOCK_ % 32 == 0, "whole warps");
   static constexpr int kBlock = BLOCK_;
   static constexpr int kIpt = IPT_;
   static constexpr int kMinCtas = MIN_CTAS_;

@@ -1,5 +1,5 @@
 """Kernels picked by the size of a launch: the tile kernel without stages (few tiles a CTA) and with tiles going round the CTAs (large
-gathered vectors) against its plain form, bit for bit; the sort's 10-bit digits."""
+gathered vectors) against its plain form, bit for bit; the warp kernel's two configurations; the sort's 10-bit digits."""
 import ctypes
 
 import numpy as np
@@ -65,6 +65,32 @@ def test_rounds_equal_runs_of_consecutive_tiles(gname, dt, bits, ctas):
     plain, whole = launch(ir, long, dtype, long.num_cols, bits, max_ctas=ctas)
     rounds, _ = launch(ir, long, dtype, 1 << 27, bits, max_ctas=ctas)
     assert not whole and plain == rounds
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float64, 1e-12)])
+@pytest.mark.parametrize("rows", [100_003, 900_007])
+def test_warp_kernel_with_few_and_many_chunks_a_warp(dtype, tol, rows):
+    """1.6 M and 14 M random edges lie on either side of the small configuration's limit; rows of 0 to 300 edges.  Against sums in
+    64 bits, relative to the sums of the terms' magnitudes."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    ln = torch.randint(0, 32, (rows,), generator=g, device="cuda")
+    ln[::5000] = 300
+    ro = torch.zeros(rows + 1, dtype=torch.int64, device="cuda")
+    torch.cumsum(ln, 0, out=ro[1:])
+    e = int(ro[-1])
+    cols = torch.randint(0, rows, (e,), generator=g, device="cuda", dtype=torch.int32)
+    vals, x = (torch.rand(k, generator=g, device="cuda", dtype=dtype) - 0.5 for k in (e, rows))
+    ext = GraphExtension(graphs.spmv_graph(), random_gather=True)
+    (y,) = ext.merged_spmv_launch(vals, x, cols, ro.to(torch.int32), rows, rows)
+    ext.check()
+    of = torch.repeat_interleave(torch.arange(rows, device="cuda"), ln)
+    terms = vals.double() * x.double()[cols.long()]
+    zero = torch.zeros(rows, dtype=torch.float64, device="cuda")
+    err = (y.double() - zero.index_add(0, of, terms)).abs()
+    assert bool((err <= tol * zero.index_add(0, of, terms.abs())).all())
+    (again,) = ext.merged_spmv_launch(vals, x, cols, ro.to(torch.int32), rows, rows)
+    assert torch.equal(y, again)
 
 
 @pytest.mark.parametrize("rows", [257, 512, 1023, 1024, 1025, (1 << 18) + 3, (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
