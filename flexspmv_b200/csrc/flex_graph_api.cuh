@@ -304,12 +304,13 @@ struct GraphApi {
     return launch_pdl(kernel, (unsigned)grid, kThreads, L::kTotal, st, p, a);
   }
 
+  static constexpr int whole_warps(int threads) { return threads < 32 ? 32 : threads / 32 * 32; }
   template <typename OffsetT, class C = CfgLean, bool SMALL = false>
   static int launch_lean(const flexspmv_desc* d, const typename G::Params& p, const void* row_offsets, void* ws,
                          const WorkspaceHeader& h, cudaStream_t st) {
     if constexpr (G::kHasReducer && kLeanBuilt) {
       // few chunks a warp (16: 500 000 power-law rows have 14 in fp32, 17 in fp64): the other kernel, on fewer warps
-      using Small = WarpCfg<C::kBlock * (sizeof(V) == 4 ? 9 : 10) / 12, C::kIpt, C::kMinCtas>;
+      using Small = WarpCfg<whole_warps(C::kBlock * (sizeof(V) == 4 ? 9 : 10) / 12), C::kIpt, C::kMinCtas>;
       auto kernel = flex_warp_kernel<G, OffsetT, C>;
       if constexpr (SMALL) kernel = flex_warp_ahead_kernel<G, OffsetT, C>;
       else if (h.num_tiles < 16ll * device_sm_count() * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
@@ -340,6 +341,7 @@ struct GraphApi {
       const long long need = (chunks + C::kWarps - 1) / C::kWarps;
       if (grid > need) grid = need;
       if (grid > kMaxWarpCarries / C::kWarps) grid = kMaxWarpCarries / C::kWarps;
+      if (SMALL && grid > WarpSmem<G, C>::template carries<OffsetT>()) grid = WarpSmem<G, C>::template carries<OffsetT>();
       if (grid < 1) grid = 1;
       WarpKernelArgs a;
       a.row_offsets = row_offsets;

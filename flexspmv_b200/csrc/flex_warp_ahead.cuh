@@ -356,13 +356,12 @@ flex_warp_ahead_kernel(const typename G::Params p, const WarpKernelArgs a) {
   __syncthreads();
   if (s_last) {
     __threadfence();
-    // all carries into shared memory first (the warps' areas are free): a row that spans many CTAs is added up there, not
-    // one round trip through L2 after the other
+    // all carries into shared memory first (nothing else is in use any more; the launch has no more CTAs than fit): a row that
+    // spans many CTAs is added up there, not one round trip through L2 after the other
     const int n_carry = (int)gridDim.x;
     const V* cvals = static_cast<const V*>(a.carry_val);
     long long* s_row = reinterpret_cast<long long*>(smem_w);
     V* s_val = reinterpret_cast<V*>(s_row + n_carry);
-    static_assert((kMaxWarpCarries / Cfg::kWarps) * (8 + kAcc * int(sizeof(V))) <= Cfg::kWarps * kWarpBytes, "the carries of all CTAs fit");
     for (int c = tid; c < n_carry; c += Cfg::kBlock) {
       s_row[c] = __ldcg(a.carry_row + c);
 #pragma unroll

@@ -51,6 +51,11 @@ struct WarpSmem {
   static constexpr int cta_bytes() {
     return Cfg::kWarps * kBytes + kMaxRuns * int(sizeof(OffsetT) + G::kAccDim * sizeof(typename G::V));
   }
+  // CTAs whose carries (a row, kAccDim partial sums) fit there, where the last CTA of a launch brings them all together
+  template <typename OffsetT>
+  static constexpr int carries() {
+    return cta_bytes<OffsetT>() / int(8 + G::kAccDim * sizeof(typename G::V));
+  }
 };
 
 constexpr int kMaxWarpCarries = 16384;            // capacity of the per-warp carry arrays in the workspace
