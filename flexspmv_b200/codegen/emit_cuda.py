@@ -133,14 +133,21 @@ def choose_config(ir: GraphIR, dtype: str) -> Tuple[int, int, int, int]:
         for ipt in (5, 3):
             if smem_bytes(ir, dtype, block, ipt, stages) <= limit:
                 return block, ipt, stages, ctas
-    # records too wide for that: small CTAs rather than one edge a thread (72 bytes staged and 8 doubles summed an edge, 2 M edges in
-    # rows of 0 - 16, us: 256 x 1 x 2 CTAs 70.5, 64 x 3 x 4 57.3, 64 x 3 x 5 64.0; 0.24 M edges 19.3, 19.1)
-    if smem_bytes(ir, dtype, 64, 3, stages) <= (227 * 1024) // 4 - 1024:
-        return 64, 3, stages, 4
     ipt = 1
     while block > 64 and smem_bytes(ir, dtype, block, ipt, stages) > 110 * 1024:
         block //= 2
     return block, ipt, stages, 2
+
+
+def wide_config(ir: GraphIR, dtype: str, chosen: Tuple[int, int, int, int]) -> Tuple[int, int, int, int]:
+    """The same tile in CTAs of 64 threads, three an SM, where ``choose_config`` is down to 256 threads with one edge each: small CTAs
+    wait for one another less at their barriers.  72 bytes staged and 8 doubles summed an edge, rows of 0 - 16 edges, us, threads x
+    edges x CTAs an SM 256 x 1 x 2 / 128 x 2 x 3 / 64 x 4 x 3 / 64 x 3 x 4: 8 M edges 278 / 219 / 203 / 219, 4 M 143 / 114 / 106 / 113, 2 M
+    72.8 / 59.1 / 56.1 / 63.5, 0.8 M 30.4 / 26.0 / 25.7 / 26.1.  The tile keeps its 256 items: a caller may ask for tiles of that many."""
+    block, ipt, stages, _ = chosen
+    if (block, ipt) == (256, 1) and smem_bytes(ir, dtype, 64, 4, stages) <= (227 * 1024) // 3 - 1024:
+        return 64, 4, stages, 3
+    return chosen
 
 
 # Tile configurations measured on B200 for the built-in benchmark graphs (block, items per thread, stages,
@@ -239,7 +246,8 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     cty, sfx = CTYPE[dtype]
     symbol = symbol or f"{ir.name}_{sfx}"
     # measured configurations are keyed by graph and value type, whatever symbol prefix the unit is emitted under
-    cfg = tuple(config or _override(symbol) or TUNED_CONFIGS.get(symbol) or TUNED_CONFIGS.get(f"{ir.name}_{sfx}") or choose_config(ir, dtype))
+    cfg = tuple(config or _override(symbol) or TUNED_CONFIGS.get(symbol) or TUNED_CONFIGS.get(f"{ir.name}_{sfx}")
+                or wide_config(ir, dtype, choose_config(ir, dtype)))
     block, ipt, stages, min_ctas = cfg[:4]
     pipeline = len(cfg) > 4 and bool(cfg[4])     # fifth field: software-pipelined tiles (TileCfg::kPipeline)
     batch_override = cfg[5] if len(cfg) > 5 else 0   # sixth field: edges per register batch in the fused row mode

@@ -70,6 +70,23 @@ def test_tile_configs_fit_shared_memory():
             assert block % 32 == 0 and ipt % 2 == 1 and block * ipt <= 65535
             assert emit_cuda.smem_bytes(ir, dt, block, ipt, stages) * ctas <= 227 * 1024 + 1024 * ctas
 
+@pytest.mark.parametrize("dtype", ["float64", "int64"])
+def test_wide_records_keep_the_tile_a_caller_may_ask_for(dtype):
+    """Graphs of wide records: small CTAs that still take tiles of 256 items, as 256 threads of one edge did, and a byte of
+    workspace more is not asked for."""
+    import ctypes
+    from flexspmv_b200.binding import Desc, load_library
+    ir = graphs.mixed_dims_graph()
+    block, ipt, stages, ctas = emit_cuda.wide_config(ir, dtype, emit_cuda.choose_config(ir, dtype))
+    assert block * ipt == 256 and block == 64 and emit_cuda.smem_bytes(ir, dtype, block, ipt, stages) * ctas <= 227 * 1024 - 1024 * ctas
+    assert emit_cuda.wide_config(ir, "float32", emit_cuda.choose_config(ir, "float32")) == emit_cuda.choose_config(ir, "float32")
+    bytes_of = getattr(load_library(), f"flexspmv_mixed_dims_{emit_cuda.CTYPE[dtype][1]}_workspace_bytes")
+    n, default = ctypes.c_size_t(), ctypes.c_size_t()
+    for tile, code in ((193, 0), (256, 0), (257, -4)):
+        assert bytes_of(ctypes.byref(Desc(1000, 9000, 1000, 32, tile, 0, 0)), ctypes.byref(n)) == code, tile
+    assert bytes_of(ctypes.byref(Desc(1000, 9000, 1000, 32, 256, 0, 0)), ctypes.byref(n)) == 0
+    assert bytes_of(ctypes.byref(Desc(1000, 9000, 1000, 32, 0, 0, 0)), ctypes.byref(default)) == 0 and n.value == default.value
+
 
 def test_algorithmic_bytes_of_the_benchmark_configs():
     p0 = problems.poisson2d(512)
