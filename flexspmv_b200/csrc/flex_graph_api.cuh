@@ -311,9 +311,13 @@ struct GraphApi {
     if constexpr (G::kHasReducer && kLeanBuilt) {
       // few chunks a warp (16: 500 000 power-law rows have 14 in fp32, 17 in fp64): the other kernel, on fewer warps
       using Small = WarpCfg<whole_warps(C::kBlock * (sizeof(V) == 4 ? 9 : 10) / 12), C::kIpt, C::kMinCtas>;
-      auto kernel = flex_warp_kernel<G, OffsetT, C>;
-      if constexpr (SMALL) kernel = flex_warp_ahead_kernel<G, OffsetT, C>;
-      else if (h.num_tiles < 16ll * device_sm_count() * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
+      if constexpr (!SMALL) {
+        if (h.num_tiles < 16ll * device_sm_count() * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
+      }
+      const auto kernel = [] {          // (the other one is not compiled for this configuration)
+        if constexpr (SMALL) return &flex_warp_ahead_kernel<G, OffsetT, C>;
+        else return &flex_warp_kernel<G, OffsetT, C>;
+      }();
       // per warp: the product slots and marker words of one chunk (WarpSmem, the layout of flex_warp_kernel)
       constexpr int kSmem = WarpSmem<G, C>::template cta_bytes<OffsetT>();
       constexpr int kMaxDevices = 64;

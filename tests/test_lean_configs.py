@@ -26,3 +26,16 @@ def compile_unit(dtype, symbol, override, tmp_path, monkeypatch):
 def test_warp_kernel_overrides_compile(dtype, override, tmp_path, monkeypatch):
     code, log = compile_unit(dtype, override.split("_lean")[0], override, tmp_path, monkeypatch)
     assert code == 0, log[-2000:]
+
+
+def test_every_compiled_warp_kernel_is_launched():
+    """The library holds one warp kernel per graph, offset width and configuration: the plain form of the configuration that the
+    emitter gives, the form for few chunks a warp of the one that the launch derives from it."""
+    import re
+    from flexspmv_b200.binding import DEFAULT_LIB
+    symbols = subprocess.run(["nm", "-C", DEFAULT_LIB], check=True, capture_output=True, text=True).stdout
+    found = {m.groups() for m in re.finditer(r"flex::(flex_warp\w*kernel)<\(anonymous namespace\)::gen_(spmv_f(?:32|64))::Graph, ([a-z ]+), "
+                                             r"flex::WarpCfg<(\d+), 5, 1> ?>", symbols)}
+    want = {(kernel, graph, offsets, threads) for graph, large, small in (("spmv_f32", "1024", "768"), ("spmv_f64", "768", "640"))
+            for kernel, threads in (("flex_warp_kernel", large), ("flex_warp_ahead_kernel", small)) for offsets in ("int", "long long")}
+    assert found == want
