@@ -88,21 +88,268 @@ struct WarpKernelArgs {
   long long num_chunks;
 };
 
+// What the kernel below and the one for few chunks a warp (flex_warp_ahead.cuh) do alike with a chunk and with the carries; the
+// two differ in the order in which they ask for their records.
+template <class G, typename OffsetT, class Cfg>
+struct WarpParts {
+  using V = typename G::V;
+  static constexpr int kAcc = G::kAccDim, IPT = Cfg::kIpt, CH = Cfg::kChunk;
+  static_assert(CH <= 255, "row numbers inside a chunk are kept in marker bytes");
+  static_assert(IPT <= 8, "a lane's markers are read as one 8-byte word");
+
+  // Marks the last edge of every row that ends inside the chunk (x0: first row, y0: first edge, nr: rows that end; row_end: the end
+  // of row x0 + lane) and finishes the rows without edges here.
+  static __device__ __forceinline__ void mark_rows(const typename G::Params& p, const OffsetT* ro, OffsetT x0, OffsetT y0, int nr,
+                                                   OffsetT row_end, unsigned char* mk, int lane, V (&carry)[kAcc]) {
+    // end of row x0 + lane relative to the chunk's first edge (rows past the chunk: unused)
+    const OffsetT* ro0 = ro + x0 + 1;
+    int rel_end = 0;
+    if (lane < nr) rel_end = (int)(row_end - y0);
+    reinterpret_cast<uint2*>(mk)[lane] = make_uint2(0xffffffffu, 0xffffffffu);
+    __syncwarp();
+
+    // rows that end inside the chunk, one lane per row: the last edge of a row is marked with the row's number;
+    // a row without edges in this chunk is finished here (row x0 then takes the whole carry)
+    const bool seed_used = __any_sync(0xffffffffu, lane == 0 && nr > 0 && rel_end == 0);
+    int before = 0;                                      // where the row before this batch's first row ended
+    for (int r0 = 0; r0 < nr; r0 += 32) {
+      const int r = r0 + lane;
+      if (r0) {
+        before = __shfl_sync(0xffffffffu, rel_end, 31);
+        rel_end = 0;
+        if (r < nr) rel_end = (int)(ro0[r] - y0);
+      }
+      int prev = __shfl_up_sync(0xffffffffu, rel_end, 1);
+      if (lane == 0) prev = before;
+      if (r < nr) {
+        if (rel_end > prev) {
+          const int q = rel_end - 1, owner = q / IPT;
+          mk[owner * 8 + (q - owner * IPT)] = (unsigned char)r;
+        } else {
+          static_for<G::kNumReducers>([&](auto R) {
+            constexpr int d = G::template red_dim<R.value>();
+            constexpr int o = G::template red_off<R.value>();
+            V* dst = G::template red_out<R.value>(p) + (size_t)((long long)x0 + r) * d;
+#pragma unroll
+            for (int j = 0; j < d; ++j) dst[j] = (r == 0) ? carry[o + j] : V(0);
+          });
+        }
+      }
+    }
+    if (seed_used) {
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j) carry[j] = V(0);
+    }
+  }
+
+  static __device__ __forceinline__ void products(const typename G::Params& p, OffsetT y0, int ne, const typename G::EReg (&er)[IPT],
+                                                  const typename G::GEdge (&ge)[IPT], V* sp, int lane) {
+    // products into this warp's slots (lanes on consecutive edges; slots past the chunk's edges hold zero)
+    typename G::GRow gr;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+      V prod[kAcc];
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j) prod[j] = V(0);
+      if (i * 32 + lane < ne) G::map(p, er[i], (long long)y0 + (i * 32 + lane), gr, ge[i], prod);
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j) sp[j * CH + i * 32 + lane] = prod[j];
+    }
+    __syncwarp();
+  }
+
+  // Sums the chunk's products, stores the rows that end inside it and leaves what is open behind it in `carry`.
+  static __device__ __forceinline__ void close_rows(const typename G::Params& p, OffsetT x0, const V* sp, const unsigned char* mk, int lane,
+                                                    V (&carry)[kAcc]) {
+    // blocked pass: every lane sums IPT consecutive items and closes the rows that end inside its span
+    V run[kAcc], first[kAcc];
+#pragma unroll
+    for (int j = 0; j < kAcc; ++j) { run[j] = V(0); first[j] = V(0); }
+    int first_row = -1;
+    {
+      V pv[IPT][kAcc];
+      int pm[IPT];
+      const uint2 mw = reinterpret_cast<const uint2*>(mk)[lane];
+#pragma unroll
+      for (int i = 0; i < IPT; ++i) {
+        pm[i] = (int)(((i < 4 ? mw.x : mw.y) >> (8 * (i & 3))) & 0xffu);
+#pragma unroll
+        for (int j = 0; j < kAcc; ++j) pv[i][j] = sp[j * CH + lane * IPT + i];
+      }
+#pragma unroll
+      for (int i = 0; i < IPT; ++i) {
+#pragma unroll
+        for (int j = 0; j < kAcc; ++j) run[j] += pv[i][j];
+        if (pm[i] != 0xff) {
+          if (first_row < 0) {                         // may have begun in earlier lanes: finished after the scan
+            first_row = pm[i];
+#pragma unroll
+            for (int j = 0; j < kAcc; ++j) first[j] = run[j];
+          } else {
+            static_for<G::kNumReducers>([&](auto R) {
+              constexpr int d = G::template red_dim<R.value>();
+              constexpr int o = G::template red_off<R.value>();
+              V* dst = G::template red_out<R.value>(p) + (size_t)((long long)x0 + pm[i]) * d;
+#pragma unroll
+              for (int j = 0; j < d; ++j) dst[j] = run[o + j];
+            });
+          }
+#pragma unroll
+          for (int j = 0; j < kAcc; ++j) run[j] = V(0);
+        }
+      }
+    }
+    // segmented inclusive scan of the open partial sums: a lane that closed a row passes on only what follows it.
+    // Which lanes closed a row is one ballot; a lane takes a value from `d` lanes down only while that lane is not
+    // before the nearest closing lane at or below it (lane 0 when there is none).
+    const unsigned closed = __ballot_sync(0xffffffffu, first_row >= 0);
+    const unsigned closed_le = closed & (0xffffffffu >> (31 - lane));
+    const int reach = lane - (closed_le ? 31 - __clz(closed_le) : 0);      // lanes below this one in its segment
+    V scan[kAcc];
+#pragma unroll
+    for (int j = 0; j < kAcc; ++j) scan[j] = run[j];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j) {
+        const V v_up = shfl_up_any(scan[j], d);
+        if (reach >= d) scan[j] = v_up + scan[j];
+      }
+    }
+    // what the lanes before this one left open (plus the warp's carry when none of them closed a row)
+    const bool f_ex = (closed_le & ~(1u << lane)) != 0;
+    V in[kAcc];
+#pragma unroll
+    for (int j = 0; j < kAcc; ++j) {
+      V v_ex = shfl_up_any(scan[j], 1);
+      if (lane == 0) v_ex = V(0);
+      in[j] = f_ex ? v_ex : carry[j] + v_ex;
+    }
+    if (first_row >= 0) {
+      static_for<G::kNumReducers>([&](auto R) {
+        constexpr int d = G::template red_dim<R.value>();
+        constexpr int o = G::template red_off<R.value>();
+        V* dst = G::template red_out<R.value>(p) + (size_t)((long long)x0 + first_row) * d;
+#pragma unroll
+        for (int j = 0; j < d; ++j) dst[j] = in[o + j] + first[o + j];
+      });
+    }
+    // the warp's new carry: what is still open behind the last lane
+    {
+      const bool f31 = closed != 0;
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j) {
+        const V v31 = __shfl_sync(0xffffffffu, scan[j], 31);
+        carry[j] = f31 ? v31 : carry[j] + v31;
+      }
+    }
+  }
+
+  // Behind all runs of the CTA (smem_w: the warps' areas; s_run_row, s_run_val: what its n_runs runs left open).
+  template <bool TOGETHER>
+  static __device__ __forceinline__ void fold_carries(const typename G::Params& p, const WarpKernelArgs& a, unsigned char* smem_w, int n_runs,
+                                                      const OffsetT* s_run_row, const V* s_run_val) {
+    __shared__ int s_last;
+    const int tid = threadIdx.x;
+    // ---- the CTA folds the carries of its runs; what its last run left open goes to the last CTA -------------------
+    {
+      const long long tail_row = n_runs ? (long long)s_run_row[n_runs - 1] : a.num_rows;
+      for (int c = tid; c < n_runs; c += Cfg::kBlock) {
+        const long long row = (long long)s_run_row[c];
+        if (c > 0 && (long long)s_run_row[c - 1] == row) continue;     // not the first carry of its row
+        V sum[kAcc];
+#pragma unroll
+        for (int i = 0; i < kAcc; ++i) sum[i] = s_run_val[c * kAcc + i];
+        for (int c2 = c + 1; c2 < n_runs && (long long)s_run_row[c2] == row; ++c2) {
+#pragma unroll
+          for (int i = 0; i < kAcc; ++i) sum[i] += s_run_val[c2 * kAcc + i];
+        }
+        if (row == tail_row) {
+          // still open at the end of the range (or no row at all): another CTA may finish it, so it waits for all of them
+          V* cv = static_cast<V*>(a.carry_val) + (size_t)blockIdx.x * kAcc;
+#pragma unroll
+          for (int i = 0; i < kAcc; ++i) cv[i] = sum[i];
+        } else {
+          // finished by a later run of this CTA: every store to it is behind the barrier above
+          static_for<G::kNumReducers>([&](auto R) {
+            constexpr int d = G::template red_dim<R.value>();
+            constexpr int o = G::template red_off<R.value>();
+            V* dst = G::template red_out<R.value>(p) + (size_t)row * d;
+#pragma unroll
+            for (int i = 0; i < d; ++i) dst[i] = dst[i] + sum[o + i];
+          });
+        }
+      }
+      if (tid == 0) a.carry_row[blockIdx.x] = tail_row;
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned t = atomicAdd(&a.header->ticket, 1u);
+      s_last = (t == gridDim.x - 1) ? 1 : 0;
+    }
+    __syncthreads();
+    if (s_last) {
+      __threadfence();
+      // TOGETHER: all carries into shared memory first (nothing else is in use any more; the launch has no more CTAs than fit): a row
+      // that spans many CTAs is added up there, not one round trip through L2 after the other
+      const int n_carry = (int)gridDim.x;
+      const V* cvals = static_cast<const V*>(a.carry_val);
+      [[maybe_unused]] long long* const s_row = reinterpret_cast<long long*>(smem_w);
+      [[maybe_unused]] V* const s_val = reinterpret_cast<V*>(s_row + n_carry);
+      if constexpr (TOGETHER) {
+        for (int c = tid; c < n_carry; c += Cfg::kBlock) {
+          s_row[c] = __ldcg(a.carry_row + c);
+#pragma unroll
+          for (int i = 0; i < kAcc; ++i) s_val[(size_t)c * kAcc + i] = __ldcg(cvals + (size_t)c * kAcc + i);
+        }
+        __syncthreads();
+      }
+      auto row_of = [&](int c) -> long long {
+        if constexpr (TOGETHER) return s_row[c];
+        else return __ldcg(a.carry_row + c);
+      };
+      auto sum_of = [&](int c, int i) -> V {
+        if constexpr (TOGETHER) return s_val[(size_t)c * kAcc + i];
+        else return __ldcg(cvals + (size_t)c * kAcc + i);
+      };
+      for (int c = tid; c < n_carry; c += Cfg::kBlock) {
+        const long long row = row_of(c);
+        if (row >= a.num_rows) continue;
+        if (c > 0 && row_of(c - 1) == row) continue;   // not the head of its run
+        V sum[kAcc];
+#pragma unroll
+        for (int i = 0; i < kAcc; ++i) sum[i] = sum_of(c, i);
+        for (int c2 = c + 1; c2 < n_carry && row_of(c2) == row; ++c2) {
+#pragma unroll
+          for (int i = 0; i < kAcc; ++i) sum[i] += sum_of(c2, i);
+        }
+        static_for<G::kNumReducers>([&](auto R) {
+          constexpr int d = G::template red_dim<R.value>();
+          constexpr int o = G::template red_off<R.value>();
+          V* dst = G::template red_out<R.value>(p) + (size_t)row * d;
+#pragma unroll
+          for (int i = 0; i < d; ++i) dst[i] = __ldcg(dst + i) + sum[o + i];
+        });
+      }
+      if (tid == 0) a.header->ticket = 0;
+    }
+  }
+};
+
 template <class G, typename OffsetT, class Cfg>
 __global__ void __launch_bounds__(Cfg::kBlock, Cfg::kMinCtas)
 flex_warp_kernel(const typename G::Params p, const WarpKernelArgs a) {
   using V = typename G::V;
+  using W = WarpParts<G, OffsetT, Cfg>;
   constexpr int kAcc = G::kAccDim;
   constexpr int IPT = Cfg::kIpt, CH = Cfg::kChunk;
   static_assert(!G::kGatherNeedsRow, "the warp kernel takes graphs whose gathers all depend on the edge");
 
   extern __shared__ __align__(16) unsigned char smem_w[];
-  __shared__ int s_last;
   __shared__ unsigned long long s_next;
   constexpr int kMaxRuns = WarpSmem<G, Cfg>::kMaxRuns;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  static_assert(CH <= 255, "row numbers inside a chunk are kept in marker bytes");
-  static_assert(IPT <= 8, "a lane's markers are read as one 8-byte word");
   constexpr int kWarpBytes = WarpSmem<G, Cfg>::kBytes;
   unsigned char* wbase = smem_w + (size_t)warp * kWarpBytes;
   V* sp = reinterpret_cast<V*>(wbase);                                   // this warp's product slots, [kAcc][CH]
@@ -212,141 +459,9 @@ flex_warp_kernel(const typename G::Params p, const WarpKernelArgs a) {
       OffsetT row_end_next = 0;
       if (k + 1 < count && lane < (int)(x2 - x1)) row_end_next = ro[(long long)x1 + 1 + lane];
 
-      // end of row x0 + lane relative to the chunk's first edge (rows past the chunk: unused)
-      const OffsetT* ro0 = ro + x0 + 1;
-      int rel_end = 0;
-      if (lane < nr) rel_end = (int)(row_end - y0);
-      reinterpret_cast<uint2*>(mk)[lane] = make_uint2(0xffffffffu, 0xffffffffu);
-      __syncwarp();
-
-      // rows that end inside the chunk, one lane per row: the last edge of a row is marked with the row's number;
-      // a row without edges in this chunk is finished here (row x0 then takes the whole carry)
-      const bool seed_used = __any_sync(0xffffffffu, lane == 0 && nr > 0 && rel_end == 0);
-      int before = 0;                                      // where the row before this batch's first row ended
-      for (int r0 = 0; r0 < nr; r0 += 32) {
-        const int r = r0 + lane;
-        if (r0) {
-          before = __shfl_sync(0xffffffffu, rel_end, 31);
-          rel_end = 0;
-          if (r < nr) rel_end = (int)(ro0[r] - y0);
-        }
-        int prev = __shfl_up_sync(0xffffffffu, rel_end, 1);
-        if (lane == 0) prev = before;
-        if (r < nr) {
-          if (rel_end > prev) {
-            const int q = rel_end - 1, owner = q / IPT;
-            mk[owner * 8 + (q - owner * IPT)] = (unsigned char)r;
-          } else {
-            static_for<G::kNumReducers>([&](auto R) {
-              constexpr int d = G::template red_dim<R.value>();
-              constexpr int o = G::template red_off<R.value>();
-              V* dst = G::template red_out<R.value>(p) + (size_t)((long long)x0 + r) * d;
-#pragma unroll
-              for (int j = 0; j < d; ++j) dst[j] = (r == 0) ? carry[o + j] : V(0);
-            });
-          }
-        }
-      }
-      if (seed_used) {
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) carry[j] = V(0);
-      }
-
-      // products into this warp's slots (lanes on consecutive edges; slots past the chunk's edges hold zero)
-      typename G::GRow gr;
-#pragma unroll
-      for (int i = 0; i < IPT; ++i) {
-        V prod[kAcc];
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) prod[j] = V(0);
-        if (i * 32 + lane < ne) G::map(p, er[i], (long long)y0 + (i * 32 + lane), gr, ge[i], prod);
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) sp[j * CH + i * 32 + lane] = prod[j];
-      }
-      __syncwarp();
-
-      // blocked pass: every lane sums IPT consecutive items and closes the rows that end inside its span
-      V run[kAcc], first[kAcc];
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j) { run[j] = V(0); first[j] = V(0); }
-      int first_row = -1;
-      {
-        V pv[IPT][kAcc];
-        int pm[IPT];
-        const uint2 mw = reinterpret_cast<const uint2*>(mk)[lane];
-#pragma unroll
-        for (int i = 0; i < IPT; ++i) {
-          pm[i] = (int)(((i < 4 ? mw.x : mw.y) >> (8 * (i & 3))) & 0xffu);
-#pragma unroll
-          for (int j = 0; j < kAcc; ++j) pv[i][j] = sp[j * CH + lane * IPT + i];
-        }
-#pragma unroll
-        for (int i = 0; i < IPT; ++i) {
-#pragma unroll
-          for (int j = 0; j < kAcc; ++j) run[j] += pv[i][j];
-          if (pm[i] != 0xff) {
-            if (first_row < 0) {                         // may have begun in earlier lanes: finished after the scan
-              first_row = pm[i];
-#pragma unroll
-              for (int j = 0; j < kAcc; ++j) first[j] = run[j];
-            } else {
-              static_for<G::kNumReducers>([&](auto R) {
-                constexpr int d = G::template red_dim<R.value>();
-                constexpr int o = G::template red_off<R.value>();
-                V* dst = G::template red_out<R.value>(p) + (size_t)((long long)x0 + pm[i]) * d;
-#pragma unroll
-                for (int j = 0; j < d; ++j) dst[j] = run[o + j];
-              });
-            }
-#pragma unroll
-            for (int j = 0; j < kAcc; ++j) run[j] = V(0);
-          }
-        }
-      }
-      // segmented inclusive scan of the open partial sums: a lane that closed a row passes on only what follows it.
-      // Which lanes closed a row is one ballot; a lane takes a value from `d` lanes down only while that lane is not
-      // before the nearest closing lane at or below it (lane 0 when there is none).
-      const unsigned closed = __ballot_sync(0xffffffffu, first_row >= 0);
-      const unsigned closed_le = closed & (0xffffffffu >> (31 - lane));
-      const int reach = lane - (closed_le ? 31 - __clz(closed_le) : 0);      // lanes below this one in its segment
-      V scan[kAcc];
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j) scan[j] = run[j];
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) {
-          const V v_up = shfl_up_any(scan[j], d);
-          if (reach >= d) scan[j] = v_up + scan[j];
-        }
-      }
-      // what the lanes before this one left open (plus the warp's carry when none of them closed a row)
-      const bool f_ex = (closed_le & ~(1u << lane)) != 0;
-      V in[kAcc];
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j) {
-        V v_ex = shfl_up_any(scan[j], 1);
-        if (lane == 0) v_ex = V(0);
-        in[j] = f_ex ? v_ex : carry[j] + v_ex;
-      }
-      if (first_row >= 0) {
-        static_for<G::kNumReducers>([&](auto R) {
-          constexpr int d = G::template red_dim<R.value>();
-          constexpr int o = G::template red_off<R.value>();
-          V* dst = G::template red_out<R.value>(p) + (size_t)((long long)x0 + first_row) * d;
-#pragma unroll
-          for (int j = 0; j < d; ++j) dst[j] = in[o + j] + first[o + j];
-        });
-      }
-      // the warp's new carry: what is still open behind the last lane
-      {
-        const bool f31 = closed != 0;
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) {
-          const V v31 = __shfl_sync(0xffffffffu, scan[j], 31);
-          carry[j] = f31 ? v31 : carry[j] + v31;
-        }
-      }
+      W::mark_rows(p, ro, x0, y0, nr, row_end, mk, lane, carry);
+      W::products(p, y0, ne, er, ge, sp, lane);
+      W::close_rows(p, x0, sp, mk, lane, carry);
       end_row = x1;
       __syncwarp();                                      // the slots are rewritten by the next chunk
 #pragma unroll
@@ -363,71 +478,8 @@ flex_warp_kernel(const typename G::Params p, const WarpKernelArgs a) {
     }
   }  // runs of this warp
 
-  // ---- the CTA folds the carries of its runs; what its last run left open goes to the last CTA -------------------
   __syncthreads();
-  {
-    const int n_runs = (int)(s_next >> 32);
-    const long long tail_row = n_runs ? (long long)s_run_row[n_runs - 1] : a.num_rows;
-    for (int c = tid; c < n_runs; c += Cfg::kBlock) {
-      const long long row = (long long)s_run_row[c];
-      if (c > 0 && (long long)s_run_row[c - 1] == row) continue;     // not the first carry of its row
-      V sum[kAcc];
-#pragma unroll
-      for (int i = 0; i < kAcc; ++i) sum[i] = s_run_val[c * kAcc + i];
-      for (int c2 = c + 1; c2 < n_runs && (long long)s_run_row[c2] == row; ++c2) {
-#pragma unroll
-        for (int i = 0; i < kAcc; ++i) sum[i] += s_run_val[c2 * kAcc + i];
-      }
-      if (row == tail_row) {
-        // still open at the end of the range (or no row at all): another CTA may finish it, so it waits for all of them
-        V* cv = static_cast<V*>(a.carry_val) + (size_t)blockIdx.x * kAcc;
-#pragma unroll
-        for (int i = 0; i < kAcc; ++i) cv[i] = sum[i];
-      } else {
-        // finished by a later run of this CTA: every store to it is behind the barrier above
-        static_for<G::kNumReducers>([&](auto R) {
-          constexpr int d = G::template red_dim<R.value>();
-          constexpr int o = G::template red_off<R.value>();
-          V* dst = G::template red_out<R.value>(p) + (size_t)row * d;
-#pragma unroll
-          for (int i = 0; i < d; ++i) dst[i] = dst[i] + sum[o + i];
-        });
-      }
-    }
-    if (tid == 0) a.carry_row[blockIdx.x] = tail_row;
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const unsigned t = atomicAdd(&a.header->ticket, 1u);
-    s_last = (t == gridDim.x - 1) ? 1 : 0;
-  }
-  __syncthreads();
-  if (s_last) {
-    __threadfence();
-    const int n_carry = (int)gridDim.x;
-    const V* cvals = static_cast<const V*>(a.carry_val);
-    for (int c = tid; c < n_carry; c += Cfg::kBlock) {
-      const long long row = __ldcg(a.carry_row + c);
-      if (row >= a.num_rows) continue;
-      if (c > 0 && __ldcg(a.carry_row + c - 1) == row) continue;   // not the head of its run
-      V sum[kAcc];
-#pragma unroll
-      for (int i = 0; i < kAcc; ++i) sum[i] = __ldcg(cvals + (size_t)c * kAcc + i);
-      for (int c2 = c + 1; c2 < n_carry && __ldcg(a.carry_row + c2) == row; ++c2) {
-#pragma unroll
-        for (int i = 0; i < kAcc; ++i) sum[i] += __ldcg(cvals + (size_t)c2 * kAcc + i);
-      }
-      static_for<G::kNumReducers>([&](auto R) {
-        constexpr int d = G::template red_dim<R.value>();
-        constexpr int o = G::template red_off<R.value>();
-        V* dst = G::template red_out<R.value>(p) + (size_t)row * d;
-#pragma unroll
-        for (int i = 0; i < d; ++i) dst[i] = __ldcg(dst + i) + sum[o + i];
-      });
-    }
-    if (tid == 0) a.header->ticket = 0;
-  }
+  W::template fold_carries<false>(p, a, smem_w, (int)(s_next >> 32), s_run_row, s_run_val);
 }
 
 }  // namespace flex
