@@ -17,6 +17,8 @@
 
 namespace flex {
 
+int device_sm_count();      // flex_core.cu
+
 constexpr int kSortKeysPerThread = 16;
 // One width of digit: bins, threads of a CTA, and with 16 keys a thread the tile.  A pass with 1024 bins has tiles of 8192
 // keys, so that a digit's keys in a tile still leave in runs of 8 and more.
@@ -261,44 +263,58 @@ __device__ __forceinline__ long long warp_lower_bound(const unsigned* __restrict
   }
   return lo;
 }
-// CSR offsets of sorted ids: offsets[r] = number of ids < r.  A block owns kOffsetRows consecutive rows: two warps find the
+// CSR offsets of sorted ids: offsets[r] = number of ids < r.  A block owns ROWS consecutive rows: two warps find the
 // run of ids of those rows (five rounds of 32 probes for 33 M ids).  Where the run is not much longer than the rows are many,
 // it is read once, side by side: a place whose id differs from the one before it is where that row begins, and a row without
-// ids begins where the next one does (a minimum from behind).  A longer run (few rows hold most edges) is bisected per row, as
-// every run was (1 M rows, 8.4 M ids: 28.6 us).
-constexpr int kOffsetRows = 1024, kOffsetThreads = 256;
-template <typename OffsetT>
+// ids begins where the next one does (a minimum from behind).  A longer run (few rows hold most edges) is bisected per row.
+// Bound by round trips unless the rows are many.  The kernel alone, us, bisected in blocks of 256 rows / read once in blocks of 256 /
+// of 1024:  8 ids a row, 10 007 rows 6.3 / 6.2 / 6.2, 100 003 6.3 / 6.2 / 7.3, 400 009 10.3 / 10.3 / 8.3, 1 M 19.5 / 16.5 / 12.4, 8 M rows
+// of one id 95 / 84 / 39;  24 ids a row, 100 003 rows 7.3 / 7.2 / 10.8, 400 009 12.5 / 12.4 / 12.4;  48 ids, 100 003 rows 8.3 / 8.3 / 16.5,
+// 400 009 16.6 / 18.6 / 18.5;  100 ids, 10 007 rows 6.3 / 10.3 / 28.  So: read once up to 24 ids a row, and blocks of 1024 rows where
+// they are two an SM and more.
+constexpr int kOffsetThreads = 256, kOffsetIdsARow = 24;
+template <typename OffsetT, int ROWS>
 __global__ void __launch_bounds__(kOffsetThreads) sorted_offsets_kernel(const unsigned* __restrict__ keys, long long n, long long num_rows,
                                                                         OffsetT* __restrict__ offsets) {
-  constexpr int kPer = kOffsetRows / kOffsetThreads;
+  constexpr int kPer = ROWS / kOffsetThreads;
   __shared__ long long s_run[2];
-  __shared__ unsigned s_begin[kOffsetRows];
+  __shared__ unsigned s_begin[ROWS];
   __shared__ unsigned s_warp[kOffsetThreads / 32];
-  const long long r0 = (long long)blockIdx.x * kOffsetRows;
+  const long long r0 = (long long)blockIdx.x * ROWS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (warp < 2) {
-    const long long at = warp_lower_bound(keys, n, r0 + kOffsetRows * warp);
+    const long long at = warp_lower_bound(keys, n, r0 + ROWS * warp);
     if (lane == 0) s_run[warp] = at;
   }
-  for (int i = tid; i < kOffsetRows; i += kOffsetThreads) s_begin[i] = 0xffffffffu;
+  for (int i = tid; i < ROWS; i += kOffsetThreads) s_begin[i] = 0xffffffffu;
   __syncthreads();
   const long long lo = s_run[0], hi = s_run[1];
-  if (hi - lo > 64 * kOffsetRows) {
-    for (int i = tid; i < kOffsetRows; i += kOffsetThreads) {
-      const long long r = r0 + i;
-      if (r > num_rows) break;
-      long long from = lo, to = hi;
-      while (from < to) {
-        const long long mid = (from + to) >> 1;
-        if ((long long)keys[mid] < r) from = mid + 1; else to = mid;
-      }
-      offsets[r] = (OffsetT)from;
+  if (hi - lo > kOffsetIdsARow * ROWS) {
+    // the thread's rows at once: one round trip a halving, whatever their number
+    long long from[kPer], to[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) { from[j] = lo; to[j] = hi; }
+    for (bool more = true; more;) {
+      more = false;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        if (from[j] < to[j]) {
+          const long long mid = (from[j] + to[j]) >> 1;
+          if ((long long)keys[mid] < r0 + j * kOffsetThreads + tid) from[j] = mid + 1; else to[j] = mid;
+          more = true;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const long long r = r0 + j * kOffsetThreads + tid;
+      if (r <= num_rows) offsets[r] = (OffsetT)from[j];
     }
     return;
   }
+#pragma unroll 4
   for (long long e = lo + tid; e < hi; e += kOffsetThreads) {
     const unsigned id = keys[e], row = id - (unsigned)r0;
-    if ((e == lo || keys[e - 1] != id) && row < (unsigned)kOffsetRows) s_begin[row] = (unsigned)e;    // (ids out of range are not in order)
+    if ((e == lo || keys[e - 1] != id) && row < (unsigned)ROWS) s_begin[row] = (unsigned)e;    // (ids out of range are not in order)
   }
   __syncthreads();
   // a row without ids: the smallest beginning behind it, or the run's end
@@ -326,6 +342,12 @@ __global__ void __launch_bounds__(kOffsetThreads) sorted_offsets_kernel(const un
     const long long r = r0 + tid * kPer + j;
     if (r <= num_rows) offsets[r] = (OffsetT)next;
   }
+}
+
+template <typename OffsetT, int ROWS>
+static int sorted_offsets(const unsigned* keys, long long n, long long num_rows, void* offsets, cudaStream_t st) {
+  sorted_offsets_kernel<OffsetT, ROWS><<<(unsigned)(num_rows / ROWS + 1), kOffsetThreads, 0, st>>>(keys, n, num_rows, static_cast<OffsetT*>(offsets));
+  return (int)cudaGetLastError();                          // (the blocks cover offsets[0 .. num_rows])
 }
 
 // dst[e] = src[perm[e]] for records of one machine word, read and written whole (T: the vector type of that width)
@@ -463,12 +485,10 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
     }
   }
   if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return (int)e;
-  const unsigned g = (unsigned)(num_rows / flex::kOffsetRows + 1);       // offsets[0 .. num_rows]
+  const bool many = num_rows >= 2048ll * flex::device_sm_count() && num_edges <= flex::kOffsetIdsARow * num_rows;
   if (offset_bits == 32)
-    flex::sorted_offsets_kernel<int><<<g, flex::kOffsetThreads, 0, st>>>(keys[cur], num_edges, num_rows, static_cast<int*>(d_row_offsets));
-  else
-    flex::sorted_offsets_kernel<long long><<<g, flex::kOffsetThreads, 0, st>>>(keys[cur], num_edges, num_rows, static_cast<long long*>(d_row_offsets));
-  return (int)cudaGetLastError();
+    return (many ? flex::sorted_offsets<int, 1024> : flex::sorted_offsets<int, 256>)(keys[cur], num_edges, num_rows, d_row_offsets, st);
+  return (many ? flex::sorted_offsets<long long, 1024> : flex::sorted_offsets<long long, 256>)(keys[cur], num_edges, num_rows, d_row_offsets, st);
 }
 
 int flexspmv_permute_edges(const void* d_src, void* d_dst, const int32_t* d_perm, int64_t num_edges, int32_t record_bytes,

@@ -136,3 +136,37 @@ def test_scratch_for_eight_bit_digits_is_enough():
             assert code == -3
         else:
             assert code == 0 and np.array_equal(perm.cpu().numpy(), np.argsort(ids, kind="stable").astype(np.int32))
+
+
+@pytest.mark.parametrize("rows", [1, 255, 256, 257, 1025, 300_000, 303_104, 303_105, 400_001])
+@pytest.mark.parametrize("ids", ["few", "limit", "above", "skewed"])
+@pytest.mark.parametrize("offset_bits", [32, 64])
+def test_offsets_read_once_or_bisected(rows, ids, offset_bits):
+    """Blocks of 256 and of 1024 rows (from two an SM on), at 24 ids a row (read once), one more in a block (bisected) and where
+    one block holds most ids; rows without ids at both ends."""
+    rng = np.random.default_rng(rows)
+    if ids == "few":
+        counts = rng.integers(0, 3, rows)
+    elif ids == "skewed":
+        counts = rng.integers(0, 4, rows)
+        counts[rows // 2:rows // 2 + 300] = 2000
+    else:
+        counts = np.full(rows, 24)
+        if ids == "above":
+            counts[rows // 3] = 25
+    if rows > 2:
+        counts[0] = counts[-1] = 0
+    of = np.repeat(np.arange(rows), counts)
+    n = of.size
+    lib = load_library()
+    need = ctypes.c_size_t()
+    assert lib.flexspmv_sort_rows_bytes(ctypes.c_int64(n), ctypes.byref(need)) == 0
+    shuffled = torch.from_numpy(of)[torch.randperm(n, generator=torch.Generator().manual_seed(rows))].cuda()
+    perm, scratch = torch.empty(max(n, 1), dtype=torch.int32, device="cuda"), torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    got = torch.full((rows + 2,), -1, dtype=torch.int32 if offset_bits == 32 else torch.int64, device="cuda")
+    status = torch.empty(1, dtype=torch.int32, device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert lib.flexspmv_sort_rows(ptr(shuffled), 64, ctypes.c_int64(n), ctypes.c_int64(rows), ptr(perm), ptr(got), offset_bits, ptr(scratch),
+                                  ctypes.c_size_t(need.value), ptr(status), None) == 0
+    want = np.concatenate([[0], np.cumsum(counts), [-1]])                  # (the word behind the last offset stays)
+    assert np.array_equal(got.cpu().numpy(), want) and int(status) == 0
