@@ -25,6 +25,9 @@ int device_sm_count() {
 // Kernels that planning has enqueued from this thread (flexspmv_plan_launches).
 static thread_local long long plan_launches = 0;
 
+static thread_local int last_kernel = FLEXSPMV_KERNEL_NONE;
+void note_kernel(int which) { last_kernel = which; }
+
 // One thread per tile boundary: coordinate of diagonal t * tile_items (clamped to rows + edges).  A plan's header goes along
 // (null: coordinates alone): a launch less in the first call on a matrix.
 template <typename OffsetT>
@@ -682,6 +685,8 @@ int flexspmv_debug_withhold_stage(void* d_workspace, uint32_t first_tile_plus_on
                                                                                first_tile_plus_one);
   return (int)cudaGetLastError();
 }
+
+int flexspmv_debug_last_kernel(void) { return flex::last_kernel; }
 
 int flexspmv_workspace_status_mirror(void* d_workspace, int32_t* pinned_host_status, void* stream) {
   if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;

@@ -21,6 +21,7 @@ namespace flex {
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,
                      int tile_items, void* d_coords, cudaStream_t stream, void* ws, const WorkspaceHeader* h);
 int device_sm_count();
+void note_kernel(int which);      // FLEXSPMV_KERNEL_*, for flexspmv_debug_last_kernel
 int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream);
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
@@ -272,6 +273,7 @@ struct GraphApi {
     int resident = 0;
     if (int e = resident_ctas<OffsetT, C, WIN>(&resident)) return e;
     const long long tiles = h.num_tiles;
+    note_kernel(FLEXSPMV_KERNEL_NONE);
     if (tiles == 0) return 0;
     long long grid = max_ctas(d, resident);
     if (grid > tiles) grid = tiles;
@@ -290,17 +292,21 @@ struct GraphApi {
       a.win_table = reinterpret_cast<const int*>(static_cast<char*>(ws) + h.win_table_offset);
       a.win_index = reinterpret_cast<const unsigned short*>(static_cast<char*>(ws) + h.win_index_offset);
     }
+    int form = FLEXSPMV_KERNEL_TILE;
     if constexpr (L::kWhole) {
       const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
       if (4 * tiles <= kSmallQuarters * grid) {
+        form = FLEXSPMV_KERNEL_TILE_SMALL;
         kernel = flex_tile_kernel<G, OffsetT, C, WIN, kSmall>;
         if (int e = resident_ctas<OffsetT, C, WIN, kSmall>(&resident)) return e;      // the grid stays the plan's
       } else if (vertices * G::kGatherRecordBytes > kKeepBytes && tiles >= grid * kTileRun) {
         a.rounds = (int)(tiles / (grid * kTileRun));
+        form = FLEXSPMV_KERNEL_TILE_ROUNDS;
         kernel = flex_tile_kernel<G, OffsetT, C, WIN, kRounds>;
         if (int e = resident_ctas<OffsetT, C, WIN, kRounds>(&resident)) return e;
       }
     }
+    note_kernel(form);
     return launch_pdl(kernel, (unsigned)grid, kThreads, L::kTotal, st, p, a);
   }
 
@@ -340,6 +346,7 @@ struct GraphApi {
       }
       if (resident < 1) return FLEXSPMV_ERR_TOO_LARGE;
       const long long chunks = h.num_tiles;
+      note_kernel(FLEXSPMV_KERNEL_NONE);
       if (chunks == 0) return 0;
       long long grid = d->max_ctas > 0 ? d->max_ctas : (long long)device_sm_count() * resident;
       const long long need = (chunks + C::kWarps - 1) / C::kWarps;
@@ -354,6 +361,7 @@ struct GraphApi {
       a.carry_row = reinterpret_cast<long long*>(static_cast<char*>(ws) + h.carry_row_offset);
       a.carry_val = static_cast<char*>(ws) + h.carry_val_offset;
       a.num_rows = d->num_rows; a.num_edges = d->num_edges; a.num_chunks = chunks;
+      note_kernel(SMALL ? FLEXSPMV_KERNEL_WARP_AHEAD : FLEXSPMV_KERNEL_WARP);
       return launch_pdl(kernel, (unsigned)grid, C::kBlock, kSmem, st, p, a);
     } else {
       (void)d; (void)p; (void)row_offsets; (void)ws; (void)h; (void)st;
@@ -412,7 +420,9 @@ struct GraphApi {
       if (d->offset_bits == 64) return launch_tiles<long long>(d, p, row_offsets, ws, h, st);
       return launch_tiles<int>(d, p, row_offsets, ws, h, st);
     } else {
+    note_kernel(FLEXSPMV_KERNEL_NONE);
     if (d->num_edges == 0 && G::kAggDim == 0) return 0;
+    note_kernel(FLEXSPMV_KERNEL_EDGE);
     const long long tile_edges = (long long)kEdgeBlock * kEdgeIpt;
     long long grid = (d->num_edges + tile_edges - 1) / tile_edges;
     const long long cap = max_ctas(d, 2048 / kEdgeBlock);

@@ -126,6 +126,18 @@ int flexspmv_row_blocks(const void *d_row_offsets, int32_t offset_bits, int64_t 
  */
 int flexspmv_debug_withhold_stage(void *d_workspace, uint32_t first_tile_plus_one, void *stream);
 
+/* Testing aid: the kernel that the calling thread's last *_launch enqueued.  No reference counterpart. */
+enum {
+  FLEXSPMV_KERNEL_NONE = 0,        /* no launch yet, or nothing to do */
+  FLEXSPMV_KERNEL_TILE = 1,        /* tile kernel, its plain form */
+  FLEXSPMV_KERNEL_TILE_SMALL = 2,  /* ... where whole rows are read straight from global memory */
+  FLEXSPMV_KERNEL_TILE_ROUNDS = 3, /* ... where tiles of whole rows go round the CTAs */
+  FLEXSPMV_KERNEL_WARP = 4,        /* warp kernel for columns without locality */
+  FLEXSPMV_KERNEL_WARP_AHEAD = 5,  /* ... for few chunks a warp */
+  FLEXSPMV_KERNEL_EDGE = 6         /* graphs without a reducer */
+};
+int flexspmv_debug_last_kernel(void);
+
 /*
  * Measurement aid: the rate at which the GPU gathers 4-byte records without locality.  Streams d_idx / d_vals
  * (num_edges entries, coalesced), gathers d_x[d_idx[e]] and accumulates; writes nothing (d_out needs `ctas` floats
