@@ -59,6 +59,10 @@ struct WorkspaceHeader {
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
 
+// Rows that each CTA of a small launch takes (flex_tile_kernel.cuh): whole warps of them.
+__host__ __device__ constexpr long long rows_a_cta(long long num_rows, long long grid) { return ((num_rows + grid - 1) / grid + 31) & ~31ll; }
+constexpr int kSmallTiles = 3;            // tiles a CTA that a small launch has at most
+
 #ifndef FLEX_WHOLE_ROW_MAX
 #define FLEX_WHOLE_ROW_MAX 32
 #endif

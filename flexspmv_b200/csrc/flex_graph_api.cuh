@@ -224,11 +224,30 @@ struct GraphApi {
     }
   }
 
-  // A launch of at most kSmallQuarters / 4 tiles a CTA is a few round trips long and takes the kernel without stages.  us, with
-  // stages / without: 5-point fp64, tiles a CTA 1.1 5.74 / 4.2, 2.1 7.13 / 5.63, 2.9 8.84 / 8.08, 3.9 10.14 / 10.46; 7-point 2.3 7.49 /
-  // 6.10, 5.4 11.98 / 14.2.  Row-mode graphs: spring-mass fp32 0.7 7.40 / 6.82, 1.9 11.4 / 11.4; Rusanov fp64 0.7 6.84 / 5.8, 1.6
-  // 11.2 / 9.9, 2.8 15.7 / 16.7; a shallow-water step (four launches) 0.2 30.7 / 24.6, 2.1 69.2 / 56.9, 5.9 124 / 129.
-  static constexpr long long kSmallQuarters = G::kGatherNeedsRow ? 9 : 12;
+  // Whether a launch takes the kernel without stages (kSmall): it is a few round trips long -- a row's ends, then its records and its
+  // gathers for every kRowBatch edges -- where stages take a tile's in one copy each, behind coordinates, copies and barriers.  That
+  // pays while the rows are short and the tiles few; and lanes that read rows a row length apart touch more lines an edge the longer
+  // the rows are.  us, with stages / without, where lines below are drawn:
+  //   tiles a CTA   5-point fp64 1.1 5.74 / 4.2, 2.1 7.13 / 5.63, 2.9 8.84 / 8.08, 3.9 10.14 / 10.46; 7-point 2.3 7.49 / 6.10, 5.4 11.98 / 14.2.
+  //                 Row-mode graphs: spring-mass fp32 0.7 7.40 / 6.82, 1.9 11.4 / 11.4; Rusanov fp64 0.7 6.84 / 5.8, 1.6 11.2 / 9.9, 2.8 15.7 / 16.7
+  //   edges a row   SpMV, 1 tile a CTA: fp32 12 4.2 / 3.8, 15 4.2 / 3.9, 16 5.3 / 5.6 (such rows begin in two banks: the plan takes the other
+  //                 loop), 27 4.8 / 5.1; fp64 10 4.5 / 4.0, 12 4.8 / 4.7, 13 4.6 / 4.4, 15 4.7 / 4.8, 18 4.9 / 5.7, 27 5.3 / 6.3.  At 2.9: fp64 12 9.6 / 7.9,
+  //                 13 9.0 / 9.2, 27 9.2 / 13.9.  Row-mode, 0.6 M items: spring-mass fp32 10 6.2 / 5.8, 14 7.4 / 7.2, 16 9.9 / 10.3; fp64 8 8.7 / 8.2,
+  //                 12 10.8 / 11.0, 16 12.8 / 14.8; Rusanov fp32 6 6.7 / 6.7, 8 7.3 / 8.8, 16 9.8 / 15.8; fp64 4 11.3 / 7.4, 6 (0.15 M) 5.8 / 6.3;
+  //                 swe_delta fp32 6 6.4 / 6.4, 8 7.1 / 8.2
+  //   rows a CTA    (several a thread, one after the other) SpMV fp64 800 7.8 / 6.6, 896 7.8 / 8.4, 1408 of one edge 8.1 / 8.9; fp32 1600 8.2 / 7.3,
+  //                 1792 8.2 / 8.2, 1914 8.3 / 10.8
+  static constexpr long long kSmallQuarters = G::kGatherNeedsRow ? 9 : 4 * kSmallTiles;
+  static constexpr int least(int a, int b) { return a < b ? a : b; }
+  static constexpr int within(int bytes_a_row) { return G::kStreamBytesPerEdge > 0 ? bytes_a_row / G::kStreamBytesPerEdge : bytes_a_row; }
+  static constexpr int kSmallRowEdges = G::kGatherNeedsRow ? least(G::kValuesStaged ? 6 : 10, within(112))
+                                                           : least(G::kLightMap ? 15 : 7, within(144));
+  static bool small_launch(const flexspmv_desc* d, long long tiles, long long grid, int threads) {
+    if (4 * tiles > kSmallQuarters * grid || d->num_edges > kSmallRowEdges * d->num_rows) return false;
+    const long long rows_a_thread = (rows_a_cta(d->num_rows, grid) + threads - 1) / threads;
+    if (!G::kGatherNeedsRow) return rows_a_thread * (long long)sizeof(V) <= 24;
+    return true;
+  }
 
   // Where the gathered vectors are larger than this, tiles of whole rows go round the CTAs (round_tile in flex_tile_kernel.cuh).
   // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its
@@ -295,7 +314,7 @@ struct GraphApi {
     int form = FLEXSPMV_KERNEL_TILE;
     if constexpr (L::kWhole) {
       const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
-      if (4 * tiles <= kSmallQuarters * grid) {
+      if (small_launch(d, tiles, grid, kThreads)) {
         form = FLEXSPMV_KERNEL_TILE_SMALL;
         kernel = flex_tile_kernel<G, OffsetT, C, WIN, kSmall>;
         if (int e = resident_ctas<OffsetT, C, WIN, kSmall>(&resident)) return e;      // the grid stays the plan's

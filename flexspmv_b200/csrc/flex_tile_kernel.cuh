@@ -293,7 +293,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   OffsetT row_from = 0, row_to = 0;
   long long small_row = 0, small_end = 0;
   if constexpr (MODE == kSmall) {
-    const long long share = ((a.num_rows + gridDim.x - 1) / gridDim.x + 31) & ~31ll;
+    const long long share = rows_a_cta(a.num_rows, gridDim.x);
     small_row = blockIdx.x * share + tid;
     small_end = (blockIdx.x + 1) * share < a.num_rows ? (blockIdx.x + 1) * share : a.num_rows;
     // (the first row begins at edge 0 whatever row_offsets[0] says)

@@ -6,22 +6,34 @@ import numpy as np
 import pytest
 import torch
 
-from flexspmv_b200 import graphs
+from flexspmv_b200 import graphs, problems
 from flexspmv_b200.binding import GraphExtension, load_library
 from flexspmv_b200.python_wrapper.dynamic_replace_submodule import sort_edges_by_row
 from oracle import ir_eval
 from parity import assert_outputs_match
-from test_gpu_parity import run_gpu
+from test_gpu_parity import NP2T, run_gpu
 from test_gpu_whole_rows import with_lengths
 
 pytestmark = pytest.mark.gpu
 
 GRAPHS = [("spmv", "float64"), ("spmv", "float32"), ("spmv", "int64"), ("spring_mass", "float32"), ("rusanov", "float64"),
           ("swe_delta", "float32"), ("swe_boundary", "float64"), ("ops_zoo", "float64")]
+TILE, SMALL, ROUNDS, WARP, AHEAD = 1, 2, 3, 4, 5      # FLEXSPMV_KERNEL_* of include/flexspmv.h
 
 
-def launch(ir, prob, dtype, num_cols, bits, **kw):
-    """Outputs (as bytes) of one launch; ``num_cols``: the number of vertices that the descriptor names."""
+def last_kernel():
+    return load_library().flexspmv_debug_last_kernel()
+
+
+def header_word(ext, i):
+    """An int32 of the header of the workspace that was planned last (struct WorkspaceHeader)."""
+    return int(next(reversed(ext._plans.values())).ws[:256].cpu().numpy().view(np.int32)[i])
+
+
+def launch(ir, prob, dtype, num_cols, bits, kernel=None, loop=None, **kw):
+    """Outputs (as bytes) of one launch and whether its plan holds whole rows; ``num_cols``: the number of vertices that the
+    descriptor names; ``kernel``: the form that the launch has to take; ``loop``: whether the plan has to choose the loop over
+    whole rows."""
     ext = GraphExtension(ir, random_gather=False, **kw)
     non_gather, gathers, index_names = graphs.operator_signature(ir)
     v = [torch.from_numpy(np.ascontiguousarray(prob.values[n].astype(dtype))).cuda() for n in non_gather + gathers]
@@ -29,25 +41,53 @@ def launch(ir, prob, dtype, num_cols, bits, **kw):
     ro = torch.from_numpy(prob.row_offsets.astype(np.int32 if bits == 32 else np.int64)).cuda()
     outs = [torch.full((prob.num_rows, d), -7, dtype=v[0].dtype, device="cuda") for _, d in ext._out_kinds]
     ext.launch_into(v, ix, ro, outs, prob.num_rows, prob.nnz, num_cols)
+    assert kernel is None or last_kernel() == kernel
     ext.check()
+    assert loop is None or header_word(ext, 39) == loop
     return [o.cpu().numpy().tobytes() for o in outs], ext.planned_whole_rows()
+
+
+def default_tile(ir, dtype):
+    return GraphExtension(ir).symbols(NP2T[dtype]).graph_info.default_tile_items
 
 
 @pytest.mark.parametrize("gname,dt", GRAPHS)
 @pytest.mark.parametrize("bits", [32, 64])
-@pytest.mark.parametrize("lengths", [[5] * 4001, [0, 3, 7, 1] * 900 + [0] * 40, [32] * 333, [1] * 31, [6, 7] * 20_000],
-                         ids=["5", "uneven", "32", "31_rows", "several_rows_a_thread"])
-def test_small_launches_equal_staged_ones(gname, dt, bits, lengths):
-    """One CTA has all the tiles (more than three: stages) against the default grid (at most one a CTA: none)."""
+@pytest.mark.parametrize("lengths,tile_items", [([3] * 8003, 0), ([0, 3, 5, 2] * 2900 + [0] * 40, 0), ([2, 1, 4] * 600, 300), ([1] * 31, 0)],
+                         ids=["3", "uneven", "small_tiles", "31_rows"])
+def test_small_launches_equal_staged_ones(gname, dt, bits, lengths, tile_items):
+    """At most one tile a CTA, and two: rows straight from global memory.  Four tiles a CTA and more: stages.  (31 rows are one tile,
+    which no grid stages.)"""
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
     prob = with_lengths(ir, lengths, 101, dtype)
-    small, whole = launch(ir, prob, dtype, prob.num_cols, bits)
-    staged, _ = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=1)
-    two, _ = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=29)       # two tiles a CTA where there are 58
-    assert small == staged == two
+    tile = tile_items or default_tile(ir, dtype)
+    tiles = -(-(prob.num_rows + prob.nnz) // tile)
+    kw = {"tile_items": tile_items} if tile_items else {}
+    loop = 0 if gname == "ops_zoo" and len(set(lengths)) > 1 else 1       # (a map that divides, lanes that would idle: the other loop)
+    small, whole = launch(ir, prob, dtype, prob.num_cols, bits, SMALL, loop, **kw)
+    assert whole and (tiles >= 8 or tiles == 1)
+    if tiles > 1:
+        two, _ = launch(ir, prob, dtype, prob.num_cols, bits, SMALL, loop, max_ctas=-(-tiles // 2), **kw)
+        staged, _ = launch(ir, prob, dtype, prob.num_cols, bits, TILE, loop, max_ctas=tiles // 4, **kw)
+        one, _ = launch(ir, prob, dtype, prob.num_cols, bits, TILE, loop, max_ctas=1, **kw)
+        assert small == staged == two == one
     ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
-    got, _ = run_gpu(GraphExtension(ir, random_gather=False), ir, prob, dtype)
+    got, _ = run_gpu(GraphExtension(ir, random_gather=False, **kw), ir, prob, dtype)
     assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} small")
+
+
+@pytest.mark.parametrize("gname,dt", GRAPHS)
+@pytest.mark.parametrize("bits", [32, 64])
+def test_small_launches_with_several_rows_a_thread(gname, dt, bits):
+    """Rows of one edge, about 600 a CTA of 288 threads: the loop asks for the ends of a thread's next row."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [1] * 5990, 107, dtype)
+    tiles = -(-(prob.num_rows + prob.nnz) // default_tile(ir, dtype))
+    grid = min(tiles, 10)
+    assert prob.num_rows / grid > 2 * 288 and tiles <= 2 * grid
+    small, whole = launch(ir, prob, dtype, prob.num_cols, bits, SMALL, 1, max_ctas=grid)
+    staged, _ = launch(ir, prob, dtype, prob.num_cols, bits, TILE, 1, max_ctas=1)
+    assert whole and small == staged
 
 
 @pytest.mark.parametrize("gname,dt", GRAPHS)
@@ -55,15 +95,15 @@ def test_small_launches_equal_staged_ones(gname, dt, bits, lengths):
 @pytest.mark.parametrize("ctas", [1, 3, 7])
 def test_rounds_equal_runs_of_consecutive_tiles(gname, dt, bits, ctas):
     """A descriptor with many vertices takes tiles in rounds of four a CTA and splits the rest; the results are those of the plain
-    order.  40 001 rows of 6 and 7 edges are 200 tiles and more."""
+    order.  40 001 rows of 6 and 7 edges are 140 tiles (2040 items) and more."""
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
     prob = with_lengths(ir, [6, 7] * 20_000 + [3], 103, dtype)
-    plain, whole = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=ctas)
-    rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, max_ctas=ctas)
+    plain, whole = launch(ir, prob, dtype, prob.num_cols, bits, TILE, max_ctas=ctas)
+    rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, ROUNDS, max_ctas=ctas)
     assert whole and plain == rounds
     long = with_lengths(ir, [6, 7] * 20_000 + [200], 103, dtype)             # not whole rows: the loop with carries in either
-    plain, whole = launch(ir, long, dtype, long.num_cols, bits, max_ctas=ctas)
-    rounds, _ = launch(ir, long, dtype, 1 << 27, bits, max_ctas=ctas)
+    plain, whole = launch(ir, long, dtype, long.num_cols, bits, TILE, max_ctas=ctas)
+    rounds, _ = launch(ir, long, dtype, 1 << 27, bits, ROUNDS, max_ctas=ctas)
     assert not whole and plain == rounds
 
 
@@ -170,3 +210,28 @@ def test_offsets_read_once_or_bisected(rows, ids, offset_bits):
                                   ctypes.c_size_t(need.value), ptr(status), None) == 0
     want = np.concatenate([[0], np.cumsum(counts), [-1]])                  # (the word behind the last offset stays)
     assert np.array_equal(got.cpu().numpy(), want) and int(status) == 0
+
+
+@pytest.mark.parametrize("gname,dt,edges,kernel", [
+    ("spmv", "float64", 12, SMALL), ("spmv", "float64", 13, TILE), ("spmv", "float32", 15, SMALL), ("spmv", "float32", 16, TILE),
+    ("spring_mass", "float32", 10, SMALL), ("spring_mass", "float64", 11, TILE), ("rusanov", "float32", 6, SMALL),
+    ("rusanov", "float32", 7, TILE), ("rusanov", "float64", 4, SMALL), ("rusanov", "float64", 5, TILE), ("swe_delta", "float32", 6, SMALL),
+    ("swe_delta", "float64", 5, TILE), ("swe_boundary", "float64", 10, SMALL), ("ops_zoo", "float32", 7, SMALL), ("ops_zoo", "float32", 8, TILE)])
+def test_rows_of_small_launches_are_short(gname, dt, edges, kernel):
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [edges] * 3001, 113, dtype)
+    default, _ = launch(ir, prob, dtype, prob.num_cols, 32, kernel)
+    staged, _ = launch(ir, prob, dtype, prob.num_cols, 32, TILE, max_ctas=1)
+    assert default == staged
+
+
+@pytest.mark.parametrize("dt,rows_a_cta,kernel", [("float64", 864, SMALL), ("float64", 896, TILE), ("int64", 896, TILE), ("float32", 1728, SMALL),
+                                                  ("float32", 1760, TILE)])
+def test_small_launches_have_few_rows_a_thread(dt, rows_a_cta, kernel):
+    """288 threads a CTA: three rows each of 8-byte values, six of 4-byte ones."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    prob = with_lengths(ir, [1] * (5 * rows_a_cta - 7), 127, dtype)
+    assert 2 * prob.num_rows <= 3 * 5 * 1280
+    default, _ = launch(ir, prob, dtype, prob.num_cols, 32, kernel, max_ctas=5)
+    staged, _ = launch(ir, prob, dtype, prob.num_cols, 32, TILE, max_ctas=1)
+    assert default == staged
