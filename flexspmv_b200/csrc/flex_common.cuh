@@ -54,7 +54,8 @@ struct WorkspaceHeader {
   uint32_t bank_degree;        // first edges lie a multiple of 32 apart
   uint32_t line_rows, line_row_lines;       // over the same groups, when the plan saw the columns: rows with an edge and the
   uint32_t line_edges, line_edge_lines;     // cache lines their middle edges gather from; consecutive edges and their lines
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4];
+  int32_t uneven_shares;       // 1: with equal shares of the rows a CTA of the plan's grid would have more than RowLoopRule allows
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
@@ -77,6 +78,10 @@ struct RowLoopRule {
   int gathers;                       // gathers whose columns the plan sees (0: none)
   const int* index[kMaxGathers];
   int record_bytes[kMaxGathers];
+  // Launches without stages (flex_tile_kernel.cuh) give every CTA as many rows: what the heaviest share may hold (0: such a launch
+  // does not come into question for the matrix).
+  long long share_items;             // rows and edges
+  int share_row_edges;               // edges a row
 };
 
 // What one tile of the tile kernel can take when a planning step moves its boundaries (in whole numbers of edges and

@@ -250,6 +250,12 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* ro
     return;
   }
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < grid && rule.share_items) {
+    const long long share = rows_a_cta(num_rows, grid), r0 = t * share < num_rows ? t * share : num_rows;
+    const long long r1 = r0 + share < num_rows ? r0 + share : num_rows;
+    const long long edges = (long long)row_offsets[r1] - (r0 ? (long long)row_offsets[r0] : 0);
+    if (r1 - r0 + edges > rule.share_items || edges > rule.share_row_edges * share) h->uneven_shares = 1;
+  }
   if (t > 0 && t < num_tiles) {
     const long long x = (long long)coords[2 * t];
     if (x < num_rows) coords[2 * t + 1] = row_offsets[x];

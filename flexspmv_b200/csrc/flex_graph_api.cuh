@@ -210,6 +210,10 @@ struct GraphApi {
         if (rule.edge_lanes && indices && d->num_edges > 0)
           rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
         for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
+        if (grid > 0 && small_launch(d, h.num_tiles, grid, Cfg::kBlock + 32)) {
+          rule.share_items = 3 * ((h.num_tiles + grid - 1) / grid) * tile_items(d) / 2;
+          rule.share_row_edges = kSmallRowEdges;
+        }
         // rows longer than kWholeRowMax on average: no need to look
         if (whole_rows && !use_win(d) && d->num_rows > 0 && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
           return whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d), rule, grid, coords, ws, st);
@@ -248,6 +252,12 @@ struct GraphApi {
     if (!G::kGatherNeedsRow) return rows_a_thread * (long long)sizeof(V) <= 24;
     return true;
   }
+  // A small launch splits the rows evenly, not the tiles.  Where a CTA's share then holds half as much again as the tiles that a CTA has at
+  // most, or longer rows than above, the plan says so (share_items and share_row_edges below, WorkspaceHeader::uneven_shares) and the loop
+  // with stages runs, 0.2 - 0.5 us behind the plain kernel, which a launch cannot choose without waiting for the plan.  us, plain / without
+  // stages / as it is now:  SpMV, 1 and 30 edges a row in the matrix's halves, fp32 6.1 / 8.4 / 6.2, 7.9 / 15.5 / 7.9 (long on average: plain), fp64 7.5 / 10.7 /
+  // 7.5; 3 and in a tenth of the rows 20 fp64 5.7 / 16.7 / 6.1; 2 and 14 fp32 5.3 / 4.3 / 4.4, 7.3 / 7.6 / 7.7, fp64 4.7 / 5.6 / 4.9, 9.0 / 13.5 / 9.1; 2 and 6 fp32 7.4 / 5.3 /
+  // 5.4, fp64 5.8 / 4.8 / 4.8.  1 and 5 edges: spring-mass fp64 7.2 / 9.7 / 7.7, Rusanov fp32 6.6 / 8.6 / 7.1, swe_delta fp64 7.7 / 8.9 / 8.2.
 
   // Where the gathered vectors are larger than this, tiles of whole rows go round the CTAs (round_tile in flex_tile_kernel.cuh).
   // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its

@@ -90,6 +90,37 @@ def test_small_launches_with_several_rows_a_thread(gname, dt, bits):
     assert whole and small == staged
 
 
+@pytest.mark.parametrize("gname,dt,row_edges", [("spmv", "float64", 12), ("spmv", "float32", 15), ("spring_mass", "float32", 10),
+                                                ("swe_delta", "float64", 4)])
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("lengths,seen", [([3] * 30_000, {0}), ([2] * 15_000 + [6] * 15_000, {0, 1}), ([1] * 15_000 + [7] * 15_000, {1}),
+                                          ([7] * 15_000 + [1] * 15_000, {1}), ([3] * 20_000 + [16] * 1000 + [3] * 9000, {1}),
+                                          ([0] * 100 + [3] * 30_000 + [0] * 3, {0})],
+                         ids=["even", "half_as_many_again", "more", "more_in_front", "one_place", "empty_ends"])
+def test_shares_of_very_different_sizes_keep_the_stages(gname, dt, row_edges, bits, lengths, seen):
+    """The plan looks at the equal shares of the rows that a small launch would give its CTAs; where one holds more than half as much
+    again as the tiles that a CTA has at most, or longer rows than a small launch takes, the kernel runs its loop with stages.  The bits
+    are the same either way."""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, lengths, 109, dtype)
+    tile = default_tile(ir, dtype)
+    grid = -(-(prob.num_rows + prob.nnz) // tile)                   # a tile a CTA
+    share = (-(-prob.num_rows // grid) + 31) // 32 * 32
+    sizes = [(len(lengths[r:r + share]), sum(lengths[r:r + share])) for r in range(0, prob.num_rows, share)]
+    uneven = int(any(rows + edges > 3 * tile // 2 or edges > row_edges * share for rows, edges in sizes))
+    assert uneven in seen
+    results = []
+    for max_ctas in (0, 1):
+        ext = GraphExtension(ir, random_gather=False, max_ctas=max_ctas)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+        ext.check()
+        assert ext.planned_whole_rows() and header_word(ext, 39) == 1
+        assert last_kernel() == (TILE if max_ctas else SMALL)
+        assert header_word(ext, 46) == (0 if max_ctas else uneven)
+        results.append([g.tobytes() for g in got])
+    assert results[0] == results[1]
+
+
 @pytest.mark.parametrize("gname,dt", GRAPHS)
 @pytest.mark.parametrize("bits", [32, 64])
 @pytest.mark.parametrize("ctas", [1, 3, 7])
