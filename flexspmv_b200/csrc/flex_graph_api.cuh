@@ -241,6 +241,9 @@ struct GraphApi {
   //                 swe_delta fp32 6 6.4 / 6.4, 8 7.1 / 8.2
   //   rows a CTA    (several a thread, one after the other) SpMV fp64 800 7.8 / 6.6, 896 7.8 / 8.4, 1408 of one edge 8.1 / 8.9; fp32 1600 8.2 / 7.3,
   //                 1792 8.2 / 8.2, 1914 8.3 / 10.8
+  //   epilogues     (as long as a row: in 8-byte values a thread's second row is as dear as a CTA's second tile) a shallow-water step, rows a
+  //                 thread and tiles a CTA fp64 1 and 1.4 49.4 / 36.8, 2 and 1.7 51.2 / 53.2, 2 and 2.0 53.4 / 55.8, 2 and 2.1 68.4 / 55.9; fp32 2 and
+  //                 0.3 37.6 / 34.8, 2 and 1 45.7 / 42.2, 2 and 1.4 57.0 / 45.8
   static constexpr long long kSmallQuarters = G::kGatherNeedsRow ? 9 : 4 * kSmallTiles;
   static constexpr int least(int a, int b) { return a < b ? a : b; }
   static constexpr int within(int bytes_a_row) { return G::kStreamBytesPerEdge > 0 ? bytes_a_row / G::kStreamBytesPerEdge : bytes_a_row; }
@@ -250,7 +253,7 @@ struct GraphApi {
     if (4 * tiles > kSmallQuarters * grid || d->num_edges > kSmallRowEdges * d->num_rows) return false;
     const long long rows_a_thread = (rows_a_cta(d->num_rows, grid) + threads - 1) / threads;
     if (!G::kGatherNeedsRow) return rows_a_thread * (long long)sizeof(V) <= 24;
-    return true;
+    return !(G::kEpilogue && sizeof(V) == 8 && rows_a_thread > 1 && rows_a_thread * grid >= tiles);
   }
   // A small launch splits the rows evenly, not the tiles.  Where a CTA's share then holds half as much again as the tiles that a CTA has at
   // most, or longer rows than above, the plan says so (share_items and share_row_edges below, WorkspaceHeader::uneven_shares) and the loop

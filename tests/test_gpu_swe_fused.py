@@ -5,10 +5,11 @@ import pytest
 import torch
 
 from flexspmv_b200 import graphs, problems
-from flexspmv_b200.binding import FlexSpmvError, GraphExtension, load_builtin
+from flexspmv_b200.binding import FlexSpmvError, GraphExtension, load_builtin, load_library
 from flexspmv_b200.shallow_water import ShallowWaterStep
 
 pytestmark = pytest.mark.gpu
+TILE, SMALL, ROUNDS = 1, 2, 3      # FLEXSPMV_KERNEL_* of include/flexspmv.h
 
 
 def mesh_of(n, dtype, split_walls):
@@ -112,3 +113,40 @@ def test_the_epilogue_refuses_a_plan_without_whole_rows(max_ctas):
         ext.check()
     assert all(torch.equal(a, b) for a, b in zip(state, before))
     assert all(torch.isnan(t).all() for t in acc + out)
+
+
+def run_stage(m, start, sums, bits, first, last, max_ctas, vertices=None):
+    """One stage through the C ABI: the kernel that the launch took, state, sums and next state as bytes."""
+    nc, ne, V = m["h"].numel(), m["src"].numel(), m["h"].dtype
+    ro = torch.searchsorted(m["dst"], torch.arange(nc + 1, dtype=torch.int32, device="cuda")).to(torch.int32 if bits == 32 else torch.int64)
+    walls = torch.searchsorted(m["bcells"], torch.arange(0, nc + 32, 32, dtype=torch.int32, device="cuda")).to(torch.int32)
+    coef = torch.tensor([1e-3, 2e-3, first, last], dtype=V)
+    ext = GraphExtension(graphs.swe_delta_graph(), symbol_prefix="swe_delta_rk", max_ctas=max_ctas)
+    state, acc = [t.clone() for t in start], [t.clone() for t in sums]
+    stage = [t.clone() for t in start]            # what the fluxes are taken of
+    out = [torch.full((nc,), float("nan"), dtype=V, device="cuda") for _ in range(3)]
+    values = [m["alpha"], m["sx"], m["sy"]] + stage + [m["area"], m["bsx"], m["bsy"], walls, m["bcells"]] + state + acc + [coef]
+    launch = ext.prepare(values, [m["src"], m["dst"]], ro, out, nc, ne, vertices or nc)
+    assert ext.planned_whole_rows()
+    launch.launch()
+    kernel = load_library().flexspmv_debug_last_kernel()
+    ext.check()
+    assert all(torch.equal(a, b) for a, b in zip(stage, start))
+    return kernel, [t.cpu().numpy().tobytes() for t in state + acc + out]
+
+
+def stage_inputs(dtype, split_walls):
+    m = mesh_of(64, dtype, split_walls)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(11)
+    rand = lambda: torch.rand(m["h"].numel(), generator=g, device="cuda", dtype=m["h"].dtype)
+    return m, [m[k] + 0.01 * rand() for k in ("h", "uh", "vh")], [rand() for _ in range(3)]
+
+
+@pytest.mark.parametrize("dtype,max_ctas,kernel", [(np.float64, 21, SMALL), (np.float64, 23, TILE), (np.float32, 13, SMALL)])
+def test_a_second_cell_a_thread_against_a_second_tile(dtype, max_ctas, kernel):
+    """8192 cells, in fp64 43 tiles: where a thread has two cells and a CTA of 23 has two tiles the stages are kept, where one of 21 has
+    three they are not.  In fp32 they are not kept either way."""
+    m, start, sums = stage_inputs(dtype, False)
+    taken, got = run_stage(m, start, sums, 32, 0.0, 0.0, max_ctas)
+    assert taken == kernel and got == run_stage(m, start, sums, 32, 0.0, 0.0, 1)[1]
