@@ -6,6 +6,7 @@
 // include/merged_spmv.cuh:22-182): no per-call device-attribute queries, no per-call temp-storage
 // allocation, one kernel launch per operator call, partition cached in the caller's workspace.
 #pragma once
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -270,29 +271,31 @@ struct GraphApi {
   static constexpr long long kKeepBytes = 40ll << 20;
 
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
-  // once for each device of the process.
+  // once for each device of the process, then one word is read (a launch asks twice, for the plan's grid and for the form that it takes).
   template <typename OffsetT, class C = Cfg, bool WIN = false, int MODE = kPlain>
   static int resident_ctas(int* out) {
     using L = TileSmemLayout<G, OffsetT, C, WIN>;
     static_assert(L::kTotal <= 227 * 1024, "tile kernel needs more shared memory than one sm_100a CTA can have");
-    auto kernel = flex_tile_kernel<G, OffsetT, C, WIN, MODE>;
-    constexpr int kThreads = C::kBlock + (G::kDirectLoads ? 0 : 32);
     constexpr int kMaxDevices = 64;
-    static std::mutex mu;
-    static int resident_of[kMaxDevices] = {};      // 0: not initialised yet
+    static std::atomic<int> resident_of[kMaxDevices];      // 0: not looked up yet
     int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= kMaxDevices) return FLEXSPMV_ERR_BAD_ARG;
-    std::lock_guard<std::mutex> lock(mu);
-    if (resident_of[dev] == 0) {
+    int resident = resident_of[dev].load(std::memory_order_acquire);
+    if (resident == 0) {
+      static std::mutex mu;
+      std::lock_guard<std::mutex> lock(mu);
+      auto kernel = flex_tile_kernel<G, OffsetT, C, WIN, MODE>;
+      constexpr int kThreads = C::kBlock + (G::kDirectLoads ? 0 : 32);
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
       int r = 0;
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kernel, kThreads, L::kTotal);
       if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
-      resident_of[dev] = r < 1 ? -1 : r;
+      resident = r < 1 ? -1 : r;
+      resident_of[dev].store(resident, std::memory_order_release);
     }
-    if (resident_of[dev] < 1) return FLEXSPMV_ERR_TOO_LARGE;
-    *out = resident_of[dev];
+    if (resident < 1) return FLEXSPMV_ERR_TOO_LARGE;
+    *out = resident;
     return 0;
   }
 
