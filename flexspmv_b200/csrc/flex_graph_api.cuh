@@ -350,10 +350,12 @@ struct GraphApi {
   static int launch_lean(const flexspmv_desc* d, const typename G::Params& p, const void* row_offsets, void* ws,
                          const WorkspaceHeader& h, cudaStream_t st) {
     if constexpr (G::kHasReducer && kLeanBuilt) {
-      // few chunks a warp (16: 500 000 power-law rows have 14 in fp32, 17 in fp64): the other kernel, on fewer warps
+      // few chunks a warp (16: 500 000 power-law rows have 14 in fp32, 17 in fp64): the other kernel, on fewer warps.  Of the grid that
+      // the launch will have: a few CTAs have many chunks each on a small matrix too.
       using Small = WarpCfg<whole_warps(C::kBlock * (sizeof(V) == 4 ? 9 : 10) / 12), C::kIpt, C::kMinCtas>;
       if constexpr (!SMALL) {
-        if (h.num_tiles < 16ll * device_sm_count() * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
+        const long long ctas = d->max_ctas > 0 ? d->max_ctas : (long long)device_sm_count() * C::kMinCtas;
+        if (h.num_tiles < 16 * ctas * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
       }
       const auto kernel = [] {          // (the other one is not compiled for this configuration)
         if constexpr (SMALL) return &flex_warp_ahead_kernel<G, OffsetT, C>;

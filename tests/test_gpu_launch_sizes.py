@@ -266,3 +266,28 @@ def test_small_launches_have_few_rows_a_thread(dt, rows_a_cta, kernel):
     default, _ = launch(ir, prob, dtype, prob.num_cols, 32, kernel, max_ctas=5)
     staged, _ = launch(ir, prob, dtype, prob.num_cols, 32, TILE, max_ctas=1)
     assert default == staged
+
+
+@pytest.mark.parametrize("dt", ["float32", "float64", "int64"])
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("kernel", [WARP, AHEAD])
+def test_both_forms_of_the_warp_kernel_match_the_oracle(dt, bits, kernel):
+    """Rows over many chunks, runs and CTAs, empty rows, odd chunk sizes, in the form for few chunks a warp (the default grid) and, on one
+    to three CTAs, in the one for many.  Integers bit for bit, the same bits twice."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    offsets = np.int32 if bits == 32 else np.int64
+    cases = [((2, 5000, 300_000), 0, 3), ((40_000, 40_000, 120_000), 0, 1), ((97, 97, 100_000), 0, 1), ((3000, 3000, 2000), 7, 1),
+             ((300, 300, 40_000), 33, 2), ((60, 60, 250_000), 159, 2), ((1, 1, 90_000), 0, 1), ((90_000, 5, 300), 0, 1)]
+    for (rows, vertices, nnz), tile_items, few_ctas in cases:
+        prob = problems.random_problem(ir, rows, vertices, nnz, seed=3000 + rows + nnz, dtype=dtype)
+        ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=8, want_abs_sums=True)
+        kw = {"tile_items": tile_items} if tile_items else {}
+        results = []
+        for _ in range(2):
+            ext = GraphExtension(ir, random_gather=True, max_ctas=few_ctas if kernel == WARP else 0, **kw)
+            got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=offsets)
+            assert last_kernel() == kernel, (rows, nnz)
+            ext.check()
+            assert_outputs_match(ir, got, ref, sums, dtype, what=f"warp kernel {kernel} {dt} {rows} x {nnz}")
+            results.append([g.tobytes() for g in got])
+        assert results[0] == results[1]
