@@ -350,12 +350,14 @@ struct GraphApi {
   static int launch_lean(const flexspmv_desc* d, const typename G::Params& p, const void* row_offsets, void* ws,
                          const WorkspaceHeader& h, cudaStream_t st) {
     if constexpr (G::kHasReducer && kLeanBuilt) {
-      // few chunks a warp (16: 500 000 power-law rows have 14 in fp32, 17 in fp64): the other kernel, on fewer warps.  Of the grid that
-      // the launch will have: a few CTAs have many chunks each on a small matrix too.
+      // Few chunks a warp: the other form, on fewer warps.  Chunks a warp, us in this form / in that: power-law rows fp32 17.4 51.0 / 45.8,
+      // 20.3 60.8 / 55.7, 24.7 64.5 / 65.6, 29 73.6 / 75.2; fp64 17.4 51.8 / 48.3, 19.2 53.5 / 52.6, 20.9 56.9 / 56.6, 24.4 63.9 / 63.7, 29.6 75.1 / 74.2.
+      // Of the grid that the launch will have: a few CTAs have many chunks each on a small matrix too.
+      constexpr int kFewChunks = 22;
       using Small = WarpCfg<whole_warps(C::kBlock * (sizeof(V) == 4 ? 9 : 10) / 12), C::kIpt, C::kMinCtas>;
       if constexpr (!SMALL) {
         const long long ctas = d->max_ctas > 0 ? d->max_ctas : (long long)device_sm_count() * C::kMinCtas;
-        if (h.num_tiles < 16 * ctas * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
+        if (h.num_tiles < kFewChunks * ctas * Small::kWarps) return launch_lean<OffsetT, Small, true>(d, p, row_offsets, ws, h, st);
       }
       const auto kernel = [] {          // (the other one is not compiled for this configuration)
         if constexpr (SMALL) return &flex_warp_ahead_kernel<G, OffsetT, C>;

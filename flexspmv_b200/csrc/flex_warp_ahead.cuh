@@ -3,10 +3,10 @@
 // The warps of such a launch all start at once, and with the gathers at the head of their own chunk they wait and compute in
 // step: on 200 003 power-law rows in fp64 the gathers alone take 11 us and the instructions 11 us, and the launch took the sum.
 // Here a warp asks for the next chunk's gathers before it sums the present one, also from one run to the next, and fewer
-// warps do the work (us, 4-byte values 1024 / 768 threads, 8-byte ones 768 / 640; power-law rows): fp64 200 003 30.8 / 27.5,
-// 70 000 20.6 / 18.4, 500 000 51.8 / 50.1; fp32 100 000 24.7 / 20.7, 300 000 36.9 / 32.4, 500 000 48.3 / 45.5.  Launches of many
-// chunks a warp drift apart by themselves and are bound by the gathers: 2^24 rows fp32 1227 / 1252, 4 M rows fp64 307 / 309.  They
-// keep the other kernel.  What is done with a chunk and with the carries is the same (WarpParts).
+// warps do the work (us, 4-byte values 1024 / 768 threads, 8-byte ones 768 / 640; power-law rows): fp64 200 003 30.8 / 27.4,
+// 70 000 20.6 / 18.4, 500 000 51.8 / 48.3; fp32 100 000 24.9 / 20.7, 300 000 36.5 / 32.1, 500 000 48.0 / 45.4, 700 000 60.8 / 55.7.  Launches
+// of many chunks a warp drift apart by themselves and are bound by the gathers: 2^24 rows fp32 1227 / 1252, 4 M rows fp64 307 / 309.
+// They keep the other form (the line: GraphApi::launch_lean).  What is done with a chunk and with the carries is the same (WarpParts).
 #pragma once
 #include <type_traits>
 

@@ -291,3 +291,14 @@ def test_both_forms_of_the_warp_kernel_match_the_oracle(dt, bits, kernel):
             assert_outputs_match(ir, got, ref, sums, dtype, what=f"warp kernel {kernel} {dt} {rows} x {nnz}")
             results.append([g.tobytes() for g in got])
         assert results[0] == results[1]
+
+
+@pytest.mark.parametrize("dt,chunks,kernel", [("float64", 439, AHEAD), ("float64", 440, WARP), ("float32", 527, AHEAD), ("float32", 528, WARP)])
+def test_chunks_a_warp_choose_the_form(dt, chunks, kernel):
+    """One CTA of 20 or 24 warps: up to 22 chunks a warp."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    prob = problems.random_problem(ir, 500, 500, chunks * 160 - 500, seed=131, dtype=dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    got, _ = run_gpu(GraphExtension(ir, random_gather=True, max_ctas=1), ir, prob, dtype)
+    assert last_kernel() == kernel
+    assert_outputs_match(ir, got, ref, sums, dtype, what=f"{chunks} chunks")
