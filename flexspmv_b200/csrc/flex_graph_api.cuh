@@ -264,11 +264,16 @@ struct GraphApi {
   // 5.4, fp64 5.8 / 4.8 / 4.8.  1 and 5 edges: spring-mass fp64 7.2 / 9.7 / 7.7, Rusanov fp32 6.6 / 8.6 / 7.1, swe_delta fp64 7.7 / 8.9 / 8.2.
 
   // Where the gathered vectors are larger than this, tiles of whole rows go round the CTAs (round_tile in flex_tile_kernel.cuh).
-  // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its
-  // neighbours in L1: 7-point fp32 145^3 (12 MB) 42.6 us in runs of its own, 45.0 in rounds; 27 columns a row fp64, 3 M rows
-  // (24 MB) 188 / 194; Rusanov fp64 1024^2 (50 MB) 80.7 / 76.7, a shallow-water step 1024^2 (50 MB) 450 / 384; 5-point fp64 3000^2
-  // (72 MB) 128 / 118.
-  static constexpr long long kKeepBytes = 40ll << 20;
+  // Smaller ones stay in L2 (126 MB, shared with the streams) whatever the order, and a CTA's own run keeps more of its neighbours in L1.
+  // us in runs of its own / in rounds, by the size of the vectors:
+  //   two-phase graphs  7-point fp32 12 MB 42.6 / 45.0, 32 112.3 / 110.6, 37 129.0 / 126.6, 43 146.9 / 146.3, 49 165.7 / 166.7, 70 247.6 / 241.4; fp64 24 MB
+  //                     55.9 / 55.7, 30 69.8 / 67.9, 36 81.4 / 80.9, 41 92.2 / 89.9, 47 105.8 / 102.6; 27 columns a row fp64 24 MB 188 / 194; 5-point
+  //                     fp64 23 MB 43.8 / 43.1, 27 51.8 / 51.2, 37 68.1 / 67.1, 42 78.5 / 76.1, 72 128 / 118: level up to 50 MB, with the losses below 25
+  //   row-mode graphs   a shallow-water step fp64 7.7 MB 92.7 / 92.7, 12 123.5 / 114.8, 17 170.4 /
+  //                     162.1, 25 247 / 227, 35 340 / 314, 50 450 / 398; spring-mass fp32 6.5 MB 32.1 / 31.4, 16 66.3 / 64.8, 20 85.0 / 81.0, 32 130.8 / 123.0,
+  //                     fp64 11.6 MB 51.0 / 50.6, 25 103.2 / 99.0, 41 164.8 / 158.0; Rusanov fp64 7.7 MB 15.7 / 15.7, 12 23.9 / 23.6, 25 42.7 / 42.1, 50 84.3 / 81.3, fp32
+  //                     13.5 MB 28.5 / 28.6, 26 51.6 / 52.2, 35 64.6 / 64.1, 54 100.4 / 97.8
+  static constexpr long long kKeepBytes = (G::kGatherNeedsRow ? 10ll : 40ll) << 20;
 
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
   // once for each device of the process, then one word is read (a launch asks twice, for the plan's grid and for the form that it takes).

@@ -302,3 +302,14 @@ def test_chunks_a_warp_choose_the_form(dt, chunks, kernel):
     got, _ = run_gpu(GraphExtension(ir, random_gather=True, max_ctas=1), ir, prob, dtype)
     assert last_kernel() == kernel
     assert_outputs_match(ir, got, ref, sums, dtype, what=f"{chunks} chunks")
+
+
+@pytest.mark.parametrize("gname,dt,record,megabytes", [("spmv", "float64", 8, 40), ("spmv", "float32", 4, 40), ("spring_mass", "float32", 8, 10),
+                                                       ("rusanov", "float64", 24, 10)])
+def test_the_size_of_the_gathered_vectors_chooses_the_order(gname, dt, record, megabytes):
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    prob = with_lengths(ir, [6, 7] * 10_000, 137, dtype)
+    most = (megabytes << 20) // record
+    plain, _ = launch(ir, prob, dtype, most, 32, TILE, max_ctas=2)
+    rounds, _ = launch(ir, prob, dtype, most + 1, 32, ROUNDS, max_ctas=2)
+    assert plain == rounds
