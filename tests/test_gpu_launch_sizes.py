@@ -313,3 +313,18 @@ def test_the_size_of_the_gathered_vectors_chooses_the_order(gname, dt, record, m
     plain, _ = launch(ir, prob, dtype, most, 32, TILE, max_ctas=2)
     rounds, _ = launch(ir, prob, dtype, most + 1, 32, ROUNDS, max_ctas=2)
     assert plain == rounds
+
+
+@pytest.mark.parametrize("dt", ["float64", "int64", "float32"])
+@pytest.mark.parametrize("lengths", [[0, 5, 16] * 1000, [300] * 60, [1] * 500 + [5000] + [0] * 300 + [7] * 200], ids=["short", "several_tiles", "one_long"])
+def test_wide_records_in_small_ctas(dt, lengths):
+    """Eight-byte values run 64 threads x 4 edges: the default tile and those that a caller may ask for, rows inside a tile and
+    over several, the default grid and two CTAs."""
+    ir, dtype = graphs.mixed_dims_graph(), np.dtype(dt)
+    prob = with_lengths(ir, lengths, 139, dtype)
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    for kw in ({}, {"tile_items": 193}, {"tile_items": 256}, {"tile_items": 255, "max_ctas": 2}, {"tile_items": 1, "max_ctas": 50}):
+        ext = GraphExtension(ir, **kw)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int64 if "max_ctas" in kw else np.int32)
+        ext.check()
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"mixed_dims {dt} {kw}")

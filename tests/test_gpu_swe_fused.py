@@ -143,6 +143,22 @@ def stage_inputs(dtype, split_walls):
     return m, [m[k] + 0.01 * rand() for k in ("h", "uh", "vh")], [rand() for _ in range(3)]
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("split_walls", [False, True, "everywhere"])
+def test_every_form_of_the_stage_gives_the_same_bits(dtype, bits, split_walls):
+    """One stage in place (the first, a middle and the last of a step) straight from global memory (the default grid), through stages
+    (one CTA and five) and with tiles going round the CTAs (a descriptor that names many vertices)."""
+    m, start, sums = stage_inputs(dtype, split_walls)
+    for first, last in ((1.0, 0.0), (0.0, 0.0), (0.0, 1.0)):
+        results = []
+        for max_ctas, vertices, kernel in ((0, None, SMALL), (1, None, TILE), (5, None, TILE), (1, 1 << 27, ROUNDS), (5, 1 << 27, ROUNDS)):
+            taken, got = run_stage(m, start, sums, bits, first, last, max_ctas, vertices)
+            assert taken == kernel
+            results.append(got)
+        assert all(r == results[0] for r in results[1:]), (first, last)
+
+
 @pytest.mark.parametrize("dtype,max_ctas,kernel", [(np.float64, 21, SMALL), (np.float64, 23, TILE), (np.float32, 13, SMALL)])
 def test_a_second_cell_a_thread_against_a_second_tile(dtype, max_ctas, kernel):
     """8192 cells, in fp64 43 tiles: where a thread has two cells and a CTA of 23 has two tiles the stages are kept, where one of 21 has
