@@ -1,7 +1,7 @@
-// Hand-written sm_100a kernel for fused graphs WITH a reduce-by-row: persistent CTAs walk contiguous
-// runs of merge-path tiles; each tile's row-end offsets, index arrays and (two-phase graphs) per-edge
-// tensors are staged into shared memory by 1-D bulk async copies (TMA, mbarrier complete_tx) that a
-// producer warp issues STAGES tiles ahead.
+// Hand-written sm_100a kernel for fused graphs WITH a reduce-by-row: persistent CTAs walk merge-path tiles, a
+// contiguous run each, or (whole rows, below) short runs in turn; each tile's row-end offsets, index arrays and
+// (two-phase graphs) per-edge tensors are staged into shared memory by 1-D bulk async copies (TMA, mbarrier
+// complete_tx) that a producer warp issues STAGES tiles ahead.
 //   Two-phase graphs (plain SpMV and every graph whose map needs no per-row data): phase 1, lanes on
 //   consecutive edges -- each thread copies IPT edges from the stage to registers, hands the stage back,
 //   gathers, runs the generated map and writes the products to shared memory; phase 2, one thread per
@@ -12,7 +12,9 @@
 //   apart, shuffle tree).  Nothing of a row-mode graph passes through a shared-memory product buffer.
 //   Whole rows (either kind of graph, when the plan found a matrix of short rows whose tiles can all hold whole rows, and
 //   that one lane per row suits): no carries at all, so no barriers either -- every warp takes 32 rows of a staged tile, one per lane,
-//   and keeps everything in registers.  The other two loops run on such tiles too, without carries between CTAs.
+//   and keeps everything in registers.  The other two loops run on such tiles too, without carries between CTAs.  No carry ties a
+//   CTA to consecutive tiles either: where the gathered vectors are large, runs of kTileRun tiles go round the CTAs (kRounds); and a
+//   small launch of short rows takes them without tiles and stages, a row per thread straight from global memory (kSmall).
 // The carry of a row that spans tiles travels inside the CTA in shared memory; the only cross-CTA state
 // is one carry per CTA, folded in by the last CTA to finish (ticket counter), in CTA order.  No atomics
 // on the output, no pre-zeroed output, run-to-run deterministic.
@@ -325,9 +327,10 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   if constexpr (MODE == kSmall) {
     if (whole && !h_stages) {
       // ---- whole rows of a small launch: one row per thread, everything straight from global memory ----------------------
-      // Bound by round trips, of which there are three -- row ends (asked for with the header), the row's edges, its gathers --
-      // without barriers, bulk copies and the producer's coordinates in front of them.  Sums run left to right as in the loop
-      // below: the same bits.
+      // Bound by round trips: the row's ends (asked for with the header), then the edges and the gathers of every kRowBatch edges, so
+      // 1 + 2 ceil(n / kRowBatch) of them for a row of n edges (5 for a 5-point row in fp64, 7 for a cell of three edges), without the barriers,
+      // bulk copies and producer's coordinates in front of a stage, whose rows need one copy and ceil(n / kRowBatch) gathers.  Which
+      // launches come here: GraphApi::small_launch.  Sums run left to right as in the loop below: the same bits.  512^2 5-point fp64 7.1 -> 5.1 us.
       LdgTile<G> tile{&p};
       constexpr int RB = Cfg::kRowBatch;
       for (; small_row < small_end; small_row += BLOCK + 32) {
@@ -623,9 +626,9 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // What the two-phase loop is bound by on short rows is the shared-memory / L1 data pipe (75 - 80 % busy at 55 % of
       // DRAM) and two CTA barriers a tile; this one moves no product through shared memory and a third of the gather lines
       // (41 % of the pipe at 70 % of DRAM), and is bound by the latency of the gathers at the registers of 4 CTAs per SM: 10 of
-      // 16 stall cycles per issue are long_scoreboard.  us a launch, two-phase / this loop: 7-point fp64 SpMV 512^3 3205 / 2564
-      // (5.65 TB/s); 145^3 fp32 54.1 / 42.6; 5-point 512^2 fp64 9.1 / 7.1; 27 columns a row fp64, 300 007 rows 26.2 / 23.9;
-      // spring-mass 1024^2 fp32 44.5 / 38.4; Rusanov 1024^2 fp64 92 / 83.5.
+      // 16 stall cycles per issue are long_scoreboard.  us a launch, two-phase / this loop with a run of tiles a CTA: 7-point fp64
+      // SpMV 512^3 3205 / 2564 (in rounds 2133); 145^3 fp32 54.1 / 42.6; 5-point 512^2 fp64 9.1 / 7.1 (without stages 5.1); 27 columns a row
+      // fp64, 300 007 rows 26.2 / 23.9; spring-mass 1024^2 fp32 44.5 / 38.4; Rusanov 1024^2 fp64 92 / 83.5.
       constexpr int RB = Cfg::kRowBatch;
       int s = 0, turn = 0;
       uint32_t parity = 0;
