@@ -36,10 +36,11 @@ if ROOT not in sys.path:
 METRIC = "fused SpMV effective GB/s"
 UNIT = "GB/s"
 # DRAM traffic of the headline kernel: dram__bytes_read.sum + dram__bytes_write.sum of ONE ncu capture of
-# flex_tile_kernel<spmv_f64, int64 offsets> on the 192^3 grid (the full-size launch holds too much memory to capture
-# with more than one pass); traffic grows in proportion to the grid, so it is scaled to the benchmarked launch by the
-# algorithmic bytes.  Part of y is still in L2 when that capture ends, so the write figure is a lower bound.
-DRAM_CAPTURE = {"grid": 192, "read_bytes": 717.6e6, "write_bytes": 25.7e6, "algorithmic_bytes": 761_757_704}
+# flex_tile_kernel<spmv_f64, int64 offsets> on the 192^3 grid, whose tiles go round the CTAs as the benchmarked launch's do (the
+# full-size launch holds too much memory to capture with more than one pass); reads are 1.006, 1.009 and 1.011 of the
+# algorithmic ones on 192^3, 240^3 and 360^3, so the figure is scaled to the benchmarked launch by the algorithmic bytes.
+# Part of y is still in L2 when that capture ends, so the write figure is a lower bound.
+DRAM_CAPTURE = {"grid": 192, "read_bytes": 709.4e6, "write_bytes": 26.0e6, "algorithmic_bytes": 761_757_704}
 
 
 def load_peaks():

@@ -268,10 +268,13 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
 
   // Tile k of the CTA where whole rows go round the CTAs: no carry ties a CTA to consecutive tiles, so in each round it takes
   // kTileRun of them, and what is left behind the last full round is split like above (the same number of tiles a CTA).  The
-  // CTAs then walk the matrix as one front.  In a run of its own a CTA meets the columns a plane (or a line) away at a time
-  // of its own: on a 512^3 grid the three places where a vector record is gathered lie 2.3 GB of traffic apart, so it is read
-  // from DRAM three times (7-point fp64 SpMV, us, own runs / rounds of 4, 8, 16, 32, 64 tiles: 2529 / 2133, 2146, 2161, 2214,
-  // 2328; 300^3 480 / 422, 429, 434, 443, 464; 400^3 fp32 905 / 821, 827, 835, 839, 846; 5-point 3000^2 128 / 118, 122, 123, 125, 126).
+  // CTAs then walk the matrix as one front.  In a run of its own a CTA meets the columns a plane (or a line) away at a time of its own,
+  // unless a plane is a whole number of runs: the three places where a vector record is gathered lie up to half the matrix of traffic
+  // apart.  DRAM reads of the 7-point fp64 SpMV, own runs / rounds: 360^3 (a plane is 1.64 runs) 5.45 / 4.71 GB, the vector's 0.37 GB three times / once;
+  // 240^3 (2.47) 1.51 / 1.39, twice / once; 300^3 (1.97) 2.72 / 2.72, once in either.  There, and on 192^3 (0.72 / 0.71 GB, 129 / 122 us cold), the front
+  // is the faster order at the same traffic: 592 CTAs read one stretch of each array, not 592.  us, own runs / rounds of 4, 8, 16, 32, 64 tiles:
+  // 512^3 2529 / 2133, 2146, 2161, 2214, 2328; 300^3 480 / 422, 429, 434, 443, 464; 400^3 fp32 905 / 821, 827, 835, 839, 846; 5-point 3000^2 128 / 118, 122, 123,
+  // 125, 126.
   auto round_tile = [&](int k) -> long long {
     if (k < a.rounds * kTileRun) return ((long long)(k / kTileRun) * gridDim.x + blockIdx.x) * kTileRun + k % kTileRun;
     return t_begin + (long long)a.rounds * kTileRun * (gridDim.x - 1 - blockIdx.x) + k;
