@@ -1,5 +1,6 @@
-"""Kernels picked by the size of a launch: the tile kernel without stages (few tiles a CTA) and with tiles going round the CTAs (large
-gathered vectors) against its plain form, bit for bit; the warp kernel's two configurations; the sort's 10-bit digits."""
+"""Kernels picked by the size of a launch, each test saying which one it means: the tile kernel without stages (few tiles a CTA, short
+rows, even shares) and with tiles going round the CTAs (large gathered vectors) against its plain form, bit for bit; the warp kernel's
+two forms; the sort's 10-bit digits and its two ways to the offsets; small CTAs for wide records."""
 import ctypes
 
 import numpy as np
