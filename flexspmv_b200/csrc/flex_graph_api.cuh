@@ -306,7 +306,7 @@ struct GraphApi {
 
   template <typename OffsetT, class C = Cfg, bool WIN = false>
   static int launch_tiles(const flexspmv_desc* d, const typename G::Params& p, const void* row_offsets, void* ws,
-                          const WorkspaceHeader& h, cudaStream_t st) {
+                          const WorkspaceHeader& h, cudaStream_t st, bool whole_rows) {
     using L = TileSmemLayout<G, OffsetT, C, WIN>;
     auto kernel = flex_tile_kernel<G, OffsetT, C, WIN>;
     constexpr int kThreads = C::kBlock + (G::kDirectLoads ? 0 : 32);   // staged mode adds the producer warp
@@ -333,7 +333,7 @@ struct GraphApi {
       a.win_index = reinterpret_cast<const unsigned short*>(static_cast<char*>(ws) + h.win_index_offset);
     }
     int form = FLEXSPMV_KERNEL_TILE;
-    if constexpr (L::kWhole) {
+    if constexpr (L::kWhole) if (whole_rows) {
       const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
       if (small_launch(d, tiles, grid, kThreads)) {
         form = FLEXSPMV_KERNEL_TILE_SMALL;
@@ -434,8 +434,9 @@ struct GraphApi {
     return 0;
   }
 
+  // `whole_rows`: false where the plan did not look for whole rows (the forms that are for them only cost such a launch).
   static int launch(const flexspmv_desc* d, const void* const* values, const void* const* indices,
-                    const void* row_offsets, void* const* outputs, void* ws, size_t ws_bytes, cudaStream_t st) {
+                    const void* row_offsets, void* const* outputs, void* ws, size_t ws_bytes, cudaStream_t st, bool whole_rows = true) {
     if (int e = check_desc(d)) return e;
     if (!ws) return FLEXSPMV_ERR_WORKSPACE;
     if ((G::kNumValues && !values) || (G::kNumIndices && !indices) || (G::kNumOutputs && !outputs)) return FLEXSPMV_ERR_BAD_ARG;
@@ -457,12 +458,12 @@ struct GraphApi {
       }
       if constexpr (G::kWindowGather && kWindowsBuilt) {
         if (use_win(d)) {
-          if (d->offset_bits == 64) return launch_tiles<long long, CfgWin, true>(d, p, row_offsets, ws, h, st);
-          return launch_tiles<int, CfgWin, true>(d, p, row_offsets, ws, h, st);
+          if (d->offset_bits == 64) return launch_tiles<long long, CfgWin, true>(d, p, row_offsets, ws, h, st, whole_rows);
+          return launch_tiles<int, CfgWin, true>(d, p, row_offsets, ws, h, st, whole_rows);
         }
       }
-      if (d->offset_bits == 64) return launch_tiles<long long>(d, p, row_offsets, ws, h, st);
-      return launch_tiles<int>(d, p, row_offsets, ws, h, st);
+      if (d->offset_bits == 64) return launch_tiles<long long>(d, p, row_offsets, ws, h, st, whole_rows);
+      return launch_tiles<int>(d, p, row_offsets, ws, h, st, whole_rows);
     } else {
     note_kernel(FLEXSPMV_KERNEL_NONE);
     if (d->num_edges == 0 && G::kAggDim == 0) return 0;
@@ -562,7 +563,7 @@ struct GraphApi {
     /* the array keeps the previous call's contents: planning rewrites the header (ticket, status) and */      \
     /* every tile coordinate this problem reads; the carry slots are written before they are read      */      \
     if (int e = Api::plan(d, nullptr, ro, ws, (size_t)(BYTES), stream, false)) return e;                             \
-    return Api::launch(d, v, ix, ro, o, ws, (size_t)(BYTES), stream);                                           \
+    return Api::launch(d, v, ix, ro, o, ws, (size_t)(BYTES), stream, false);                                    \
   }                                                                                                             \
   extern "C" int flexspmv_##SYM##_static_device_status(int32_t* d_out, void* st) {                              \
     void* ws = nullptr;                                                                                         \

@@ -84,6 +84,22 @@ def test_static_scratch_entry_matches_workspace_entry_twice_in_a_row():
         assert torch.equal(_static_result(lib, flagged, vals, x, cols, ro), expect)
 
 
+def test_static_scratch_entry_takes_the_plain_kernel():
+    """Its plan does not look for whole rows, so the forms of the kernel that are for them would only cost the call: neither the one for
+    small launches nor the one for large vectors."""
+    lib = load_library()
+    lib.flexspmv_spmv_f64_launch_static.restype = ctypes.c_int
+    lib.flexspmv_spmv_f64_static_device_status.restype = ctypes.c_int
+    prob = problems.poisson2d(96)
+    vals, x, cols, ro = _device_problem(prob, np.int32)
+    for cols_named, max_ctas, workspace_kernel in ((prob.num_cols, 0, 2), (1 << 27, 1, 3)):      # FLEXSPMV_KERNEL_TILE_SMALL, _ROUNDS
+        desc = Desc(prob.num_rows, prob.nnz, cols_named, 32, 0, max_ctas, 0)
+        expect = _workspace_result(lib, desc, vals, x, cols, ro)
+        assert lib.flexspmv_debug_last_kernel() == workspace_kernel
+        got = _static_result(lib, desc, vals, x, cols, ro)
+        assert lib.flexspmv_debug_last_kernel() == 1 and torch.equal(got, expect)
+
+
 def test_static_scratch_entry_refuses_oversized_problems():
     lib = load_library()
     lib.flexspmv_spmv_f64_launch_static.restype = ctypes.c_int
