@@ -54,7 +54,8 @@ struct WorkspaceHeader {
   uint32_t bank_degree;        // first edges lie a multiple of 32 apart
   uint32_t line_rows, line_row_lines;       // over the same groups, when the plan saw the columns: rows with an edge and the
   uint32_t line_edges, line_edge_lines;     // cache lines their middle edges gather from; consecutive edges and their lines
-  int32_t uneven_shares;       // 1: with equal shares of the rows a CTA of the plan's grid would have more than RowLoopRule allows
+  int32_t uneven_shares;       // 1: with equal shares of the rows a CTA of the plan's grid would have more than RowLoopRule allows; 2 is added
+                               // while a test withholds a stage (not 0: a small launch runs its loop with stages)
   char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");

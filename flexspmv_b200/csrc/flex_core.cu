@@ -320,7 +320,10 @@ __global__ void header_init_kernel(WorkspaceHeader* dst, const WorkspaceHeader h
   if (threadIdx.x == 0 && blockIdx.x == 0) *dst = h;
 }
 __global__ void debug_withhold_kernel(WorkspaceHeader* h, uint32_t first_tile_plus_one) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) h->debug[7] = first_tile_plus_one;
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    h->debug[7] = first_tile_plus_one;
+    h->uneven_shares = (h->uneven_shares & 1) | (first_tile_plus_one ? 2 : 0);
+  }
 }
 __global__ void window_ready_kernel(WorkspaceHeader* h) {
   if (threadIdx.x == 0 && blockIdx.x == 0) h->win_ready = 1;

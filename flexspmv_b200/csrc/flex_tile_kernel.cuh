@@ -310,8 +310,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   const int h_bits = a.header->offset_bits;
   const long long h_rows = a.header->num_rows, h_edges = a.header->num_edges, h_tiles = a.header->num_tiles;
   const int h_snapped = a.header->snapped_grid, h_whole = a.header->whole_rows, h_row_loop = a.header->row_loop;
-  // (a test that withholds a stage means the loops with stages)
-  const bool h_stages = MODE == kSmall && (a.header->debug[7] != 0 || a.header->uneven_shares != 0);
+  const bool h_stages = MODE == kSmall && a.header->uneven_shares != 0;
   // a workspace that was never planned for this problem holds no usable coordinates: every CTA
   // sees the same header, so all of them leave here and the ticket stays untouched
   if (h_magic != kMagic || h_tiles != a.num_tiles || h_rows != a.num_rows || h_edges != a.num_edges || h_bits != (int)(8 * sizeof(OffsetT))) {
