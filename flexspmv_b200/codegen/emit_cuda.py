@@ -379,14 +379,20 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w("  }")
     # a row's finished sums: to the reducers' outputs, or through the epilogue
     w(f"  static constexpr bool kEpilogue = {'true' if swe_rk else 'false'};")
-    w("  __device__ __forceinline__ static void finish_row(const Params& p, long long row, const V* v) {")
+    w(f"  using GOwn = {'flex::SweRkOwn<V>' if swe_rk else 'flex::NoOwn'};")
+    w("  __device__ __forceinline__ static void load_own(const Params& p, long long row, GOwn& own) {")
     if swe_rk:
-        w("    flex::swe_rk_row<V>(p, row, v);")
+        w("    flex::swe_rk_load<V>(p, row, own);")
+    w("    (void)p; (void)row; (void)own;")
+    w("  }")
+    w("  __device__ __forceinline__ static void finish_row(const Params& p, long long row, const V* v, const GOwn& own) {")
+    if swe_rk:
+        w("    flex::swe_rk_row<V>(p, row, v, own);")
     else:
         for n, d, off, _ in reducers:
             for j in range(d):
                 w(f"    p.out_{n}[row * {d} + {j}] = v[{off + j}];")
-        w("    (void)p; (void)row; (void)v;")
+        w("    (void)p; (void)row; (void)v; (void)own;")
     w("  }")
     w("  __device__ __forceinline__ static void prefetch_rows(const Params& p, long long row0, long long row1, int lane) {")
     if swe_rk:      # one array per lane: the cell's own records and what the epilogue reads (the running sums from stage 2 on)

@@ -29,6 +29,8 @@
 
 namespace flex {
 
+struct NoOwn {};       // what finish_row reads of a row itself in graphs without an epilogue
+
 template <int BLOCK_, int IPT_, int STAGES_, int MIN_CTAS_, int BATCH_ = 8, bool PIPELINE_ = false, int ROW_BATCH_ = BATCH_>
 struct TileCfg {
   // software pipelining across tiles (gathers of tile k in flight while tile k-1 is reduced); measured
@@ -358,7 +360,9 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
             if (e0 + b < n) G::map(p, er[b], e_from + e0 + b, grow, ge[b], sum);
         }
         if (small_row + BLOCK + 32 < small_end) { row_from = row_offsets[small_row + BLOCK + 32]; row_to = row_offsets[small_row + BLOCK + 33]; }
-        G::finish_row(p, small_row, sum);
+        typename G::GOwn own;
+        G::load_own(p, small_row, own);
+        G::finish_row(p, small_row, sum, own);
       }
       return;
     }
@@ -698,7 +702,11 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
           }
-          if (r < c.nrows) G::finish_row(p, c.row0 + r, sum);
+          if (r < c.nrows) {
+            typename G::GOwn own;
+            G::load_own(p, c.row0 + r, own);
+            G::finish_row(p, c.row0 + r, sum, own);
+          }
         }
         turn = (turn + groups) % Cfg::kWarps;
         if (++s == L::kRowStages) { s = 0; parity ^= 1u; }
