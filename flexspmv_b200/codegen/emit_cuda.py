@@ -172,6 +172,17 @@ TUNED_CONFIGS = {
 }
 
 
+# Row-mode graphs: one large CTA an SM for large launches of short rows (GraphApi::use_big; consumer threads, merge items per thread,
+# stages, CTAs per SM).  A tile of 4 items a thread is a row of three edges a thread, less one item each.  us on meshes of 1024^2
+# squares, CTAs an SM x warps: the shallow-water step 3 x 9 368, 1 x 24 332 (tiles of 3 items a thread 367, of 5 370), 1 x 28 367, 2 x 12
+# 363, 1 x 20 363; Rusanov fp64 3 x 9 76.3, 1 x 24 74.0, 1 x 28 77.0, 2 x 12 76.2; fp32 4 x 9 48.9, 1 x 32 45.8, 1 x 28 48.0, 1 x 24 52.0.
+TUNED_BIG_CONFIGS = {
+    "rusanov_f64": (736, 4, 2, 1),
+    "rusanov_f32": (992, 4, 2, 1),
+    "swe_delta_f64": (736, 4, 2, 1),
+}
+
+
 # Configuration of the warp kernel for matrices whose gathers have no locality (csrc/flex_warp_kernel.cuh):
 # (threads per CTA, merge items per lane, min CTAs per SM).  It is built for graphs whose gathers all depend on the
 # edge and whose accumulator is at most 16 bytes wide (its one shared-memory buffer holds a product per item, and
@@ -721,6 +732,12 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         w(f"using CfgLean = flex::WarpCfg<{lb}, {li}, {lm}>;      // the warp kernel for matrices with random columns")
     else:
         w("using CfgLean = flex::NoLean;")
+    big = _override(symbol + "_big") or TUNED_BIG_CONFIGS.get(f"{ir.name}_{sfx}")
+    if big:
+        bb, bi, bs, bm = big[:4]
+        w(f"using CfgBig = flex::TileCfg<{bb}, {bi}, {bs}, {bm}, {batch}, false, {row_batch}>;      // for large launches")
+    else:
+        w("using CfgBig = flex::NoBig;")
     w(f"}}  // namespace gen_{symbol}")
     w("}  // namespace")
     for i_, line in enumerate(L):
@@ -729,7 +746,7 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         elif line == "@@GROW_BODY@@":
             L[i_] = "\n".join(row_body) if grow_fields else "    // (nothing to evaluate per row)"
     ns = f"gen_{symbol}::"
-    w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean)")
+    w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns}CfgBig)")
     if static_scratch_bytes:
         w(f"FLEXSPMV_DEFINE_STATIC_SCRATCH_LAUNCH({symbol}, {ns}Graph, {ns}Cfg, {int(static_scratch_bytes)})")
     return "\n".join(L) + "\n"

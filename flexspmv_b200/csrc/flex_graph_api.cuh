@@ -1,5 +1,5 @@
 // Host side of one generated graph: workspace sizing, planning (merge-path partition into the
-// workspace), launch.  FLEXSPMV_DEFINE_GRAPH(symbol_suffix, GraphStruct, Cfg) emits the five
+// workspace), launch.  FLEXSPMV_DEFINE_GRAPH(symbol_suffix, GraphStruct, Cfg...) emits the five
 // extern "C" entry points declared by FLEXSPMV_DECLARE_GRAPH in include/flexspmv.h.
 //
 // Replaces the reference's host dispatch (merged_spmv_dispatch / merged_spmv_launch,
@@ -62,8 +62,13 @@ struct NoLean {      // in place of CfgLean: the warp kernel for matrices with r
   static constexpr int kChunk = 0;
 };
 
-template <class G, class Cfg, class CfgWin = Cfg, class CfgLean = NoLean>
+struct NoBig {       // in place of CfgBig: one configuration of the tile kernel for launches of every size
+  static constexpr int kTile = 0, kIpt = 0, kMinCtas = 1;
+};
+
+template <class G, class Cfg, class CfgWin = Cfg, class CfgLean = NoLean, class CfgBig = NoBig>
 struct GraphApi {
+  static constexpr bool kBigBuilt = !std::is_same_v<CfgBig, NoBig>;
   static constexpr bool kWindowsBuilt = !std::is_same_v<CfgWin, NoWindows>;
   static constexpr bool kLeanBuilt = !std::is_same_v<CfgLean, NoLean>;
   using V = typename G::V;
@@ -87,6 +92,37 @@ struct GraphApi {
     if constexpr (G::kHasReducer && kLeanBuilt) return (d->reserved & FLEXSPMV_FLAG_RANDOM_GATHER) != 0;
     return false;
   }
+  // Launches of more than a tile for each SM, of rows about as short as the configuration was made for, run one large CTA an SM
+  // (CfgBig), unless the launch is a small one.  The row-mode loop is bound by what an SM has in flight: its 24 warps at the 80
+  // registers of one CTA of 768 threads spill nothing (three CTAs of 288: 72 registers, 48 - 156 bytes), share one stage of a group
+  // of 32 rows for every warp, and the one producer's book-keeping is per 735 rows instead of 191 or 255.  us, CfgBig / Cfg:
+  //   shallow-water step fp64  260^2 45.0 / 49.4, 310^2 52.8 / 66.7, 400^2 78.0 / 88.3, 520^2 102.9 / 121.4, 800^2 221 / 248, 1024^2 332 / 368, 1200^2
+  //                            455 / 503; 200^2, a small launch there: 32.8 / 28.4
+  //   Rusanov fp64             400^2 15.3 / 15.6, 450^2 18.7 / 19.8, 520^2 23.4 / 24.6, 800^2 48.0 / 50.0, 1024^2 74.0 / 76.3, 1200^2 100 / 106
+  //   Rusanov fp32             450^2 11.4 / 12.3, 520^2 14.1 / 15.8, 800^2 29.4 / 32.9, 1024^2 45.8 / 48.9, 1200^2 59.3 / 64.0
+  // A tile has to hold about a row a thread (7 to 11 for ten), or warps wait for a stage, or go round it twice.  8 M items: rows of 8 Rusanov fp64
+  // 116 / 103, fp32 59.4 / 56.8, swe_delta fp64 102 / 98; of 6 81.8 / 85.0, 47.7 / 46.4, 68.9 / 76.9; of 4 76.7 / 83.6, 45.4 / 46.4, 64.9 / 71.8; of 1 - 7
+  // 103.8 / 114.4, 59.4 / 67.3, 77.6 / 89.8; of 2 76.6 / 81.8, 47.7 / 49.2, 70.6 / 65.4 (3 M items: 32.9 / 36.7, 20.7 / 20.1, 30.4 / 28.4); of 3, one of them of 40
+  // (not whole rows) 98.0 / 104.3, 64.6 / 67.5, 77.2 / 94.1 (1 M items, swe_delta: 21.8 / 21.1).
+  // Callers that name a tile or a number of CTAs get the configuration that they know.
+  static constexpr int kBigTile = CfgBig::kTile - CfgBig::kIpt;
+  static bool use_big(const flexspmv_desc* d) {
+    if constexpr (kBigBuilt) {
+      const long long sms = device_sm_count(), items = d->num_rows + d->num_edges;
+      if (d->tile_items > 0 || d->max_ctas > 0 || use_lean(d) || use_win(d)) return false;
+      const long long ten_rows = 10 * d->num_rows * kBigTile, each_a_row = items * CfgBig::kBlock;
+      if (items <= sms * CfgBig::kMinCtas * kBigTile || ten_rows < 7 * each_a_row || ten_rows > 11 * each_a_row) return false;
+      const long long tiles = (items + kDefaultTile - 1) / kDefaultTile, slots = sms * Cfg::kMinCtas;
+      return !small_launch(d, tiles, tiles < slots ? tiles : slots, Cfg::kBlock + 32);
+    }
+    return false;
+  }
+  // Up to 16 tiles a CTA are made equal in number: with tiles of one size 7.07 a CTA are as long as 8.
+  static int big_tile(const flexspmv_desc* d) {
+    const long long ctas = (long long)device_sm_count() * CfgBig::kMinCtas, items = d->num_rows + d->num_edges;
+    const long long each = (items + ctas * kBigTile - 1) / (ctas * kBigTile);
+    return (int)(each <= 16 ? (items + ctas * each - 1) / (ctas * each) : kBigTile);
+  }
   static int compiled_tile(const flexspmv_desc* d) {
     if (use_lean(d)) return CfgLean::kChunk;
     return use_win(d) ? CfgWin::kTile : Cfg::kTile;
@@ -98,6 +134,7 @@ struct GraphApi {
   static int tile_items(const flexspmv_desc* d) {
     if (d->tile_items > 0) return d->tile_items;
     if (use_lean(d)) return CfgLean::kChunk;
+    if (use_big(d)) return big_tile(d);
     return use_win(d) ? CfgWin::kTile : kDefaultTile;
   }
   static int max_ctas(const flexspmv_desc* d, int resident) {
@@ -170,6 +207,11 @@ struct GraphApi {
     return room;
   }
 
+  static TileRoom room_of(const flexspmv_desc* d) {
+    if constexpr (kBigBuilt) if (use_big(d)) return tile_room<CfgBig>(d);
+    return tile_room<Cfg>(d);
+  }
+
   // `whole_rows`: also look for a matrix of short rows whose tiles can all hold whole rows.
   // `indices` (may be null): the launch's index arrays, which the choice of the loop on such tiles looks at.
   static int plan(const flexspmv_desc* d, const void* const* indices, const void* row_offsets, void* ws, size_t ws_bytes, cudaStream_t st,
@@ -198,7 +240,12 @@ struct GraphApi {
         if constexpr (G::kWindowGather && kWindowsBuilt) {
           if (win) e = d->offset_bits == 64 ? resident_ctas<long long, CfgWin, true>(&resident) : resident_ctas<int, CfgWin, true>(&resident);
         }
-        if (!win) e = d->offset_bits == 64 ? resident_ctas<long long>(&resident) : resident_ctas<int>(&resident);
+        bool big = false;
+        if constexpr (kBigBuilt) {
+          big = use_big(d);
+          if (big) e = d->offset_bits == 64 ? resident_ctas<long long, CfgBig>(&resident) : resident_ctas<int, CfgBig>(&resident);
+        }
+        if (!win && !big) e = d->offset_bits == 64 ? resident_ctas<long long>(&resident) : resident_ctas<int>(&resident);
         if (e) return e;
         const long long most = max_ctas(d, resident);
         grid = (int)(most < h.num_tiles ? most : h.num_tiles);
@@ -211,16 +258,16 @@ struct GraphApi {
         if (rule.edge_lanes && indices && d->num_edges > 0)
           rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
         for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
-        if (grid > 0 && small_launch(d, h.num_tiles, grid, Cfg::kBlock + 32)) {
+        if (grid > 0 && !use_big(d) && small_launch(d, h.num_tiles, grid, Cfg::kBlock + 32)) {
           rule.share_items = 3 * ((h.num_tiles + grid - 1) / grid) * tile_items(d) / 2;
           rule.share_row_edges = kSmallRowEdges;
         }
         // rows longer than kWholeRowMax on average: no need to look
         if (whole_rows && !use_win(d) && d->num_rows > 0 && d->num_edges <= (long long)kWholeRowMax * d->num_rows)
-          return whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, tile_room<Cfg>(d), rule, grid, coords, ws, st);
+          return whole_rows_launch(row_offsets, d->offset_bits, d->num_rows, d->num_edges, h.num_tiles, room_of(d), rule, grid, coords, ws, st);
       }
       // boundaries between the CTAs of that grid moved onto row ends where the tiles have room
-      TileRoom room = tile_room<Cfg>(d);
+      TileRoom room = room_of(d);
       if constexpr (G::kWindowGather && kWindowsBuilt) { if (win) room = tile_room<CfgWin>(d); }
       return snap_cta_boundaries_launch(row_offsets, d->offset_bits, d->num_rows, h.num_tiles, grid, room, coords, ws, st);
     } else {
@@ -335,12 +382,17 @@ struct GraphApi {
     int form = FLEXSPMV_KERNEL_TILE;
     if constexpr (L::kWhole) if (whole_rows) {
       const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
-      if (small_launch(d, tiles, grid, kThreads)) {
-        form = FLEXSPMV_KERNEL_TILE_SMALL;
-        kernel = flex_tile_kernel<G, OffsetT, C, WIN, kSmall>;
-        if (int e = resident_ctas<OffsetT, C, WIN, kSmall>(&resident)) return e;      // the grid stays the plan's
-      } else if (vertices * G::kGatherRecordBytes > kKeepBytes && tiles >= grid * kTileRun) {
-        a.rounds = (int)(tiles / (grid * kTileRun));
+      bool small = false;
+      if constexpr (!std::is_same_v<C, CfgBig>) {
+        small = small_launch(d, tiles, grid, kThreads);
+        if (small) {
+          form = FLEXSPMV_KERNEL_TILE_SMALL;
+          kernel = flex_tile_kernel<G, OffsetT, C, WIN, kSmall>;
+          if (int e = resident_ctas<OffsetT, C, WIN, kSmall>(&resident)) return e;      // the grid stays the plan's
+        }
+      }
+      if (!small && vertices * G::kGatherRecordBytes > kKeepBytes && tiles >= grid * C::kTileRun) {
+        a.rounds = (int)(tiles / (grid * C::kTileRun));
         form = FLEXSPMV_KERNEL_TILE_ROUNDS;
         kernel = flex_tile_kernel<G, OffsetT, C, WIN, kRounds>;
         if (int e = resident_ctas<OffsetT, C, WIN, kRounds>(&resident)) return e;
@@ -462,6 +514,12 @@ struct GraphApi {
           return launch_tiles<int, CfgWin, true>(d, p, row_offsets, ws, h, st, whole_rows);
         }
       }
+      if constexpr (kBigBuilt) {
+        if (use_big(d)) {
+          if (d->offset_bits == 64) return launch_tiles<long long, CfgBig>(d, p, row_offsets, ws, h, st, whole_rows);
+          return launch_tiles<int, CfgBig>(d, p, row_offsets, ws, h, st, whole_rows);
+        }
+      }
       if (d->offset_bits == 64) return launch_tiles<long long>(d, p, row_offsets, ws, h, st, whole_rows);
       return launch_tiles<int>(d, p, row_offsets, ws, h, st, whole_rows);
     } else {
@@ -490,28 +548,28 @@ struct GraphApi {
 
 }  // namespace flex
 
-#define FLEXSPMV_DEFINE_GRAPH(SYM, GRAPH, CFG, CFGWIN, CFGLEAN)                                                          \
+#define FLEXSPMV_DEFINE_GRAPH(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG)                                                          \
   extern "C" {                                                                                                  \
-  int flexspmv_##SYM##_info(flexspmv_graph_info* info) { return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::info(info); } \
+  int flexspmv_##SYM##_info(flexspmv_graph_info* info) { return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::info(info); } \
   int flexspmv_##SYM##_workspace_bytes(const flexspmv_desc* d, size_t* b) {                                     \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::workspace_bytes(d, b);                                           \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::workspace_bytes(d, b);                                           \
   }                                                                                                             \
   int flexspmv_##SYM##_plan(const flexspmv_desc* d, const void* ro, void* ws, size_t wb, void* st) {            \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan(d, nullptr, ro, ws, wb, static_cast<cudaStream_t>(st));     \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::plan(d, nullptr, ro, ws, wb, static_cast<cudaStream_t>(st));     \
   }                                                                                                             \
   int flexspmv_##SYM##_plan_indexed(const flexspmv_desc* d, const void* const* ix, const void* ro, void* ws, size_t wb, void* st) { \
     if (!ix) return FLEXSPMV_ERR_BAD_ARG;                                                                       \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan(d, ix, ro, ws, wb, static_cast<cudaStream_t>(st));          \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::plan(d, ix, ro, ws, wb, static_cast<cudaStream_t>(st));          \
   }                                                                                                             \
   int flexspmv_##SYM##_plan_windows(const flexspmv_desc* d, const void* const* ix, void* ws, size_t wb, void* st) { \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::plan_windows(d, ix, ws, wb, static_cast<cudaStream_t>(st));      \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::plan_windows(d, ix, ws, wb, static_cast<cudaStream_t>(st));      \
   }                                                                                                             \
   int flexspmv_##SYM##_launch(const flexspmv_desc* d, const void* const* v, const void* const* ix,              \
                               const void* ro, void* const* o, void* ws, size_t wb, void* st) {                  \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st));  \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st));  \
   }                                                                                                             \
   int flexspmv_##SYM##_device_status(const void* ws, int32_t* out, void* st) {                                  \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN>::device_status(ws, out, static_cast<cudaStream_t>(st));           \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::device_status(ws, out, static_cast<cudaStream_t>(st));           \
   }                                                                                                             \
   }
 

@@ -45,6 +45,9 @@ struct TileCfg {
   static constexpr int kWarps = BLOCK_ / 32;
   static constexpr int kBatch = BATCH_;   // edges of one row whose gathers are in flight together (short-row tiles)
   static constexpr int kRowBatch = ROW_BATCH_;   // the same in the loop over whole rows
+  // consecutive tiles of a CTA where whole rows go round the CTAs (TileKernelArgs::rounds); large tiles go round one by one: 1024^2
+  // shallow-water step 333 us, in runs of two 336, of four 353; Rusanov 74.0, 76.6, 77.7
+  static constexpr int kTileRun = kTile >= 2560 ? 1 : 4;
 };
 
 // Whether the plan may move all tile boundaries of the graph to row starts, and the kernel has the loop over whole rows, one
@@ -55,7 +58,6 @@ struct WholeRows {
   static constexpr bool value = !WIN && !G::kDirectLoads && !Cfg::kPipeline && !G::kStoresPerEdge;
 };
 
-constexpr int kTileRun = 4;               // consecutive tiles of a CTA where whole rows go round the CTAs (TileKernelArgs::rounds)
 constexpr int kMaxCtas = 2048;            // capacity of the per-CTA carry arrays in the workspace
 #ifndef FLEX_SHORT_ROW_MAX
 #define FLEX_SHORT_ROW_MAX 64
@@ -277,6 +279,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
   // is the faster order at the same traffic: 592 CTAs read one stretch of each array, not 592.  us, own runs / rounds of 4, 8, 16, 32, 64 tiles:
   // 512^3 2529 / 2133, 2146, 2161, 2214, 2328; 300^3 480 / 422, 429, 434, 443, 464; 400^3 fp32 905 / 821, 827, 835, 839, 846; 5-point 3000^2 128 / 118, 122, 123,
   // 125, 126.
+  constexpr int kTileRun = Cfg::kTileRun;
   auto round_tile = [&](int k) -> long long {
     if (k < a.rounds * kTileRun) return ((long long)(k / kTileRun) * gridDim.x + blockIdx.x) * kTileRun + k % kTileRun;
     return t_begin + (long long)a.rounds * kTileRun * (gridDim.x - 1 - blockIdx.x) + k;
