@@ -736,8 +736,6 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     if big:
         bb, bi, bs, bm = big[:4]
         w(f"using CfgBig = flex::TileCfg<{bb}, {bi}, {bs}, {bm}, {batch}, false, {row_batch}>;      // for large launches")
-    else:
-        w("using CfgBig = flex::NoBig;")
     w(f"}}  // namespace gen_{symbol}")
     w("}  // namespace")
     for i_, line in enumerate(L):
@@ -746,7 +744,10 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         elif line == "@@GROW_BODY@@":
             L[i_] = "\n".join(row_body) if grow_fields else "    // (nothing to evaluate per row)"
     ns = f"gen_{symbol}::"
-    w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns}CfgBig)")
+    if big:
+        w(f"FLEXSPMV_DEFINE_GRAPH_BIG({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns}CfgBig)")
+    else:
+        w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean)")
     if static_scratch_bytes:
         w(f"FLEXSPMV_DEFINE_STATIC_SCRATCH_LAUNCH({symbol}, {ns}Graph, {ns}Cfg, {int(static_scratch_bytes)})")
     return "\n".join(L) + "\n"

@@ -548,7 +548,9 @@ struct GraphApi {
 
 }  // namespace flex
 
-#define FLEXSPMV_DEFINE_GRAPH(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG)                                                          \
+// a graph with one configuration of the tile kernel
+#define FLEXSPMV_DEFINE_GRAPH(SYM, GRAPH, CFG, CFGWIN, CFGLEAN) FLEXSPMV_DEFINE_GRAPH_BIG(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, flex::NoBig)
+#define FLEXSPMV_DEFINE_GRAPH_BIG(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG)                                                          \
   extern "C" {                                                                                                  \
   int flexspmv_##SYM##_info(flexspmv_graph_info* info) { return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::info(info); } \
   int flexspmv_##SYM##_workspace_bytes(const flexspmv_desc* d, size_t* b) {                                     \
