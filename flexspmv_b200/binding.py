@@ -144,6 +144,7 @@ class _Symbols:
         gi = GraphInfo()
         check(lib, self.info(ctypes.byref(gi)), f"{sym}_info")
         self.graph_info = gi
+        self.also, self.name = fn, lambda what: f"flexspmv_{sym}_{what}"
 
 
 class GraphExtension:
@@ -382,6 +383,18 @@ class GraphExtension:
             plan, desc = self._plan_for(syms, values, indices, row_end_offsets, num_rows, num_edges, num_cols, device)
         return PreparedLaunch(self, syms, desc, list(values), list(indices), row_end_offsets if self._has_reducer else None,
                               list(outputs), plan)
+
+    def prepare_step(self, values: Sequence[torch.Tensor], indices: Sequence[torch.Tensor], row_end_offsets: torch.Tensor,
+                     outputs: Sequence[torch.Tensor], num_rows: int, num_edges: int, num_cols: int = 0) -> "Optional[PreparedLaunch]":
+        """``prepare`` for a graph whose unit has a launch over all stages of a step (include/flexspmv.h,
+        swe_delta_rk_T_step); None where the problem does not fit that launch."""
+        syms = self._by_type(values[0].dtype)
+        launch = self.prepare(values, indices, row_end_offsets, outputs, num_rows, num_edges, num_cols)
+        with torch.cuda.device(values[0].device):
+            if not syms.also("step_fits")(ctypes.byref(launch._desc)):
+                return None
+        launch._fn = _LAUNCH((syms.name("step"), self.lib))
+        return launch
 
     def device_status(self, dtype: torch.dtype, row_end_offsets: Optional[torch.Tensor] = None) -> int:
         """Reads back the status word of the most recently used workspace (synchronises)."""

@@ -311,6 +311,7 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w('#include "flex_graph_api.cuh"')
     if swe_rk:
         w('#include "flex_swe_rk.cuh"')
+        w('#include "flex_swe_step.cuh"')
     extra = SWE_RK_FIELDS if swe_rk else []
     w("namespace {")
     w(f"namespace gen_{symbol} {{      // several generated units may share one translation unit")
@@ -443,10 +444,14 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     if not edge_sel:
         w("    int unused;")
     w("  };")
+    # a launch over several stages gathers what it has written itself
+    gather = "fx::gather_vec<FIXED, V, {}>" if swe_rk else "fx::ldg_vec<V, {}>"
+    if swe_rk:
+        w("  template <bool FIXED = true>      // nothing writes the gathered vectors during the launch")
     w("  __device__ __forceinline__ static void gather_row(const Params& p, long long row, GRow& g) {")
     for s in row_sel:
         d = dim_of(s["shape"])
-        w(f"    g.{s['name']} = fx::ldg_vec<V, {d}>(p.{s['target']} + row * {d});")
+        w(f"    g.{s['name']} = {gather.format(d)}(p.{s['target']} + row * {d});")
     w("@@GROW_BODY@@")
     w("    (void)p; (void)row; (void)g;")
     w("  }")
@@ -520,10 +525,12 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
     w("    (void)indices; (void)index; (void)record_bytes; (void)most;")
     w("    return n;")
     w("  }")
+    if swe_rk:
+        w("  template <bool FIXED = true>")
     w("  __device__ __forceinline__ static void gather_edge(const Params& p, const EReg& r, GEdge& g) {")
     for s_ in edge_sel:
         d = dim_of(s_["shape"])
-        w(f"    g.{s_['name']} = fx::ldg_vec<V, {d}>(p.{s_['target']} + (long long)r.idx_{s_['selector_name']} * {d});")
+        w(f"    g.{s_['name']} = {gather.format(d)}(p.{s_['target']} + (long long)r.idx_{s_['selector_name']} * {d});")
     w("    (void)p; (void)r; (void)g;")
     w("  }")
     # gather windows: a two-phase graph with exactly one index array and one gathered tensor whose record is a
@@ -748,6 +755,8 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         w(f"FLEXSPMV_DEFINE_GRAPH_BIG({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns}CfgBig)")
     else:
         w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean)")
+    if swe_rk:
+        w(f"FLEXSPMV_DEFINE_STEP({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns + 'CfgBig' if big else 'flex::NoBig'})")
     if static_scratch_bytes:
         w(f"FLEXSPMV_DEFINE_STATIC_SCRATCH_LAUNCH({symbol}, {ns}Graph, {ns}Cfg, {int(static_scratch_bytes)})")
     return "\n".join(L) + "\n"

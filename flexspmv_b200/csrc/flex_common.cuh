@@ -56,7 +56,9 @@ struct WorkspaceHeader {
   uint32_t line_edges, line_edge_lines;     // cache lines their middle edges gather from; consecutive edges and their lines
   int32_t uneven_shares;       // 1: with equal shares of the rows a CTA of the plan's grid would have more than RowLoopRule allows; 2 is added
                                // while a test withholds a stage (not 0: a small launch runs its loop with stages)
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4];
+  int32_t unused;
+  uint64_t step_barrier;       // CTAs that have come to a barrier of a whole-step launch (flex_swe_step.cuh), over all launches
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4 - 4 - 8];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"

@@ -232,6 +232,12 @@ __device__ __forceinline__ Vec<V, D> ld_vec(P p) {   // plain load through anyth
   for (int i = 0; i < D; ++i) r.v[i] = p[i];
   return r;
 }
+// A gathered record: through the read-only path where nothing writes it during the launch (FIXED).
+template <bool FIXED, typename V, int D>
+__device__ __forceinline__ Vec<V, D> gather_vec(const V* p) {
+  if constexpr (FIXED) return ldg_vec<V, D>(p);
+  else return ld_vec<V, D>(p);
+}
 
 template <typename V, int D>
 __device__ __forceinline__ void st_vec(V* p, const Vec<V, D>& a) {

@@ -10,7 +10,9 @@ stage's per-cell arithmetic -- wall terms, ``-(...)/area``, the Runge-Kutta upda
 cell's finished flux sums (csrc/flex_swe_rk.cuh), bound once with ``GraphExtension.prepare``.  Meshes whose
 cells are too irregular for that kernel (a cell with more than 32 edges), and steps with operator objects of the
 caller's, run a stage as three launches with the same results, bit for bit: ``swe_delta``, ``swe_boundary``,
-``flexspmv_swe_rk_stage``.  ``capture()`` records the whole step (4 launches, or 12) into one CUDA graph.
+``flexspmv_swe_rk_stage``.  Meshes that fit the chip (about 290 000 cells in fp64) run all four stages in one cooperative
+launch (csrc/flex_swe_step.cuh), again with the same bits.  ``capture()`` records the whole step (1 launch, 4, or 12) into one
+CUDA graph.
 
 Edges must be sorted by destination cell and ``bcells`` ascending: both Reducers then see sorted indices,
 which is what the merge-path kernels need (python_wrapper/dynamic_replace_submodule.py:20-41 makes the
@@ -81,6 +83,7 @@ class ShallowWaterStep:
         other = new(3)
         state = [m["h"], m["uh"], m["vh"]]
         launches = []
+        self._step = None
         self._coef, self._coef_dt = [], float(self.dt)
         for k, (c, first, last) in enumerate(self._coefficients()):
             src = state if k == 0 else (self.stage if k % 2 else other)
@@ -92,6 +95,12 @@ class ShallowWaterStep:
             launches.append(ext.prepare(values, [m["src"], m["dst"]], self.ro, dst, self.nc, self.ne, self.nc))
             if k == 0 and not ext.planned_whole_rows():
                 return None
+        # meshes that fit the chip: the four stages in one launch (csrc/flex_swe_step.cuh); the coefficients side by side
+        all_coef = torch.stack(self._coef).contiguous()
+        values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [all_coef]
+        self._step = ext.prepare_step(values, [m["src"], m["dst"]], self.ro, self.stage + other, self.nc, self.ne, self.nc)
+        if self._step is not None:
+            self._coef = list(all_coef)            # rows of it: set where the time step changes
         return launches
 
     def _bind(self, h, uh, vh):
@@ -120,7 +129,7 @@ class ShallowWaterStep:
                 for coef, (c, first, last) in zip(self._coef, self._coefficients()):
                     coef.copy_(torch.tensor([c, dt / 6, first, last], dtype=coef.dtype, device="cpu"))
                 self._coef_dt = dt
-            for launch in self._fused:
+            for launch in [self._step] if self._step is not None else self._fused:
                 launch.launch()
             return
         for k, (c, first, last) in enumerate(self._coefficients()):

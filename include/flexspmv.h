@@ -134,7 +134,8 @@ enum {
   FLEXSPMV_KERNEL_TILE_ROUNDS = 3, /* ... where tiles of whole rows go round the CTAs */
   FLEXSPMV_KERNEL_WARP = 4,        /* warp kernel for columns without locality */
   FLEXSPMV_KERNEL_WARP_AHEAD = 5,  /* ... for few chunks a warp */
-  FLEXSPMV_KERNEL_EDGE = 6         /* graphs without a reducer */
+  FLEXSPMV_KERNEL_EDGE = 6,        /* graphs without a reducer */
+  FLEXSPMV_KERNEL_STEP = 7         /* whole step of the shallow-water model (swe_delta_rk_*) */
 };
 int flexspmv_debug_last_kernel(void);
 
@@ -350,7 +351,24 @@ FLEXSPMV_DECLARE_GRAPH(edge_copy_i64)
  * The workspace's plan must hold whole rows (flexspmv_workspace_whole_rows): otherwise launch raises
  * FLEXSPMV_ERR_NOT_PLANNED in the workspace status and writes nothing.  flexspmv_b200/shallow_water.py binds a step.
  */
-#define FLEXSPMV_DECLARE_EPILOGUE_GRAPH(G) FLEXSPMV_DECLARE_GRAPH(G)
+/*
+ * swe_delta_rk_T_step: the four stages of a step in one cooperative launch, for meshes whose edges' records and cells' sums fit
+ * the shared memory of all SMs.  The arrays of the first stage's launch, with
+ *   values[3..5] and values[11..13]   the state at the beginning of the step, advanced in place
+ *   values[14..16]                    scratch
+ *   values[17]                        a HOST pointer to four times four T: c, w, first, last of every stage
+ *   outputs[0..2]                     the state that the second and fourth stage's fluxes are evaluated at (scratch)
+ *   outputs[3..5]                     and the third one's
+ * on a workspace that was planned with whole rows (FLEXSPMV_ERR_NOT_PLANNED in its status otherwise, nothing written).  Results
+ * are those of the four launches, bit for bit.  FLEXSPMV_ERR_TOO_LARGE where the mesh does not fit; swe_delta_rk_T_step_fits
+ * says so beforehand (1: it fits).  A wait of the launch's CTAs for one another that takes more than a second raises
+ * FLEXSPMV_ERR_TIMEOUT in the workspace status; later launches on the workspace then do nothing until it is planned again.
+ */
+#define FLEXSPMV_DECLARE_EPILOGUE_GRAPH(G)                                                                                  \
+  FLEXSPMV_DECLARE_GRAPH(G)                                                                                                 \
+  int flexspmv_##G##_step_fits(const flexspmv_desc *desc);                                                                  \
+  int flexspmv_##G##_step(const flexspmv_desc *desc, const void *const *values, const void *const *indices, const void *row_offsets, \
+                          void *const *outputs, void *workspace, size_t workspace_bytes, void *stream);
 FLEXSPMV_DECLARE_EPILOGUE_GRAPH(swe_delta_rk_f64)
 FLEXSPMV_DECLARE_EPILOGUE_GRAPH(swe_delta_rk_f32)
 

@@ -1,0 +1,116 @@
+"""A whole step of the shallow-water model in one cooperative launch against the launches of a stage each: the same bits."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from flexspmv_b200 import graphs
+from flexspmv_b200.binding import FlexSpmvError, GraphExtension, load_library
+from flexspmv_b200.shallow_water import ShallowWaterStep
+from test_gpu_swe_fused import mesh_of
+
+pytestmark = pytest.mark.gpu
+STEP = 7            # FLEXSPMV_KERNEL_STEP of include/flexspmv.h
+STATE = ("h", "uh", "vh")
+
+
+def both(mesh, steps=2, dt=1e-4):
+    """The state after some steps in one launch each, and in four; what ran last in the first form."""
+    a, b = mesh, {k: v.clone() for k, v in mesh.items()}
+    one, four = ShallowWaterStep(a, dt=dt), ShallowWaterStep(b, dt=dt)
+    assert one._step is not None and four._fused is not None
+    four._step = None
+    for launch, coef in zip(four._fused, one._coef):        # (the coefficients that four launches read are their own)
+        launch._keep[0][-1].copy_(coef)
+    for _ in range(steps):
+        one.forward()
+        kernel = load_library().flexspmv_debug_last_kernel()
+        four.forward()
+    torch.cuda.synchronize()
+    return a, b, kernel
+
+
+@pytest.mark.parametrize("n,walls", [(16, True), (33, "everywhere"), (97, False), (150, True), (200, "everywhere"), (270, False), (330, True)])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_one_launch_equals_four(n, walls, dtype):
+    """One cell a thread and several rounds, in CTAs of both sizes; cells with no, one and several wall records."""
+    a, b, kernel = both(mesh_of(n, dtype, walls), dt=0.01 / n)
+    assert kernel == STEP
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_edges_that_a_cta_cannot_keep(dtype):
+    """Cells of 25 edges side by side: their CTAs have more edges than shared memory was claimed for, and read the others in place."""
+    m = mesh_of(160, dtype, True)
+    cells = m["h"].numel()
+    many = torch.arange(20_000, 21_000, dtype=torch.int32, device="cuda").repeat_interleave(22)
+    src = torch.randint(0, cells, (many.numel(),), generator=torch.Generator().manual_seed(3)).to(torch.int32).cuda()
+    order = torch.argsort(torch.cat([m["dst"], many]).long(), stable=True)
+    for k, extra in (("src", src), ("dst", many)):
+        m[k] = torch.cat([m[k], extra])[order].contiguous()
+    for k, c in (("alpha", 0.5), ("sx", 1e-7), ("sy", -2e-7)):
+        m[k] = torch.cat([m[k], torch.full((many.numel(),), c, dtype=m[k].dtype, device="cuda")])[order].contiguous()
+    a, b, kernel = both(m, dt=1e-4)
+    assert kernel == STEP
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n,fits", [(380, True), (400, False)])
+def test_meshes_that_do_not_fit_take_four_launches(n, fits):
+    """About 1980 cells of three edges an SM in fp64."""
+    step = ShallowWaterStep(mesh_of(n, np.float64, False), dt=1e-5)
+    assert step._fused is not None and (step._step is not None) == fits
+    step.forward()
+    assert (load_library().flexspmv_debug_last_kernel() == STEP) == fits
+
+
+def bind(m, bits):
+    """The step through the operator object with 32- or 64-bit offsets; scratch filled with NaN."""
+    nc, ne, V = m["h"].numel(), m["src"].numel(), m["h"].dtype
+    ro = torch.searchsorted(m["dst"], torch.arange(nc + 1, dtype=torch.int32, device="cuda")).to(torch.int32 if bits == 32 else torch.int64)
+    walls = torch.searchsorted(m["bcells"], torch.arange(0, nc + 32, 32, dtype=torch.int32, device="cuda")).to(torch.int32)
+    state = [m[k] for k in STATE]
+    nan = lambda k: [torch.full((nc,), float("nan"), dtype=V, device="cuda") for _ in range(k)]
+    coef = torch.tensor([[5e-5, 2e-5, 1, 0], [5e-5, 2e-5, 0, 0], [1e-4, 2e-5, 0, 0], [0, 2e-5, 0, 1]], dtype=V)
+    values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], walls, m["bcells"]] + state + nan(3) + [coef]
+    ext = GraphExtension(graphs.swe_delta_graph(), symbol_prefix="swe_delta_rk")
+    return ext, ext.prepare_step(values, [m["src"], m["dst"]], ro, nan(6), nc, ne, nc)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_offsets_of_either_width(dtype):
+    a, b = mesh_of(70, dtype, True), mesh_of(70, dtype, True)
+    for m, bits in ((a, 32), (b, 64)):
+        ext, step = bind(m, bits)
+        step.launch()
+        ext.check()
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+
+
+def test_a_barrier_that_stays_shut_runs_out():
+    """A CTA that never arrives (testing aid): the others wait for a second, the status says so, the context stays usable, a later launch
+    on the workspace writes nothing, and a newly planned one runs."""
+    m = mesh_of(64, np.float64, False)
+    before = {k: m[k].clone() for k in STATE}
+    ext, step = bind(m, 32)
+    lib, ws = load_library(), step._keep[-1]
+    lib.flexspmv_debug_withhold_stage.restype = ctypes.c_int
+    assert lib.flexspmv_debug_withhold_stage(ctypes.c_void_p(ws.data_ptr()), ctypes.c_uint32(1), None) == 0
+    torch.cuda.synchronize()
+    step.launch()
+    with pytest.raises(FlexSpmvError, match="status -6"):
+        ext.check()
+    assert all(torch.equal(m[k], before[k]) for k in STATE)
+    step._plan._flag_view[0] = 0                 # as if the host had not noticed
+    step.launch()
+    torch.cuda.synchronize()
+    assert all(torch.equal(m[k], before[k]) for k in STATE)
+    ext, step = bind(m, 32)
+    step.launch()
+    ext.check()
+    assert not torch.equal(m["h"], before["h"]) and torch.isfinite(m["h"]).all()
