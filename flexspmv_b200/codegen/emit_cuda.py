@@ -180,6 +180,9 @@ TUNED_BIG_CONFIGS = {
     "rusanov_f64": (736, 4, 2, 1),
     "rusanov_f32": (992, 4, 2, 1),
     "swe_delta_f64": (736, 4, 2, 1),
+    # lattices of eight edges a particle, 1024^2: fp32 992 x 8 35.9 (x 9 36.2), fp64 736 x 7 62.0 (x 8 63.8, x 9 62.1)
+    "spring_mass_f32": (992, 8, 2, 1),
+    "spring_mass_f64": (736, 7, 2, 1),
 }
 
 
@@ -503,6 +506,33 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
                 w(f"    r.{s_['selector_name']} = fx::ldg_vec<V, {d_}>(p.{s_['target']} + e * {d_});")
     w("    (void)p; (void)t; (void)le; (void)e; (void)r;")
     w("  }")
+    # the records of four consecutive edges as 16-byte words, for the configuration of large launches: `e` (and `le`) count from a
+    # multiple of four; `wide`: the edge tensors' addresses are multiples of 16 bytes and they hold all four
+    grouped = dtype == "float32" and needs_row and not staged_values and bool(edge_regs_list) and \
+        all(dim_of(s_["shape"]) == 1 and s_["target"] not in inplace_targets for s_ in edge_regs_list)
+    w(f"  static constexpr int kGroup = {4 if grouped else 1};")
+    if grouped:
+        tensors = list(dict.fromkeys((s_["selector_name"], s_["target"]) for s_ in edge_regs_list))
+        w("  static __device__ __forceinline__ bool groups_aligned(const Params& p) {")
+        w("    return ((" + " | ".join(f"reinterpret_cast<uintptr_t>(p.{t_})" for _, t_ in tensors) + ") & 15u) == 0;")
+        w("  }")
+        w("  template <class Tile>")
+        w("  __device__ __forceinline__ static void load_group(const Params& p, const Tile& t, int le, long long e, long long num_edges, bool wide, EReg (&r)[kGroup]) {")
+        for n_ in idx_names:
+            w(f"    {{ const fx::Four<int> q = fx::ld_four(t.template stream<{stream_of['idx:' + n_]}, int>(le));")
+            w("#pragma unroll")
+            w(f"      for (int i = 0; i < kGroup; ++i) r[i].idx_{n_} = q.v[i]; }}")
+        w("    if (wide) {")
+        for n_, t_ in tensors:
+            w(f"      {{ const fx::Four<V> q = fx::ldg_four(p.{t_} + e);")
+            w("#pragma unroll")
+            w(f"        for (int i = 0; i < kGroup; ++i) r[i].{n_}.v[0] = q.v[i]; }}")
+        w("    } else {")
+        w("#pragma unroll")
+        w("      for (int i = 0; i < kGroup; ++i)")
+        w("        if (e + i < num_edges) load_edge_vals(p, t, le + i, e + i, r[i]);")
+        w("    }")
+        w("  }")
     # edge tensors that are NOT staged are read straight from global memory by the consumers; the producer warp
     # prefetches the tile's part of them into L2 when it stages the tile, STAGES tiles ahead of their use
     w("  __device__ __forceinline__ static void prefetch_direct(const Params& p, long long nz0, long long nz1, int lane) {")
@@ -751,12 +781,10 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         elif line == "@@GROW_BODY@@":
             L[i_] = "\n".join(row_body) if grow_fields else "    // (nothing to evaluate per row)"
     ns = f"gen_{symbol}::"
-    if big:
-        w(f"FLEXSPMV_DEFINE_GRAPH_BIG({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns}CfgBig)")
-    else:
-        w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean)")
+    configs = f"{ns}Cfg, {ns}CfgWin, {ns}CfgLean" + (f", {ns}CfgBig" if big else "")
+    w(f"FLEXSPMV_DEFINE_GRAPH({symbol}, {ns}Graph, {configs})")
     if swe_rk:
-        w(f"FLEXSPMV_DEFINE_STEP({symbol}, {ns}Graph, {ns}Cfg, {ns}CfgWin, {ns}CfgLean, {ns + 'CfgBig' if big else 'flex::NoBig'})")
+        w(f"FLEXSPMV_DEFINE_STEP({symbol}, {ns}Graph, {configs})")
     if static_scratch_bytes:
         w(f"FLEXSPMV_DEFINE_STATIC_SCRATCH_LAUNCH({symbol}, {ns}Graph, {ns}Cfg, {int(static_scratch_bytes)})")
     return "\n".join(L) + "\n"

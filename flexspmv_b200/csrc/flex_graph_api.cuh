@@ -99,19 +99,23 @@ struct GraphApi {
   //   shallow-water step fp64  260^2 45.0 / 49.4, 310^2 52.8 / 66.7, 400^2 78.0 / 88.3, 520^2 102.9 / 121.4, 800^2 221 / 248, 1024^2 332 / 368, 1200^2
   //                            455 / 503; 200^2, a small launch there: 32.8 / 28.4
   //   Rusanov fp64             400^2 15.3 / 15.6, 450^2 18.7 / 19.8, 520^2 23.4 / 24.6, 800^2 48.0 / 50.0, 1024^2 74.0 / 76.3, 1200^2 100 / 106
+  //   spring-mass fp64         600^2 26.1 / 32.2, 1024^2 62.0 / 70.2, 1500^2 123 / 135; fp32 (with words of four edges) 600^2 14.8 / 16.2, 1024^2 35.9 / 38.3,
+  //                            1500^2 65.9 / 72.7
   //   Rusanov fp32             450^2 11.4 / 12.3, 520^2 14.1 / 15.8, 800^2 29.4 / 32.9, 1024^2 45.8 / 48.9, 1200^2 59.3 / 64.0
   // A tile has to hold about a row a thread (7 to 11 for ten), or warps wait for a stage, or go round it twice.  8 M items: rows of 8 Rusanov fp64
   // 116 / 103, fp32 59.4 / 56.8, swe_delta fp64 102 / 98; of 6 81.8 / 85.0, 47.7 / 46.4, 68.9 / 76.9; of 4 76.7 / 83.6, 45.4 / 46.4, 64.9 / 71.8; of 1 - 7
   // 103.8 / 114.4, 59.4 / 67.3, 77.6 / 89.8; of 2 76.6 / 81.8, 47.7 / 49.2, 70.6 / 65.4 (3 M items: 32.9 / 36.7, 20.7 / 20.1, 30.4 / 28.4); of 3, one of them of 40
   // (not whole rows) 98.0 / 104.3, 64.6 / 67.5, 77.2 / 94.1 (1 M items, swe_delta: 21.8 / 21.1).
+  // Spring-mass fp32, 9 M items: rows of 8 31.3 / 42.3, of 4 - 12 46.7 / 52.4, of 9 38.6 / 36.5 (three words for a row, which single indices read
+  // without conflicts): 8.5 rows for ten threads at least; one row of 40 among rows of 8 50.9 / 46.9, fp64 94.4 / 98.1.
   // Callers that name a tile or a number of CTAs get the configuration that they know.
-  static constexpr int kBigTile = CfgBig::kTile - CfgBig::kIpt;
+  static constexpr int kBigTile = CfgBig::kTile - CfgBig::kIpt, kLeastRows = G::kGroup > 1 ? 17 : 14;      // rows a tile, for 20 threads
   static bool use_big(const flexspmv_desc* d) {
     if constexpr (kBigBuilt) {
       const long long sms = device_sm_count(), items = d->num_rows + d->num_edges;
       if (d->tile_items > 0 || d->max_ctas > 0 || use_lean(d) || use_win(d)) return false;
       const long long ten_rows = 10 * d->num_rows * kBigTile, each_a_row = items * CfgBig::kBlock;
-      if (items <= sms * CfgBig::kMinCtas * kBigTile || ten_rows < 7 * each_a_row || ten_rows > 11 * each_a_row) return false;
+      if (items <= sms * CfgBig::kMinCtas * kBigTile || 2 * ten_rows < kLeastRows * each_a_row || ten_rows > 11 * each_a_row) return false;
       const long long tiles = (items + kDefaultTile - 1) / kDefaultTile, slots = sms * Cfg::kMinCtas;
       return !small_launch(d, tiles, tiles < slots ? tiles : slots, Cfg::kBlock + 32);
     }
@@ -548,30 +552,29 @@ struct GraphApi {
 
 }  // namespace flex
 
-// a graph with one configuration of the tile kernel
-#define FLEXSPMV_DEFINE_GRAPH(SYM, GRAPH, CFG, CFGWIN, CFGLEAN) FLEXSPMV_DEFINE_GRAPH_BIG(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, flex::NoBig)
-#define FLEXSPMV_DEFINE_GRAPH_BIG(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG)                                                          \
+// (behind CFGWIN: the configuration of the warp kernel, and where there is one that of large launches)
+#define FLEXSPMV_DEFINE_GRAPH(SYM, GRAPH, CFG, CFGWIN, ...)                                                          \
   extern "C" {                                                                                                  \
-  int flexspmv_##SYM##_info(flexspmv_graph_info* info) { return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::info(info); } \
+  int flexspmv_##SYM##_info(flexspmv_graph_info* info) { return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::info(info); } \
   int flexspmv_##SYM##_workspace_bytes(const flexspmv_desc* d, size_t* b) {                                     \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::workspace_bytes(d, b);                                           \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::workspace_bytes(d, b);                                           \
   }                                                                                                             \
   int flexspmv_##SYM##_plan(const flexspmv_desc* d, const void* ro, void* ws, size_t wb, void* st) {            \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::plan(d, nullptr, ro, ws, wb, static_cast<cudaStream_t>(st));     \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::plan(d, nullptr, ro, ws, wb, static_cast<cudaStream_t>(st));     \
   }                                                                                                             \
   int flexspmv_##SYM##_plan_indexed(const flexspmv_desc* d, const void* const* ix, const void* ro, void* ws, size_t wb, void* st) { \
     if (!ix) return FLEXSPMV_ERR_BAD_ARG;                                                                       \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::plan(d, ix, ro, ws, wb, static_cast<cudaStream_t>(st));          \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::plan(d, ix, ro, ws, wb, static_cast<cudaStream_t>(st));          \
   }                                                                                                             \
   int flexspmv_##SYM##_plan_windows(const flexspmv_desc* d, const void* const* ix, void* ws, size_t wb, void* st) { \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::plan_windows(d, ix, ws, wb, static_cast<cudaStream_t>(st));      \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::plan_windows(d, ix, ws, wb, static_cast<cudaStream_t>(st));      \
   }                                                                                                             \
   int flexspmv_##SYM##_launch(const flexspmv_desc* d, const void* const* v, const void* const* ix,              \
                               const void* ro, void* const* o, void* ws, size_t wb, void* st) {                  \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st));  \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st));  \
   }                                                                                                             \
   int flexspmv_##SYM##_device_status(const void* ws, int32_t* out, void* st) {                                  \
-    return flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>::device_status(ws, out, static_cast<cudaStream_t>(st));           \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::device_status(ws, out, static_cast<cudaStream_t>(st));           \
   }                                                                                                             \
   }
 

@@ -285,11 +285,11 @@ struct StepApi {
 
 }  // namespace flex
 
-#define FLEXSPMV_DEFINE_STEP(SYM, GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG)                                                                 \
+#define FLEXSPMV_DEFINE_STEP(SYM, GRAPH, CFG, CFGWIN, ...)                                                                 \
   extern "C" int flexspmv_##SYM##_step_fits(const flexspmv_desc* d) {                                                                  \
-    return flex::StepApi<GRAPH, flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>>::fits(d);                                          \
+    return flex::StepApi<GRAPH, flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>>::fits(d);                                          \
   }                                                                                                                                    \
   extern "C" int flexspmv_##SYM##_step(const flexspmv_desc* d, const void* const* v, const void* const* ix, const void* ro, void* const* o, \
                                        void* ws, size_t wb, void* st) {                                                                \
-    return flex::StepApi<GRAPH, flex::GraphApi<GRAPH, CFG, CFGWIN, CFGLEAN, CFGBIG>>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st)); \
+    return flex::StepApi<GRAPH, flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st)); \
   }

@@ -232,6 +232,17 @@ __device__ __forceinline__ Vec<V, D> ld_vec(P p) {   // plain load through anyth
   for (int i = 0; i < D; ++i) r.v[i] = p[i];
   return r;
 }
+// Four consecutive 4-byte values as one word, from a multiple of 16 bytes.
+template <typename T>
+struct alignas(16) Four { T v[4]; };
+template <typename T>
+__device__ __forceinline__ Four<T> ld_four(const T* p) { return *reinterpret_cast<const Four<T>*>(p); }
+template <typename T>
+__device__ __forceinline__ Four<T> ldg_four(const T* p) {
+  Four<T> r;
+  *reinterpret_cast<int4*>(r.v) = __ldg(reinterpret_cast<const int4*>(p));
+  return r;
+}
 // A gathered record: through the read-only path where nothing writes it during the launch (FIXED).
 template <bool FIXED, typename V, int D>
 __device__ __forceinline__ Vec<V, D> gather_vec(const V* p) {

@@ -47,7 +47,8 @@ struct TileCfg {
   static constexpr int kRowBatch = ROW_BATCH_;   // the same in the loop over whole rows
   // consecutive tiles of a CTA where whole rows go round the CTAs (TileKernelArgs::rounds); large tiles go round one by one: 1024^2
   // shallow-water step 333 us, in runs of two 336, of four 353; Rusanov 74.0, 76.6, 77.7
-  static constexpr int kTileRun = kTile >= 2560 ? 1 : 4;
+  static constexpr bool kLarge = kTile >= 2560;
+  static constexpr int kTileRun = kLarge ? 1 : 4;
 };
 
 // Whether the plan may move all tile boundaries of the graph to row starts, and the kernel has the loop over whole rows, one
@@ -639,6 +640,9 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // SpMV 512^3 3205 / 2564 (in rounds 2133); 145^3 fp32 54.1 / 42.6; 5-point 512^2 fp64 9.1 / 7.1 (without stages 5.1); 27 columns a row
       // fp64, 300 007 rows 26.2 / 23.9; spring-mass 1024^2 fp32 44.5 / 38.4; Rusanov 1024^2 fp64 92 / 83.5.
       constexpr int RB = Cfg::kRowBatch;
+      constexpr bool GROUPS = G::kGroup > 1 && Cfg::kLarge;
+      [[maybe_unused]] bool groups_wide = false;
+      if constexpr (GROUPS) groups_wide = G::groups_aligned(p);
       int s = 0, turn = 0;
       uint32_t parity = 0;
       for (int k = 0; k < count; ++k) {
@@ -681,6 +685,25 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
           for (int j = 0; j < kAcc; ++j) sum[j] = V(0);
           typename G::GRow grow;
           if constexpr (G::kGatherNeedsRow) { if (lo < hi) G::gather_row(p, c.row0 + r, grow); }
+          if constexpr (GROUPS) {
+            // Four edges' records a word of every array, from a multiple of four on: lanes a row of eight edges apart meet in four banks with
+            // single indices (8-way), and read a line each for every edge tensor.  Lattices fp32 600^2 15.3 -> 14.8 us, 1024^2 36.4 -> 35.9, 1500^2 70.6 -> 65.9.  In the
+            // smaller configuration, where four edges more in registers spill, no gain: 38.3 -> 38.4, 430^2 9.8 -> 10.0; neither for pairs
+            // of 8-byte values, 600^2 26.1 -> 28.5.
+            constexpr int N = G::kGroup;
+            const int lead = (int)((unsigned)c.nz0 % (unsigned)N);
+            for (int e0 = lo - (lo + lead) % N; e0 < hi; e0 += N) {
+              typename G::EReg er[N];
+              typename G::GEdge ge[N];
+              G::load_group(p, tile, e0, c.nz0 + e0, a.num_edges, groups_wide && c.nz0 + e0 + N <= a.num_edges, er);
+#pragma unroll
+              for (int b = 0; b < N; ++b)
+                if (e0 + b >= lo && e0 + b < hi) G::gather_edge(p, er[b], ge[b]);
+#pragma unroll
+              for (int b = 0; b < N; ++b)
+                if (e0 + b >= lo && e0 + b < hi) G::map(p, er[b], c.nz0 + e0 + b, grow, ge[b], sum);
+            }
+          } else
           for (int e0 = lo; e0 < hi; e0 += RB) {
             typename G::EReg er[RB];
             typename G::GEdge ge[RB];

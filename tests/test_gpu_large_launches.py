@@ -13,7 +13,9 @@ from test_gpu_launch_sizes import ROUNDS, default_tile, header_word, launch, run
 
 pytestmark = pytest.mark.gpu
 
-LARGE = [("rusanov", "float64", 736), ("rusanov", "float32", 992), ("swe_delta", "float64", 736)]
+# graph, type, threads and items of each that take rows, edges a row that suit, and rows that are too short and too long
+LARGE = [("rusanov", "float64", 736, 4, 3), ("rusanov", "float32", 992, 4, 3), ("swe_delta", "float64", 736, 4, 3),
+         ("spring_mass", "float64", 736, 7, 7), ("spring_mass", "float32", 992, 8, 8)]
 
 
 def sms():
@@ -23,21 +25,22 @@ def sms():
 def small_limit(ir, dtype):
     """Items up to which a launch of short rows takes the kernel without stages: 9 tiles for four CTAs, of which an SM holds three
     or four."""
-    return 9 * sms() * (3 if dtype == np.float64 else 4) * default_tile(ir, dtype) // 4
+    resident = 3 if dtype == np.float64 and ir.name != "spring_mass" else 4
+    return 9 * sms() * resident * default_tile(ir, dtype) // 4
 
 
-@pytest.mark.parametrize("gname,dt,threads", LARGE)
+@pytest.mark.parametrize("gname,dt,threads,ipt,edges", LARGE)
 @pytest.mark.parametrize("bits", [32, 64])
-@pytest.mark.parametrize("tiles,lengths", [(0, [3]), (1, [3]), (3, [4, 0, 4, 3, 5]), (5, [2, 4]), (16, [3]), (17, [3])],
+@pytest.mark.parametrize("tiles,lengths", [(0, [0]), (1, [0]), (3, [1, -3, 1, 0, 2]), (5, [-1, 1]), (16, [0]), (17, [0])],
                          ids=["small", "above", "uneven", "five", "sixteen", "seventeen"])
-def test_large_launches_equal_those_of_the_other_configuration(gname, dt, threads, bits, tiles, lengths):
+def test_large_launches_equal_those_of_the_other_configuration(gname, dt, threads, ipt, edges, bits, tiles, lengths):
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
-    tile = threads * 4 - 4
+    tile, lengths = threads * ipt - ipt, [edges + more for more in lengths]
     if tiles > 5 and (bits == 64 or (gname, dt) != ("rusanov", "float64")):
         pytest.skip("one graph and width at the large sizes")
     # the last small launch and the first one that is not; up to `tiles` tiles a CTA
     items = small_limit(ir, dtype) + (4 if tiles else 0) if tiles < 2 else sms() * tile * tiles - 7 + (60 if tiles == 17 else 0)
-    rows = items // (sum(lengths) // len(lengths) + 1) // len(lengths) * len(lengths)
+    rows = items // (sum(lengths) // len(lengths) + 1) // len(lengths) * len(lengths) + (len(lengths) if tiles == 1 else 0)
     prob = with_lengths(ir, lengths * (rows // len(lengths)), 211, dtype)
     items = prob.num_rows + prob.nnz
     ext = GraphExtension(ir, random_gather=False)
@@ -59,13 +62,13 @@ def test_large_launches_equal_those_of_the_other_configuration(gname, dt, thread
         assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} large")
 
 
-@pytest.mark.parametrize("gname,dt,threads", LARGE)
+@pytest.mark.parametrize("gname,dt,threads,ipt,edges", LARGE)
 @pytest.mark.parametrize("bits", [32, 64])
-def test_large_launches_without_whole_rows(gname, dt, threads, bits):
+def test_large_launches_without_whole_rows(gname, dt, threads, ipt, edges, bits):
     """A row of 40 edges, one of 900 and one of 20 000 among rows of three: the loop with carries, in tiles of both kinds."""
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
-    rows = small_limit(ir, dtype) // 4
-    lengths = np.full(rows, 3)
+    rows = small_limit(ir, dtype) // (edges + 1) + 1000
+    lengths = np.full(rows, edges)
     lengths[[100, rows // 2, rows - 7]] = [40, 900, 20_000]
     prob = with_lengths(ir, lengths.tolist(), 223, dtype)
     ext = GraphExtension(ir, random_gather=False)
@@ -76,13 +79,45 @@ def test_large_launches_without_whole_rows(gname, dt, threads, bits):
     assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} large, long rows")
 
 
-@pytest.mark.parametrize("gname,dt,threads", LARGE)
-def test_rows_of_which_the_large_tiles_hold_too_few_or_too_many(gname, dt, threads):
-    """Seven to eleven rows a tile for ten threads: three or four edges a row (of 4 items a thread)."""
+@pytest.mark.parametrize("gname,dt,held", [("rusanov", "float64", {2: 0, 3: 1, 4: 1, 5: 0}), ("rusanov", "float32", {2: 0, 3: 1, 4: 1, 5: 0}),
+                                           ("swe_delta", "float64", {2: 0, 3: 1, 4: 1, 5: 0}), ("spring_mass", "float64", {5: 0, 6: 1, 8: 1, 9: 0}),
+                                           ("spring_mass", "float32", {6: 0, 7: 1, 8: 1, 9: 0})])
+def test_rows_of_which_the_large_tiles_hold_too_few_or_too_many(gname, dt, held):
+    """Seven (words of four edges: 8.5) to eleven rows a tile for ten threads."""
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
-    for edges, large in ((2, False), (3, True), (4, True), (5, False)):
+    for edges, large in held.items():
         rows = (small_limit(ir, dtype) + 4000) // (edges + 1)
         prob = with_lengths(ir, [edges] * rows, 227, dtype)
         ext = GraphExtension(ir, random_gather=False)
         run_gpu(ext, ir, prob, dtype)
         assert (header_word(ext, 10) > default_tile(ir, dtype)) == large, edges
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("skip", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("last", [8, 9, 10, 11])
+def test_words_of_four_edges_at_odd_places(bits, skip, last):
+    """Rows that begin and end at any edge of a word of four, a last word that the arrays do not fill, edge tensors at any multiple of
+    four bytes (an operator takes views), against the configuration that reads edge by edge."""
+    ir, dtype = graphs.spring_mass_graph(), np.dtype("float32")
+    lengths = [8, 7, 9, 8, 5, 11, 0, 16] * ((small_limit(ir, dtype) + 5000) // 72) + [last]
+    prob = with_lengths(ir, lengths, 229, dtype)
+    non_gather, gathers, index_names = graphs.operator_signature(ir)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    def shifted(a):
+        t = torch.full((a.size + skip,), float("nan"), device="cuda")
+        t[skip:] = dev(a.astype(np.float32))
+        return t[skip:]
+    values = [shifted(prob.values[n]) for n in non_gather] + [dev(prob.values[n].astype(np.float32)) for n in gathers]
+    indices = [dev(prob.indices[n]) for n in index_names]
+    ro = dev(prob.row_offsets.astype(np.int32 if bits == 32 else np.int64))
+    outs = []
+    for max_ctas in (0, 4 * sms()):
+        ext = GraphExtension(ir, max_ctas=max_ctas)
+        out = torch.full((prob.num_rows, 2), float("nan"), device="cuda")
+        ext.launch_into(values, indices, ro, [out], prob.num_rows, prob.nnz, prob.num_cols)
+        ext.check()
+        assert (header_word(ext, 10) > default_tile(ir, dtype)) == (max_ctas == 0)
+        outs.append(out.cpu().numpy().tobytes())
+    assert outs[0] == outs[1]
