@@ -73,8 +73,8 @@ struct SmemTile {
     static_for<G::kNumStreams>([&](auto I) { base[I.value] += (size_t)records * G::template stream_bytes<I.value>(); });
   }
   template <int I, class T>
-  __device__ __forceinline__ const T* stream(int le) const {
-    return reinterpret_cast<const T*>(base[I] + (size_t)le * G::template stream_bytes<I>());
+  __device__ __forceinline__ fx::Staged<T> stream(int le) const {
+    return fx::Staged<T>{reinterpret_cast<const T*>(base[I] + (size_t)le * G::template stream_bytes<I>())};
   }
 };
 
