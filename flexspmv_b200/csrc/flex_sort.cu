@@ -5,9 +5,9 @@
 // the per-edge arrays are permuted with it, and the CSR offsets come from the sorted ids.
 //
 // Least-significant-digit radix sort on the row ids, which are dense: ceil(log2(num_rows)) bits in as few passes as cover
-// them, every pass the same width (20 bits: 2 x 10).  A pass is three launches: digit counts per tile of keys, one CTA per
+// them, every pass the same width (21 bits: 3 x 7).  A pass is three launches: digit counts per tile of keys, one CTA per
 // digit that scans that digit's counts over the tiles, and the stable scatter.  No block waits for another one.  Digits have
-// up to 8 bits, or up to 10 where that saves a pass (SortShape).  The first pass reads the caller's ids and takes the
+// up to 8 bits, or up to 10 where that saves a pass that costs more (flexspmv_sort_rows); every width is compiled by itself.  The first pass reads the caller's ids and takes the
 // positions as values, so there is no separate initialisation; the passes alternate between two buffers so that the last one
 // writes the caller's permutation.  Equal digits keep their input order in every pass (see sort_scatter_kernel), so the
 // permutation equals a stable argsort (bit-exact against numpy.argsort(kind="stable")).
@@ -20,7 +20,7 @@ namespace flex {
 int device_sm_count();      // flex_core.cu
 
 constexpr int kSortKeysPerThread = 16;
-// One width of digit: bins, threads of a CTA, and with 16 keys a thread the tile.  A pass with 1024 bins has tiles of 8192
+// One width of digit: bins, threads of a CTA, and with 16 keys a thread the tile.  A pass with 512 or 1024 bins has tiles of 8192
 // keys, so that a digit's keys in a tile still leave in runs of 8 and more.
 template <int BITS_, int THREADS_>
 struct SortShape {
@@ -31,8 +31,10 @@ struct SortShape {
   // shared memory of the scatter: tile in digit order, global place of every digit, counters by warp
   static constexpr int kSmem = kTile * 8 + kBins * 4 + kWarps * kCntPitch * 2;
 };
-using SortNarrow = SortShape<8, 256>;
-using SortWide = SortShape<10, 512>;
+template <int BITS>
+using SortNarrow = SortShape<BITS, 256>;
+template <int BITS>
+using SortWide = SortShape<BITS, 512>;
 
 template <typename KeyT>
 __device__ __forceinline__ unsigned digit_of(KeyT key, int shift, unsigned mask) { return ((unsigned)key >> shift) & mask; }
@@ -41,30 +43,29 @@ __device__ __forceinline__ unsigned digit_of(KeyT key, int shift, unsigned mask)
 // [0, num_rows).
 template <typename KeyT, bool CHECK, class S>
 __global__ void __launch_bounds__(S::kThreads) sort_count_kernel(const KeyT* __restrict__ keys, long long n, long long num_rows,
-                                                                 int shift, unsigned mask, int num_tiles,
-                                                                 unsigned* __restrict__ hist, int* status) {
+                                                                 int shift, int num_tiles, unsigned* __restrict__ hist, int* status) {
+  constexpr unsigned mask = S::kBins - 1;
   __shared__ unsigned s_cnt[S::kBins];
   const int tid = threadIdx.x;
   for (int d = tid; d < S::kBins; d += S::kThreads) s_cnt[d] = 0;
   __syncthreads();
   const long long base = (long long)blockIdx.x * S::kTile + tid;
+  const int left = (int)(n - base < S::kTile ? n - base : S::kTile);      // key i of the thread lies inside the input: i * kThreads < left
+  const KeyT* const in = keys + base;
   bool bad = false;
   KeyT k[kSortKeysPerThread];           // all loads before the first atomic
 #pragma unroll
-  for (int i = 0; i < kSortKeysPerThread; ++i) {
-    const long long e = base + i * S::kThreads;
-    k[i] = e < n ? keys[e] : KeyT(0);
-  }
+  for (int i = 0; i < kSortKeysPerThread; ++i) k[i] = i * S::kThreads < left ? in[i * S::kThreads] : KeyT(0);
 #pragma unroll
   for (int i = 0; i < kSortKeysPerThread; ++i) {
-    if (base + i * S::kThreads < n) {
+    if (i * S::kThreads < left) {
       if (CHECK) bad |= (long long)k[i] < 0 || (long long)k[i] >= num_rows;
       atomicAdd(&s_cnt[digit_of(k[i], shift, mask)], 1u);     // integer counts: order does not matter
     }
   }
   if (CHECK && bad) atomicCAS(status, 0, FLEXSPMV_ERR_BAD_ARG);
   __syncthreads();
-  for (int d = tid; d <= (int)mask; d += S::kThreads) hist[(size_t)d * num_tiles + blockIdx.x] = s_cnt[d];
+  for (int d = tid; d < S::kBins; d += S::kThreads) hist[(size_t)d * num_tiles + blockIdx.x] = s_cnt[d];
 }
 
 // Exclusive scan over the CTA's 32 * WARPS threads; `total` is the sum of all.  s_warp: WARPS words.
@@ -120,14 +121,17 @@ __global__ void __launch_bounds__(kScanThreads) sort_scan_kernel(unsigned* __res
 // below), the tile is put in digit order in shared memory and leaves from there, so that a digit's keys are stored side by
 // side.  Storing straight from the ranks would touch a sector per key.  Order: warps own consecutive runs of keys, a warp's
 // rounds follow one another and lanes are ranked in order, so equal digits never change places.  FIRST: the values are the
-// positions.  Bound by the instructions of the ranking and the moves (135 for 32 keys a pass with 7-bit digits, half of the
-// issue slots) and by shared memory's wavefronts (52 %), so what helps is a pass less.
+// positions.  Bound by the instructions of the ranking and the moves and by shared memory's wavefronts (52 %).  With the width and whole tiles
+// known to the compiler a vote is four instructions, not seven, and no key asks whether it lies inside: 8.4 M ids in three
+// passes of 7 bits 306 -> 283 us with the counts, offsets and a permutation.  Measured and left out: two passes of 11 bits in ranges of
+// tiles a CTA, lanes meeting in shared memory instead of by votes (331: 2048 counters a warp, 48 wavefronts for 32 keys).
 template <typename KeyT, bool FIRST, class S>
 __global__ void __launch_bounds__(S::kThreads, 1024 / S::kThreads)
-sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ vals_in, long long n, int shift, unsigned mask,
+sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ vals_in, long long n, int shift,
                     int num_tiles, const unsigned* __restrict__ hist, const unsigned* __restrict__ totals,
                     unsigned* __restrict__ keys_out, int* __restrict__ vals_out) {
   constexpr int KPT = kSortKeysPerThread, T = S::kThreads, W = S::kWarps, WPT = S::kWordsPerThread;
+  constexpr unsigned mask = S::kBins - 1;
   extern __shared__ __align__(16) unsigned char s_sort[];
   uint2* const s_pair = reinterpret_cast<uint2*>(s_sort);                                  // [kTile] the tile in digit order
   unsigned* const s_out = reinterpret_cast<unsigned*>(s_pair + S::kTile);                  // [kBins] where the digit's run goes, less its place in the tile
@@ -136,44 +140,48 @@ sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ va
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long tile0 = (long long)blockIdx.x * S::kTile;
   const int count = (int)(n - tile0 < S::kTile ? n - tile0 : S::kTile);
+  const int mine = warp * (32 * KPT) + lane;      // place of the lane's first key in the tile
+  const int left = count - mine;                  // key i of the thread lies inside the input: i * 32 < left
   for (int i = tid; i < W * S::kCntPitch / 2; i += T) reinterpret_cast<unsigned*>(s_cnt)[i] = 0;
   unsigned k[KPT];
-  const int mine = warp * (32 * KPT) + lane;      // place of the lane's first key in the tile
+  const KeyT* const in = keys_in + tile0 + mine;
 #pragma unroll
-  for (int i = 0; i < KPT; ++i) {
-    const int at = mine + i * 32;
-    k[i] = at < count ? (unsigned)keys_in[tile0 + at] : 0u;
-  }
+  for (int i = 0; i < KPT; ++i) k[i] = i * 32 < left ? (unsigned)in[i * 32] : 0u;
   __syncthreads();
   unsigned short* const cnt = s_cnt + warp * S::kCntPitch;
+  const unsigned below_mask = (1u << lane) - 1u;
   unsigned rank[KPT / 2];                          // two 16-bit ranks a register
+  auto rank_keys = [&](auto full) {
 #pragma unroll
-  for (int i = 0; i < KPT; ++i) {
-    const bool in = mine + i * 32 < count;
-    const unsigned d = in ? digit_of(k[i], shift, mask) : (unsigned)S::kBins;
-    unsigned same = __ballot_sync(0xffffffffu, in);
-    if (!in) same = ~same;
+    for (int i = 0; i < KPT; ++i) {
+      unsigned d = (k[i] >> shift) & mask, same = 0xffffffffu;
+      bool inside = true;
+      if constexpr (!full.value) {
+        inside = i * 32 < left;
+        same = __ballot_sync(0xffffffffu, inside);
+        if (!inside) same = ~same;
+      }
 #pragma unroll
-    for (int b = 0; b < S::kBits; ++b) {
-      if ((mask >> b) == 0) break;                              // the same for every lane
-      const unsigned set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-      same &= (d >> b) & 1u ? set : ~set;
+      for (int b = 0; b < S::kBits; ++b) {
+        const bool bit = (d & (1u << b)) != 0;
+        const unsigned set = __ballot_sync(0xffffffffu, bit);
+        same &= set ^ (bit ? 0u : 0xffffffffu);
+      }
+      if constexpr (!full.value) if (!inside) d = (unsigned)S::kBins;
+      const unsigned below = __popc(same & below_mask);
+      const unsigned seen = cnt[d];
+      __syncwarp();
+      if (below == 0) cnt[d] = (unsigned short)(seen + __popc(same));
+      __syncwarp();
+      rank[i / 2] = i & 1 ? rank[i / 2] | (seen + below) << 16 : seen + below;
     }
-    const unsigned below = __popc(same & ((1u << lane) - 1u));
-    const unsigned seen = cnt[d];
-    __syncwarp();
-    if (below == 0) cnt[d] = (unsigned short)(seen + __popc(same));
-    __syncwarp();
-    rank[i / 2] = i & 1 ? rank[i / 2] | (seen + below) << 16 : seen + below;
-  }
+  };
+  if (count == S::kTile) rank_keys(IntC<1>{}); else rank_keys(IntC<0>{});
   __syncthreads();
   // values: needed last, requested now
   int v[KPT];
 #pragma unroll
-  for (int i = 0; i < KPT; ++i) {
-    const int at = mine + i * 32;
-    v[i] = FIRST ? (int)(tile0 + at) : (at < count ? vals_in[tile0 + at] : 0);
-  }
+  for (int i = 0; i < KPT; ++i) v[i] = FIRST ? (int)(tile0 + mine + i * 32) : (i * 32 < left ? vals_in[tile0 + mine + i * 32] : 0);
   {
     // two digits a word: the warps' counts become places in the tile -- behind the digits before, behind the warps before
     unsigned* const words = reinterpret_cast<unsigned*>(s_cnt);
@@ -188,8 +196,8 @@ sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ va
       if (has) {
 #pragma unroll
         for (int w = 0; w < W; ++w) sum[j] += words[w * kPitch + w0 + j];
-        if (2 * (w0 + j) <= (int)mask) tot[2 * j] = totals[2 * (w0 + j)];
-        if (2 * (w0 + j) + 1 <= (int)mask) tot[2 * j + 1] = totals[2 * (w0 + j) + 1];
+        tot[2 * j] = totals[2 * (w0 + j)];
+        tot[2 * j + 1] = totals[2 * (w0 + j) + 1];
       }
       digits += (sum[j] & 0xffffu) + (sum[j] >> 16);
       global += tot[2 * j] + tot[2 * j + 1];
@@ -202,8 +210,8 @@ sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ va
       for (int j = 0; j < WPT; ++j) {
         const int d = 2 * (w0 + j);
         const unsigned second = place + (sum[j] & 0xffffu);
-        if (d <= (int)mask) s_out[d] = to + hist[(size_t)d * num_tiles + blockIdx.x] - place;
-        if (d + 1 <= (int)mask) s_out[d + 1] = to + tot[2 * j] + hist[(size_t)(d + 1) * num_tiles + blockIdx.x] - second;
+        s_out[d] = to + hist[(size_t)d * num_tiles + blockIdx.x] - place;
+        s_out[d + 1] = to + tot[2 * j] + hist[(size_t)(d + 1) * num_tiles + blockIdx.x] - second;
         unsigned at = place | second << 16;        // places are at most a tile: no carry between the halves
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -219,15 +227,15 @@ sort_scatter_kernel(const KeyT* __restrict__ keys_in, const int* __restrict__ va
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < KPT; ++i)
-    if (mine + i * 32 < count) {
-      const unsigned at = cnt[digit_of(k[i], shift, mask)] + (i & 1 ? rank[i / 2] >> 16 : rank[i / 2] & 0xffffu);
+    if (i * 32 < left) {
+      const unsigned at = cnt[(k[i] >> shift) & mask] + (i & 1 ? rank[i / 2] >> 16 : rank[i / 2] & 0xffffu);
       s_pair[at] = make_uint2(k[i], (unsigned)v[i]);
     }
   __syncthreads();
 #pragma unroll 4
   for (int j = tid; j < count; j += T) {
     const uint2 q = s_pair[j];
-    const unsigned to = s_out[digit_of(q.x, shift, mask)] + (unsigned)j;
+    const unsigned to = s_out[(q.x >> shift) & mask] + (unsigned)j;
     keys_out[to] = q.x;
     vals_out[to] = (int)q.y;
   }
@@ -383,43 +391,40 @@ __global__ void permute_kernel(const unsigned* __restrict__ src, unsigned* __res
 
 // One pass over `keys` (FIRST: the values are the positions, and the ids are checked).
 template <typename KeyT, bool FIRST, class S>
-static int sort_pass(const KeyT* keys, const int* vals, long long n, long long num_rows, int shift, unsigned mask, unsigned* hist,
-                     unsigned* totals, unsigned* keys_out, int* vals_out, int* status, cudaStream_t st) {
+static int sort_pass(const KeyT* keys, const int* vals, long long n, long long num_rows, int shift, unsigned* hist, unsigned* totals,
+                     unsigned* keys_out, int* vals_out, int* status, cudaStream_t st) {
   const int tiles = (int)((n + S::kTile - 1) / S::kTile);
   auto scatter = sort_scatter_kernel<KeyT, FIRST, S>;
   if (S::kSmem > 48 * 1024)
     if (cudaError_t e = cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem); e != cudaSuccess) return (int)e;
-  sort_count_kernel<KeyT, FIRST, S><<<tiles, S::kThreads, 0, st>>>(keys, n, num_rows, shift, mask, tiles, hist, status);
-  sort_scan_kernel<<<mask + 1, kScanThreads, 0, st>>>(hist, tiles, totals);
-  scatter<<<tiles, S::kThreads, S::kSmem, st>>>(keys, vals, n, shift, mask, tiles, hist, totals, keys_out, vals_out);
+  sort_count_kernel<KeyT, FIRST, S><<<tiles, S::kThreads, 0, st>>>(keys, n, num_rows, shift, tiles, hist, status);
+  sort_scan_kernel<<<S::kBins, kScanThreads, 0, st>>>(hist, tiles, totals);
+  scatter<<<tiles, S::kThreads, S::kSmem, st>>>(keys, vals, n, shift, tiles, hist, totals, keys_out, vals_out);
   return (int)cudaGetLastError();
 }
 
-// All passes; `cur` says which of the two key buffers holds the sorted ids.
+// All passes of S::kBits each (one alone may have fewer); `cur` says which of the two key buffers holds the sorted ids.
 template <class S>
-static int sort_passes(const void* ids, int id_bits, long long n, long long num_rows, int bits, int* perm, unsigned* const keys[2],
+static int sort_passes(const void* ids, int id_bits, long long n, long long num_rows, int passes, int* perm, unsigned* const keys[2],
                        int* spare, unsigned* hist, unsigned* totals, int* status, cudaStream_t st, int& cur) {
-  const int passes = (bits + S::kBits - 1) / S::kBits, width = (bits + passes - 1) / passes;
-  const unsigned mask = (1u << width) - 1u;
   // the last pass writes the caller's permutation; the ones before it alternate with the spare buffer
   int* vals[2] = {(passes & 1) ? spare : perm, (passes & 1) ? perm : spare};
   for (int p = 0; p < passes; ++p) {
-    const int to = cur ^ 1;
+    const int to = cur ^ 1, shift = p * S::kBits;
     int e;
     if (p > 0)
-      e = sort_pass<unsigned, false, S>(keys[cur], vals[cur], n, num_rows, p * width, mask, hist, totals, keys[to], vals[to], status, st);
+      e = sort_pass<unsigned, false, S>(keys[cur], vals[cur], n, num_rows, shift, hist, totals, keys[to], vals[to], status, st);
     else if (id_bits == 32)
-      e = sort_pass<int, true, S>(static_cast<const int*>(ids), nullptr, n, num_rows, 0, mask, hist, totals, keys[to], vals[to], status, st);
+      e = sort_pass<int, true, S>(static_cast<const int*>(ids), nullptr, n, num_rows, 0, hist, totals, keys[to], vals[to], status, st);
     else
-      e = sort_pass<long long, true, S>(static_cast<const long long*>(ids), nullptr, n, num_rows, 0, mask, hist, totals, keys[to], vals[to],
-                                        status, st);
+      e = sort_pass<long long, true, S>(static_cast<const long long*>(ids), nullptr, n, num_rows, 0, hist, totals, keys[to], vals[to], status, st);
     if (e) return e;
     cur = to;
   }
   return 0;
 }
 
-// Bytes of the counts and totals of a pass.
+// Bytes of the counts and totals of a pass with digits of up to BITS bits.
 template <class S>
 static uint64_t sort_count_bytes(long long n) {
   return align_up((uint64_t)((n + S::kTile - 1) / S::kTile) * S::kBins * 4u, 256) + S::kBins * 4u;
@@ -440,7 +445,7 @@ int flexspmv_sort_rows_bytes(int64_t num_edges, size_t* bytes) {
   if (!bytes || num_edges < 0) return FLEXSPMV_ERR_BAD_ARG;
   if (num_edges > 0x7fffffffLL) return FLEXSPMV_ERR_TOO_LARGE;
   // keys (2 buffers), values (1 extra buffer; the other is the caller's permutation array), digit x tile counts, digit totals
-  const uint64_t wide = flex::sort_count_bytes<flex::SortWide>(num_edges), narrow = flex::sort_count_bytes<flex::SortNarrow>(num_edges);
+  const uint64_t wide = flex::sort_count_bytes<flex::SortWide<10>>(num_edges), narrow = flex::sort_count_bytes<flex::SortNarrow<8>>(num_edges);
   *bytes = (size_t)(flex::align_up((uint64_t)num_edges * 4u, 256) * 3 + (wide > narrow ? wide : narrow));
   return 0;
 }
@@ -454,8 +459,8 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
   if (num_edges > 0x7fffffffLL || num_rows > 0x7fffffffLL) return FLEXSPMV_ERR_TOO_LARGE;
   const uint64_t seg = flex::align_up((uint64_t)num_edges * 4u, 256);
   // scratch for 8-bit digits is enough; with less than flexspmv_sort_rows_bytes says the wider ones are not taken
-  const uint64_t narrow_bytes = 3 * seg + flex::sort_count_bytes<flex::SortNarrow>(num_edges);
-  const uint64_t wide_bytes = 3 * seg + flex::sort_count_bytes<flex::SortWide>(num_edges);
+  const uint64_t narrow_bytes = 3 * seg + flex::sort_count_bytes<flex::SortNarrow<8>>(num_edges);
+  const uint64_t wide_bytes = 3 * seg + flex::sort_count_bytes<flex::SortWide<10>>(num_edges);
   if (!d_scratch || scratch_bytes < narrow_bytes) return FLEXSPMV_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(d_scratch) & 15u) return FLEXSPMV_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -468,10 +473,12 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
   if (num_edges > 0) {
     int bits = 0;
     while (bits < 31 && (1ll << bits) < num_rows) ++bits;
-    // 10-bit digits where they save a pass
-    const bool wide = scratch_bytes >= wide_bytes && (bits + 9) / 10 < (bits + 7) / 8;
+    // 10-bit digits where they save a pass: always the second one, a third (or fourth) one up to 5 M ids, where passes are short.  us, the
+    // whole sort and a permutation, wide / narrow digits: 3.2 M ids, 17 and 18 bits 140 / 152, 137 / 152; 8.4 M, 20 bits 295 / 284; 30 M, 19 bits
+    // 1163 / 1095.
+    const bool wide = scratch_bytes >= wide_bytes && (bits + 9) / 10 < (bits + 7) / 8 && (bits <= 10 || num_edges <= 5ll << 20);
     // the totals are the last words of the scratch that the shape takes
-    unsigned* totals = reinterpret_cast<unsigned*>(base + (wide ? wide_bytes : narrow_bytes)) - (wide ? flex::SortWide::kBins : flex::SortNarrow::kBins);
+    unsigned* totals = reinterpret_cast<unsigned*>(base + (wide ? wide_bytes : narrow_bytes)) - (wide ? flex::SortWide<10>::kBins : flex::SortNarrow<8>::kBins);
     if (bits == 0) {
       const int g = flex::grid_for(num_edges, 256);
       if (id_bits == 32)
@@ -480,8 +487,18 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
         flex::sort_identity_kernel<long long><<<g, 256, 0, st>>>(static_cast<const long long*>(d_row_ids), num_edges, num_rows, keys[0],
                                                                  d_perm, d_status);
     } else {
-      auto sort = wide ? flex::sort_passes<flex::SortWide> : flex::sort_passes<flex::SortNarrow>;
-      if (int e = sort(d_row_ids, id_bits, num_edges, num_rows, bits, d_perm, keys, spare, hist, totals, d_status, st, cur)) return e;
+      const int passes = (bits + (wide ? 9 : 7)) / (wide ? 10 : 8), width = (bits + passes - 1) / passes;
+      auto sort = flex::sort_passes<flex::SortNarrow<4>>;             // 1 to 4 bits
+      switch (width) {
+        case 5: sort = flex::sort_passes<flex::SortNarrow<5>>; break;
+        case 6: sort = flex::sort_passes<flex::SortNarrow<6>>; break;
+        case 7: sort = flex::sort_passes<flex::SortNarrow<7>>; break;
+        case 8: sort = flex::sort_passes<flex::SortNarrow<8>>; break;
+        case 9: sort = flex::sort_passes<flex::SortWide<9>>; break;
+        case 10: sort = flex::sort_passes<flex::SortWide<10>>; break;
+        default: break;
+      }
+      if (int e = sort(d_row_ids, id_bits, num_edges, num_rows, passes, d_perm, keys, spare, hist, totals, d_status, st, cur)) return e;
     }
   }
   if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return (int)e;
