@@ -172,8 +172,8 @@ TUNED_CONFIGS = {
 }
 
 
-# Row-mode graphs: one large CTA an SM for large launches of short rows (GraphApi::use_big; consumer threads, merge items per thread,
-# stages, CTAs per SM).  A tile of 4 items a thread is a row of three edges a thread, less one item each.  us on meshes of 1024^2
+# Other configurations for large launches (GraphApi::use_big; consumer threads, merge items per thread, stages, CTAs per SM[, edges a
+# batch in the loop over whole rows]).  Row-mode graphs: one large CTA an SM on short rows.  A tile of 4 items a thread is a row of three edges a thread, less one item each.  us on meshes of 1024^2
 # squares, CTAs an SM x warps: the shallow-water step 3 x 9 368, 1 x 24 332 (tiles of 3 items a thread 367, of 5 370), 1 x 28 367, 2 x 12
 # 363, 1 x 20 363; Rusanov fp64 3 x 9 76.3, 1 x 24 74.0, 1 x 28 77.0, 2 x 12 76.2; fp32 4 x 9 48.9, 1 x 32 45.8, 1 x 28 48.0, 1 x 24 52.0.
 TUNED_BIG_CONFIGS = {
@@ -184,6 +184,21 @@ TUNED_BIG_CONFIGS = {
     "spring_mass_f32": (992, 8, 2, 1),
     "spring_mass_f64": (736, 7, 2, 1),
 }
+
+
+def big_config(ir: GraphIR, dtype: str):
+    """The configuration for large launches: as measured for a graph, or that of longer rows for any graph of SpMV's shape (one value and
+    one gathered value an edge, one sum a row, a light map).  27 columns, 1 M rows, batches of 8 / 9 / 10 / 12: fp32 41.7 / 39.8 / 40.5 / 42.9 us
+    (480 threads x 7, 3 stages, batch 4 39.8; the usual configuration 49.9), fp64 62.0 / 60.3 / 60.7 / 82.1 (992 x 5 x 1, batch 4 66.6; 65.4)."""
+    named = TUNED_BIG_CONFIGS.get(f"{ir.name}_{CTYPE[dtype][1]}")
+    if named or dtype == "int64" or not ir.has_reducer or not light_map(ir) or stores_per_edge(ir):
+        return named
+    gathered = [s_ for s_ in ir.selector_register if s_.get("selector") == 1]
+    edge = {s_["target"]: dim_of(s_["shape"]) for s_ in ir.selector_register if s_.get("selector") != 1}
+    sums = sum(dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer")
+    if any(s_.get("row_identity") for s_ in gathered) or [dim_of(s_["shape"]) for s_ in gathered] != [1] or list(edge.values()) != [1] or sums != 1:
+        return None
+    return (352, 10, 2, 2, 9) if VBYTES[dtype] == 4 else (352, 8, 2, 2, 9)
 
 
 # Configuration of the warp kernel for matrices whose gathers have no locality (csrc/flex_warp_kernel.cuh):
@@ -769,10 +784,10 @@ def emit_graph(ir: GraphIR, dtype: str, symbol: str | None = None, config=None, 
         w(f"using CfgLean = flex::WarpCfg<{lb}, {li}, {lm}>;      // the warp kernel for matrices with random columns")
     else:
         w("using CfgLean = flex::NoLean;")
-    big = _override(symbol + "_big") or TUNED_BIG_CONFIGS.get(f"{ir.name}_{sfx}")
+    big = _override(symbol + "_big") or big_config(ir, dtype)
     if big:
         bb, bi, bs, bm = big[:4]
-        w(f"using CfgBig = flex::TileCfg<{bb}, {bi}, {bs}, {bm}, {batch}, false, {row_batch}>;      // for large launches")
+        w(f"using CfgBig = flex::TileCfg<{bb}, {bi}, {bs}, {bm}, {batch}, false, {big[4] if len(big) > 4 else row_batch}>;      // for large launches")
     w(f"}}  // namespace gen_{symbol}")
     w("}  // namespace")
     for i_, line in enumerate(L):

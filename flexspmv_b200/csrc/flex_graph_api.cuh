@@ -109,13 +109,24 @@ struct GraphApi {
   // Spring-mass fp32, 9 M items: rows of 8 31.3 / 42.3, of 4 - 12 46.7 / 52.4, of 9 38.6 / 36.5 (three words for a row, which single indices read
   // without conflicts): 8.5 rows for ten threads at least; one row of 40 among rows of 8 50.9 / 46.9, fp64 94.4 / 98.1.
   // Callers that name a tile or a number of CTAs get the configuration that they know.
-  static constexpr int kBigTile = CfgBig::kTile - CfgBig::kIpt, kLeastRows = G::kGroup > 1 ? 17 : 14;      // rows a tile, for 20 threads
+  static constexpr int kBigTile = CfgBig::kTile - (G::kGatherNeedsRow ? CfgBig::kIpt : 0), kLeastRows = G::kGroup > 1 ? 17 : 14;      // rows a tile, for 20 threads
+  // Two-phase graphs (SpMV): rows of 21 to 32 edges on average.  A tile of 1280 items holds 45 rows of 27, so that a warp has 32 of them or 13, and
+  // a row takes seven rounds of four gathers; two CTAs of 12 warps leave registers for nine at a time and hold 100 or 125 rows.  us, CfgBig / Cfg,
+  // 27 columns a row: fp32 300 007 rows 15.3 / 18.4, 1 M 39.8 / 49.9, 3 M 116 / 149; fp64 21.8 / 23.6, 60.3 / 65.4, 175 / 189.  12 M items, columns side by side, fp32
+  // and fp64: rows of 24 29.2 / 30.6, 42.4 / 43.9; of 31 20.6 / 25.4, 28.8 / 31.8; of 32 61.7 / 67.3, 64.7 / 65.3; of 20 - 32 22.8 / 25.8, 33.5 / 33.8.  Shorter ones gain where
+  // they begin in many banks, and lose where they do not: of 18 18.4 / 24.1, 26.3 / 29.0, of 20 21.7 / 22.4, 31.4 / 30.1 (3 M items fp32 9.4 / 8.8), of 16 42.4 / 40.7, 64.5 / 63.8.
+  static constexpr int kBigRowEdges = 21;
   static bool use_big(const flexspmv_desc* d) {
     if constexpr (kBigBuilt) {
       const long long sms = device_sm_count(), items = d->num_rows + d->num_edges;
       if (d->tile_items > 0 || d->max_ctas > 0 || use_lean(d) || use_win(d)) return false;
-      const long long ten_rows = 10 * d->num_rows * kBigTile, each_a_row = items * CfgBig::kBlock;
-      if (items <= sms * CfgBig::kMinCtas * kBigTile || 2 * ten_rows < kLeastRows * each_a_row || ten_rows > 11 * each_a_row) return false;
+      if (items <= sms * CfgBig::kMinCtas * kBigTile) return false;
+      if constexpr (G::kGatherNeedsRow) {
+        const long long ten_rows = 10 * d->num_rows * kBigTile, each_a_row = items * CfgBig::kBlock;
+        if (2 * ten_rows < kLeastRows * each_a_row || ten_rows > 11 * each_a_row) return false;
+      } else if (d->num_edges < (long long)kBigRowEdges * d->num_rows || d->num_edges > (long long)kWholeRowMax * d->num_rows) {
+        return false;
+      }
       const long long tiles = (items + kDefaultTile - 1) / kDefaultTile, slots = sms * Cfg::kMinCtas;
       return !small_launch(d, tiles, tiles < slots ? tiles : slots, Cfg::kBlock + 32);
     }

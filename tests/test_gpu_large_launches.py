@@ -121,3 +121,37 @@ def test_words_of_four_edges_at_odd_places(bits, skip, last):
         assert (header_word(ext, 10) > default_tile(ir, dtype)) == (max_ctas == 0)
         outs.append(out.cpu().numpy().tobytes())
     assert outs[0] == outs[1]
+
+
+@pytest.mark.parametrize("dt,tile", [("float64", 352 * 8), ("float32", 352 * 10)])
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("lengths,large", [([27], True), ([21], True), ([32], True), ([20], False), ([33], False), ([30, 0, 32, 9, 31, 32, 28, 10], True),
+                                           ([27] * 5000 + [40], True), ([25] * 3000 + [900, 0, 0], True)],
+                         ids=["27", "21", "32", "20", "33", "uneven", "one_of_40", "long"])
+def test_longer_rows_of_spmv(dt, tile, bits, lengths, large):
+    """21 to 32 edges a row on average: batches of nine in two CTAs of 12 warps, or the loop with carries where a row is longer than 32."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    times = int(2 * sms() * tile * 1.3 / (sum(lengths) + len(lengths))) + 1
+    prob = with_lengths(ir, lengths * times, 233, dtype)
+    items = prob.num_rows + prob.nnz
+    ext = GraphExtension(ir, random_gather=False)
+    got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+    ext.check()
+    each = -(-items // (2 * sms() * tile))
+    assert header_word(ext, 10) == (-(-items // (2 * sms() * each)) if large else default_tile(ir, dtype))
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    assert_outputs_match(ir, got, ref, sums, dtype, what=f"spmv {dt}")
+    if large and max(lengths) <= 32:
+        named, whole = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=4 * sms())
+        rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, ROUNDS)
+        assert whole and [g.tobytes() for g in got] == named == rounds
+
+
+@pytest.mark.parametrize("dt,tile", [("float64", 352 * 8), ("float32", 352 * 10)])
+def test_a_tile_a_cta_of_longer_rows_keeps_the_other_configuration(dt, tile):
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    for more, large in ((0, False), (28, True)):
+        prob = with_lengths(ir, [27] * ((2 * sms() * tile + more) // 28), 239, dtype)
+        ext = GraphExtension(ir, random_gather=False)
+        run_gpu(ext, ir, prob, dtype)
+        assert (header_word(ext, 10) != default_tile(ir, dtype)) == large
