@@ -118,15 +118,17 @@ struct GraphApi {
   static constexpr int kBigRowEdges = 21;
   static bool use_big(const flexspmv_desc* d) {
     if constexpr (kBigBuilt) {
-      const long long sms = device_sm_count(), items = d->num_rows + d->num_edges;
-      if (d->tile_items > 0 || d->max_ctas > 0 || use_lean(d) || use_win(d)) return false;
-      if (items <= sms * CfgBig::kMinCtas * kBigTile) return false;
+      // (a launch asks several times: what needs no look at the device first)
+      const long long items = d->num_rows + d->num_edges;
+      if (items <= kBigTile || d->tile_items > 0 || d->max_ctas > 0 || use_lean(d) || use_win(d)) return false;
       if constexpr (G::kGatherNeedsRow) {
         const long long ten_rows = 10 * d->num_rows * kBigTile, each_a_row = items * CfgBig::kBlock;
         if (2 * ten_rows < kLeastRows * each_a_row || ten_rows > 11 * each_a_row) return false;
       } else if (d->num_edges < (long long)kBigRowEdges * d->num_rows || d->num_edges > (long long)kWholeRowMax * d->num_rows) {
         return false;
       }
+      const long long sms = device_sm_count();
+      if (items <= sms * CfgBig::kMinCtas * kBigTile) return false;
       const long long tiles = (items + kDefaultTile - 1) / kDefaultTile, slots = sms * Cfg::kMinCtas;
       return !small_launch(d, tiles, tiles < slots ? tiles : slots, Cfg::kBlock + 32);
     }
@@ -337,6 +339,14 @@ struct GraphApi {
   //                     13.5 MB 28.5 / 28.6, 26 51.6 / 52.2, 35 64.6 / 64.1, 54 100.4 / 97.8
   static constexpr long long kKeepBytes = (G::kGatherNeedsRow ? 10ll : 40ll) << 20;
 
+  // SpMV on rows of four to five edges on average (five-point grids): batches of five, so that a row is one round of gathers instead of two, in
+  // launches without stages and in tiles a CTA's own run.  us, batches of four / five: 512^2 fp64 4.9 / 4.6, 600^2 8.05 / 7.50, fp32 5.8 / 4.8; 700^2 fp64 10.05 /
+  // 9.2, 1500^2 34.5 / 33.5, fp32 26.1 / 24.0.  Not in rounds, where more gathers at a time leave L2 earlier: 2500^2 fp64 83.0 / 86.1.  Of any other
+  // length it gains less than it loses: 1.2 M items without stages fp64, rows of 4 5.25 / 5.40, of 6 6.0 / 6.4, 62^3 7-point 6.76 / 7.06; 145^3 55.2 / 58.0, fp32 42.1 / 44.2.
+  template <class C>
+  static constexpr bool kFiveBuilt = !G::kGatherNeedsRow && G::kLightMap && G::kAccDim == 1 && C::kRowBatch == 4 && !C::kPipeline && !C::kLarge;
+  static bool rows_of_five(const flexspmv_desc* d) { return d->num_edges > 4 * d->num_rows && d->num_edges <= 5 * d->num_rows; }
+
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
   // once for each device of the process, then one word is read (a launch asks twice, for the plan's grid and for the form that it takes).
   template <typename OffsetT, class C = Cfg, bool WIN = false, int MODE = kPlain>
@@ -411,6 +421,19 @@ struct GraphApi {
         form = FLEXSPMV_KERNEL_TILE_ROUNDS;
         kernel = flex_tile_kernel<G, OffsetT, C, WIN, kRounds>;
         if (int e = resident_ctas<OffsetT, C, WIN, kRounds>(&resident)) return e;
+      }
+    }
+    if constexpr (L::kWhole && !WIN && kFiveBuilt<C>) {
+      if (whole_rows && form != FLEXSPMV_KERNEL_TILE_ROUNDS && rows_of_five(d)) {
+        using Five = TileCfg<C::kBlock, C::kIpt, C::kStages, C::kMinCtas, C::kBatch, false, 5>;         // (the same stages and tiles)
+        static_assert(TileSmemLayout<G, OffsetT, Five>::kTotal == L::kTotal);
+        if (form == FLEXSPMV_KERNEL_TILE_SMALL) {
+          kernel = flex_tile_kernel<G, OffsetT, Five, false, kSmall>;
+          if (int e = resident_ctas<OffsetT, Five, false, kSmall>(&resident)) return e;
+        } else {
+          kernel = flex_tile_kernel<G, OffsetT, Five, false, kPlain>;
+          if (int e = resident_ctas<OffsetT, Five, false, kPlain>(&resident)) return e;
+        }
       }
     }
     note_kernel(form);

@@ -329,3 +329,33 @@ def test_wide_records_in_small_ctas(dt, lengths):
         got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int64 if "max_ctas" in kw else np.int32)
         ext.check()
         assert_outputs_match(ir, got, ref, sums, dtype, what=f"mixed_dims {dt} {kw}")
+
+
+@pytest.mark.parametrize("dt", ["float64", "float32", "int64"])
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("lengths", [[5], [4, 5], [3, 4, 5, 6, 7], [0, 10, 5, 5], [1, 9, 4, 5, 5, 0, 6]], ids=["5", "4_5", "3_to_7", "0_10", "1_to_9"])
+@pytest.mark.parametrize("rows,kernel", [(9000, SMALL), (600_000, TILE)])
+def test_rows_of_five_edges_in_one_round(dt, bits, lengths, rows, kernel):
+    """Four to five edges a row on average are taken five at a time; the same rows in front of others that bring the average out of that
+    range are taken four at a time.  The same bits."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    mine = (lengths * (rows // len(lengths) + 1))[:rows]
+    others = [8] * (rows // 3)
+    prob = with_lengths(ir, mine + others, 241, dtype)
+    n, e = len(mine), sum(mine)
+    assert 4 * n < e <= 5 * n and prob.nnz > 5 * prob.num_rows
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    non_gather, gathers, index_names = graphs.operator_signature(ir)
+    x = dev(prob.values[gathers[0]].astype(dtype))
+    results = []
+    for count, edges in ((n, e), (prob.num_rows, prob.nnz)):
+        ext = GraphExtension(ir, random_gather=False)
+        y = torch.full((count,), 7, dtype=x.dtype, device="cuda")
+        ext.launch_into([dev(prob.values[non_gather[0]][:edges].astype(dtype)), x], [dev(prob.indices[index_names[0]][:edges])],
+                        dev(prob.row_offsets[:count + 1].astype(np.int32 if bits == 32 else np.int64)), [y], count, edges, prob.num_cols)
+        if count == n:
+            assert last_kernel() == kernel
+        ext.check()
+        assert ext.planned_whole_rows()
+        results.append(y[:n].cpu().numpy().tobytes())
+    assert results[0] == results[1]
