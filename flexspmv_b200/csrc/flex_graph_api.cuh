@@ -339,13 +339,17 @@ struct GraphApi {
   //                     13.5 MB 28.5 / 28.6, 26 51.6 / 52.2, 35 64.6 / 64.1, 54 100.4 / 97.8
   static constexpr long long kKeepBytes = (G::kGatherNeedsRow ? 10ll : 40ll) << 20;
 
-  // SpMV on rows of four to five edges on average (five-point grids): batches of five, so that a row is one round of gathers instead of two, in
-  // launches without stages and in tiles a CTA's own run.  us, batches of four / five: 512^2 fp64 4.9 / 4.6, 600^2 8.05 / 7.50, fp32 5.8 / 4.8; 700^2 fp64 10.05 /
-  // 9.2, 1500^2 34.5 / 33.5, fp32 26.1 / 24.0.  Not in rounds, where more gathers at a time leave L2 earlier: 2500^2 fp64 83.0 / 86.1.  Of any other
-  // length it gains less than it loses: 1.2 M items without stages fp64, rows of 4 5.25 / 5.40, of 6 6.0 / 6.4, 62^3 7-point 6.76 / 7.06; 145^3 55.2 / 58.0, fp32 42.1 / 44.2.
+  // SpMV on rows of four to five edges on average (five-point grids), and of five to seven in 4-byte values (seven-point ones): batches of as
+  // many, so that a row is one round of gathers instead of two, in launches without stages and in tiles a CTA's own run.  us, batches of
+  // four / five: 512^2 fp64 4.9 / 4.6, 600^2 7.9 / 7.5, fp32 5.7 / 4.8; 700^2 fp64 10.1 / 9.3, 1500^2 34.5 / 33.4, fp32 26.1 / 24.0; four / seven, fp32: 60^3 4.46 / 4.18, 80^3 10.2 /
+  // 9.9, 145^3 42.1 / 40.9, 200^3 110.5 / 107.5, rows of 6, 8 M items 16.6 / 16.1.  Not in rounds, where more gathers at a time leave L2 earlier: 2500^2 fp64
+  // 83.0 / 86.1, 240^3 fp32 182 / 192.  Other lengths gain less than they lose: five at a time fp64, 1.2 M items without stages, rows of 4 5.25 / 5.40, of 6
+  // 6.0 / 6.4, 145^3 55.2 / 58.0; seven at a time fp32, 8 M items, rows of 3 16.3 / 18.2, of 8 23.4 / 24.9, 0 - 30 22.0 / 22.8, fp64 145^3 55.2 / 68.7.
   template <class C>
-  static constexpr bool kFiveBuilt = !G::kGatherNeedsRow && G::kLightMap && G::kAccDim == 1 && C::kRowBatch == 4 && !C::kPipeline && !C::kLarge;
-  static bool rows_of_five(const flexspmv_desc* d) { return d->num_edges > 4 * d->num_rows && d->num_edges <= 5 * d->num_rows; }
+  static constexpr bool kOneRoundBuilt = !G::kGatherNeedsRow && G::kLightMap && G::kAccDim == 1 && C::kRowBatch == 4 && !C::kPipeline && !C::kLarge;
+  static bool row_edges_within(const flexspmv_desc* d, int above, int most) {
+    return d->num_edges > above * d->num_rows && d->num_edges <= most * d->num_rows;
+  }
 
   // CTAs of the tile kernel that one SM holds.  The shared-memory opt-in and the occupancy are per device: looked up
   // once for each device of the process, then one word is read (a launch asks twice, for the plan's grid and for the form that it takes).
@@ -423,17 +427,19 @@ struct GraphApi {
         if (int e = resident_ctas<OffsetT, C, WIN, kRounds>(&resident)) return e;
       }
     }
-    if constexpr (L::kWhole && !WIN && kFiveBuilt<C>) {
-      if (whole_rows && form != FLEXSPMV_KERNEL_TILE_ROUNDS && rows_of_five(d)) {
-        using Five = TileCfg<C::kBlock, C::kIpt, C::kStages, C::kMinCtas, C::kBatch, false, 5>;         // (the same stages and tiles)
-        static_assert(TileSmemLayout<G, OffsetT, Five>::kTotal == L::kTotal);
-        if (form == FLEXSPMV_KERNEL_TILE_SMALL) {
-          kernel = flex_tile_kernel<G, OffsetT, Five, false, kSmall>;
-          if (int e = resident_ctas<OffsetT, Five, false, kSmall>(&resident)) return e;
-        } else {
-          kernel = flex_tile_kernel<G, OffsetT, Five, false, kPlain>;
-          if (int e = resident_ctas<OffsetT, Five, false, kPlain>(&resident)) return e;
-        }
+    if constexpr (L::kWhole && !WIN && kOneRoundBuilt<C>) {
+      auto batch_of = [&](auto edges) -> int {
+        using One = TileCfg<C::kBlock, C::kIpt, C::kStages, C::kMinCtas, C::kBatch, false, edges.value>;      // (the same stages and tiles)
+        static_assert(TileSmemLayout<G, OffsetT, One>::kTotal == L::kTotal);
+        const bool small = form == FLEXSPMV_KERNEL_TILE_SMALL;
+        kernel = small ? flex_tile_kernel<G, OffsetT, One, false, kSmall> : flex_tile_kernel<G, OffsetT, One, false, kPlain>;
+        return small ? resident_ctas<OffsetT, One, false, kSmall>(&resident) : resident_ctas<OffsetT, One, false, kPlain>(&resident);
+      };
+      if (whole_rows && form != FLEXSPMV_KERNEL_TILE_ROUNDS) {
+        int e = 0;
+        if (row_edges_within(d, 4, 5)) e = batch_of(IntC<5>{});
+        else if constexpr (sizeof(V) == 4) { if (row_edges_within(d, 5, 7)) e = batch_of(IntC<7>{}); }
+        if (e) return e;
       }
     }
     note_kernel(form);

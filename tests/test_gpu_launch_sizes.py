@@ -333,17 +333,18 @@ def test_wide_records_in_small_ctas(dt, lengths):
 
 @pytest.mark.parametrize("dt", ["float64", "float32", "int64"])
 @pytest.mark.parametrize("bits", [32, 64])
-@pytest.mark.parametrize("lengths", [[5], [4, 5], [3, 4, 5, 6, 7], [0, 10, 5, 5], [1, 9, 4, 5, 5, 0, 6]], ids=["5", "4_5", "3_to_7", "0_10", "1_to_9"])
+@pytest.mark.parametrize("lengths", [[5], [4, 5], [3, 4, 5, 6, 7], [0, 10, 5, 5], [1, 9, 4, 5, 5, 0, 6], [7], [6, 7, 7, 5], [0, 14, 6, 8, 3]],
+                         ids=["5", "4_5", "3_to_7", "0_10", "1_to_9", "7", "5_to_7", "0_14"])
 @pytest.mark.parametrize("rows,kernel", [(9000, SMALL), (600_000, TILE)])
-def test_rows_of_five_edges_in_one_round(dt, bits, lengths, rows, kernel):
-    """Four to five edges a row on average are taken five at a time; the same rows in front of others that bring the average out of that
-    range are taken four at a time.  The same bits."""
+def test_short_rows_in_one_round(dt, bits, lengths, rows, kernel):
+    """Four to five edges a row on average are taken five at a time, and five to seven (4-byte values) seven; the same rows in front of
+    others that bring the average out of those ranges are taken four at a time.  The same bits."""
     ir, dtype = graphs.spmv_graph(), np.dtype(dt)
     mine = (lengths * (rows // len(lengths) + 1))[:rows]
-    others = [8] * (rows // 3)
+    others = [12] * rows
     prob = with_lengths(ir, mine + others, 241, dtype)
     n, e = len(mine), sum(mine)
-    assert 4 * n < e <= 5 * n and prob.nnz > 5 * prob.num_rows
+    assert 4 * n < e <= 7 * n and prob.nnz > 7 * prob.num_rows
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
     non_gather, gathers, index_names = graphs.operator_signature(ir)
     x = dev(prob.values[gathers[0]].astype(dtype))
