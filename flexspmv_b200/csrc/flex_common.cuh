@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <cstdlib>
 
 #include "flexspmv.h"   // the public C header (include/ of the project; the build passes -I for it)
 
@@ -255,6 +256,27 @@ __device__ __forceinline__ T shfl_up_any(T v, int delta) {
 template <typename T>
 __device__ __forceinline__ T shfl_down_any(T v, int delta) {
   return __shfl_down_sync(0xffffffffu, v, delta);
+}
+
+// ---- host: launches ----------------------------------------------------------------------------
+// FLEXSPMV_NO_PDL=1 in the environment launches the kernels without the programmatic-dependent-launch attribute.
+inline bool pdl_enabled() {
+  static const bool on = [] { const char* e = getenv("FLEXSPMV_NO_PDL"); return !(e && e[0] == '1'); }();
+  return on;
+}
+
+// Launches with the programmatic-dependent-launch attribute: the CTAs may be placed while the kernel before this one on
+// the stream drains; the kernels touch no global memory before their griddepcontrol.wait.  Back-to-back launches of
+// small problems (a time-stepping loop) then overlap one launch's set-up with the tail of the one before.
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3((unsigned)block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace flex

@@ -210,6 +210,42 @@ def test_scratch_for_eight_bit_digits_is_enough():
             assert code == 0 and np.array_equal(perm.cpu().numpy(), np.argsort(ids, kind="stable").astype(np.int32))
 
 
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("n,rows", [(5, 3), (4097, 1), (20_011, 200), (300_007, 10_007), (600_011, 600_000)])
+def test_sorts_behind_one_another_share_scratch(n, rows, captured):
+    """The kernels of a sort start while the ones before them drain: sorts of new ids over the same scratch and outputs,
+    nothing between them but the stream's order."""
+    lib = load_library()
+    need = ctypes.c_size_t()
+    assert lib.flexspmv_sort_rows_bytes(ctypes.c_int64(n), ctypes.byref(need)) == 0
+    rng = np.random.default_rng(n)
+    scratch, ids_now = torch.empty(need.value, dtype=torch.uint8, device="cuda"), torch.zeros(n, dtype=torch.int64, device="cuda")
+    perm, crow = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+    status = torch.empty(1, dtype=torch.int32, device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def sort():
+        assert lib.flexspmv_sort_rows(ptr(ids_now), 64, ctypes.c_int64(n), ctypes.c_int64(rows), ptr(perm), ptr(crow), 32, ptr(scratch),
+                                      ctypes.c_size_t(need.value), ptr(status), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+    graph = torch.cuda.CUDAGraph()
+    if captured:
+        with torch.cuda.graph(graph):
+            sort()
+    ids = [rng.integers(0, rows, n) for _ in range(6)]
+    on_device = [torch.from_numpy(i).cuda() for i in ids]
+    got = []
+    for i in on_device:
+        ids_now.copy_(i)
+        graph.replay() if captured else sort()
+        got.append((perm.clone(), crow.clone()))
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    for i, (p, c) in zip(ids, got):
+        assert np.array_equal(p.cpu().numpy(), np.argsort(i, kind="stable").astype(np.int32))
+        assert np.array_equal(c.cpu().numpy(), np.searchsorted(np.sort(i), np.arange(rows + 1)))
+
+
 @pytest.mark.parametrize("rows", [1, 255, 256, 257, 1025, 300_000, 303_104, 303_105, 400_001])
 @pytest.mark.parametrize("ids", ["few", "limit", "above", "skewed"])
 @pytest.mark.parametrize("offset_bits", [32, 64])
