@@ -4,10 +4,10 @@
 // stands for (the swe_boundary graph's pow / mul / sum and flexspmv_swe_rk_stage), so the states are bit-identical to
 // theirs.  In the flux kernel the sums never leave their registers and the wall terms cost nothing on cells without a
 // wall: per cell 16 bytes of memory traffic a sum, 32 a wall sum and two launches a stage less.
-// Bound by the latency of the gathers and of the cell's own records (26 warps per SM at 72 registers, 51 % of DRAM); the
+// Bound by the latency of the gathers and of the cell's own records (23 warps per SM at 80 registers, 57 % of DRAM); the
 // producer warp therefore asks for those records in L2 when it stages a tile (prefetch_rows: 510 -> 454 us a step).  A step of
-// the model on 2 097 152 cells, fp64: 606 us as 12 launches, 369 us as 4 (1024 x 1024 squares); on 20 402 cells
-// 57.4 -> 23.8 us (30.8 with stages).
+// the model on 2 097 152 cells, fp64: 606 us as 12 launches, 333 us as 4 (1024 x 1024 squares; 369 in three CTAs of 9 warps, GraphApi::use_big);
+// on 20 402 cells 57.4 -> 23.8 us (30.8 with stages), as one launch (flex_swe_step.cuh) 20.5.
 // fp64 batches of 1 / 2 edges per thread at 3 CTAs per SM, 3 at 2, 1 at 4 (before the prefetch): 510 / 546 / 625 / 555 us;
 // fp32, 4 CTAs per SM, batches of 4 / 1: 327 / 286 us.
 #pragma once

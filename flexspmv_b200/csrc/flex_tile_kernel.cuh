@@ -636,7 +636,7 @@ flex_tile_kernel(const typename G::Params p, const TileKernelArgs a) {
       // What the two-phase loop is bound by on short rows is the shared-memory / L1 data pipe (75 - 80 % busy at 55 % of
       // DRAM) and two CTA barriers a tile; this one moves no product through shared memory and a third of the gather lines
       // (41 % of the pipe at 70 % of DRAM), and is bound by the latency of the gathers at the registers of 4 CTAs per SM: 10 of
-      // 16 stall cycles per issue are long_scoreboard.  us a launch, two-phase / this loop with a run of tiles a CTA: 7-point fp64
+      // 16 stall cycles per issue are long_scoreboard (row-mode graphs, and longer rows in large launches: GraphApi::use_big).  us a launch, two-phase / this loop with a run of tiles a CTA: 7-point fp64
       // SpMV 512^3 3205 / 2564 (in rounds 2133); 145^3 fp32 54.1 / 42.6; 5-point 512^2 fp64 9.1 / 7.1 (without stages 5.1); 27 columns a row
       // fp64, 300 007 rows 26.2 / 23.9; spring-mass 1024^2 fp32 44.5 / 38.4; Rusanov 1024^2 fp64 92 / 83.5.
       constexpr int RB = Cfg::kRowBatch;
