@@ -457,7 +457,7 @@ class PreparedLaunch:
             with torch.cuda.device(self._device):
                 return self.launch()
         if self._plan._flag_view[0]:
-            _raise_if_failed(self.ext.lib, self._plan, "launch")
+            self.raise_if_failed()
         stream = _raw_stream(self._device)
         if stream not in self._ordered:                       # first use on another stream: after the plan
             if torch.cuda.is_current_stream_capturing():
@@ -474,6 +474,11 @@ class PreparedLaunch:
             self.ext.check()
 
     __call__ = launch
+
+    def raise_if_failed(self, what: str = "launch") -> None:
+        """Raises FlexSpmvError where a kernel has given up on this object's workspace, as far as the host has been told
+        (one read of host memory, no synchronisation)."""
+        _raise_if_failed(self.ext.lib, self._plan, what)
 
 
 def load_builtin(name: str, **kw) -> GraphExtension:

@@ -55,6 +55,7 @@ class ShallowWaterStep:
         self.stage = new(3)                               # the state the next delta is evaluated at
         self.acc = new(3)                                 # running sum of the increments
         self._graph: Optional[torch.cuda.CUDAGraph] = None
+        self._step = None
         self._fused = None if own else self._bind_fused(new)
         if self._fused is not None:
             return
@@ -83,7 +84,6 @@ class ShallowWaterStep:
         other = new(3)
         state = [m["h"], m["uh"], m["vh"]]
         launches = []
-        self._step = None
         self._coef, self._coef_dt = [], float(self.dt)
         for k, (c, first, last) in enumerate(self._coefficients()):
             src = state if k == 0 else (self.stage if k % 2 else other)
@@ -158,9 +158,28 @@ class ShallowWaterStep:
         self._graph = g
 
     def replay(self) -> None:
+        """One captured step.  Raises FlexSpmvError, as ``forward`` does, where an earlier one failed on the device: the launches
+        of a graph leave a workspace whose status is raised without doing anything, and the state would stand still."""
         if self._graph is None:
             raise RuntimeError("capture() first")
+        self._raise_if_failed("replay")
         self._graph.replay()
+
+    # -- errors --------------------------------------------------------------------------------------------
+    def _bound_launches(self):
+        if self._fused is not None:
+            return self._fused if self._step is None else [self._step] + self._fused
+        return list(self._on_state + self._on_stage)
+
+    def _raise_if_failed(self, what: str) -> None:
+        for launch in self._bound_launches():
+            launch.raise_if_failed(what)
+
+    def check(self) -> None:
+        """Waits for the steps enqueued so far and raises FlexSpmvError if one of them gave up on the device (a bounded wait
+        ran out).  The state is undefined then: cells may be at different stages of a step."""
+        torch.cuda.synchronize(self.m["h"].device)
+        self._raise_if_failed("check")
 
 
 def assemble_shallow_water(mesh: Dict[str, torch.Tensor]) -> Dict[str, torch.Tensor]:

@@ -114,3 +114,25 @@ def test_a_barrier_that_stays_shut_runs_out():
     step.launch()
     ext.check()
     assert not torch.equal(m["h"], before["h"]) and torch.isfinite(m["h"]).all()
+
+
+def test_replays_after_a_run_out_raise():
+    """The launches of a captured step return at once on a workspace whose status is raised; the host has the status word and says so,
+    in ``replay`` and in ``check``."""
+    m = mesh_of(64, np.float64, False)
+    step = ShallowWaterStep(m, dt=1e-4)
+    assert step._step is not None
+    step.capture()
+    step.replay()
+    step.check()
+    before = {k: m[k].clone() for k in STATE}
+    lib = load_library()
+    assert lib.flexspmv_debug_withhold_stage(ctypes.c_void_p(step._step._keep[-1].data_ptr()), ctypes.c_uint32(1), None) == 0
+    torch.cuda.synchronize()
+    step.replay()
+    with pytest.raises(FlexSpmvError, match="check.*status -6"):
+        step.check()
+    for call in (step.replay, step.forward):
+        with pytest.raises(FlexSpmvError, match="status -6"):
+            call()
+    assert all(torch.equal(m[k], before[k]) for k in STATE)

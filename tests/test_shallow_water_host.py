@@ -1,0 +1,51 @@
+"""Host side of the shallow-water step, without a GPU."""
+import pytest
+
+from flexspmv_b200 import shallow_water
+from flexspmv_b200.binding import FlexSpmvError, PreparedLaunch, load_library
+
+
+class FakePlan:
+    def __init__(self):
+        self._flag_view = [0]
+
+    def status(self):
+        return self._flag_view[0]
+
+
+class FakeGraph:
+    replays = 0
+
+    def replay(self):
+        self.replays += 1
+
+
+def bare_launch(plan):
+    launch = PreparedLaunch.__new__(PreparedLaunch)
+    launch.ext = type("Ext", (), {"lib": load_library()})
+    launch._plan = plan
+    return launch
+
+
+def bare_step(**attributes):
+    step = shallow_water.ShallowWaterStep.__new__(shallow_water.ShallowWaterStep)
+    step.__dict__.update(_step=None, _fused=None, _graph=FakeGraph(), **attributes)
+    return step
+
+
+@pytest.mark.parametrize("form", ["one", "four", "twelve"])
+def test_replay_raises_where_an_earlier_step_failed(form):
+    plan = FakePlan()
+    step = bare_step()
+    if form == "twelve":
+        step._on_state, step._on_stage = (bare_launch(FakePlan()), bare_launch(FakePlan())), (bare_launch(FakePlan()), bare_launch(plan))
+    else:
+        step._fused = [bare_launch(plan) for _ in range(4)]
+        if form == "one":
+            step._step = bare_launch(plan)
+    step.replay()
+    assert step._graph.replays == 1
+    plan._flag_view[0] = -6
+    with pytest.raises(FlexSpmvError, match="replay.*status -6"):
+        step.replay()
+    assert step._graph.replays == 1
