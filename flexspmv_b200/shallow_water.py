@@ -72,6 +72,11 @@ class ShallowWaterStep:
         of the sum."""
         return ((0.5 * self.dt, 1, 0), (0.5 * self.dt, 0, 0), (self.dt, 0, 0), (0.0, 0, 1))
 
+    def _set_coefficients(self):
+        self._coef_dt = float(self.dt)
+        self._coef.copy_(torch.tensor([[c, self._coef_dt / 6, first, last] for c, first, last in self._coefficients()], device="cpu",
+                                      dtype=self._coef.dtype))
+
     def _bind_fused(self, new):
         """The four launches of a step, or None when the mesh was not planned with whole rows.  A stage reads one
         state and writes the next, and neighbours read what a cell wrote, so the states alternate between two sets
@@ -84,23 +89,19 @@ class ShallowWaterStep:
         other = new(3)
         state = [m["h"], m["uh"], m["vh"]]
         launches = []
-        self._coef, self._coef_dt = [], float(self.dt)
-        for k, (c, first, last) in enumerate(self._coefficients()):
+        # a row for each stage, in host memory that is read when a launch is made; both forms of the step read the same rows
+        self._coef = torch.empty(4, 4, dtype=dt_, device="cpu")
+        self._set_coefficients()
+        for k in range(4):
             src = state if k == 0 else (self.stage if k % 2 else other)
             dst = other if k % 2 else self.stage          # the last stage writes the state itself
-            # host memory, read when a launch is made
-            coef = torch.tensor([c, self.dt / 6, first, last], dtype=dt_, device="cpu")
-            self._coef.append(coef)
-            values = [m["alpha"], m["sx"], m["sy"]] + src + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [coef]
+            values = [m["alpha"], m["sx"], m["sy"]] + src + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [self._coef[k]]
             launches.append(ext.prepare(values, [m["src"], m["dst"]], self.ro, dst, self.nc, self.ne, self.nc))
             if k == 0 and not ext.planned_whole_rows():
                 return None
-        # meshes that fit the chip: the four stages in one launch (csrc/flex_swe_step.cuh); the coefficients side by side
-        all_coef = torch.stack(self._coef).contiguous()
-        values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [all_coef]
+        # meshes that fit the chip: the four stages in one launch (csrc/flex_swe_step.cuh)
+        values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [self._coef]
         self._step = ext.prepare_step(values, [m["src"], m["dst"]], self.ro, self.stage + other, self.nc, self.ne, self.nc)
-        if self._step is not None:
-            self._coef = list(all_coef)            # rows of it: set where the time step changes
         return launches
 
     def _bind(self, h, uh, vh):
@@ -124,11 +125,8 @@ class ShallowWaterStep:
         """swe_main.py:121-146: four delta evaluations (:86-119), each followed by its stage update.  ``dt`` may be set
         between calls (a step captured by ``capture`` keeps the one it was captured with)."""
         if self._fused is not None:
-            dt = float(self.dt)
-            if dt != self._coef_dt:
-                for coef, (c, first, last) in zip(self._coef, self._coefficients()):
-                    coef.copy_(torch.tensor([c, dt / 6, first, last], dtype=coef.dtype, device="cpu"))
-                self._coef_dt = dt
+            if float(self.dt) != self._coef_dt:
+                self._set_coefficients()
             for launch in [self._step] if self._step is not None else self._fused:
                 launch.launch()
             return

@@ -21,8 +21,6 @@ def both(mesh, steps=2, dt=1e-4):
     one, four = ShallowWaterStep(a, dt=dt), ShallowWaterStep(b, dt=dt)
     assert one._step is not None and four._fused is not None
     four._step = None
-    for launch, coef in zip(four._fused, one._coef):        # (the coefficients that four launches read are their own)
-        launch._keep[0][-1].copy_(coef)
     for _ in range(steps):
         one.forward()
         kernel = load_library().flexspmv_debug_last_kernel()
@@ -136,3 +134,18 @@ def test_replays_after_a_run_out_raise():
         with pytest.raises(FlexSpmvError, match="status -6"):
             call()
     assert all(torch.equal(m[k], before[k]) for k in STATE)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_the_time_step_reaches_both_forms(dtype):
+    """``dt`` set after binding: the four launches of a step whose one launch is left out take it too."""
+    a, b = mesh_of(40, dtype, True), mesh_of(40, dtype, True)
+    one, four = ShallowWaterStep(a, dt=1e-3), ShallowWaterStep(b, dt=1e-3)
+    assert one._step is not None
+    four._step = None
+    for dt in (1e-3, 2e-3, 0.5e-3):
+        one.dt = four.dt = dt
+        one.forward()
+        four.forward()
+        for k in STATE:
+            assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), (dt, k)
