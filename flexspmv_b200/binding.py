@@ -56,7 +56,11 @@ class GraphInfo(ctypes.Structure):
 
 
 class FlexSpmvError(RuntimeError):
-    pass
+    """``status``: the library's status behind the error, 0 where there is none."""
+
+    def __init__(self, message: str = "", status: int = 0):
+        super().__init__(message)
+        self.status = status
 
 
 _libs: Dict[str, ctypes.CDLL] = {}
@@ -79,7 +83,7 @@ def load_library(path: Optional[str] = None) -> ctypes.CDLL:
 
 def check(lib, status: int, what: str):
     if status != 0:
-        raise FlexSpmvError(f"{what} failed: {lib.flexspmv_error_string(status).decode()} (status {status})")
+        raise FlexSpmvError(f"{what} failed: {lib.flexspmv_error_string(status).decode()} (status {status})", status)
 
 
 _CHECK_EVERY_CALL = os.environ.get("FLEXSPMV_CHECK_STATUS", "0") == "1"
@@ -104,7 +108,7 @@ def _raise_if_failed(lib, plan: "_Plan", what: str):
     st = plan.status()
     if st != 0:
         raise FlexSpmvError(f"{what}: an earlier launch on this workspace failed on the device: "
-                            f"{lib.flexspmv_error_string(st).decode()} (status {st}); its outputs are undefined")
+                            f"{lib.flexspmv_error_string(st).decode()} (status {st}); its outputs are undefined", st)
 
 
 def _stream_ptr() -> ctypes.c_void_p:

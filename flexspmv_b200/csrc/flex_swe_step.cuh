@@ -242,13 +242,40 @@ struct StepApi {
   using V = typename G::V;
   static int fits(const flexspmv_desc* d) {
     StepShape<G> s;
-    return Api::check_desc(d) == 0 && s.fit(d, device_sm_count()) ? 1 : 0;
+    if (Api::check_desc(d) != 0 || !s.fit(d, device_sm_count())) return 0;
+    return d->offset_bits == 64 ? resident<long long>(s.more) : resident<int>(s.more);
+  }
+  template <typename OffsetT>
+  static auto kernel_of(bool more) {
+    return more ? flex_swe_step_kernel<G, OffsetT, kStepMoreThreads> : flex_swe_step_kernel<G, OffsetT, kStepThreads>;
+  }
+  // Whether the device launches cooperatively and an SM holds the largest CTA (looked up once for each device of the process; 1 where
+  // there is none to ask).
+  template <typename OffsetT>
+  static int resident(bool more) {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> known[2][kMaxDevices];       // 0: not looked up yet, 1: yes, -1: no
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return 1; }
+    if (dev < 0 || dev >= kMaxDevices) return 0;
+    int answer = known[more][dev].load(std::memory_order_acquire);
+    if (answer == 0) {
+      int cooperative = 0, ctas = 0;
+      const auto kernel = kernel_of<OffsetT>(more);
+      const bool held = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && cooperative &&
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem) == cudaSuccess &&
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kernel, more ? kStepMoreThreads : kStepThreads, kStepSmem) == cudaSuccess && ctas > 0;
+      if (!held) (void)cudaGetLastError();
+      answer = held ? 1 : -1;
+      known[more][dev].store(answer, std::memory_order_release);
+    }
+    return answer > 0;
   }
   template <typename OffsetT>
   static int launch_as(const flexspmv_desc* d, const typename G::Params& p, const StepStages<V>& st, const void* row_offsets, void* ws, cudaStream_t stream) {
     StepShape<G> s;
     if (!s.fit(d, device_sm_count())) return FLEXSPMV_ERR_TOO_LARGE;
-    auto kernel = s.more ? flex_swe_step_kernel<G, OffsetT, kStepMoreThreads> : flex_swe_step_kernel<G, OffsetT, kStepThreads>;
+    const auto kernel = kernel_of<OffsetT>(s.more);
     if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem); e != cudaSuccess) return (int)e;
     StepArgs a;
     a.row_offsets = row_offsets; a.header = static_cast<WorkspaceHeader*>(ws);
@@ -261,7 +288,10 @@ struct StepApi {
     attr[0].id = cudaLaunchAttributeCooperative;        // all CTAs at once: they wait for one another
     attr[0].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, p, st, a);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, st, a);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return (int)e;
+    (void)cudaGetLastError();                 // the context has fewer SMs than the device: nothing was enqueued
+    return FLEXSPMV_ERR_TOO_LARGE;
   }
   static int launch(const flexspmv_desc* d, const void* const* values, const void* const* indices, const void* row_offsets, void* const* outputs,
                     void* ws, size_t ws_bytes, cudaStream_t stream) {

@@ -26,9 +26,11 @@ import ctypes
 
 import torch
 
-from .binding import GraphExtension, check, load_builtin
+from .binding import FlexSpmvError, GraphExtension, check, load_builtin
 from .graphs import swe_delta_graph
 from .python_wrapper.dynamic_replace_submodule import coo_rows_to_csr_ptr
+
+_ERR_TOO_LARGE = -4          # FLEXSPMV_ERR_TOO_LARGE of include/flexspmv.h
 
 
 class ShallowWaterStep:
@@ -127,7 +129,14 @@ class ShallowWaterStep:
         if self._fused is not None:
             if float(self.dt) != self._coef_dt:
                 self._set_coefficients()
-            for launch in [self._step] if self._step is not None else self._fused:
+            if self._step is not None:
+                try:
+                    return self._step.launch()
+                except FlexSpmvError as error:
+                    if error.status != _ERR_TOO_LARGE:
+                        raise
+                    self._step = None            # the context does not hold all of its CTAs at once; nothing was enqueued
+            for launch in self._fused:
                 launch.launch()
             return
         for k, (c, first, last) in enumerate(self._coefficients()):

@@ -360,8 +360,8 @@ FLEXSPMV_DECLARE_GRAPH(edge_copy_i64)
  *   outputs[0..2]                     the state that the second and fourth stage's fluxes are evaluated at (scratch)
  *   outputs[3..5]                     and the third one's
  * on a workspace that was planned with whole rows (FLEXSPMV_ERR_NOT_PLANNED in its status otherwise, nothing written).  Results
- * are those of the four launches, bit for bit.  FLEXSPMV_ERR_TOO_LARGE where the mesh does not fit; swe_delta_rk_T_step_fits
- * says so beforehand (1: it fits).  A wait of the launch's CTAs for one another that takes more than a second raises
+ * are those of the four launches, bit for bit.  FLEXSPMV_ERR_TOO_LARGE, with nothing enqueued, where the mesh does not fit or
+ * the context cannot hold all CTAs at once; swe_delta_rk_T_step_fits says beforehand what the mesh and the device allow (1: it fits).  A wait of the launch's CTAs for one another that takes more than a second raises
  * FLEXSPMV_ERR_TIMEOUT in the workspace status; later launches on the workspace then do nothing until it is planned again.  The
  * state at values[3..5] is undefined after it: a CTA that gave up has not written its cells, another one may have advanced its own.
  */

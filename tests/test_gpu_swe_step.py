@@ -149,3 +149,21 @@ def test_the_time_step_reaches_both_forms(dtype):
         four.forward()
         for k in STATE:
             assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), (dt, k)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_refused_launch_is_four_launches(captured):
+    """A context with fewer SMs than the device refuses the cooperative launch (here: in its place a function that answers so)."""
+    a, b = mesh_of(40, np.float64, True), mesh_of(40, np.float64, True)
+    refused, other = ShallowWaterStep(a, dt=1e-3), ShallowWaterStep(b, dt=1e-3)
+    asked = []
+    refused._step._fn = lambda *args: asked.append(1) or -4
+    if captured:
+        refused.capture()
+    for _ in range(2):
+        refused.replay() if captured else refused.forward()
+        other.forward()
+    assert len(asked) == 1 and refused._step is None
+    refused.check()
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k

@@ -49,3 +49,27 @@ def test_replay_raises_where_an_earlier_step_failed(form):
     with pytest.raises(FlexSpmvError, match="replay.*status -6"):
         step.replay()
     assert step._graph.replays == 1
+
+
+@pytest.mark.parametrize("status,launches", [(-4, 4), (-3, 0), (1, 0)])
+def test_only_a_launch_that_does_not_fit_is_replaced_by_four(status, launches):
+    """FLEXSPMV_ERR_TOO_LARGE of the whole step; other errors are raised."""
+    made = []
+
+    class Refused:
+        def launch(self):
+            raise FlexSpmvError("refused", status)
+
+    class Stage:
+        def launch(self):
+            made.append(1)
+
+    step = bare_step(dt=1.0, _coef_dt=1.0)
+    step._step, step._fused = Refused(), [Stage() for _ in range(4)]
+    if launches:
+        step.forward()
+        assert step._step is None
+    else:
+        with pytest.raises(FlexSpmvError, match="refused"):
+            step.forward()
+    assert len(made) == launches
