@@ -35,11 +35,12 @@ struct StepShape {
   int threads;                        // a cell each, a round
   bool more;
   size_t bytes;
-  // False where a CTA's cells and about as many edges do not fit.
+  // False where a CTA's cells and about as many edges do not fit.  A CTA an SM, or as many as the descriptor caps them at.
   bool fit(const flexspmv_desc* d, long long sms) {
     if (d->num_rows < 1) return false;
+    const long long most = d->max_ctas > 0 && d->max_ctas < sms ? d->max_ctas : sms;
     grid = (d->num_rows + 31) / 32;
-    if (grid > sms) grid = sms;
+    if (grid > most) grid = most;
     share = rows_a_cta(d->num_rows, grid);
     const long long mean = share * d->num_edges / d->num_rows + 1, left = kStepSmem - share * kCellBytes;
     if (mean * kEdgeBytes > left) return false;

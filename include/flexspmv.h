@@ -359,7 +359,10 @@ FLEXSPMV_DECLARE_GRAPH(edge_copy_i64)
  *   values[17]                        a HOST pointer to four times four T: c, w, first, last of every stage
  *   outputs[0..2]                     the state that the second and fourth stage's fluxes are evaluated at (scratch)
  *   outputs[3..5]                     and the third one's
- * on a workspace that was planned with whole rows (FLEXSPMV_ERR_NOT_PLANNED in its status otherwise, nothing written).  Results
+ * on a workspace that was planned with whole rows (FLEXSPMV_ERR_NOT_PLANNED in its status otherwise, nothing written).  It has a
+ * CTA for every SM, or desc->max_ctas of them; they are on the chip together, so the launch waits until other streams' kernels leave
+ * it that room, and with a CTA an SM and more than about 400 threads or half of the shared memory each it shares no SM with a
+ * second such launch.  Results
  * are those of the four launches, bit for bit.  FLEXSPMV_ERR_TOO_LARGE, with nothing enqueued, where the mesh does not fit or
  * the context cannot hold all CTAs at once; swe_delta_rk_T_step_fits says beforehand what the mesh and the device allow (1: it fits).  A wait of the launch's CTAs for one another that takes more than a second raises
  * FLEXSPMV_ERR_TIMEOUT in the workspace status; later launches on the workspace then do nothing until it is planned again.  The

@@ -15,6 +15,10 @@ STEP = 7            # FLEXSPMV_KERNEL_STEP of include/flexspmv.h
 STATE = ("h", "uh", "vh")
 
 
+def sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
 def both(mesh, steps=2, dt=1e-4):
     """The state after some steps in one launch each, and in four; what ran last in the first form."""
     a, b = mesh, {k: v.clone() for k, v in mesh.items()}
@@ -66,7 +70,7 @@ def test_meshes_that_do_not_fit_take_four_launches(n, fits):
     assert (load_library().flexspmv_debug_last_kernel() == STEP) == fits
 
 
-def bind(m, bits):
+def bind(m, bits, max_ctas=0):
     """The step through the operator object with 32- or 64-bit offsets; scratch filled with NaN."""
     nc, ne, V = m["h"].numel(), m["src"].numel(), m["h"].dtype
     ro = torch.searchsorted(m["dst"], torch.arange(nc + 1, dtype=torch.int32, device="cuda")).to(torch.int32 if bits == 32 else torch.int64)
@@ -75,7 +79,7 @@ def bind(m, bits):
     nan = lambda k: [torch.full((nc,), float("nan"), dtype=V, device="cuda") for _ in range(k)]
     coef = torch.tensor([[5e-5, 2e-5, 1, 0], [5e-5, 2e-5, 0, 0], [1e-4, 2e-5, 0, 0], [0, 2e-5, 0, 1]], dtype=V)
     values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], walls, m["bcells"]] + state + nan(3) + [coef]
-    ext = GraphExtension(graphs.swe_delta_graph(), symbol_prefix="swe_delta_rk")
+    ext = GraphExtension(graphs.swe_delta_graph(), symbol_prefix="swe_delta_rk", max_ctas=max_ctas)
     return ext, ext.prepare_step(values, [m["src"], m["dst"]], ro, nan(6), nc, ne, nc)
 
 
@@ -165,5 +169,18 @@ def test_a_refused_launch_is_four_launches(captured):
         other.forward()
     assert len(asked) == 1 and refused._step is None
     refused.check()
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("max_ctas", [1, 5, 33, 1000])
+def test_the_descriptor_caps_the_ctas(max_ctas):
+    a, b = mesh_of(30, np.float64, True), mesh_of(30, np.float64, True)
+    (ext, capped), (_, usual) = bind(a, 32, max_ctas), bind(b, 32)
+    for step in (capped, usual):
+        step.launch()
+    ext.check()
+    arrivals = int(capped._keep[-1][:256].cpu().numpy().view(np.uint64)[24])          # step_barrier of struct WorkspaceHeader
+    assert arrivals == 3 * min(max_ctas, -(-2 * 30 * 30 // 32), sms())
     for k in STATE:
         assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k

@@ -1,8 +1,10 @@
 """Host side of the shallow-water step, without a GPU."""
+import ctypes
+
 import pytest
 
 from flexspmv_b200 import shallow_water
-from flexspmv_b200.binding import FlexSpmvError, PreparedLaunch, load_library
+from flexspmv_b200.binding import Desc, FlexSpmvError, PreparedLaunch, load_library
 
 
 class FakePlan:
@@ -73,3 +75,10 @@ def test_only_a_launch_that_does_not_fit_is_replaced_by_four(status, launches):
         with pytest.raises(FlexSpmvError, match="refused"):
             step.forward()
     assert len(made) == launches
+
+
+@pytest.mark.parametrize("cells,max_ctas,fits", [(40_000, 0, 1), (40_000, 1000, 1), (40_000, 21, 1), (40_000, 19, 0), (1900, 1, 1), (2100, 1, 0)])
+def test_a_cap_on_the_ctas_leaves_each_more_cells(cells, max_ctas, fits):
+    """About 1980 cells of three edges a CTA in fp64."""
+    d = Desc(cells, 3 * cells, cells, 32, 0, max_ctas, 0)
+    assert bool(load_library().flexspmv_swe_delta_rk_f64_step_fits(ctypes.byref(d))) == bool(fits)
