@@ -391,12 +391,14 @@ class GraphExtension:
     def prepare_step(self, values: Sequence[torch.Tensor], indices: Sequence[torch.Tensor], row_end_offsets: torch.Tensor,
                      outputs: Sequence[torch.Tensor], num_rows: int, num_edges: int, num_cols: int = 0) -> "Optional[PreparedLaunch]":
         """``prepare`` for a graph whose unit has a launch over all stages of a step (include/flexspmv.h,
-        swe_delta_rk_T_step); None where the problem does not fit that launch."""
+        swe_delta_rk_T_step); None where the problem does not fit that launch.  ``rows_a_cta`` of the result: the consecutive rows
+        that each of its CTAs takes."""
         syms = self._by_type(values[0].dtype)
         launch = self.prepare(values, indices, row_end_offsets, outputs, num_rows, num_edges, num_cols)
         with torch.cuda.device(values[0].device):
-            if not syms.also("step_fits")(ctypes.byref(launch._desc)):
-                return None
+            launch.rows_a_cta = int(syms.also("step_fits")(ctypes.byref(launch._desc)))
+        if not launch.rows_a_cta:
+            return None
         launch._fn = _LAUNCH((syms.name("step"), self.lib))
         return launch
 

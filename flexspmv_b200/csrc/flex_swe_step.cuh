@@ -36,6 +36,7 @@ struct StepShape {
   bool more;
   size_t bytes;
   // False where a CTA's cells and about as many edges do not fit.  A CTA an SM, or as many as the descriptor caps them at.
+  // (Goes by the mesh's mean; what heavy cells cost: ShallowWaterStep._shares_are_even.)
   bool fit(const flexspmv_desc* d, long long sms) {
     if (d->num_rows < 1) return false;
     const long long most = d->max_ctas > 0 && d->max_ctas < sms ? d->max_ctas : sms;
@@ -244,7 +245,7 @@ struct StepApi {
   static int fits(const flexspmv_desc* d) {
     StepShape<G> s;
     if (Api::check_desc(d) != 0 || !s.fit(d, device_sm_count())) return 0;
-    return d->offset_bits == 64 ? resident<long long>(s.more) : resident<int>(s.more);
+    return (d->offset_bits == 64 ? resident<long long>(s.more) : resident<int>(s.more)) ? (int)s.share : 0;
   }
   template <typename OffsetT>
   static auto kernel_of(bool more) {

@@ -33,6 +33,14 @@ from .python_wrapper.dynamic_replace_submodule import coo_rows_to_csr_ptr
 _ERR_TOO_LARGE = -4          # FLEXSPMV_ERR_TOO_LARGE of include/flexspmv.h
 
 
+def shares_are_even(cells: int, num_cells: int, num_edges: int, most: int, longest: int) -> bool:
+    """No share of ``cells`` consecutive cells with more than half as many edges again as the mean, and no cell with more edges than
+    its share hides (see ``ShallowWaterStep._shares_are_even``)."""
+    if 2 * most * num_cells > 3 * cells * num_edges:
+        return False
+    return cells >= 320 or longest <= -(-num_edges // num_cells) * (1 + cells / 64)
+
+
 class ShallowWaterStep:
     def __init__(self, mesh: Dict[str, torch.Tensor], dt: float = 0.005,
                  delta_ext: Optional[GraphExtension] = None, boundary_ext: Optional[GraphExtension] = None):
@@ -101,10 +109,24 @@ class ShallowWaterStep:
             launches.append(ext.prepare(values, [m["src"], m["dst"]], self.ro, dst, self.nc, self.ne, self.nc))
             if k == 0 and not ext.planned_whole_rows():
                 return None
-        # meshes that fit the chip: the four stages in one launch (csrc/flex_swe_step.cuh)
+        # meshes that fit the chip in even shares: the four stages in one launch (csrc/flex_swe_step.cuh)
         values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [self._coef]
-        self._step = ext.prepare_step(values, [m["src"], m["dst"]], self.ro, self.stage + other, self.nc, self.ne, self.nc)
+        step = ext.prepare_step(values, [m["src"], m["dst"]], self.ro, self.stage + other, self.nc, self.ne, self.nc)
+        if step is not None and self._shares_are_even(step.rows_a_cta):
+            self._step = step
         return launches
+
+    def _shares_are_even(self, cells: int) -> bool:
+        """Whether the whole-step launch is the faster form with ``cells`` consecutive cells a CTA (one look at the row offsets when
+        the model is bound).  Its stages wait for the CTA with the most edges, and a cell's edges are a chain of gathers that takes
+        0.23 us an edge and step of each stage, 0.14 in the four launches; with more cells a CTA there is other work to hide it.
+        us a step, one launch / four, fp64, n x n squares: 330^2 with 1000 cells of 25 edges side by side 457 / 92, 700 of 8 (the
+        largest share 1.8 times the mean) 64 / 60, half of the cells with 6 (1.3) 39 / 53 on 260^2; one cell of 25 on 64^2 (64 a CTA)
+        41 / 37, on 101^2 (160) 37 / 35, on 160^2 (352) 37 / 43; of 12 on 64^2 29 / 25, on 101^2 25 / 29; six cells of 5 on 40^2 (32)
+        25 / 23.  fp32 alike (330^2 174 / 56; one of 25 on 64^2 35 / 29)."""
+        ends = self.ro[torch.arange(0, self.nc + cells, cells, device=self.ro.device).clamp_(max=self.nc)]
+        most, longest = torch.stack([(ends[1:] - ends[:-1]).max(), (self.ro[1:] - self.ro[:-1]).max()]).tolist()
+        return shares_are_even(cells, self.nc, self.ne, most, longest)
 
     def _bind(self, h, uh, vh):
         m = self.m

@@ -364,7 +364,9 @@ FLEXSPMV_DECLARE_GRAPH(edge_copy_i64)
  * it that room, and with a CTA an SM and more than about 400 threads or half of the shared memory each it shares no SM with a
  * second such launch.  Results
  * are those of the four launches, bit for bit.  FLEXSPMV_ERR_TOO_LARGE, with nothing enqueued, where the mesh does not fit or
- * the context cannot hold all CTAs at once; swe_delta_rk_T_step_fits says beforehand what the mesh and the device allow (1: it fits).  A wait of the launch's CTAs for one another that takes more than a second raises
+ * the context cannot hold all CTAs at once; swe_delta_rk_T_step_fits says beforehand what the mesh and the device allow: the number of
+ * consecutive cells that each CTA takes, or 0.  It goes by the mean number of edges; every stage lasts as long as the CTA with the most,
+ * so that four launches are faster where some share has half as many edges again as the mean, or, in small shares, a few rows are long.  A wait of the launch's CTAs for one another that takes more than a second raises
  * FLEXSPMV_ERR_TIMEOUT in the workspace status; later launches on the workspace then do nothing until it is planned again.  The
  * state at values[3..5] is undefined after it: a CTA that gave up has not written its cells, another one may have advanced its own.
  */

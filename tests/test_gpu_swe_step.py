@@ -44,21 +44,46 @@ def test_one_launch_equals_four(n, walls, dtype):
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-def test_edges_that_a_cta_cannot_keep(dtype):
-    """Cells of 25 edges side by side: their CTAs have more edges than shared memory was claimed for, and read the others in place."""
-    m = mesh_of(160, dtype, True)
+def test_edges_that_a_cta_cannot_keep(dtype, monkeypatch):
+    """Cells of 25 edges side by side: their CTAs have more edges than shared memory was claimed for, and read the others in place.
+    (Four launches are faster there, and are what such a mesh takes.)"""
+    m = heavy_cells(mesh_of(160, dtype, True), torch.arange(20_000, 21_000), 22)
+    assert ShallowWaterStep(m, dt=1e-4)._step is None
+    monkeypatch.setattr(ShallowWaterStep, "_shares_are_even", lambda *a: True)
+    a, b, kernel = both(m, dt=1e-4)
+    assert kernel == STEP
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n,cells,extra,even", [(64, 0, 0, True), (64, 1, 3, True), (64, 1, 4, False), (160, 1, 22, True), (330, 50, 22, True), (330, 700, 5, False)])
+def test_cells_that_hold_the_others_up(n, cells, extra, even):
+    """What decides is measured in ``_shares_are_even``; the step has the same bits in either form."""
+    m = mesh_of(n, np.float64, True)
+    if cells:
+        m = heavy_cells(m, torch.arange(n * n, n * n + cells), extra)
+    b = {k: v.clone() for k, v in m.items()}
+    step, four = ShallowWaterStep(m, dt=1e-4), ShallowWaterStep(b, dt=1e-4)
+    assert four._fused is not None and (step._step is not None) == even
+    four._step = None
+    step.forward()
+    assert (load_library().flexspmv_debug_last_kernel() == STEP) == even
+    four.forward()
+    for k in STATE:
+        assert torch.isfinite(m[k]).all() and torch.equal(m[k], b[k]), k
+
+
+def heavy_cells(m, at, extra):
+    """The mesh with ``extra`` more edges into each of the cells ``at``."""
     cells = m["h"].numel()
-    many = torch.arange(20_000, 21_000, dtype=torch.int32, device="cuda").repeat_interleave(22)
+    many = at.to(torch.int32).repeat_interleave(extra).cuda()
     src = torch.randint(0, cells, (many.numel(),), generator=torch.Generator().manual_seed(3)).to(torch.int32).cuda()
     order = torch.argsort(torch.cat([m["dst"], many]).long(), stable=True)
     for k, extra in (("src", src), ("dst", many)):
         m[k] = torch.cat([m[k], extra])[order].contiguous()
     for k, c in (("alpha", 0.5), ("sx", 1e-7), ("sy", -2e-7)):
         m[k] = torch.cat([m[k], torch.full((many.numel(),), c, dtype=m[k].dtype, device="cuda")])[order].contiguous()
-    a, b, kernel = both(m, dt=1e-4)
-    assert kernel == STEP
-    for k in STATE:
-        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+    return m
 
 
 @pytest.mark.parametrize("n,fits", [(380, True), (400, False)])

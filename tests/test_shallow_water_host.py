@@ -82,3 +82,17 @@ def test_a_cap_on_the_ctas_leaves_each_more_cells(cells, max_ctas, fits):
     """About 1980 cells of three edges a CTA in fp64."""
     d = Desc(cells, 3 * cells, cells, 32, 0, max_ctas, 0)
     assert bool(load_library().flexspmv_swe_delta_rk_f64_step_fits(ctypes.byref(d))) == bool(fits)
+
+
+def test_the_cells_of_a_cta():
+    """step_fits: whole warps of cells, over 148 SMs where there is no device to ask."""
+    for cells, max_ctas, share in ((101, 4, 32), (101, 1, 128), (1900, 1, 1920)):
+        d = Desc(cells, 3 * cells, cells, 64, 0, max_ctas, 0)
+        assert load_library().flexspmv_swe_delta_rk_f32_step_fits(ctypes.byref(d)) == share
+
+
+@pytest.mark.parametrize("cells,most,longest,even", [(64, 192, 3, True), (64, 288, 6, True), (64, 289, 6, False), (64, 192, 7, False), (32, 96, 4, True),
+                                                     (32, 96, 5, False), (160, 480, 10, True), (160, 480, 11, False), (320, 960, 32, True), (320, 1441, 4, False)])
+def test_shares_of_cells(cells, most, longest, even):
+    """On a mesh of 9000 cells with three edges each."""
+    assert shallow_water.shares_are_even(cells, 9000, 27000, most, longest) == even
