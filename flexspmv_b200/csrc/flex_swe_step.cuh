@@ -295,6 +295,23 @@ struct StepApi {
     (void)cudaGetLastError();                 // the context has fewer SMs than the device: nothing was enqueued
     return FLEXSPMV_ERR_TOO_LARGE;
   }
+  // What the launch writes lies apart from what other cells read meanwhile: the state that it advances, the two states in between and
+  // the wall terms from one another, and from the state that the first stage gathers what that stage writes.
+  static bool apart(long long cells, const void* const* values, void* const* outputs) {
+    uintptr_t at[3 + 6 + 2];
+    for (int i = 0; i < 6; ++i) at[i] = reinterpret_cast<uintptr_t>(outputs[i]);
+    for (int i = 0; i < 2; ++i) at[6 + i] = reinterpret_cast<uintptr_t>(values[15 + i]);
+    for (int i = 0; i < 3; ++i) at[8 + i] = reinterpret_cast<uintptr_t>(values[11 + i]);
+    const uintptr_t bytes = (uintptr_t)cells * sizeof(V);
+    auto meet = [&](uintptr_t a, uintptr_t b) { return (a > b ? a - b : b - a) < bytes; };
+    for (int i = 0; i < 11; ++i)
+      for (int j = 0; j < i; ++j)
+        if (meet(at[i], at[j])) return false;
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 8; ++j)
+        if ((j < 3 || j >= 6) && meet(reinterpret_cast<uintptr_t>(values[3 + i]), at[j])) return false;
+    return true;
+  }
   static int launch(const flexspmv_desc* d, const void* const* values, const void* const* indices, const void* row_offsets, void* const* outputs,
                     void* ws, size_t ws_bytes, cudaStream_t stream) {
     if (int e = Api::check_desc(d)) return e;
@@ -305,6 +322,7 @@ struct StepApi {
     for (int i = 0; i < G::kNumValues; ++i) if (!values[i]) return FLEXSPMV_ERR_BAD_ARG;
     for (int i = 0; i < G::kNumIndices; ++i) if (!indices[i]) return FLEXSPMV_ERR_BAD_ARG;
     for (int i = 0; i < 6; ++i) if (!outputs[i]) return FLEXSPMV_ERR_BAD_ARG;
+    if (!apart(d->num_rows, values, outputs)) return FLEXSPMV_ERR_BAD_ARG;
     const typename G::Params p = G::make_params(values, indices, outputs);
     if (!G::pointers_aligned(p) || !aligned16(row_offsets)) return FLEXSPMV_ERR_ALIGN;
     StepStages<V> st;

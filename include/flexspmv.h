@@ -354,21 +354,26 @@ FLEXSPMV_DECLARE_GRAPH(edge_copy_i64)
 /*
  * swe_delta_rk_T_step: the four stages of a step in one cooperative launch, for meshes whose edges' records and cells' sums fit
  * the shared memory of all SMs.  The arrays of the first stage's launch, with
- *   values[3..5] and values[11..13]   the state at the beginning of the step, advanced in place
+ *   values[3..5]                      the state that the first stage's fluxes are evaluated at
+ *   values[11..13]                    the state at the beginning of the step (as a rule the same arrays), advanced in place
  *   values[14..16]                    scratch
  *   values[17]                        a HOST pointer to four times four T: c, w, first, last of every stage
  *   outputs[0..2]                     the state that the second and fourth stage's fluxes are evaluated at (scratch)
  *   outputs[3..5]                     and the third one's
- * on a workspace that was planned with whole rows (FLEXSPMV_ERR_NOT_PLANNED in its status otherwise, nothing written).  It has a
- * CTA for every SM, or desc->max_ctas of them; they are on the chip together, so the launch waits until other streams' kernels leave
- * it that room, and with a CTA an SM and more than about 400 threads or half of the shared memory each it shares no SM with a
- * second such launch.  Results
- * are those of the four launches, bit for bit.  FLEXSPMV_ERR_TOO_LARGE, with nothing enqueued, where the mesh does not fit or
- * the context cannot hold all CTAs at once; swe_delta_rk_T_step_fits says beforehand what the mesh and the device allow: the number of
- * consecutive cells that each CTA takes, or 0.  It goes by the mean number of edges; every stage lasts as long as the CTA with the most,
- * so that four launches are faster where some share has half as many edges again as the mean, or, in small shares, a few rows are long.  A wait of the launch's CTAs for one another that takes more than a second raises
- * FLEXSPMV_ERR_TIMEOUT in the workspace status; later launches on the workspace then do nothing until it is planned again.  The
- * state at values[3..5] is undefined after it: a CTA that gave up has not written its cells, another one may have advanced its own.
+ * on a workspace that was planned with whole rows (FLEXSPMV_ERR_NOT_PLANNED in its status otherwise, nothing written).  Results are
+ * those of the four launches, bit for bit.  values[11..13], values[15..16] and the outputs must not overlap one another, nor
+ * values[3..5] the outputs[0..2] or values[15..16] (FLEXSPMV_ERR_BAD_ARG).
+ *
+ * The launch has a CTA for every SM, or desc->max_ctas of them.  They are on the chip together, so it waits until other streams'
+ * kernels leave it that room, and shares no SM with a second such launch where its CTAs have more than 400 threads or half of the
+ * shared memory.  FLEXSPMV_ERR_TOO_LARGE, with nothing enqueued, where the mesh does not fit or the context cannot hold all CTAs at once;
+ * swe_delta_rk_T_step_fits says beforehand what the mesh and the device allow: the number of consecutive cells that each CTA takes,
+ * or 0.  It goes by the mean number of edges; every stage lasts as long as the CTA with the most, so that four launches are faster where
+ * some share has half as many edges again as the mean, or, in small shares, a few rows are long.
+ *
+ * A wait of the CTAs for one another that takes more than a second raises FLEXSPMV_ERR_TIMEOUT in the workspace status; later launches
+ * on the workspace then do nothing until it is planned again.  The state at values[11..13] is undefined after it: a CTA that gave up
+ * has not written its cells, another one may have advanced its own.
  */
 #define FLEXSPMV_DECLARE_EPILOGUE_GRAPH(G)                                                                                  \
   FLEXSPMV_DECLARE_GRAPH(G)                                                                                                 \

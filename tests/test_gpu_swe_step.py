@@ -209,3 +209,30 @@ def test_the_descriptor_caps_the_ctas(max_ctas):
     assert arrivals == 3 * min(max_ctas, -(-2 * 30 * 30 // 32), sms())
     for k in STATE:
         assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_a_first_state_of_its_own(dtype):
+    """The first stage's fluxes may be evaluated at other arrays than the ones that are advanced, as in four launches."""
+    results = []
+    for whole in (True, False):
+        m = mesh_of(50, dtype, True)
+        x = [m[k] + 0.01 * (i + 1) for i, k in enumerate(STATE)]
+        m["h"], first = m["h"].clone(), [m[k] * 1.01 for k in STATE]
+        nc, ne, V = m["h"].numel(), m["src"].numel(), m["h"].dtype
+        ro = torch.searchsorted(m["dst"], torch.arange(nc + 1, dtype=torch.int32, device="cuda")).to(torch.int32)
+        walls = torch.searchsorted(m["bcells"], torch.arange(0, nc + 32, 32, dtype=torch.int32, device="cuda")).to(torch.int32)
+        stage, other, acc = ([torch.zeros(nc, dtype=V, device="cuda") for _ in range(3)] for _ in range(3))
+        coef = torch.tensor([[5e-5, 2e-5, 1, 0], [5e-5, 2e-5, 0, 0], [1e-4, 2e-5, 0, 0], [0, 2e-5, 0, 1]], dtype=V)
+        ext = GraphExtension(graphs.swe_delta_graph(), symbol_prefix="swe_delta_rk")
+        values = lambda src, c: [m["alpha"], m["sx"], m["sy"]] + src + [m["area"], m["bsx"], m["bsy"], walls, m["bcells"]] + x + acc + [c]
+        if whole:
+            ext.prepare_step(values(first, coef), [m["src"], m["dst"]], ro, stage + other, nc, ne, nc).launch()
+        else:
+            for k in range(4):
+                src, dst = first if k == 0 else (stage if k % 2 else other), other if k % 2 else stage
+                ext.prepare(values(src, coef[k]), [m["src"], m["dst"]], ro, dst, nc, ne, nc).launch()
+        ext.check()
+        results.append(x)
+    for a, b in zip(*results):
+        assert torch.isfinite(a).all() and torch.equal(a, b)

@@ -96,3 +96,33 @@ def test_the_cells_of_a_cta():
 def test_shares_of_cells(cells, most, longest, even):
     """On a mesh of 9000 cells with three edges each."""
     assert shallow_water.shares_are_even(cells, 9000, 27000, most, longest) == even
+
+
+@pytest.mark.parametrize("dtype,size", [("f32", 4), ("f64", 8)])
+def test_the_whole_step_refuses_arrays_that_overlap(dtype, size):
+    """Checked before anything is enqueued, so that addresses which nothing reads will do.  -2: the arrays pass, the row offsets' address
+    does not."""
+    lib, cells = load_library(), 1000
+    d = Desc(cells, 3 * cells, cells, 32, 0, 0, 0)
+    need = ctypes.c_size_t()
+    assert getattr(lib, f"flexspmv_swe_delta_rk_{dtype}_workspace_bytes")(ctypes.byref(d), ctypes.byref(need)) == 0
+    step = getattr(lib, f"flexspmv_swe_delta_rk_{dtype}_step")
+    far, coef = 1 << 20, (ctypes.c_double * 16)()
+
+    def call(**places):
+        at = {f"v{i}": far * (1 + i) for i in range(18)}
+        at.update({f"o{i}": far * (31 + i) for i in range(6)}, v11=far * 4, v12=far * 5, v13=far * 6, v17=ctypes.addressof(coef))
+        at.update(places)
+        values = (ctypes.c_void_p * 18)(*[at[f"v{i}"] for i in range(18)])
+        outputs = (ctypes.c_void_p * 6)(*[at[f"o{i}"] for i in range(6)])
+        indices = (ctypes.c_void_p * 2)(far * 40, far * 41)
+        return step(ctypes.byref(d), values, indices, ctypes.c_void_p(8), outputs, ctypes.c_void_p(far), need, None)
+
+    last = (cells - 1) * size
+    assert call() == -2
+    for accepted in ({"v11": far * 50, "v12": far * 51, "v13": far * 52}, {"v14": far * 31}, {"o0": far * 20, "o1": far * 20 + cells * size},
+                     {"v11": far * 50, "v12": far * 51, "v13": far * 52, "o3": far * 4}):
+        assert call(**accepted) == -2
+    for refused in ({"o0": far * 4}, {"o5": far * 5}, {"o1": far * 4 + last}, {"o3": far * 31}, {"o2": far * 16}, {"v15": far * 17}, {"v16": far * 6 + last},
+                    {"v12": far * 4}, {"v11": far * 50, "v12": far * 51, "v13": far * 52, "o0": far * 4}):
+        assert call(**refused) == -1, refused
