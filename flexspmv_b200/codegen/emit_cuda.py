@@ -173,32 +173,42 @@ TUNED_CONFIGS = {
 
 
 # Other configurations for large launches (GraphApi::use_big; consumer threads, merge items per thread, stages, CTAs per SM[, edges a
-# batch in the loop over whole rows]).  Row-mode graphs: one large CTA an SM on short rows.  A tile of 4 items a thread is a row of three edges a thread, less one item each.  us on meshes of 1024^2
-# squares, CTAs an SM x warps: the shallow-water step 3 x 9 368, 1 x 24 332 (tiles of 3 items a thread 367, of 5 370), 1 x 28 367, 2 x 12
-# 363, 1 x 20 363; Rusanov fp64 3 x 9 76.3, 1 x 24 74.0, 1 x 28 77.0, 2 x 12 76.2; fp32 4 x 9 48.9, 1 x 32 45.8, 1 x 28 48.0, 1 x 24 52.0.
-TUNED_BIG_CONFIGS = {
-    "rusanov_f64": (736, 4, 2, 1),
-    "rusanov_f32": (992, 4, 2, 1),
-    "swe_delta_f64": (736, 4, 2, 1),
-    # lattices of eight edges a particle, 1024^2: fp32 992 x 8 35.9 (x 9 36.2), fp64 736 x 7 62.0 (x 8 63.8, x 9 62.1)
-    "spring_mass_f32": (992, 8, 2, 1),
-    "spring_mass_f64": (736, 7, 2, 1),
+# batch in the loop over whole rows]).  Row-mode graphs: one large CTA an SM on short rows.  They are picked by what a graph moves and
+# computes, whatever its name: (widths of the edge tensors, of the records gathered by edge, of those gathered by row, sums a row), and as
+# measured with (map operations an edge, by component; divisions, pow, exp and norm among them; value bytes).  A tile of 4 items a thread is
+# a row of three edges a thread, less one item each.  us on meshes of 1024^2 squares, CTAs an SM x warps: the shallow-water step 3 x 9 368,
+# 1 x 24 332 (tiles of 3 items a thread 367, of 5 370), 1 x 28 367, 2 x 12 363, 1 x 20 363; Rusanov fp64 3 x 9 76.3, 1 x 24 74.0, 1 x 28 77.0,
+# 2 x 12 76.2; fp32 4 x 9 48.9, 1 x 32 45.8, 1 x 28 48.0, 1 x 24 52.0.  Lattices of eight edges a particle, 1024^2: fp32 992 x 8 35.9 (x 9
+# 36.2), fp64 736 x 7 62.0 (x 8 63.8, x 9 62.1).
+ROW_BIG_CONFIGS = {
+    ((3,), (3,), (3,), 3): (64, 4, {4: (992, 4, 2, 1), 8: (736, 4, 2, 1)}),                  # a finite-volume flux: Rusanov
+    ((1, 1, 1), (1, 1, 1), (1, 1, 1), 3): (29, 2, {8: (736, 4, 2, 1)}),                      # the shallow-water model's delta
+    ((1, 1), (2,), (2,), 2): (9, 3, {4: (992, 8, 2, 1), 8: (736, 7, 2, 1)}),                 # a force along an edge: spring-mass
 }
+MAX_SMEM = 227 * 1024
 
 
 def big_config(ir: GraphIR, dtype: str):
-    """The configuration for large launches: as measured for a graph, or that of longer rows for any graph of SpMV's shape (one value and
-    one gathered value an edge, one sum a row, a light map).  27 columns, 1 M rows, batches of 8 / 9 / 10 / 12: fp32 41.7 / 39.8 / 40.5 / 42.9 us
-    (480 threads x 7, 3 stages, batch 4 39.8; the usual configuration 49.9), fp64 62.0 / 60.3 / 60.7 / 82.1 (992 x 5 x 1, batch 4 66.6; 65.4)."""
-    named = TUNED_BIG_CONFIGS.get(f"{ir.name}_{CTYPE[dtype][1]}")
-    if named or dtype == "int64" or not ir.has_reducer or not light_map(ir) or stores_per_edge(ir):
-        return named
-    gathered = [s_ for s_ in ir.selector_register if s_.get("selector") == 1]
-    edge = {s_["target"]: dim_of(s_["shape"]) for s_ in ir.selector_register if s_.get("selector") != 1}
-    sums = sum(dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer")
-    if any(s_.get("row_identity") for s_ in gathered) or [dim_of(s_["shape"]) for s_ in gathered] != [1] or list(edge.values()) != [1] or sums != 1:
+    """The configuration for large launches, or None: of a row-mode graph as in ``ROW_BIG_CONFIGS``, where no more is computed and the
+    tile's stages have room (``smem_bytes``); that of longer rows for any graph of SpMV's shape (one value and one gathered value an edge, one
+    sum a row, a light map).  27 columns, 1 M rows, batches of 8 / 9 / 10 / 12: fp32 41.7 / 39.8 / 40.5 / 42.9 us (480 threads x 7, 3 stages,
+    batch 4 39.8; the usual configuration 49.9), fp64 62.0 / 60.3 / 60.7 / 82.1 (992 x 5 x 1, batch 4 66.6; 65.4)."""
+    if dtype == "int64" or not ir.has_reducer or stores_per_edge(ir):
         return None
-    return (352, 10, 2, 2, 9) if VBYTES[dtype] == 4 else (352, 8, 2, 2, 9)
+    gathers = {(s_["selector_name"], s_["target"]): s_ for s_ in ir.selector_register if s_.get("selector") == 1}.values()
+    edge = {s_["target"]: dim_of(s_["shape"]) for s_ in ir.selector_register if s_.get("selector") != 1}
+    widths = lambda row: tuple(sorted(dim_of(s_["shape"]) for s_ in gathers if bool(s_.get("row_identity")) == row))
+    sums = sum(dim_of(o["shape"]) for o in ir.outputs if str(o["target"]) == "reducer")
+    shape = (tuple(sorted(edge.values())), widths(False), widths(True), sums)
+    if shape == ((1,), (1,), (), 1) and light_map(ir):
+        return (352, 10, 2, 2, 9) if VBYTES[dtype] == 4 else (352, 8, 2, 2, 9)
+    most, most_heavy, configs = ROW_BIG_CONFIGS.get(shape, (0, 0, {}))
+    config = configs.get(VBYTES[dtype])
+    width = lambda ops: sum(dim_of(op_["shape"]) for op_ in ir.map_operations if ops(op_["op"]))
+    if config is None or width(lambda op: op != "reducer") > most or width(lambda op: op in ("truediv", "pow", "exp", "norm")) > most_heavy or \
+            smem_bytes(ir, dtype, *config[:3]) > MAX_SMEM:
+        return None
+    return config
 
 
 # Configuration of the warp kernel for matrices whose gathers have no locality (csrc/flex_warp_kernel.cuh):

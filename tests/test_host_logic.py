@@ -1,9 +1,12 @@
 """Host-side logic that needs no GPU: IR -> operator signature, the CUDA emitter, tile configuration,
 problem generators and the algorithmic-bytes figures of the benchmark configurations."""
+import os
+
 import numpy as np
 import pytest
 
 from flexspmv_b200 import graphs, problems
+from flexspmv_b200.build import NVCC, NVCC_FLAGS
 from flexspmv_b200.codegen import emit_cuda
 
 
@@ -188,3 +191,51 @@ def test_the_package_imports_without_torchs_cuda_internals():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
     assert r.returncode == 0 and "not found" in r.stdout, r.stderr
+
+
+def _wider(name):
+    """A graph under a built-in one's name whose records are wider."""
+    import copy
+    ir = copy.deepcopy(graphs.ALL_GRAPHS[name]())
+    if name == "rusanov":                # eight values a face, of which the map takes three
+        for s_ in ir.inputs + ir.selector_register:
+            if "face" in (s_["name"], s_.get("selector_name")):
+                s_["shape"] = (8,)
+        return ir
+    width = (1,) if name == "spring_mass" else (2,)
+    ir.inputs.insert(0, graphs.placeholder("c", width))
+    ir.selector_register.insert(0, graphs.edge_register("c", width))
+    last = next(op_ for op_ in ir.map_operations if op_["op"] == "mul")
+    if name == "spring_mass":
+        last["args"] = ["c" if a == "k" else a for a in last["args"]]
+    return ir
+
+
+@pytest.mark.parametrize("name,dtypes", [("spring_mass", ("float32", "float64")), ("swe_delta", ("float64",)), ("rusanov", ("float32", "float64"))])
+def test_large_tiles_go_by_what_a_graph_moves(name, dtypes):
+    """A graph takes the configuration for large launches by its records and operations: another one under the same name does not, the
+    same one under another name does."""
+    import copy
+    for dt in dtypes:
+        assert "CfgBig" in emit_cuda.emit_graph(graphs.ALL_GRAPHS[name](), dt, "it")
+        other = copy.deepcopy(graphs.ALL_GRAPHS[name]())
+        other.name = "traced"
+        config = emit_cuda.big_config(other, dt)
+        assert config == emit_cuda.big_config(graphs.ALL_GRAPHS[name](), dt) and emit_cuda.smem_bytes(other, dt, *config[:3]) <= emit_cuda.MAX_SMEM
+        wider = _wider(name)
+        assert emit_cuda.smem_bytes(wider, dt, *config[:3]) > emit_cuda.MAX_SMEM
+        assert emit_cuda.big_config(wider, dt) is None
+        longer = copy.deepcopy(other)       # more work an edge than was measured
+        longer.map_operations.insert(-1, dict(longer.map_operations[0], name="more"))
+        assert emit_cuda.big_config(longer, dt) is None
+    assert emit_cuda.big_config(graphs.ALL_GRAPHS[name](), "int64") is None
+
+
+@pytest.mark.skipif(not os.path.exists(NVCC), reason="needs nvcc")
+@pytest.mark.parametrize("name,dt", [("spring_mass", "float32"), ("spring_mass", "float64"), ("swe_delta", "float64"), ("rusanov", "float64")])
+def test_wider_records_under_a_built_in_name_compile(name, dt, tmp_path):
+    import subprocess
+    src = tmp_path / "unit.cu"
+    src.write_text(emit_cuda.emit_graph(_wider(name), dt, "wider", windows=False))
+    run = subprocess.run([NVCC] + NVCC_FLAGS + ["-cuda", str(src), "-o", str(tmp_path / "unit.ii")], capture_output=True, text=True)
+    assert run.returncode == 0, run.stderr[-2000:]
