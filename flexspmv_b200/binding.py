@@ -142,7 +142,7 @@ class _Symbols:
             f.restype = ctypes.c_int
             return f
         self.info, self.workspace_bytes, self.plan = fn("info"), fn("workspace_bytes"), fn("plan_indexed")
-        self.plan_windows = fn("plan_windows")
+        self.plan_windows, self.uses_longest_row = fn("plan_windows"), fn("uses_longest_row")
         fn("launch")
         self.launch, self.device_status = _LAUNCH((f"flexspmv_{sym}_launch", lib)), fn("device_status")
         gi = GraphInfo()
@@ -159,8 +159,12 @@ class GraphExtension:
 
     def __init__(self, ir: GraphIR, lib_path: Optional[str] = None, symbol_prefix: Optional[str] = None,
                  tile_items: int = 0, max_ctas: int = 0, gather_windows: Optional[bool] = None,
-                 random_gather: Optional[bool] = None):
-        """``random_gather``: run the kernel for matrices whose columns have no locality (include/flexspmv.h,
+                 random_gather: Optional[bool] = None, longest_row: Optional[int] = None):
+        """``longest_row``: the edges of the longest row where the caller knows that all tiles hold whole rows (include/flexspmv.h,
+        FLEXSPMV_LONGEST_ROW), 0 = unknown.  None = asked of the plan where launches of the size go by it (one device-to-host read,
+        at plan time only; not while the stream is captured).
+
+        ``random_gather``: run the kernel for matrices whose columns have no locality (include/flexspmv.h,
         FLEXSPMV_FLAG_RANDOM_GATHER), for graphs built with it.  None = decide per matrix the first time it is
         planned, from a sample of its index array (one device-to-host read, at plan time only): the flag is set
         when 32 consecutive edges gather from more than 16 different cache lines on average.  The environment
@@ -181,6 +185,7 @@ class GraphExtension:
         if random_gather is None and os.environ.get("FLEXSPMV_RANDOM_GATHER") in ("0", "1"):
             random_gather = os.environ["FLEXSPMV_RANDOM_GATHER"] == "1"
         self.random_gather = random_gather
+        self.longest_row = longest_row
         self._locality: Dict[tuple, bool] = {}
         edge_sel = [s_ for s_ in ir.selector_register if s_.get("selector") == 1 and not s_.get("row_identity")]
         self._gather_dim = dim_of(edge_sel[0]["shape"]) if edge_sel else 1
@@ -274,12 +279,38 @@ class GraphExtension:
             self._plans.move_to_end(key)
             if plan.desc.num_vertices == num_cols:
                 return plan, plan.desc
-            return plan, Desc(num_rows, num_edges, num_cols, bits, self.tile_items, self.max_ctas, flags)
-        desc = Desc(num_rows, num_edges, num_cols, bits, self.tile_items, self.max_ctas, flags)
-        return self._make_plan(key, syms, desc, ro, device, indices), desc
+            return plan, Desc(num_rows, num_edges, num_cols, bits, self.tile_items, self.max_ctas, plan.desc.reserved)
+        described = lambda longest: Desc(num_rows, num_edges, num_cols, bits, self.tile_items, self.max_ctas, flags | longest << 8)
+        plan = self._make_plan(syms, described, ro, device, indices)
+        self._plans[key] = plan
+        while len(self._plans) > self.PLAN_CACHE_ENTRIES:
+            self._plans.popitem(last=False)
+        return plan, plan.desc
 
-    def _make_plan(self, key, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device,
-                   indices: Sequence[torch.Tensor] = ()) -> "_Plan":
+    def _make_plan(self, syms: _Symbols, described, ro: Optional[torch.Tensor], device, indices: Sequence[torch.Tensor] = ()) -> "_Plan":
+        """A plan for ``described(longest)``, the descriptor that names the longest row.  Where its tiles go by that, they are those of
+        whole rows until the plan says that it has none."""
+        if self.longest_row is not None:
+            return self._plan_once(syms, described(int(self.longest_row)), ro, device, indices)
+        unknown = described(0)
+        by_row = syms.uses_longest_row(ctypes.byref(unknown))
+        if not by_row or torch.cuda.is_current_stream_capturing():
+            return self._plan_once(syms, unknown, ro, device, indices)
+        plan = self._plan_once(syms, described(32), ro, device, indices)
+        longest = self._longest_row(plan)
+        if longest == 0:
+            return self._plan_once(syms, unknown, ro, device, indices)
+        plan.desc = described(longest)
+        return plan
+
+    def _longest_row(self, plan: "_Plan") -> int:
+        out = torch.empty(1, dtype=torch.int32, device=plan.ws.device)
+        self.lib.flexspmv_workspace_longest_row.restype = ctypes.c_int
+        check(self.lib, self.lib.flexspmv_workspace_longest_row(ctypes.c_void_p(plan.ws_ptr), ctypes.c_void_p(out.data_ptr()), _stream_ptr()),
+              "workspace_longest_row")
+        return int(out.item())
+
+    def _plan_once(self, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device, indices: Sequence[torch.Tensor]) -> "_Plan":
         nbytes = ctypes.c_size_t()
         check(self.lib, syms.workspace_bytes(ctypes.byref(desc), ctypes.byref(nbytes)), "workspace_bytes")
         ws = torch.empty(nbytes.value, dtype=torch.uint8, device=device)
@@ -297,9 +328,6 @@ class GraphExtension:
                                                                   ctypes.c_void_p(plan.flag.data_ptr()), _stream_ptr()),
               "workspace_status_mirror")
         self.launches += self.lib.flexspmv_plan_launches() - before
-        self._plans[key] = plan
-        while len(self._plans) > self.PLAN_CACHE_ENTRIES:
-            self._plans.popitem(last=False)
         return plan
 
     # -- the operator --------------------------------------------------------------------------------

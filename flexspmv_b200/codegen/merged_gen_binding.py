@@ -79,6 +79,7 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w("struct PlanEntry {")
     w("  const void* ro_ptr; uint32_t ro_version; int64_t num_rows, ne; int offset_bits, device; cudaStream_t stream; int type_tag;")
     w("  torch::Tensor ws, ro_keep;")
+    w("  int32_t reserved;                   // of the descriptor that the workspace was planned for")
     w("};")
     w("std::mutex g_mu;")
     w("std::list<PlanEntry> g_plans;          // most recently used first")
@@ -88,15 +89,18 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w("  int (*workspace_bytes)(const flexspmv_desc*, size_t*);")
     w("  int (*plan)(const flexspmv_desc*, const void* const*, const void*, void*, size_t, void*);")
     w("  int (*launch)(const flexspmv_desc*, const void* const*, const void* const*, const void*, void* const*, void*, size_t, void*);")
+    w("  int (*uses_longest_row)(const flexspmv_desc*);")
     w("  int (*device_status)(const void*, int32_t*, void*);")
     w("  int type_tag;")
     w("};")
     for i, dt in enumerate(dtypes):
         s = f"{symbol}_{CTYPE[dt][1]}"
         w(f"const Entry kEntry_{CTYPE[dt][1]} = {{flexspmv_{s}_workspace_bytes, flexspmv_{s}_plan_indexed, flexspmv_{s}_launch, "
-          f"flexspmv_{s}_device_status, {i}}};")
+          f"flexspmv_{s}_uses_longest_row, flexspmv_{s}_device_status, {i}}};")
     w("")
-    w("torch::Tensor planned_workspace(const Entry& e, const flexspmv_desc& d, const void* const* indices, const torch::Tensor& ro,")
+    w("// A planned workspace; `d.reserved` becomes that of the descriptor it was planned for.  Where the tiles go by the longest row they")
+    w("// are those of whole rows, unless the plan says that it has none (one read back at plan time, not while the stream is captured).")
+    w("torch::Tensor planned_workspace(const Entry& e, flexspmv_desc& d, const void* const* indices, const torch::Tensor& ro,")
     w("                                bool has_rows, const torch::Tensor& like, cudaStream_t stream) {")
     w("  const void* ro_ptr = has_rows ? ro.data_ptr() : nullptr;")
     w("  const uint32_t ver = has_rows ? ro._version() : 0u;")
@@ -106,17 +110,35 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w("    if (it->ro_ptr == ro_ptr && it->ro_version == ver && it->num_rows == d.num_rows && it->ne == d.num_edges &&")
     w("        it->offset_bits == d.offset_bits && it->device == device && it->stream == stream && it->type_tag == e.type_tag) {")
     w("      g_plans.splice(g_plans.begin(), g_plans, it);")
+    w("      d.reserved = g_plans.front().reserved;")
     w("      return g_plans.front().ws;")
     w("    }")
     w("  }")
-    w("  size_t bytes = 0;")
-    w("  int st = e.workspace_bytes(&d, &bytes);")
-    w('  TORCH_CHECK(st == 0, "merged_spmv_launch (workspace size) failed: ", flexspmv_error_string(st));')
-    w("  torch::Tensor ws = torch::empty({(int64_t)bytes}, torch::TensorOptions().dtype(torch::kUInt8).device(like.device()));")
-    w("  st = e.plan(&d, indices, ro_ptr, ws.data_ptr(), bytes, stream);")
-    w('  TORCH_CHECK(st == 0, "merged_spmv_launch (plan) failed: ", flexspmv_error_string(st));')
+    w("  torch::Tensor ws;")
+    w("  auto plan = [&] {")
+    w("    size_t bytes = 0;")
+    w("    int st = e.workspace_bytes(&d, &bytes);")
+    w('    TORCH_CHECK(st == 0, "merged_spmv_launch (workspace size) failed: ", flexspmv_error_string(st));')
+    w("    ws = torch::empty({(int64_t)bytes}, torch::TensorOptions().dtype(torch::kUInt8).device(like.device()));")
+    w("    st = e.plan(&d, indices, ro_ptr, ws.data_ptr(), bytes, stream);")
+    w('    TORCH_CHECK(st == 0, "merged_spmv_launch (plan) failed: ", flexspmv_error_string(st));')
+    w("  };")
+    w("  const int32_t unknown = d.reserved;")
+    w("  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;")
+    w("  if (has_rows && e.uses_longest_row(&d) && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {")
+    w("    d.reserved = unknown | FLEXSPMV_LONGEST_ROW(32);")
+    w("    plan();")
+    w("    torch::Tensor out = torch::empty({1}, torch::TensorOptions().dtype(torch::kInt).device(like.device()));")
+    w("    const int st = flexspmv_workspace_longest_row(ws.data_ptr(), out.data_ptr<int32_t>(), stream);")
+    w('    TORCH_CHECK(st == 0, "merged_spmv_launch (longest row) failed: ", flexspmv_error_string(st));')
+    w("    const int longest = out.item<int32_t>();")
+    w("    d.reserved = longest ? unknown | FLEXSPMV_LONGEST_ROW(longest) : unknown;")
+    w("    if (!longest) plan();")
+    w("  } else {")
+    w("    plan();")
+    w("  }")
     w("  g_plans.push_front(PlanEntry{ro_ptr, ver, d.num_rows, d.num_edges, d.offset_bits, device, stream, e.type_tag, ws,")
-    w("                               has_rows ? ro : torch::Tensor()});")
+    w("                               has_rows ? ro : torch::Tensor(), d.reserved});")
     w("  while (g_plans.size() > kMaxPlans) g_plans.pop_back();")
     w("  return ws;")
     w("}")

@@ -57,9 +57,11 @@ struct WorkspaceHeader {
   uint32_t line_edges, line_edge_lines;     // cache lines their middle edges gather from; consecutive edges and their lines
   int32_t uneven_shares;       // 1: with equal shares of the rows a CTA of the plan's grid would have more than RowLoopRule allows; 2 is added
                                // while a test withholds a stage (not 0: a small launch runs its loop with stages)
-  int32_t unused;
+  int32_t longest_row;         // where whole_rows is 1 and the rows suit the plan's tiles (RowLoopRule): the edges of the longest one (else 0
+                               // once the plan is complete)
   uint64_t step_barrier;       // CTAs that have come to a barrier of a whole-step launch (flex_swe_step.cuh), over all launches
-  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4 - 4 - 8];
+  uint64_t lane_slots;         // row_slots without the lanes that have no row
+  char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4 - 4 - 8 - 8];
 };
 static_assert(sizeof(WorkspaceHeader) == 256, "header is one 256-byte block");
 constexpr uint32_t kMagic = 0x464c5831u;  // "FLX1"
@@ -86,6 +88,9 @@ struct RowLoopRule {
   // does not come into question for the matrix).
   long long share_items;             // rows and edges
   int share_row_edges;               // edges a row
+  // Large tiles of row-mode graphs (GraphApi::use_big): the longest row, and steps of lanes with a row for 100 edges, that suit them (0: any).
+  long long most_row;
+  int most_slots;
 };
 
 // What one tile of the tile kernel can take when a planning step moves its boundaries (in whole numbers of edges and

@@ -120,16 +120,18 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
                                                          long long num_tiles, const TileRoom room, const RowLoopRule rule,
                                                          const OffsetT* __restrict__ coords, WorkspaceHeader* h) {
   constexpr int kAhead = 4;                 // loads in flight
-  __shared__ unsigned long long s_slots;
+  __shared__ unsigned long long s_slots, s_lane_slots;
   __shared__ unsigned s_seen[6];            // the header's bank_groups .. line_edge_lines
-  if (threadIdx.x == 0) s_slots = 0;
+  __shared__ int s_most;
+  if (threadIdx.x == 0) { s_slots = s_lane_slots = 0; s_most = 0; }
   if (threadIdx.x < 6) s_seen[threadIdx.x] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   const long long step = num_tiles / 1024 + 1;                              // tiles whose first 32 rows are looked at closely
-  unsigned long long slots = 0;
+  unsigned long long slots = 0, lane_slots = 0;
   unsigned seen[6] = {0, 0, 0, 0, 0, 0};
+  int most = 0;                             // edges of the longest row
   bool bad = false;
   long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   OffsetT next[4] = {0, 0, 0, 0};           // coordinates are requested a tile ahead
@@ -172,7 +174,9 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
         const int counted = !in ? 0 : (inside && (unsigned)len <= (unsigned)kWholeRowMax ? len : kWholeRowMax + 1);
         const int longest = __reduce_max_sync(0xffffffffu, counted);
         bad |= longest > kWholeRowMax;
+        most = most > longest ? most : longest;
         slots += 32u * (unsigned)longest;
+        lane_slots += (unsigned)(rows - r0 - 32 * j < 32 ? rows - r0 - 32 * j : 32) * (unsigned)longest;
         if (j == 0 && r0 == 0 && t % step == 0 && !bad) {
           const int bank = (int)(y0 + from) & 31;
           const bool row = counted > 0, edge = lane < edges;
@@ -205,14 +209,18 @@ __global__ void __launch_bounds__(256) whole_rows_kernel(const OffsetT* __restri
   }
   if (lane == 0) {
     if (bad) h->whole_rows = -1;
-    if (!bad && slots) atomicAdd(&s_slots, slots);
+    if (!bad && slots) { atomicAdd(&s_slots, slots); atomicAdd(&s_lane_slots, lane_slots); atomicMax(&s_most, most); }
     if (!bad && seen[0]) {
 #pragma unroll
       for (int i = 0; i < 6; ++i) atomicAdd(&s_seen[i], seen[i]);
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && s_slots) atomicAdd(reinterpret_cast<unsigned long long*>(&h->row_slots), s_slots);
+  if (threadIdx.x == 0 && s_slots) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(&h->row_slots), s_slots);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&h->lane_slots), s_lane_slots);
+    atomicMax(&h->longest_row, s_most);
+  }
   if (threadIdx.x < 6 && s_seen[threadIdx.x]) atomicAdd(&h->bank_groups + threadIdx.x, s_seen[threadIdx.x]);
 }
 // Moves the boundaries when the kernel above found nothing against it and at least two fifths of the thread-steps have
@@ -246,6 +254,7 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* ro
                                                                OffsetT* coords, WorkspaceHeader* h) {
   // whole_rows is read by this kernel only as "-1 or not"
   if (*reinterpret_cast<volatile int32_t*>(&h->whole_rows) == -1 || 2 * (unsigned long long)h->row_slots > 5 * (unsigned long long)num_edges) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) h->longest_row = 0;      // (counted up to the refusal)
     if (blockIdx.x == 0) snap_cta_boundaries(row_offsets, num_rows, num_tiles, grid, room, coords, h);
     return;
   }
@@ -267,6 +276,9 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* ro
     const long long lines_more = 32ll * h->line_row_lines * h->line_edges - 32ll * h->line_edge_lines * h->line_rows;   // x rows x edges
     const bool edges_share_lines = lines_more * rule.gathers > 22ll * rule.accumulators * h->line_rows * h->line_edges;
     const bool lanes_idle = num_edges > 7 * num_rows || 9 * (long long)h->row_slots > 10 * num_edges;
+    if ((rule.most_row && h->longest_row > rule.most_row) ||
+        (rule.most_slots && 100 * (unsigned long long)h->lane_slots > (unsigned long long)rule.most_slots * (unsigned long long)num_edges))
+      h->longest_row = 0;
     h->row_loop = !(rule.edge_lanes && (same_bank || edges_share_lines || (rule.heavy && lanes_idle)));
   }
 }
@@ -717,6 +729,13 @@ int flexspmv_workspace_whole_rows(const void* d_workspace, int32_t* d_out, void*
   if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;
   if (!d_out) return FLEXSPMV_ERR_BAD_ARG;
   const char* src = static_cast<const char*>(d_workspace) + offsetof(flex::WorkspaceHeader, whole_rows);
+  return (int)cudaMemcpyAsync(d_out, src, sizeof(int32_t), cudaMemcpyDefault, static_cast<cudaStream_t>(stream));
+}
+
+int flexspmv_workspace_longest_row(const void* d_workspace, int32_t* d_out, void* stream) {
+  if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;
+  if (!d_out) return FLEXSPMV_ERR_BAD_ARG;
+  const char* src = static_cast<const char*>(d_workspace) + offsetof(flex::WorkspaceHeader, longest_row);
   return (int)cudaMemcpyAsync(d_out, src, sizeof(int32_t), cudaMemcpyDefault, static_cast<cudaStream_t>(stream));
 }
 

@@ -88,6 +88,20 @@ struct GraphApi {
   // (not whole rows) 98.0 / 104.3, 64.6 / 67.5, 77.2 / 94.1 (1 M items, swe_delta: 21.8 / 21.1).
   // Spring-mass fp32, 9 M items: rows of 8 31.3 / 42.3, of 4 - 12 46.7 / 52.4, of 9 38.6 / 36.5 (three words for a row, which single indices read
   // without conflicts): 8.5 rows for ten threads at least; one row of 40 among rows of 8 50.9 / 46.9, fp64 94.4 / 98.1.
+  // So a row of more than kWholeRowMax edges, or rows too uneven for one a thread, cost a launch more there (the loop with carries, one barrier for
+  // 24 warps), and nothing in the description tells: a caller who has seen the plan names the longest row (FLEXSPMV_LONGEST_ROW), and others get
+  // the usual configuration.  Units with an epilogue take plans of whole rows only.  us, CfgBig / Cfg, without whole rows: one row of 40 among rows of 8,
+  // spring-mass fp32 9 M items 47.7 / 44.0, fp64 1.8 M 28.4 / 25.6; of 0 - 16 fp64 3 M 41.6 / 38.8; among rows of 3 Rusanov fp64 2 M 33.5 / 32.1; SpMV, one
+  // of 40 among rows of 27 fp64 2.2 M 10.0 / 9.9, 4.5 M 16.0 / 15.3, 6 M 19.5 / 18.8, fp32 2.2 M 9.6 / 8.4, 3 M 9.8 / 10.1; one of 900 among rows of 31 fp64 1.6 M
+  // 11.2 / 9.4, 4.5 M 15.9 / 20.0, fp32 2.2 M 12.2 / 8.8, 6 M 18.0 / 21.2: either way by size, and no line.
+  // Nor do whole rows alone: the plan says that there is no longest row where one has more than three times the mean's edges, and lanes
+  // idle behind it, or where the rows are so uneven that of 32 in a warp some always idle (RowLoopRule::most_row, most_slots).  That costs graphs which read
+  // edge tensors in place at any size -- spring-mass, rows of 7 - 9 fp32 4 M items 28.9 / 24.5, 9 M 50.6 / 47.1, fp64 2.2 M 26.1 / 23.4, 9 M 78.7 / 77.4; of
+  // 6 - 10 32.1 / 25.9, 56.0 / 49.8, 29.7 / 26.3, 92.2 / 90.7; of 0 - 16 44.5 / 40.7, 82.0 / 81.7, 45.1 / 40.4, 144.6 / 146.6 --, and graphs which stage them only
+  // in 8-byte values where the tile has as many rows as the CTA threads: Rusanov fp64 rows of 0 - 6, 8 M (735 of 736) 124.8 / 122.7, 3 M (724) 50.9 / 54.0, 4 M (675)
+  // 63.6 / 71.4, of 0 - 8 8 M (588) 119.7 / 127.2; swe_delta of 2 - 4 1.3 M (732) 16.3 / 15.7, 3 M 29.0 / 32.0, of 2 - 5 8 M 64.8 / 72.1; Rusanov fp32 rows of 0 - 6, 3 M
+  // 28.3 / 32.5, 8 M 69.3 / 77.0.  One long row among even ones: spring-mass, 16 edges fp32 4 M 20.1 / 21.2, fp64 33.6 / 35.3, 24 20.8 / 21.1, 35.0 / 35.3, 32 22.4 /
+  // 20.9, 37.6 / 35.9; Rusanov fp64 3 M, 6 28.8 / 30.7, 12 30.0 / 30.8, 24 34.0 / 33.3.
   // Callers that name a tile or a number of CTAs get the configuration that they know.
   static constexpr int kBigTile = CfgBig::kTile - (G::kGatherNeedsRow ? CfgBig::kIpt : 0), kLeastRows = G::kGroup > 1 ? 17 : 14;      // rows a tile, for 20 threads
   // Two-phase graphs (SpMV): rows of 21 to 32 edges on average.  A tile of 1280 items holds 45 rows of 27, so that a warp has 32 of them or 13, and
@@ -96,8 +110,19 @@ struct GraphApi {
   // and fp64: rows of 24 29.2 / 30.6, 42.4 / 43.9; of 31 20.6 / 25.4, 28.8 / 31.8; of 32 61.7 / 67.3, 64.7 / 65.3; of 20 - 32 22.8 / 25.8, 33.5 / 33.8.  Shorter ones gain where
   // they begin in many banks, and lose where they do not: of 18 18.4 / 24.1, 26.3 / 29.0, of 20 21.7 / 22.4, 31.4 / 30.1 (3 M items fp32 9.4 / 8.8), of 16 42.4 / 40.7, 64.5 / 63.8.
   static constexpr int kBigRowEdges = 21;
+  static int longest_row(const flexspmv_desc* d) {
+    const int n = (d->reserved >> 8) & 63;
+    return n <= kWholeRowMax ? n : 0;
+  }
+  static int uses_longest_row(const flexspmv_desc* d) {
+    if (!G::kHasReducer || check_desc(d) != 0) return 0;
+    flexspmv_desc known = *d;
+    known.reserved = (d->reserved & 255) | FLEXSPMV_LONGEST_ROW(kWholeRowMax);
+    return !G::kEpilogue && use_big(&known) ? 1 : 0;
+  }
   static bool use_big(const flexspmv_desc* d) {
     if constexpr (kBigBuilt) {
+      if (!G::kEpilogue && !longest_row(d)) return false;
       // (a launch asks several times: what needs no look at the device first)
       const long long items = d->num_rows + d->num_edges;
       if (items <= kBigTile || d->tile_items > 0 || d->max_ctas > 0 || use_lean(d) || use_win(d)) return false;
@@ -113,6 +138,19 @@ struct GraphApi {
       return !small_launch(d, tiles, tiles < slots ? tiles : slots, Cfg::kBlock + 32);
     }
     return false;
+  }
+  struct LargeTileRows { long long most_row = 0; int most_slots = 0; };
+  static LargeTileRows large_tile_rows(const flexspmv_desc* d) {
+    LargeTileRows r;
+    if constexpr (kBigBuilt && G::kGatherNeedsRow && !G::kEpilogue) {
+      if (use_big(d)) {
+        const long long items = d->num_rows + d->num_edges;
+        const bool spare = sizeof(V) == 4 || 1000 * d->num_rows * big_tile(d) <= 985ll * CfgBig::kBlock * items;
+        r.most_row = 3 * d->num_edges / d->num_rows;
+        r.most_slots = G::kValuesStaged && spare ? 0 : 105;
+      }
+    }
+    return r;
   }
   // Up to 16 tiles a CTA are made equal in number: with tiles of one size 7.07 a CTA are as long as 8.
   static int big_tile(const flexspmv_desc* d) {
@@ -255,6 +293,7 @@ struct GraphApi {
         if (rule.edge_lanes && indices && d->num_edges > 0)
           rule.gathers = G::gathers(indices, rule.index, rule.record_bytes, RowLoopRule::kMaxGathers);
         for (int i = 0; i < rule.gathers; ++i) if (!rule.index[i]) return FLEXSPMV_ERR_BAD_ARG;
+        if (const LargeTileRows suits = large_tile_rows(d); suits.most_row) { rule.most_row = suits.most_row; rule.most_slots = suits.most_slots; }
         if (grid > 0 && !use_big(d) && small_launch(d, h.num_tiles, grid, Cfg::kBlock + 32)) {
           rule.share_items = 3 * ((h.num_tiles + grid - 1) / grid) * tile_items(d) / 2;
           rule.share_row_edges = kSmallRowEdges;
@@ -592,6 +631,9 @@ struct GraphApi {
   int flexspmv_##SYM##_launch(const flexspmv_desc* d, const void* const* v, const void* const* ix,              \
                               const void* ro, void* const* o, void* ws, size_t wb, void* st) {                  \
     return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::launch(d, v, ix, ro, o, ws, wb, static_cast<cudaStream_t>(st));  \
+  }                                                                                                             \
+  int flexspmv_##SYM##_uses_longest_row(const flexspmv_desc* d) {                                               \
+    return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::uses_longest_row(d);                                \
   }                                                                                                             \
   int flexspmv_##SYM##_device_status(const void* ws, int32_t* out, void* st) {                                  \
     return flex::GraphApi<GRAPH, CFG, CFGWIN, __VA_ARGS__>::device_status(ws, out, static_cast<cudaStream_t>(st));           \

@@ -57,7 +57,8 @@ typedef struct flexspmv_desc {
   int32_t max_ctas;      /* cap on persistent CTAs; 0 = SM count x resident CTAs per SM.  plan() lays the tile
                             boundaries between the CTAs of THIS grid on row ends where it can; a launch with
                             another value still works but hands carries between its CTAs            */
-  int32_t reserved;      /* flags: 0 or an OR of the FLEXSPMV_FLAG_* below (field name kept from ABI 1) */
+  int32_t reserved;      /* flags: 0 or an OR of the FLEXSPMV_FLAG_* and one FLEXSPMV_LONGEST_ROW below (field name
+                            kept from ABI 1) */
 } flexspmv_desc;
 
 /*
@@ -86,6 +87,16 @@ typedef struct flexspmv_desc {
  * with that kernel.  On stencil / banded matrices the plain path is faster.
  */
 #define FLEXSPMV_FLAG_RANDOM_GATHER 2
+
+/*
+ * The longest row (no reference counterpart).  A caller who knows that the matrix has no row of more than n edges, 1 <= n <= 32, and that
+ * its tiles hold whole rows, names n in the descriptor (the same for workspace_bytes, plan and launch).  Launches of graphs and sizes for
+ * which flexspmv_<graph>_uses_longest_row is not 0 then take larger tiles (bit 0 of its answer), which are faster on even rows
+ * and up to a quarter slower on others.  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
+ * later launches; where it says 0, plan without, and launch without.  Results of launches on whole rows are the same bits in either
+ * form.
+ */
+#define FLEXSPMV_LONGEST_ROW(n) ((n) << 8)
 
 /* ---- library-wide ----------------------------------------------------------------------------- */
 
@@ -242,6 +253,10 @@ int64_t flexspmv_plan_launches(void);
  * accepts the workspace. */
 int flexspmv_workspace_whole_rows(const void *d_workspace, int32_t *d_out, void *stream);
 
+/* The same for the edges of the longest row of such a plan; 0 where it has found no whole rows, or rows that do not suit the larger tiles
+ * it was made for (FLEXSPMV_LONGEST_ROW). */
+int flexspmv_workspace_longest_row(const void *d_workspace, int32_t *d_out, void *stream);
+
 /* ---- per fused graph ---------------------------------------------------------------------------
  * One set of symbols per (graph, value type); the per-edge map is compiled into the kernel, so
  * a graph is identified by its symbol prefix.  For graph G and value type T (f32 | f64 | i64):
@@ -265,6 +280,7 @@ int flexspmv_workspace_whole_rows(const void *d_workspace, int32_t *d_out, void 
  *                                cuda_template/reducer/merged_agent_spmv_template.cuh:350-445, and
  *                                the aggregator flavour cuda_template/aggregator/...:348-409).
  *                                Every output element is written (outputs need no zero fill).
+ *   flexspmv_G_T_uses_longest_row  what launches of the descriptor choose by FLEXSPMV_LONGEST_ROW: bit 0 the tiles (host only)
  *   flexspmv_G_T_device_status   copies the workspace's device status word into *d_status_out
  *                                (int32 in device or page-locked host memory) without synchronising
  *
@@ -303,6 +319,7 @@ typedef struct flexspmv_graph_info {
                             const void *const *indices, const void *d_row_offsets,                  \
                             void *const *outputs, void *d_workspace, size_t workspace_bytes,        \
                             void *stream);                                                          \
+  int flexspmv_##G##_uses_longest_row(const flexspmv_desc *desc);                                   \
   int flexspmv_##G##_device_status(const void *d_workspace, int32_t *d_status_out, void *stream);
 
 /* graphs built into libflexspmv_b200.so (the benchmark configurations and the unit-test graphs) */

@@ -71,3 +71,26 @@ def test_generated_binding_builds_and_matches(gname, dt, make):
     other = torch.float32 if dt == "float64" else torch.float64
     with pytest.raises(RuntimeError, match="Unsupported dtype"):
         ext.merged_spmv_launch(*[v.to(other) for v in vals], *idxs, ro, prob.num_rows, prob.num_cols)
+
+
+@pytest.mark.parametrize("long_row,large", [(0, True), (40, False)])
+def test_generated_binding_asks_its_plan_for_the_longest_row(long_row, large):
+    """A lattice large enough for large tiles, and the same with a row of 40 edges: the shim chooses as the ctypes operator does."""
+    if shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"):
+        pytest.skip("needs nvcc to build the generated extension")
+    from test_gpu_launch_sizes import default_tile, header_word
+    from test_gpu_whole_rows import with_lengths
+    ir, dtype = graphs.spring_mass_graph(), np.dtype("float32")
+    project_root = os.path.join(ROOT, "build", "jit", "binding_spring_mass_float32")
+    os.makedirs(project_root, exist_ok=True)
+    ext = merged_gen_binding.load_binding(ir, project_root, dtypes=("float32",))
+    lengths = [8] * 400_000
+    lengths[1000] = long_row or 8
+    prob = with_lengths(ir, lengths, 7, dtype)
+    vals, idxs, ro, _ = _device_args(ir, prob, dtype)
+    same = GraphExtension(ir)
+    for _ in range(2):                      # planned, and from the cache
+        (a,), (b,) = (e.merged_spmv_launch(*vals, *idxs, ro, prob.num_rows, prob.num_cols) for e in (ext, same))
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))      # (an edge from a particle to itself has a NaN)
+    same.check()
+    assert ext.device_status() == 0 and (header_word(same, 10) > default_tile(ir, dtype)) == large

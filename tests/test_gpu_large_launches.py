@@ -22,6 +22,11 @@ def sms():
     return torch.cuda.get_device_properties(0).multi_processor_count
 
 
+def longest_row_of(ext):
+    plan = next(reversed(ext._plans.values()))
+    return ext._longest_row(plan)
+
+
 def small_limit(ir, dtype):
     """Items up to which a launch of short rows takes the kernel without stages: 9 tiles for four CTAs, of which an SM holds three
     or four."""
@@ -43,7 +48,8 @@ def test_large_launches_equal_those_of_the_other_configuration(gname, dt, thread
     rows = items // (sum(lengths) // len(lengths) + 1) // len(lengths) * len(lengths) + (len(lengths) if tiles == 1 else 0)
     prob = with_lengths(ir, lengths * (rows // len(lengths)), 211, dtype)
     items = prob.num_rows + prob.nnz
-    ext = GraphExtension(ir, random_gather=False)
+    longest = max(lengths)            # named, so that the rows' evenness does not come into it
+    ext = GraphExtension(ir, random_gather=False, longest_row=longest)
     run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
     ext.check()
     each, took = -(-items // (sms() * tile)), header_word(ext, 10)
@@ -51,10 +57,10 @@ def test_large_launches_equal_those_of_the_other_configuration(gname, dt, thread
         assert took == default_tile(ir, dtype)
         return
     assert took == (-(-items // (sms() * each)) if each <= 16 else tile)
-    large, whole = launch(ir, prob, dtype, prob.num_cols, bits)
+    large, whole = launch(ir, prob, dtype, prob.num_cols, bits, longest_row=longest)
     named, also = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=3 * sms())
     assert whole and also and large == named
-    rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, ROUNDS)           # the same tiles going round the CTAs
+    rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, ROUNDS, longest_row=longest)           # the same tiles going round the CTAs
     assert rounds == large
     if tiles == 3:
         ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
@@ -65,18 +71,21 @@ def test_large_launches_equal_those_of_the_other_configuration(gname, dt, thread
 @pytest.mark.parametrize("gname,dt,threads,ipt,edges", LARGE)
 @pytest.mark.parametrize("bits", [32, 64])
 def test_large_launches_without_whole_rows(gname, dt, threads, ipt, edges, bits):
-    """A row of 40 edges, one of 900 and one of 20 000 among rows of three: the loop with carries, in tiles of both kinds."""
+    """A row of 40 edges, one of 900 and one of 20 000 among rows of three: the loop with carries, which large tiles make slower.  Both
+    kinds give the oracle's sums; the plan's look at the rows brings the usual one."""
     ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
     rows = small_limit(ir, dtype) // (edges + 1) + 1000
     lengths = np.full(rows, edges)
     lengths[[100, rows // 2, rows - 7]] = [40, 900, 20_000]
     prob = with_lengths(ir, lengths.tolist(), 223, dtype)
-    ext = GraphExtension(ir, random_gather=False)
-    got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
-    ext.check()
-    assert not ext.planned_whole_rows() and header_word(ext, 10) > 3 * default_tile(ir, dtype) // 2
     ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
-    assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} large, long rows")
+    for longest_row in (None, 0, 32):
+        ext = GraphExtension(ir, random_gather=False, longest_row=longest_row)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+        ext.check()
+        assert not ext.planned_whole_rows() and longest_row_of(ext) == 0
+        assert (header_word(ext, 10) > 3 * default_tile(ir, dtype) // 2) == (longest_row == 32)
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"{gname} large, long rows")
 
 
 @pytest.mark.parametrize("gname,dt,held", [("rusanov", "float64", {2: 0, 3: 1, 4: 1, 5: 0}), ("rusanov", "float32", {2: 0, 3: 1, 4: 1, 5: 0}),
@@ -91,6 +100,27 @@ def test_rows_of_which_the_large_tiles_hold_too_few_or_too_many(gname, dt, held)
         ext = GraphExtension(ir, random_gather=False)
         run_gpu(ext, ir, prob, dtype)
         assert (header_word(ext, 10) > default_tile(ir, dtype)) == large, edges
+
+
+@pytest.mark.parametrize("gname,dt,lengths,tiles,suits", [
+    ("spring_mass", "float32", [8], 3.0, True), ("spring_mass", "float32", [8] * 9999 + [24], 3.0, True), ("spring_mass", "float32", [8] * 9999 + [25], 3.0, False),
+    ("spring_mass", "float32", [7, 8, 9], 3.0, False), ("spring_mass", "float64", [8], 3.5, True), ("spring_mass", "float64", [8] * 640 + [9] * 32, 3.5, True),
+    ("spring_mass", "float64", [6, 10], 3.5, False), ("rusanov", "float64", [3] * 999 + [9], 2.9, True), ("rusanov", "float64", [3] * 999 + [10], 2.9, False),
+    ("rusanov", "float64", [0, 6, 3], 2.9, True), ("rusanov", "float64", [0, 6, 3], 3.0, False), ("rusanov", "float32", [0, 6, 3], 3.0, True),
+    ("swe_delta", "float64", [2, 5], 3.0, True), ("swe_delta", "float64", [2, 4], 17.0, False)])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_rows_that_suit_large_tiles(gname, dt, lengths, tiles, suits, bits):
+    """Whole rows of about one length, and none of more than three times the mean; graphs that stage their edge tensors take uneven ones in
+    tiles of fewer rows than threads.  (``tiles`` a CTA, of which the last part is the margin.)"""
+    ir, dtype = graphs.ALL_GRAPHS[gname](), np.dtype(dt)
+    _, _, threads, ipt, _ = next(c for c in LARGE if c[:2] == (gname, dt))
+    times = int((sms() * (threads - 1) * ipt * tiles - 50) / (sum(lengths) + len(lengths)))
+    prob = with_lengths(ir, lengths * times, 251, dtype)
+    ext = GraphExtension(ir, random_gather=False)
+    run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+    ext.check()
+    assert ext.planned_whole_rows() and (header_word(ext, 10) > 3 * default_tile(ir, dtype) // 2) == suits
+    assert next(reversed(ext._plans.values())).desc.reserved >> 8 == (max(lengths) if suits else 0)
 
 
 @pytest.mark.parametrize("bits", [32, 64])
@@ -114,7 +144,7 @@ def test_words_of_four_edges_at_odd_places(bits, skip, last):
     ro = dev(prob.row_offsets.astype(np.int32 if bits == 32 else np.int64))
     outs = []
     for max_ctas in (0, 4 * sms()):
-        ext = GraphExtension(ir, max_ctas=max_ctas)
+        ext = GraphExtension(ir, max_ctas=max_ctas, longest_row=max(lengths))
         out = torch.full((prob.num_rows, 2), float("nan"), device="cuda")
         ext.launch_into(values, indices, ro, [out], prob.num_rows, prob.nnz, prob.num_cols)
         ext.check()
@@ -129,18 +159,21 @@ def test_words_of_four_edges_at_odd_places(bits, skip, last):
                                            ([27] * 5000 + [40], True), ([25] * 3000 + [900, 0, 0], True)],
                          ids=["27", "21", "32", "20", "33", "uneven", "one_of_40", "long"])
 def test_longer_rows_of_spmv(dt, tile, bits, lengths, large):
-    """21 to 32 edges a row on average: batches of nine in two CTAs of 12 warps, or the loop with carries where a row is longer than 32."""
+    """21 to 32 edges a row on average: batches of nine in two CTAs of 12 warps, unless a row is longer than 32."""
     ir, dtype = graphs.spmv_graph(), np.dtype(dt)
     times = int(2 * sms() * tile * 1.3 / (sum(lengths) + len(lengths))) + 1
     prob = with_lengths(ir, lengths * times, 233, dtype)
     items = prob.num_rows + prob.nnz
-    ext = GraphExtension(ir, random_gather=False)
-    got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
-    ext.check()
-    each = -(-items // (2 * sms() * tile))
-    assert header_word(ext, 10) == (-(-items // (2 * sms() * each)) if large else default_tile(ir, dtype))
+    each, longest = -(-items // (2 * sms() * tile)), max(lengths) if max(lengths) <= 32 else 0
     ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
-    assert_outputs_match(ir, got, ref, sums, dtype, what=f"spmv {dt}")
+    for known in (0, 32, None):
+        ext = GraphExtension(ir, random_gather=False, longest_row=known)
+        got, _ = run_gpu(ext, ir, prob, dtype, offsets_dtype=np.int32 if bits == 32 else np.int64)
+        ext.check()
+        assert longest_row_of(ext) == longest
+        takes = large and (longest > 0 if known is None else known > 0)
+        assert header_word(ext, 10) == (-(-items // (2 * sms() * each)) if takes else default_tile(ir, dtype))
+        assert_outputs_match(ir, got, ref, sums, dtype, what=f"spmv {dt}")
     if large and max(lengths) <= 32:
         named, whole = launch(ir, prob, dtype, prob.num_cols, bits, max_ctas=4 * sms())
         rounds, _ = launch(ir, prob, dtype, 1 << 27, bits, ROUNDS)

@@ -239,3 +239,49 @@ def test_wider_records_under_a_built_in_name_compile(name, dt, tmp_path):
     src.write_text(emit_cuda.emit_graph(_wider(name), dt, "wider", windows=False))
     run = subprocess.run([NVCC] + NVCC_FLAGS + ["-cuda", str(src), "-o", str(tmp_path / "unit.ii")], capture_output=True, text=True)
     assert run.returncode == 0, run.stderr[-2000:]
+
+
+@pytest.mark.parametrize("graph,edges,uses", [("spring_mass_f32", 8, 1), ("spring_mass_f64", 8, 1), ("rusanov_f64", 3, 1), ("swe_delta_f64", 3, 1),
+                                              ("swe_delta_rk_f64", 3, 0), ("spmv_f64", 27, 1), ("spmv_f32", 27, 1), ("spmv_i64", 27, 0), ("spmv_f64", 33, 0),
+                                              ("spmv_f64", 12, 0), ("rusanov_f64", 9, 0), ("edge_sum_f32", 3, 0)])
+def test_which_launches_go_by_the_longest_row(graph, edges, uses):
+    """On a million rows over 148 SMs: the workspace of a descriptor that names the longest row has fewer, larger tiles where the library
+    says that it matters, and is the same one elsewhere.  What is no row length is nothing known."""
+    import ctypes
+    from flexspmv_b200.binding import Desc, load_library
+    lib = load_library()
+
+    def bytes_of(reserved, **kw):
+        d, n = Desc(1 << 20, edges << 20, 1 << 20, 32, kw.get("tile_items", 0), kw.get("max_ctas", 0), reserved), ctypes.c_size_t()
+        assert getattr(lib, f"flexspmv_{graph}_workspace_bytes")(ctypes.byref(d), ctypes.byref(n)) == 0
+        return n.value, getattr(lib, f"flexspmv_{graph}_uses_longest_row")(ctypes.byref(d))
+
+    (unknown, asked), (known, also) = bytes_of(0), bytes_of(edges << 8)
+    assert asked == also == uses and (known < unknown) == bool(uses)
+    assert bytes_of(33 << 8)[0] == unknown
+    for kw in ({"max_ctas": 7}, {"tile_items": 64}):
+        assert bytes_of(edges << 8, **kw)[1] == 0 and bytes_of(edges << 8, **kw) == bytes_of(0, **kw)
+
+
+@pytest.mark.parametrize("given,uses,longest,planned,described", [(None, 0, 9, [0], 0), (None, 1, 9, [32], 9), (None, 1, 0, [32, 0], 0), (0, 1, 9, [0], 0),
+                                                                  (7, 1, 9, [7], 7)])
+def test_a_plan_is_asked_for_the_longest_row(given, uses, longest, planned, described, monkeypatch):
+    from flexspmv_b200.binding import Desc, GraphExtension
+    import torch
+    made = []
+
+    def plan_once(syms, desc, *rest):
+        made.append(desc.reserved >> 8)
+        return type("Plan", (), {"desc": desc})()
+
+    ext = GraphExtension(graphs.spring_mass_graph(), longest_row=given)
+    monkeypatch.setattr(ext, "_plan_once", plan_once)
+    monkeypatch.setattr(ext, "_longest_row", lambda plan: longest)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    syms = type("Syms", (), {"uses_longest_row": staticmethod(lambda desc: uses)})()
+    plan = ext._make_plan(syms, lambda n: Desc(10, 20, 10, 32, 0, 0, n << 8), None, None)
+    assert made == planned and plan.desc.reserved >> 8 == described
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    made.clear()
+    plan = ext._make_plan(syms, lambda n: Desc(10, 20, 10, 32, 0, 0, n << 8), None, None)
+    assert made == [given or 0] and plan.desc.reserved >> 8 == (given or 0)
