@@ -88,7 +88,7 @@ struct RowLoopRule {
   // does not come into question for the matrix).
   long long share_items;             // rows and edges
   int share_row_edges;               // edges a row
-  // Large tiles of row-mode graphs (GraphApi::use_big): the longest row, and steps of lanes with a row for 100 edges, that suit them (0: any).
+  // Large tiles of row-mode graphs (GraphApi::use_big): the longest row, and steps of lanes with a row for 1000 edges, that suit them (0: any).
   long long most_row;
   int most_slots;
 };

@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256) whole_rows_apply_kernel(const OffsetT* ro
     const bool edges_share_lines = lines_more * rule.gathers > 22ll * rule.accumulators * h->line_rows * h->line_edges;
     const bool lanes_idle = num_edges > 7 * num_rows || 9 * (long long)h->row_slots > 10 * num_edges;
     if ((rule.most_row && h->longest_row > rule.most_row) ||
-        (rule.most_slots && 100 * (unsigned long long)h->lane_slots > (unsigned long long)rule.most_slots * (unsigned long long)num_edges))
+        (rule.most_slots && 1000 * (unsigned long long)h->lane_slots > (unsigned long long)rule.most_slots * (unsigned long long)num_edges))
       h->longest_row = 0;
     h->row_loop = !(rule.edge_lanes && (same_bank || edges_share_lines || (rule.heavy && lanes_idle)));
   }

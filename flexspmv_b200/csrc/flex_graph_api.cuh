@@ -43,7 +43,7 @@ struct NoLean {      // in place of CfgLean: the warp kernel for matrices with r
 };
 
 struct NoBig {       // in place of CfgBig: one configuration of the tile kernel for launches of every size
-  static constexpr int kTile = 0, kIpt = 0, kMinCtas = 1;
+  static constexpr int kTile = 0, kIpt = 0, kMinCtas = 1, kWarps = 1;
 };
 
 template <class G, class Cfg, class CfgWin = Cfg, class CfgLean = NoLean, class CfgBig = NoBig>
@@ -88,20 +88,18 @@ struct GraphApi {
   // (not whole rows) 98.0 / 104.3, 64.6 / 67.5, 77.2 / 94.1 (1 M items, swe_delta: 21.8 / 21.1).
   // Spring-mass fp32, 9 M items: rows of 8 31.3 / 42.3, of 4 - 12 46.7 / 52.4, of 9 38.6 / 36.5 (three words for a row, which single indices read
   // without conflicts): 8.5 rows for ten threads at least; one row of 40 among rows of 8 50.9 / 46.9, fp64 94.4 / 98.1.
-  // So a row of more than kWholeRowMax edges, or rows too uneven for one a thread, cost a launch more there (the loop with carries, one barrier for
-  // 24 warps), and nothing in the description tells: a caller who has seen the plan names the longest row (FLEXSPMV_LONGEST_ROW), and others get
-  // the usual configuration.  Units with an epilogue take plans of whole rows only.  us, CfgBig / Cfg, without whole rows: one row of 40 among rows of 8,
-  // spring-mass fp32 9 M items 47.7 / 44.0, fp64 1.8 M 28.4 / 25.6; of 0 - 16 fp64 3 M 41.6 / 38.8; among rows of 3 Rusanov fp64 2 M 33.5 / 32.1; SpMV, one
-  // of 40 among rows of 27 fp64 2.2 M 10.0 / 9.9, 4.5 M 16.0 / 15.3, 6 M 19.5 / 18.8, fp32 2.2 M 9.6 / 8.4, 3 M 9.8 / 10.1; one of 900 among rows of 31 fp64 1.6 M
-  // 11.2 / 9.4, 4.5 M 15.9 / 20.0, fp32 2.2 M 12.2 / 8.8, 6 M 18.0 / 21.2: either way by size, and no line.
-  // Nor do whole rows alone: the plan says that there is no longest row where one has more than three times the mean's edges, and lanes
-  // idle behind it, or where the rows are so uneven that of 32 in a warp some always idle (RowLoopRule::most_row, most_slots).  That costs graphs which read
-  // edge tensors in place at any size -- spring-mass, rows of 7 - 9 fp32 4 M items 28.9 / 24.5, 9 M 50.6 / 47.1, fp64 2.2 M 26.1 / 23.4, 9 M 78.7 / 77.4; of
-  // 6 - 10 32.1 / 25.9, 56.0 / 49.8, 29.7 / 26.3, 92.2 / 90.7; of 0 - 16 44.5 / 40.7, 82.0 / 81.7, 45.1 / 40.4, 144.6 / 146.6 --, and graphs which stage them only
-  // in 8-byte values where the tile has as many rows as the CTA threads: Rusanov fp64 rows of 0 - 6, 8 M (735 of 736) 124.8 / 122.7, 3 M (724) 50.9 / 54.0, 4 M (675)
-  // 63.6 / 71.4, of 0 - 8 8 M (588) 119.7 / 127.2; swe_delta of 2 - 4 1.3 M (732) 16.3 / 15.7, 3 M 29.0 / 32.0, of 2 - 5 8 M 64.8 / 72.1; Rusanov fp32 rows of 0 - 6, 3 M
-  // 28.3 / 32.5, 8 M 69.3 / 77.0.  One long row among even ones: spring-mass, 16 edges fp32 4 M 20.1 / 21.2, fp64 33.6 / 35.3, 24 20.8 / 21.1, 35.0 / 35.3, 32 22.4 /
-  // 20.9, 37.6 / 35.9; Rusanov fp64 3 M, 6 28.8 / 30.7, 12 30.0 / 30.8, 24 34.0 / 33.3.
+  // So a row of more than kWholeRowMax edges costs a launch far more there (the loop with carries, one barrier for 24 warps), and nothing in the
+  // description tells: a caller who has seen the plan names the longest row (FLEXSPMV_LONGEST_ROW), and others get the usual configuration.  Units
+  // with an epilogue take plans of whole rows only.  us, CfgBig / Cfg, without whole rows, columns within 300 rows: one row in 1000 of 40 edges among rows of 3, 8 M
+  // items Rusanov fp64 270 / 227, fp32 170 / 131, swe_delta 215 / 172; one in 5000 of 1000 531 / 276, 271 / 172, 338 / 194 (one in 100 of 40 384 / 397, 216 / 212, 284 /
+  // 338; one in ten of 14 among rows of 2 238 / 250, 130 / 158, 173 / 187); one row of 40 among rows of 8, spring-mass fp32 9 M 51.9 / 46.9, fp64 4 M 51.2 / 48.8; SpMV, one
+  // of 40 among rows of 27 fp64 4.5 M 16.0 / 15.3, fp32 2.2 M 9.6 / 8.4, 3 M 9.8 / 10.1, of 900 among rows of 31 2.2 M 12.2 / 8.8, 6 M 18.0 / 21.2.
+  // Of whole rows the plan says that there is no longest one where it has more than four times the mean's edges, behind which lanes idle (RowLoopRule::most_row):
+  // one row of 12, 24 among rows of 3 Rusanov fp64 3 M items 30.0 / 30.8, 34.0 / 33.3; of 32 among rows of 8 spring-mass 9 M fp32 33.2 / 42.2, fp64 69.3 / 79.9 -- and for
+  // 8-byte values of graphs that read edge tensors in place where rows are uneven (most_slots: more than 1.005 lane-steps an edge): lattices with one edge in 20
+  // left out, spring-mass fp64 500^2 20.8 / 19.1, 600^2 27.4 / 30.2, 1024^2 65.4 / 63.3, 1300^2 101.6 / 92.8, one in ten 64.5 / 61.8 and 103 / 90; one in 100 1300^2 103 / 99.
+  // (fp32 one in 20 600^2 16.0 / 18.3, 1024^2 39.9 / 43.8, one in five 38.3 / 39.8, though rows of 6 - 10 with columns side by side 4 M items 32.1 / 25.9.  Graphs that stage
+  // their edge tensors: rows of 0 - 6 fp64 Rusanov 3 M items 53.5 / 57.6, 8 M 131 / 133, swe_delta 41.3 / 42.1, 98.6 / 98.7, fp32 Rusanov 28.5 / 33.3.)
   // Callers that name a tile or a number of CTAs get the configuration that they know.
   static constexpr int kBigTile = CfgBig::kTile - (G::kGatherNeedsRow ? CfgBig::kIpt : 0), kLeastRows = G::kGroup > 1 ? 17 : 14;      // rows a tile, for 20 threads
   // Two-phase graphs (SpMV): rows of 21 to 32 edges on average.  A tile of 1280 items holds 45 rows of 27, so that a warp has 32 of them or 13, and
@@ -134,6 +132,21 @@ struct GraphApi {
       }
       const long long sms = device_sm_count();
       if (items <= sms * CfgBig::kMinCtas * kBigTile) return false;
+      if constexpr (G::kGatherNeedsRow) {
+        // No more rows a tile than threads, or a warp goes round it for one group of 32.  us, triangles of 1024^2 squares, one edge in 100 left out: Rusanov fp64 (741
+        // rows for 736) 82.4 / 79.0, swe_delta 72.9 / 69.0, in 20 (764) 72.6 / 68.0; Rusanov fp32 45.7 / 50.2 (998 for 992), 54.1 / 50.2 (1030).
+        const long long ctas = sms * CfgBig::kMinCtas, tile = big_tile(d);
+        if (100 * d->num_rows * tile > (sizeof(V) == 4 ? 101ll : 100ll) * CfgBig::kBlock * items) return false;
+        // A CTA's warps take its tiles' groups of 32 rows in turns; a last turn that leaves 215 of 1000 of all their lanes without a row costs 8-byte values of
+        // graphs that stage their edge tensors what the large tiles gain, up to four turns: by the share with a row, Rusanov fp64 0.75 16.4 / 15.9, 0.76 15.6 / 14.9, 0.78 16.7 /
+        // 16.2, 0.79 17.1 / 17.3, 0.80 12.9 / 13.6; swe_delta 0.74 10.8 / 10.5, 0.775 13.4 / 13.0, 0.79 13.5 / 14.1.  (Spring-mass lattices fp64 0.67 19.1 / 19.8, 0.73 20.6 / 20.3,
+        // 0.75 25.1 / 27.0; a stage of the shallow-water step, 406^2 squares, 0.76 17.9 / 21.2.)
+        if constexpr (G::kValuesStaged && sizeof(V) == 8 && !G::kEpilogue) {
+          const long long each = (items + ctas * kBigTile - 1) / (ctas * kBigTile), tile_rows = (d->num_rows * tile + items - 1) / items;
+          const long long turns = (each * ((tile_rows + 31) / 32) + CfgBig::kWarps - 1) / CfgBig::kWarps;
+          if (1000 * d->num_rows < 785 * 32 * ctas * turns * CfgBig::kWarps) return false;
+        }
+      }
       const long long tiles = (items + kDefaultTile - 1) / kDefaultTile, slots = sms * Cfg::kMinCtas;
       return !small_launch(d, tiles, tiles < slots ? tiles : slots, Cfg::kBlock + 32);
     }
@@ -144,10 +157,8 @@ struct GraphApi {
     LargeTileRows r;
     if constexpr (kBigBuilt && G::kGatherNeedsRow && !G::kEpilogue) {
       if (use_big(d)) {
-        const long long items = d->num_rows + d->num_edges;
-        const bool spare = sizeof(V) == 4 || 1000 * d->num_rows * big_tile(d) <= 985ll * CfgBig::kBlock * items;
-        r.most_row = 3 * d->num_edges / d->num_rows;
-        r.most_slots = G::kValuesStaged && spare ? 0 : 105;
+        r.most_row = 4 * d->num_edges / d->num_rows;
+        r.most_slots = G::kValuesStaged || sizeof(V) == 4 ? 0 : 1005;
       }
     }
     return r;

@@ -91,8 +91,8 @@ typedef struct flexspmv_desc {
 /*
  * The longest row (no reference counterpart).  A caller who knows that the matrix has no row of more than n edges, 1 <= n <= 32, and that
  * its tiles hold whole rows, names n in the descriptor (the same for workspace_bytes, plan and launch).  Launches of graphs and sizes for
- * which flexspmv_<graph>_uses_longest_row is not 0 then take larger tiles (bit 0 of its answer), which are faster on even rows
- * and up to a quarter slower on others.  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
+ * which flexspmv_<graph>_uses_longest_row is not 0 then take larger tiles (bit 0 of its answer), which are faster on whole rows
+ * of about one length, and take up to twice as long on others.  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
  * later launches; where it says 0, plan without, and launch without.  Results of launches on whole rows are the same bits in either
  * form.
  */
