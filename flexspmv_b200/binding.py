@@ -288,8 +288,8 @@ class GraphExtension:
         return plan, plan.desc
 
     def _make_plan(self, syms: _Symbols, described, ro: Optional[torch.Tensor], device, indices: Sequence[torch.Tensor] = ()) -> "_Plan":
-        """A plan for ``described(longest)``, the descriptor that names the longest row.  Where its tiles go by that, they are those of
-        whole rows until the plan says that it has none."""
+        """A plan for ``described(longest)``, the descriptor that names the longest row.  Where its tiles go by that (bit 0 of
+        ``uses_longest_row``), they are those of whole rows until the plan says that it has none."""
         if self.longest_row is not None:
             return self._plan_once(syms, described(int(self.longest_row)), ro, device, indices)
         unknown = described(0)
@@ -298,7 +298,7 @@ class GraphExtension:
             return self._plan_once(syms, unknown, ro, device, indices)
         plan = self._plan_once(syms, described(32), ro, device, indices)
         longest = self._longest_row(plan)
-        if longest == 0:
+        if longest == 0 and by_row & 1:
             return self._plan_once(syms, unknown, ro, device, indices)
         plan.desc = described(longest)
         return plan

@@ -125,7 +125,8 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w("  };")
     w("  const int32_t unknown = d.reserved;")
     w("  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;")
-    w("  if (has_rows && e.uses_longest_row(&d) && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {")
+    w("  const int by_row = has_rows ? e.uses_longest_row(&d) : 0;        // bit 0: the tiles do")
+    w("  if (by_row && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {")
     w("    d.reserved = unknown | FLEXSPMV_LONGEST_ROW(32);")
     w("    plan();")
     w("    torch::Tensor out = torch::empty({1}, torch::TensorOptions().dtype(torch::kInt).device(like.device()));")
@@ -133,7 +134,7 @@ def binding_source(ir: GraphIR, symbol: str, dtypes: Iterable[str]) -> str:
     w('    TORCH_CHECK(st == 0, "merged_spmv_launch (longest row) failed: ", flexspmv_error_string(st));')
     w("    const int longest = out.item<int32_t>();")
     w("    d.reserved = longest ? unknown | FLEXSPMV_LONGEST_ROW(longest) : unknown;")
-    w("    if (!longest) plan();")
+    w("    if (!longest && (by_row & 1)) plan();")
     w("  } else {")
     w("    plan();")
     w("  }")

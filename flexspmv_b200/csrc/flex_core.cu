@@ -25,8 +25,8 @@ int device_sm_count() {
 // Kernels that planning has enqueued from this thread (flexspmv_plan_launches).
 static thread_local long long plan_launches = 0;
 
-static thread_local int last_kernel = FLEXSPMV_KERNEL_NONE;
-void note_kernel(int which) { last_kernel = which; }
+static thread_local int last_kernel = FLEXSPMV_KERNEL_NONE, last_row_batch = 0;
+void note_kernel(int which, int row_batch) { last_kernel = which; last_row_batch = row_batch; }
 
 // One thread per tile boundary: coordinate of diagonal t * tile_items (clamped to rows + edges).  A plan's header goes along
 // (null: coordinates alone): a launch less in the first call on a matrix.
@@ -708,6 +708,8 @@ int flexspmv_debug_withhold_stage(void* d_workspace, uint32_t first_tile_plus_on
 }
 
 int flexspmv_debug_last_kernel(void) { return flex::last_kernel; }
+
+int flexspmv_debug_last_row_batch(void) { return flex::last_row_batch; }
 
 int flexspmv_workspace_status_mirror(void* d_workspace, int32_t* pinned_host_status, void* stream) {
   if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;

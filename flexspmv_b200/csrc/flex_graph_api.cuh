@@ -22,7 +22,7 @@ namespace flex {
 int partition_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_edges,
                      int tile_items, void* d_coords, cudaStream_t stream, void* ws, const WorkspaceHeader* h);
 int device_sm_count();
-void note_kernel(int which);      // FLEXSPMV_KERNEL_*, for flexspmv_debug_last_kernel
+void note_kernel(int which, int row_batch = 0);      // for flexspmv_debug_last_kernel, flexspmv_debug_last_row_batch
 int header_init_launch(void* ws, const WorkspaceHeader& h, cudaStream_t stream);
 int snap_cta_boundaries_launch(const void* d_row_offsets, int offset_bits, long long num_rows, long long num_tiles, int grid,
                                const TileRoom& room, void* d_coords, void* ws, cudaStream_t stream);
@@ -113,10 +113,14 @@ struct GraphApi {
     return n <= kWholeRowMax ? n : 0;
   }
   static int uses_longest_row(const flexspmv_desc* d) {
-    if (!G::kHasReducer || check_desc(d) != 0) return 0;
-    flexspmv_desc known = *d;
-    known.reserved = (d->reserved & 255) | FLEXSPMV_LONGEST_ROW(kWholeRowMax);
-    return !G::kEpilogue && use_big(&known) ? 1 : 0;
+    if constexpr (G::kHasReducer) {
+      if (check_desc(d) != 0) return 0;
+      flexspmv_desc known = *d;
+      known.reserved = (d->reserved & 255) | FLEXSPMV_LONGEST_ROW(kWholeRowMax);
+      if (use_big(&known)) return G::kEpilogue ? 0 : 1;
+      if (kOneRoundBuilt<Cfg> && !use_lean(d) && !use_win(d)) return row_edges_within(d, 4, sizeof(V) == 4 ? 7 : 5) ? 2 : 0;
+    }
+    return 0;
   }
   static bool use_big(const flexspmv_desc* d) {
     if constexpr (kBigBuilt) {
@@ -369,12 +373,15 @@ struct GraphApi {
   //                     13.5 MB 28.5 / 28.6, 26 51.6 / 52.2, 35 64.6 / 64.1, 54 100.4 / 97.8
   static constexpr long long kKeepBytes = (G::kGatherNeedsRow ? 10ll : 40ll) << 20;
 
-  // SpMV on rows of four to five edges on average (five-point grids), and of five to seven in 4-byte values (seven-point ones): batches of as
-  // many, so that a row is one round of gathers instead of two, in launches without stages and in tiles a CTA's own run.  us, batches of
+  // SpMV on rows of more than four edges on average and five at most (five-point grids), and in 4-byte values seven at most (seven-point ones):
+  // batches of as many, so that a row is one round of gathers instead of two, in launches without stages and in tiles a CTA's own run.  us, batches of
   // four / five: 512^2 fp64 4.9 / 4.6, 600^2 7.9 / 7.5, fp32 5.7 / 4.8; 700^2 fp64 10.1 / 9.3, 1500^2 34.5 / 33.4, fp32 26.1 / 24.0; four / seven, fp32: 60^3 4.46 / 4.18, 80^3 10.2 /
   // 9.9, 145^3 42.1 / 40.9, 200^3 110.5 / 107.5, rows of 6, 8 M items 16.6 / 16.1.  Not in rounds, where more gathers at a time leave L2 earlier: 2500^2 fp64
   // 83.0 / 86.1, 240^3 fp32 182 / 192.  Other lengths gain less than they lose: five at a time fp64, 1.2 M items without stages, rows of 4 5.25 / 5.40, of 6
-  // 6.0 / 6.4, 145^3 55.2 / 58.0; seven at a time fp32, 8 M items, rows of 3 16.3 / 18.2, of 8 23.4 / 24.9, 0 - 30 22.0 / 22.8, fp64 145^3 55.2 / 68.7.
+  // 6.0 / 6.4, 145^3 55.2 / 58.0; seven at a time fp32, 8 M items, rows of 3 16.3 / 18.2, of 8 23.4 / 24.9, 0 - 30 22.0 / 22.8, fp64 145^3 55.2 / 68.7.  A longer row takes
+  // two rounds either way, the first of which then waits for more: five at a time, fp64 rows of 4 - 6 3 M items 10.1 / 10.9, 8 M 21.1 / 23.3, 3 - 7 10.2 / 10.9, 21.8 /
+  // 22.7; seven, fp32 6 - 8 8 M 16.0 / 18.2, 4 - 9 18.4 / 19.5.  So the caller has to name the longest row, which the plan knows (FLEXSPMV_LONGEST_ROW).  int64 as fp64: rows
+  // of 5 3 M 10.4 / 9.3, 8 M 21.2 / 19.9, of 4 - 5 23.3 / 21.2; fp32 rows of 2 - 7 seven at a time 8 M 17.8 / 16.9 (five 19.0), one in ten of 7 among rows of 4 17.7 / 16.9.
   template <class C>
   static constexpr bool kOneRoundBuilt = !G::kGatherNeedsRow && G::kLightMap && G::kAccDim == 1 && C::kRowBatch == 4 && !C::kPipeline && !C::kLarge;
   static bool row_edges_within(const flexspmv_desc* d, int above, int most) {
@@ -438,7 +445,7 @@ struct GraphApi {
       a.win_table = reinterpret_cast<const int*>(static_cast<char*>(ws) + h.win_table_offset);
       a.win_index = reinterpret_cast<const unsigned short*>(static_cast<char*>(ws) + h.win_index_offset);
     }
-    int form = FLEXSPMV_KERNEL_TILE;
+    int form = FLEXSPMV_KERNEL_TILE, row_batch = C::kRowBatch;
     if constexpr (L::kWhole) if (whole_rows) {
       const long long vertices = d->num_vertices > d->num_rows ? d->num_vertices : d->num_rows;
       bool small = false;
@@ -465,14 +472,15 @@ struct GraphApi {
         kernel = small ? flex_tile_kernel<G, OffsetT, One, false, kSmall> : flex_tile_kernel<G, OffsetT, One, false, kPlain>;
         return small ? resident_ctas<OffsetT, One, false, kSmall>(&resident) : resident_ctas<OffsetT, One, false, kPlain>(&resident);
       };
-      if (whole_rows && form != FLEXSPMV_KERNEL_TILE_ROUNDS) {
+      const int longest = longest_row(d);
+      if (whole_rows && form != FLEXSPMV_KERNEL_TILE_ROUNDS && longest && row_edges_within(d, 4, longest)) {
         int e = 0;
-        if (row_edges_within(d, 4, 5)) e = batch_of(IntC<5>{});
-        else if constexpr (sizeof(V) == 4) { if (row_edges_within(d, 5, 7)) e = batch_of(IntC<7>{}); }
+        if (longest <= 5) { e = batch_of(IntC<5>{}); row_batch = 5; }
+        else if constexpr (sizeof(V) == 4) { if (longest <= 7) { e = batch_of(IntC<7>{}); row_batch = 7; } }
         if (e) return e;
       }
     }
-    note_kernel(form);
+    note_kernel(form, row_batch);
     return launch_pdl(kernel, (unsigned)grid, kThreads, L::kTotal, st, p, a);
   }
 

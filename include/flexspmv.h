@@ -92,8 +92,8 @@ typedef struct flexspmv_desc {
  * The longest row (no reference counterpart).  A caller who knows that the matrix has no row of more than n edges, 1 <= n <= 32, and that
  * its tiles hold whole rows, names n in the descriptor (the same for workspace_bytes, plan and launch).  Launches of graphs and sizes for
  * which flexspmv_<graph>_uses_longest_row is not 0 then take larger tiles (bit 0 of its answer), which are faster on whole rows
- * of about one length, and take up to twice as long on others.  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
- * later launches; where it says 0, plan without, and launch without.  Results of launches on whole rows are the same bits in either
+ * of about one length, and take up to twice as long on others, or take rows of four to seven edges in one round of gathers (bit 1).  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
+ * later launches; where it says 0, launch without, and where bit 0 is set plan without before that.  Results of launches on whole rows are the same bits in either
  * form.
  */
 #define FLEXSPMV_LONGEST_ROW(n) ((n) << 8)
@@ -149,6 +149,9 @@ enum {
   FLEXSPMV_KERNEL_STEP = 7         /* whole step of the shallow-water model (swe_delta_rk_*) */
 };
 int flexspmv_debug_last_kernel(void);
+
+/* Testing aid: the edges of a row that it takes together where it runs a loop over whole rows (0: another kernel). */
+int flexspmv_debug_last_row_batch(void);
 
 /*
  * Measurement aid: the rate at which the GPU gathers 4-byte records without locality.  Streams d_idx / d_vals
@@ -280,7 +283,8 @@ int flexspmv_workspace_longest_row(const void *d_workspace, int32_t *d_out, void
  *                                cuda_template/reducer/merged_agent_spmv_template.cuh:350-445, and
  *                                the aggregator flavour cuda_template/aggregator/...:348-409).
  *                                Every output element is written (outputs need no zero fill).
- *   flexspmv_G_T_uses_longest_row  what launches of the descriptor choose by FLEXSPMV_LONGEST_ROW: bit 0 the tiles (host only)
+ *   flexspmv_G_T_uses_longest_row  what launches of the descriptor choose by FLEXSPMV_LONGEST_ROW: bit 0 the tiles, bit 1
+ *                                the edges that they gather for together (host only)
  *   flexspmv_G_T_device_status   copies the workspace's device status word into *d_status_out
  *                                (int32 in device or page-locked host memory) without synchronising
  *

@@ -373,8 +373,8 @@ def test_wide_records_in_small_ctas(dt, lengths):
                          ids=["5", "4_5", "3_to_7", "0_10", "1_to_9", "7", "5_to_7", "0_14"])
 @pytest.mark.parametrize("rows,kernel", [(9000, SMALL), (600_000, TILE)])
 def test_short_rows_in_one_round(dt, bits, lengths, rows, kernel):
-    """Four to five edges a row on average are taken five at a time, and five to seven (4-byte values) seven; the same rows in front of
-    others that bring the average out of those ranges are taken four at a time.  The same bits."""
+    """Four to five edges a row on average, and no row of more, are taken five at a time, and up to seven (4-byte values) seven; the same
+    rows in front of others that bring the average out of those ranges are taken four at a time.  The same bits."""
     ir, dtype = graphs.spmv_graph(), np.dtype(dt)
     mine = (lengths * (rows // len(lengths) + 1))[:rows]
     others = [12] * rows
@@ -390,9 +390,31 @@ def test_short_rows_in_one_round(dt, bits, lengths, rows, kernel):
         y = torch.full((count,), 7, dtype=x.dtype, device="cuda")
         ext.launch_into([dev(prob.values[non_gather[0]][:edges].astype(dtype)), x], [dev(prob.indices[index_names[0]][:edges])],
                         dev(prob.row_offsets[:count + 1].astype(np.int32 if bits == 32 else np.int64)), [y], count, edges, prob.num_cols)
+        longest, most = max(lengths), 7 if dt == "float32" else 5
+        batch = 4 if count > n or longest > most else 5 if longest <= 5 else 7
+        assert load_library().flexspmv_debug_last_row_batch() == batch
         if count == n:
             assert last_kernel() == kernel
         ext.check()
         assert ext.planned_whole_rows()
         results.append(y[:n].cpu().numpy().tobytes())
     assert results[0] == results[1]
+
+
+@pytest.mark.parametrize("dt,lengths,known,batch", [("float64", [5], None, 5), ("float64", [5], 0, 4), ("float64", [4] * 99 + [5], None, 5), ("float64", [4], None, 4),
+                                                    ("float64", [5] * 999 + [6, 4], None, 4), ("float64", [6, 7], None, 4), ("float32", [5] * 9 + [6, 4], None, 7),
+                                                    ("float32", [7], None, 7), ("float32", [7] * 999 + [8, 6], None, 4), ("float32", [7, 7, 8], None, 4),
+                                                    ("int64", [5], None, 5), ("int64", [6], None, 4)])
+def test_the_longest_row_decides_how_many_edges_go_together(dt, lengths, known, batch):
+    """Averages at, just above and just below the lines, each with a longest row that a batch holds and with one more; and tiles that go round
+    the CTAs take four."""
+    ir, dtype = graphs.spmv_graph(), np.dtype(dt)
+    prob = with_lengths(ir, lengths * (60_000 // len(lengths)), 263, dtype)
+    ext = GraphExtension(ir, random_gather=False, longest_row=known)
+    got, _ = run_gpu(ext, ir, prob, dtype)
+    ext.check()
+    assert load_library().flexspmv_debug_last_row_batch() == batch
+    ref, _, sums = ir_eval.run_graph(ir, prob, dtype, num_threads=4, want_abs_sums=True)
+    assert_outputs_match(ir, got, ref, sums, dtype, what=f"spmv {dt}")
+    launch(ir, prob, dtype, 1 << 27, 32, ROUNDS, max_ctas=4)
+    assert load_library().flexspmv_debug_last_row_batch() == 4

@@ -243,7 +243,8 @@ def test_wider_records_under_a_built_in_name_compile(name, dt, tmp_path):
 
 @pytest.mark.parametrize("graph,edges,uses", [("spring_mass_f32", 8, 1), ("spring_mass_f64", 8, 1), ("rusanov_f64", 3, 1), ("swe_delta_f64", 3, 1),
                                               ("swe_delta_rk_f64", 3, 0), ("spmv_f64", 27, 1), ("spmv_f32", 27, 1), ("spmv_i64", 27, 0), ("spmv_f64", 33, 0),
-                                              ("spmv_f64", 12, 0), ("rusanov_f64", 9, 0), ("edge_sum_f32", 3, 0)])
+                                              ("spmv_f64", 12, 0), ("rusanov_f64", 9, 0), ("edge_sum_f32", 3, 0), ("spmv_f64", 5, 2), ("spmv_i64", 5, 2), ("spmv_f64", 6, 0),
+                                              ("spmv_f32", 7, 2), ("spmv_f32", 4, 0), ("spmv_f32", 8, 0), ("swe_boundary_f64", 5, 0)])
 def test_which_launches_go_by_the_longest_row(graph, edges, uses):
     """On a million rows over 148 SMs: the workspace of a descriptor that names the longest row has fewer, larger tiles where the library
     says that it matters, and is the same one elsewhere.  What is no row length is nothing known."""
@@ -257,14 +258,14 @@ def test_which_launches_go_by_the_longest_row(graph, edges, uses):
         return n.value, getattr(lib, f"flexspmv_{graph}_uses_longest_row")(ctypes.byref(d))
 
     (unknown, asked), (known, also) = bytes_of(0), bytes_of(edges << 8)
-    assert asked == also == uses and (known < unknown) == bool(uses)
+    assert asked == also == uses and (known < unknown) == bool(uses & 1)
     assert bytes_of(33 << 8)[0] == unknown
     for kw in ({"max_ctas": 7}, {"tile_items": 64}):
-        assert bytes_of(edges << 8, **kw)[1] == 0 and bytes_of(edges << 8, **kw) == bytes_of(0, **kw)
+        assert bytes_of(edges << 8, **kw)[1] == uses & 2 and bytes_of(edges << 8, **kw) == bytes_of(0, **kw)
 
 
 @pytest.mark.parametrize("given,uses,longest,planned,described", [(None, 0, 9, [0], 0), (None, 1, 9, [32], 9), (None, 1, 0, [32, 0], 0), (0, 1, 9, [0], 0),
-                                                                  (7, 1, 9, [7], 7)])
+                                                                  (7, 1, 9, [7], 7), (None, 2, 5, [32], 5), (None, 2, 0, [32], 0)])
 def test_a_plan_is_asked_for_the_longest_row(given, uses, longest, planned, described, monkeypatch):
     from flexspmv_b200.binding import Desc, GraphExtension
     import torch
