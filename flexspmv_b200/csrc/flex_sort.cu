@@ -7,7 +7,7 @@
 // Least-significant-digit radix sort on the row ids, which are dense: ceil(log2(num_rows)) bits in as few passes as cover
 // them, every pass the same width (21 bits: 3 x 7).  A pass is three launches: digit counts per tile of keys, one CTA per
 // digit that scans that digit's counts over the tiles, and the stable scatter.  No block waits for another one.  Digits have
-// up to 8 bits, or up to 10 where that saves a pass that costs more (flexspmv_sort_rows); every width is compiled by itself.  The first pass reads the caller's ids and takes the
+// up to 8 bits, or 9 and 10 where that saves a pass that costs more (flexspmv_sort_rows); every width is compiled by itself.  The first pass reads the caller's ids and takes the
 // positions as values, so there is no separate initialisation; the passes alternate between two buffers so that the last one
 // writes the caller's permutation.  Equal digits keep their input order in every pass (see sort_scatter_kernel), so the
 // permutation equals a stable argsort (bit-exact against numpy.argsort(kind="stable")).
@@ -482,10 +482,13 @@ int flexspmv_sort_rows(const void* d_row_ids, int32_t id_bits, int64_t num_edges
   if (num_edges > 0) {
     int bits = 0;
     while (bits < 31 && (1ll << bits) < num_rows) ++bits;
-    // 10-bit digits where they save a pass: always the second one, a third (or fourth) one up to 5 M ids, where passes are short.  us, the
-    // whole sort and a permutation, wide / narrow digits: 3.2 M ids, 17 and 18 bits 140 / 152, 137 / 152; 8.4 M, 20 bits 295 / 284; 30 M, 19 bits
-    // 1163 / 1095.
-    const bool wide = scratch_bytes >= wide_bytes && (bits + 9) / 10 < (bits + 7) / 8 && (bits <= 10 || num_edges <= 5ll << 20);
+    // 9- and 10-bit digits where one of them is enough, and two of 9 bits for three of 6 from 3 M to 5 M ids.  us, the whole sort and a
+    // permutation, wide / narrow digits.  9 and 10 bits: 0.3 M ids 75 / 77, 85 / 87; 5 M 122 / 120, 132 / 133; 30 M 749 / 750, 822 / 822.  17 bits: 0.5 M 110 / 97, 2 M
+    // 123 / 115, 3.2 M 141 / 146, 4 M 153 / 156, 5 M 176 / 179, 5.6 M 188 / 188, 6.5 M 208 / 204, 8.4 M 247 / 253, 30 M 1009 / 1024; 18 bits: 1 M 103 / 96, 3.2 M 130 / 133, 4 M
+    // 147 / 154, 5 M 173 / 176, 6.5 M 207 / 205, 30 M 1030 / 1035.  Pairs of 10 bits (19 and 20) lose at every size: 1 M 118 / 102, 2 M 121 / 118, 4 M 170 / 154, 8.4 M 282 / 265,
+    // 12 M 438 / 396; three of 9 bits for four of 7: 26 bits 4 M 320 / 312, 12 M 599 / 594, 28 bits 5 M 1081 / 985.
+    const bool wide = scratch_bytes >= wide_bytes &&
+        (bits == 9 || bits == 10 || ((bits == 17 || bits == 18) && num_edges >= 3'000'000 && num_edges <= 5ll << 20));
     // the totals are the last words of the scratch that the shape takes
     unsigned* totals = reinterpret_cast<unsigned*>(base + (wide ? wide_bytes : narrow_bytes)) - (wide ? flex::SortWide<10>::kBins : flex::SortNarrow<8>::kBins);
     if (bits == 0) {

@@ -52,3 +52,14 @@ def test_counts_of_more_than_a_thousand_tiles_and_records_beyond_one_sweep():
     for dtype in (np.float64, np.float32):
         src = np.random.default_rng(89).random(n).astype(dtype)
         assert np.array_equal(permute_edges(torch.from_numpy(src).cuda(), perm).cpu().numpy(), src[want])
+
+
+@pytest.mark.parametrize("rows,n", [(1 << 17, 2_999_999), (1 << 17, 3_000_000), ((1 << 17) + 1, 5 << 20), ((1 << 18) - 5, (5 << 20) + 1), (1 << 20, 3_000_001),
+                                    (1 << 10, 200_003), ((1 << 9) - 1, 200_003)])
+def test_lines_between_digit_widths(rows, n):
+    """Two digits of nine bits between 3 M and 5 M ids of 17 and 18 bits, one of nine or ten, narrow ones elsewhere."""
+    ids = np.random.default_rng(97).integers(0, rows, n)
+    perm, ro = sort_edges_by_row(torch.from_numpy(ids.astype(np.int32)).cuda(), rows)
+    want = np.argsort(ids, kind="stable")
+    assert np.array_equal(perm.cpu().numpy(), want)
+    assert np.array_equal(ro.cpu().numpy(), np.searchsorted(ids[want], np.arange(rows + 1)))
