@@ -115,8 +115,9 @@ def test_the_epilogue_refuses_a_plan_without_whole_rows(max_ctas):
     assert all(torch.isnan(t).all() for t in acc + out)
 
 
-def run_stage(m, start, sums, bits, first, last, max_ctas, vertices=None):
-    """One stage through the C ABI: the kernel that the launch took, state, sums and next state as bytes."""
+def run_stage(m, start, sums, bits, first, last, max_ctas, vertices=None, tiles=None):
+    """One stage through the C ABI: the kernel that the launch took, state, sums and next state as bytes.  ``tiles``: takes the items of
+    the plan's tiles."""
     nc, ne, V = m["h"].numel(), m["src"].numel(), m["h"].dtype
     ro = torch.searchsorted(m["dst"], torch.arange(nc + 1, dtype=torch.int32, device="cuda")).to(torch.int32 if bits == 32 else torch.int64)
     walls = torch.searchsorted(m["bcells"], torch.arange(0, nc + 32, 32, dtype=torch.int32, device="cuda")).to(torch.int32)
@@ -131,12 +132,14 @@ def run_stage(m, start, sums, bits, first, last, max_ctas, vertices=None):
     launch.launch()
     kernel = load_library().flexspmv_debug_last_kernel()
     ext.check()
+    if tiles is not None:
+        tiles.append(int(launch._keep[-1][:256].cpu().numpy().view(np.int32)[10]))
     assert all(torch.equal(a, b) for a, b in zip(stage, start))
     return kernel, [t.cpu().numpy().tobytes() for t in state + acc + out]
 
 
-def stage_inputs(dtype, split_walls):
-    m = mesh_of(64, dtype, split_walls)
+def stage_inputs(dtype, split_walls, n=64):
+    m = mesh_of(n, dtype, split_walls)
     g = torch.Generator(device="cuda")
     g.manual_seed(11)
     rand = lambda: torch.rand(m["h"].numel(), generator=g, device="cuda", dtype=m["h"].dtype)
@@ -166,3 +169,37 @@ def test_a_second_cell_a_thread_against_a_second_tile(dtype, max_ctas, kernel):
     m, start, sums = stage_inputs(dtype, False)
     taken, got = run_stage(m, start, sums, 32, 0.0, 0.0, max_ctas)
     assert taken == kernel and got == run_stage(m, start, sums, 32, 0.0, 0.0, 1)[1]
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("split_walls", [False, "everywhere"])
+def test_stages_in_large_tiles(bits, split_walls):
+    """fp64 on 231 200 cells: large tiles, in a CTA's own run and going round the CTAs one by one, against the usual ones (a descriptor that names
+    the CTAs)."""
+    m, start, sums = stage_inputs(np.float64, split_walls, 340)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for first, last in ((1.0, 0.0), (0.0, 0.0), (0.0, 1.0)):
+        results, tiles = [], []
+        for max_ctas, vertices, kernel in ((0, None, TILE), (0, 1 << 27, ROUNDS), (3 * sms, None, TILE), (3 * sms, 1 << 27, TILE)):
+            taken, got = run_stage(m, start, sums, bits, first, last, max_ctas, vertices, tiles)
+            assert taken == kernel
+            results.append(got)
+        assert min(tiles[:2]) > 2 * max(tiles[2:])
+        assert all(r == results[0] for r in results[1:]), (first, last)
+
+
+@pytest.mark.parametrize("split_walls", [False, "everywhere"])
+def test_a_step_in_large_tiles_that_go_round(split_walls):
+    """460 800 cells, whose gathered states are beyond 10 MB: the kernel that large meshes take, against three launches a stage."""
+    a, b = mesh_of(480, np.float64, split_walls), mesh_of(480, np.float64, split_walls)
+    fused = ShallowWaterStep(a, dt=1e-5)
+    apart = ShallowWaterStep(b, dt=1e-5, delta_ext=load_builtin("swe_delta"), boundary_ext=load_builtin("swe_boundary"))
+    assert fused._fused is not None and fused._step is None and apart._fused is None
+    for _ in range(2):
+        fused.forward()
+        assert load_library().flexspmv_debug_last_kernel() == ROUNDS
+        apart.forward()
+    assert int(fused._fused[0]._keep[-1][:256].cpu().numpy().view(np.int32)[10]) > 2000          # items a tile; 765 in the usual ones
+    fused.check()
+    for name in ("h", "uh", "vh"):
+        assert torch.isfinite(a[name]).all() and torch.equal(a[name], b[name]), name

@@ -236,3 +236,35 @@ def test_a_first_state_of_its_own(dtype):
         results.append(x)
     for a, b in zip(*results):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [60, 200])      # CTAs of which an SM holds two, and one
+@pytest.mark.parametrize("captured", [False, True])
+def test_two_models_on_two_streams(n, captured):
+    """Whole-step launches of two models that meet on the chip: each waits for room for all of its CTAs, none for the other's."""
+    meshes = [mesh_of(n, np.float64, True) for _ in range(3)]
+    meshes[1]["h"] += 0.01
+    start = {k: meshes[1][k].clone() for k in STATE}
+    models = [ShallowWaterStep(m, dt=1e-5) for m in meshes[:2]]
+    assert all(model._step is not None for model in models)
+    if captured:
+        for model in models:
+            model.capture()
+    streams = [torch.cuda.Stream() for _ in models]
+    torch.cuda.synchronize()
+    for _ in range(40):
+        for model, stream in zip(models, streams):
+            with torch.cuda.stream(stream):
+                model.replay() if captured else model.forward()
+    for model in models:
+        model.check()
+    alone = ShallowWaterStep(meshes[2], dt=1e-5)
+    for m, state in ((meshes[0], None), (meshes[1], start)):
+        if state is not None:
+            for k in STATE:
+                meshes[2][k].copy_(state[k])
+        for _ in range(40):
+            alone.forward()
+        torch.cuda.synchronize()
+        for k in STATE:
+            assert torch.isfinite(m[k]).all() and torch.equal(m[k], meshes[2][k]), k
