@@ -91,13 +91,13 @@ _CHECK_EVERY_CALL = os.environ.get("FLEXSPMV_CHECK_STATUS", "0") == "1"
 
 class _Plan:
     """One planned workspace: the scratch tensor, its size, the tensors whose addresses it depends on, and
-    the page-locked int the kernels copy their error status to."""
+    the page-locked ints, to the first of which the kernels copy their error status."""
     __slots__ = ("ws", "nbytes", "keep", "flag", "_flag_view", "desc", "ws_ptr")
 
     def __init__(self, ws, nbytes, keep, desc):
         self.ws, self.nbytes, self.keep = ws, nbytes, keep
         self.desc, self.ws_ptr = desc, ws.data_ptr()
-        self.flag = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.flag = torch.zeros(2, dtype=torch.int32).pin_memory()          # the status, and what _longest_row reads back
         self._flag_view = self.flag.numpy()
 
     def status(self) -> int:
@@ -304,11 +304,14 @@ class GraphExtension:
         return plan
 
     def _longest_row(self, plan: "_Plan") -> int:
-        out = torch.empty(1, dtype=torch.int32, device=plan.ws.device)
+        """Part of the first call on a matrix: one copy to page-locked memory and a wait for the stream, 25 us (through a device tensor and
+        its ``item`` 40; with the first launch enqueued in front of the wait, and again where the tiles turn out to be others, 23)."""
+        stream = torch.cuda.current_stream(plan.ws.device)
         self.lib.flexspmv_workspace_longest_row.restype = ctypes.c_int
-        check(self.lib, self.lib.flexspmv_workspace_longest_row(ctypes.c_void_p(plan.ws_ptr), ctypes.c_void_p(out.data_ptr()), _stream_ptr()),
-              "workspace_longest_row")
-        return int(out.item())
+        check(self.lib, self.lib.flexspmv_workspace_longest_row(ctypes.c_void_p(plan.ws_ptr), ctypes.c_void_p(plan.flag.data_ptr() + 4),
+                                                                ctypes.c_void_p(stream.cuda_stream)), "workspace_longest_row")
+        stream.synchronize()
+        return int(plan._flag_view[1])
 
     def _plan_once(self, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device, indices: Sequence[torch.Tensor]) -> "_Plan":
         nbytes = ctypes.c_size_t()
