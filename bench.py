@@ -15,7 +15,7 @@ One JSON line is printed by rank 0.  At N = 1 it also carries the per-configurat
 four single-GPU configurations (kernel-only, warm and with L2 flushed between launches) and the CPU
 baseline: the reference's own generated CPU operator (OmpMergeSystem, compiled from the reference's
 sources into oracle/_ref) timed on a bounded slab of the same matrix on the host cores.
-`--impl reference` times only that CPU operator.
+`--impl reference` times only that CPU operator, and says so where it has not been built.
 """
 from __future__ import annotations
 
@@ -211,6 +211,11 @@ def cpu_reference(grid: int, steps: int, warmup: int, planes=None) -> dict:
 def run_reference(args) -> None:
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    from oracle import ref_run
+    if not ref_run.available("spmv"):                            # (the restatement of its operator is no reference)
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's compiled operator (oracle/_ref) is not here, and its sources are needed to build it"}),
+              flush=True)
         return
     steps, warmup = max(1, args.steps), max(args.warmup, 3)      # exactly the K and W of the CUDA arm (0.15 s per call)
     r = cpu_reference(args.grid, steps, warmup, planes=args.cpu_planes)

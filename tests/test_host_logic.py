@@ -286,3 +286,16 @@ def test_a_plan_is_asked_for_the_longest_row(given, uses, longest, planned, desc
     made.clear()
     plan = ext._make_plan(syms, lambda n: Desc(10, 20, 10, 32, 0, 0, n << 8), None, None)
     assert made == [given or 0] and plan.desc.reserved >> 8 == (given or 0)
+
+
+def test_the_reference_arm_times_no_restatement():
+    import json
+    import subprocess
+    import sys
+    from oracle import ref_run
+    if ref_run.available("spmv"):
+        pytest.skip("the reference's operator is here")
+    bench = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "bench.py")
+    run = subprocess.run([sys.executable, bench, "--impl", "reference", "--grid", "16", "--steps", "1", "--warmup", "3"], capture_output=True, text=True)
+    line = json.loads(run.stdout.strip().splitlines()[-1])
+    assert run.returncode == 0 and line["impl"] == "reference" and line["unavailable"] and "value" not in line
