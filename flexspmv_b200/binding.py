@@ -291,7 +291,7 @@ class GraphExtension:
         """A plan for ``described(longest)``, the descriptor that names the longest row.  Where its tiles go by that (bit 0 of
         ``uses_longest_row``), they are those of whole rows until the plan says that it has none."""
         if self.longest_row is not None:
-            return self._plan_once(syms, described(int(self.longest_row)), ro, device, indices)
+            return self._plan_once(syms, described(self.longest_row if 0 < self.longest_row <= 32 else 0), ro, device, indices)
         unknown = described(0)
         by_row = syms.uses_longest_row(ctypes.byref(unknown))
         if not by_row or torch.cuda.is_current_stream_capturing():

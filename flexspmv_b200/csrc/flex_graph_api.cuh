@@ -73,9 +73,11 @@ struct GraphApi {
     return false;
   }
   // Launches of more than a tile for each SM, of rows about as short as the configuration was made for, run one large CTA an SM
-  // (CfgBig), unless the launch is a small one.  The row-mode loop is bound by what an SM has in flight: its 24 warps at the 80
-  // registers of one CTA of 768 threads spill nothing (three CTAs of 288: 72 registers, 48 - 156 bytes), share one stage of a group
-  // of 32 rows for every warp, and the one producer's book-keeping is per 735 rows instead of 191 or 255.  us, CfgBig / Cfg:
+  // (CfgBig), unless the launch is a small one.  The row-mode loop is bound by what an SM has in flight: its 24 warps in
+  // one CTA of 768 threads have 80 registers each (three CTAs of 288: 72; bytes spilled there and here, the stage of the shallow-water step 48 and 0,
+  // swe_delta 60 and 16, Rusanov fp64 68 and 28 - 32, spring-mass fp64 in 56 and 72 registers 88 and 0), share one stage of a group
+  // of 32 rows for every warp, and the one producer's book-keeping is per 735 rows instead of 191 or 255.  us, CfgBig / Cfg (steps: one model
+  // replayed):
   //   shallow-water step fp64  260^2 45.0 / 49.4, 310^2 52.8 / 66.7, 400^2 78.0 / 88.3, 520^2 102.9 / 121.4, 800^2 221 / 248, 1024^2 332 / 368, 1200^2
   //                            455 / 503; 200^2, a small launch there: 32.8 / 28.4
   //   Rusanov fp64             400^2 15.3 / 15.6, 450^2 18.7 / 19.8, 520^2 23.4 / 24.6, 800^2 48.0 / 50.0, 1024^2 74.0 / 76.3, 1200^2 100 / 106
@@ -84,10 +86,9 @@ struct GraphApi {
   //   Rusanov fp32             450^2 11.4 / 12.3, 520^2 14.1 / 15.8, 800^2 29.4 / 32.9, 1024^2 45.8 / 48.9, 1200^2 59.3 / 64.0
   // A tile has to hold about a row a thread (7 to 11 for ten), or warps wait for a stage, or go round it twice.  8 M items: rows of 8 Rusanov fp64
   // 116 / 103, fp32 59.4 / 56.8, swe_delta fp64 102 / 98; of 6 81.8 / 85.0, 47.7 / 46.4, 68.9 / 76.9; of 4 76.7 / 83.6, 45.4 / 46.4, 64.9 / 71.8; of 1 - 7
-  // 103.8 / 114.4, 59.4 / 67.3, 77.6 / 89.8; of 2 76.6 / 81.8, 47.7 / 49.2, 70.6 / 65.4 (3 M items: 32.9 / 36.7, 20.7 / 20.1, 30.4 / 28.4); of 3, one of them of 40
-  // (not whole rows) 98.0 / 104.3, 64.6 / 67.5, 77.2 / 94.1 (1 M items, swe_delta: 21.8 / 21.1).
+  // 103.8 / 114.4, 59.4 / 67.3, 77.6 / 89.8; of 2 76.6 / 81.8, 47.7 / 49.2, 70.6 / 65.4 (3 M items: 32.9 / 36.7, 20.7 / 20.1, 30.4 / 28.4).
   // Spring-mass fp32, 9 M items: rows of 8 31.3 / 42.3, of 4 - 12 46.7 / 52.4, of 9 38.6 / 36.5 (three words for a row, which single indices read
-  // without conflicts): 8.5 rows for ten threads at least; one row of 40 among rows of 8 50.9 / 46.9, fp64 94.4 / 98.1.
+  // without conflicts): 8.5 rows for ten threads at least.
   // So a row of more than kWholeRowMax edges costs a launch far more there (the loop with carries, one barrier for 24 warps), and nothing in the
   // description tells: a caller who has seen the plan names the longest row (FLEXSPMV_LONGEST_ROW), and others get the usual configuration.  Units
   // with an epilogue take plans of whole rows only.  us, CfgBig / Cfg, without whole rows, columns within 300 rows: one row in 1000 of 40 edges among rows of 3, 8 M
@@ -109,8 +110,8 @@ struct GraphApi {
   // they begin in many banks, and lose where they do not: of 18 18.4 / 24.1, 26.3 / 29.0, of 20 21.7 / 22.4, 31.4 / 30.1 (3 M items fp32 9.4 / 8.8), of 16 42.4 / 40.7, 64.5 / 63.8.
   static constexpr int kBigRowEdges = 21;
   static int longest_row(const flexspmv_desc* d) {
-    const int n = (d->reserved >> 8) & 63;
-    return n <= kWholeRowMax ? n : 0;
+    const unsigned n = (unsigned)d->reserved >> 8;
+    return n <= (unsigned)kWholeRowMax ? (int)n : 0;
   }
   static int uses_longest_row(const flexspmv_desc* d) {
     if constexpr (G::kHasReducer) {

@@ -90,9 +90,9 @@ typedef struct flexspmv_desc {
 
 /*
  * The longest row (no reference counterpart).  A caller who knows that the matrix has no row of more than n edges, 1 <= n <= 32, and that
- * its tiles hold whole rows, names n in the descriptor (the same for workspace_bytes, plan and launch).  Launches of graphs and sizes for
- * which flexspmv_<graph>_uses_longest_row is not 0 then take larger tiles (bit 0 of its answer), which are faster on whole rows
- * of about one length, and take up to twice as long on others, or take rows of four to seven edges in one round of gathers (bit 1).  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
+ * its tiles hold whole rows, names n in the descriptor (the same for workspace_bytes, plan and launch).  Where
+ * flexspmv_<graph>_uses_longest_row is not 0, launches then take larger tiles (bit 0 of its answer), which are faster on whole rows of about
+ * one length and take up to twice as long on others, or rows of five to seven edges in one round of gathers (bit 1).  Plan with FLEXSPMV_LONGEST_ROW(32), ask flexspmv_workspace_longest_row for n, and name it in
  * later launches; where it says 0, launch without, and where bit 0 is set plan without before that.  Results of launches on whole rows are the same bits in either
  * form.
  */
