@@ -176,7 +176,7 @@ TUNED_CONFIGS = {
 # batch in the loop over whole rows]).  Row-mode graphs: one large CTA an SM on short rows.  They are picked by what a graph moves and
 # computes, whatever its name: (widths of the edge tensors, of the records gathered by edge, of those gathered by row, sums a row), and as
 # measured with (map operations an edge, by component; divisions, pow, exp and norm among them; value bytes).  A tile of 4 items a thread is
-# a row of three edges a thread, less one item each.  us on meshes of 1024^2 squares, CTAs an SM x warps: the shallow-water step 3 x 9 368,
+# a row of three edges a thread, less one item each.  us on meshes of 1024^2 squares, CTAs an SM x warps: the shallow-water step (one model replayed) 3 x 9 368,
 # 1 x 24 332 (tiles of 3 items a thread 367, of 5 370), 1 x 28 367, 2 x 12 363, 1 x 20 363; Rusanov fp64 3 x 9 76.3, 1 x 24 74.0, 1 x 28 77.0,
 # 2 x 12 76.2; fp32 4 x 9 48.9, 1 x 32 45.8, 1 x 28 48.0, 1 x 24 52.0.  Lattices of eight edges a particle, 1024^2: fp32 992 x 8 35.9 (x 9
 # 36.2), fp64 736 x 7 62.0 (x 8 63.8, x 9 62.1).

@@ -6,7 +6,8 @@
 // wall: per cell 16 bytes of memory traffic a sum, 32 a wall sum and two launches a stage less.
 // Bound by the latency of the gathers and of the cell's own records (23 warps per SM at 80 registers, 57 % of DRAM); the
 // producer warp therefore asks for those records in L2 when it stages a tile (prefetch_rows: 510 -> 454 us a step).  A step of
-// the model on 2 097 152 cells, fp64: 606 us as 12 launches, 333 us as 4 (1024 x 1024 squares; 369 in three CTAs of 9 warps, GraphApi::use_big);
+// the model on 2 097 152 cells, fp64: 606 us as 12 launches, 329 - 333 us as 4 (1024 x 1024 squares, one model replayed, three in turn 348; 369 in three CTAs of 9
+// warps, GraphApi::use_big);
 // on 20 402 cells 57.4 -> 23.8 us (30.8 with stages), as one launch (flex_swe_step.cuh) 20.5.
 // fp64 batches of 1 / 2 edges per thread at 3 CTAs per SM, 3 at 2, 1 at 4 (before the prefetch): 510 / 546 / 625 / 555 us;
 // fp32, 4 CTAs per SM, batches of 4 / 1: 327 / 286 us.

@@ -46,7 +46,7 @@ struct TileCfg {
   static constexpr int kBatch = BATCH_;   // edges of one row whose gathers are in flight together (short-row tiles)
   static constexpr int kRowBatch = ROW_BATCH_;   // the same in the loop over whole rows
   // consecutive tiles of a CTA where whole rows go round the CTAs (TileKernelArgs::rounds); large tiles go round one by one: 1024^2
-  // shallow-water step 333 us, in runs of two 336, of four 353; Rusanov 74.0, 76.6, 77.7
+  // shallow-water step (one model replayed) 333 us, in runs of two 336, of four 353; Rusanov 74.0, 76.6, 77.7
   static constexpr bool kLarge = kTile >= 2560;
   static constexpr int kTileRun = kLarge ? 1 : 4;
 };
