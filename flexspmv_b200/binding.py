@@ -433,6 +433,12 @@ class GraphExtension:
         launch._fn = _LAUNCH((syms.name("step"), self.lib))
         return launch
 
+    def longest_row_of(self, launch: "PreparedLaunch") -> int:
+        """The edges of the longest row of a prepared problem whose plan holds whole rows (include/flexspmv.h,
+        flexspmv_workspace_longest_row), else 0.  Waits for the plan."""
+        with torch.cuda.device(launch._device):
+            return self._longest_row(launch._plan)
+
     def device_status(self, dtype: torch.dtype, row_end_offsets: Optional[torch.Tensor] = None) -> int:
         """Reads back the status word of the most recently used workspace (synchronises)."""
         if not self._plans:
@@ -512,9 +518,13 @@ class PreparedLaunch:
 
     __call__ = launch
 
+    def failed(self) -> bool:
+        """Whether a kernel has given up on this object's workspace, as far as the host has been told (one read of host
+        memory, no synchronisation)."""
+        return self._plan._flag_view[0] != 0
+
     def raise_if_failed(self, what: str = "launch") -> None:
-        """Raises FlexSpmvError where a kernel has given up on this object's workspace, as far as the host has been told
-        (one read of host memory, no synchronisation)."""
+        """Raises FlexSpmvError where ``failed()``."""
         _raise_if_failed(self.ext.lib, self._plan, what)
 
 

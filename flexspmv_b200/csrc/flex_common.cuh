@@ -59,7 +59,7 @@ struct WorkspaceHeader {
                                // while a test withholds a stage (not 0: a small launch runs its loop with stages)
   int32_t longest_row;         // where whole_rows is 1 and the rows suit the plan's tiles (RowLoopRule): the edges of the longest one (else 0
                                // once the plan is complete)
-  uint64_t step_barrier;       // CTAs that have come to a barrier of a whole-step launch (flex_swe_step.cuh), over all launches
+  uint64_t step_barrier;       // the barriers of whole-step launches (flex_swe_step.cuh), over all launches
   uint64_t lane_slots;         // row_slots without the lanes that have no row
   char pad[256 - 4 * 4 - 3 * 8 - 2 * 4 - 4 * 8 - 8 * 4 - 2 * 8 - 2 * 4 - 8 - 8 - 8 * 4 - 4 - 4 - 8 - 8];
 };

@@ -99,11 +99,14 @@ __device__ __noinline__ WallTerms<V> swe_step_wall(const V* h, const int* wall_c
 }
 
 // A barrier of the grid in two halves: what the CTA's threads wrote before step_arrive is seen by every CTA behind its step_wait.  One
-// counter in the header that only grows; every launch adds a whole number of grids to it, and the barrier is open at `all`.  The wait
+// counter in the header that only grows, by kStepBarrier a barrier whatever the launch's grid (the first CTA counts for those that it
+// does not have), so that launches of different grids may follow one another on a workspace; the barrier is open at `all`.  The wait
 // is bounded (a second) and ends in FLEXSPMV_ERR_TIMEOUT.
+constexpr uint64_t kStepBarrier = 1u << 20;
 __device__ __forceinline__ void step_arrive(WorkspaceHeader* h, bool withhold) {
   __syncthreads();
-  if (threadIdx.x == 0 && !withhold) asm volatile("fence.acq_rel.gpu;\n\tred.release.gpu.global.add.u64 [%0], 1;" ::"l"(&h->step_barrier) : "memory");
+  const uint64_t n = blockIdx.x == 0 ? kStepBarrier - (gridDim.x - 1) : 1;
+  if (threadIdx.x == 0 && !withhold) asm volatile("fence.acq_rel.gpu;\n\tred.release.gpu.global.add.u64 [%0], %1;" ::"l"(&h->step_barrier), "l"(n) : "memory");
 }
 __device__ __forceinline__ bool step_wait(WorkspaceHeader* h, uint64_t all, int* s_ok) {
   if (threadIdx.x == 0) {
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) flex_swe_step_kernel(const typ
   for (int i = tid; i < cells; i += threads) s_wall[i] = -1;
   if (__syncthreads_or(h->status != 0)) return;    // an earlier launch gave up: its counter says nothing
   // as this CTA has not come to a barrier yet, fewer than all have come to the first one
-  uint64_t all = count / gridDim.x * gridDim.x;
+  uint64_t all = count / kStepBarrier * kStepBarrier;
   const int kept = (int)(e_last - e_first < a.edges ? e_last - e_first : a.edges);
   for (int j = j_first + tid; j < j_last; j += threads) {
     const int cell = __ldg(params.wall_cell + j), before = j > j_first ? __ldg(params.wall_cell + j - 1) : -1;
@@ -193,7 +196,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) flex_swe_step_kernel(const typ
       p.h = even ? st.state[1][0] : st.state[0][0];
       p.uh = even ? st.state[1][1] : st.state[0][1];
       p.vh = even ? st.state[1][2] : st.state[0][2];
-      all += gridDim.x;
+      all += kStepBarrier;
       step_arrive(a.header, withhold);
       walls(p.h);                     // of the thread's own cells, while the other CTAs arrive
       if (!step_wait(a.header, all, &s_ok)) return;

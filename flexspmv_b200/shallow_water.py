@@ -112,20 +112,20 @@ class ShallowWaterStep:
         # meshes that fit the chip in even shares: the four stages in one launch (csrc/flex_swe_step.cuh)
         values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [self._coef]
         step = ext.prepare_step(values, [m["src"], m["dst"]], self.ro, self.stage + other, self.nc, self.ne, self.nc)
-        if step is not None and self._shares_are_even(step.rows_a_cta):
+        if step is not None and self._shares_are_even(step.rows_a_cta, ext.longest_row_of(step)):
             self._step = step
         return launches
 
-    def _shares_are_even(self, cells: int) -> bool:
-        """Whether the whole-step launch is the faster form with ``cells`` consecutive cells a CTA (one look at the row offsets when
-        the model is bound).  Its stages wait for the CTA with the most edges, and a cell's edges are a chain of gathers that takes
+    def _shares_are_even(self, cells: int, longest: int) -> bool:
+        """Whether the whole-step launch is the faster form with ``cells`` consecutive cells a CTA and ``longest`` edges in a cell at most (one
+        look at the row offsets when the model is bound).  Its stages wait for the CTA with the most edges, and a cell's edges are a chain of gathers that takes
         0.23 us an edge and step of each stage, 0.14 in the four launches; with more cells a CTA there is other work to hide it.
         us a step, one launch / four, fp64, n x n squares: 330^2 with 1000 cells of 25 edges side by side 457 / 92, 700 of 8 (the
         largest share 1.8 times the mean) 64 / 60, half of the cells with 6 (1.3) 39 / 53 on 260^2; one cell of 25 on 64^2 (64 a CTA)
         41 / 37, on 101^2 (160) 37 / 35, on 160^2 (352) 37 / 43; of 12 on 64^2 29 / 25, on 101^2 25 / 29; six cells of 5 on 40^2 (32)
         25 / 23.  fp32 alike (330^2 174 / 56; one of 25 on 64^2 35 / 29)."""
-        ends = self.ro[torch.arange(0, self.nc + cells, cells, device=self.ro.device).clamp_(max=self.nc)]
-        most, longest = torch.stack([(ends[1:] - ends[:-1]).max(), (self.ro[1:] - self.ro[:-1]).max()]).tolist()
+        begins = self.ro[:self.nc:cells].tolist()
+        most = max(e - b for b, e in zip(begins, begins[1:] + [self.ne]))
         return shares_are_even(cells, self.nc, self.ne, most, longest)
 
     def _bind(self, h, uh, vh):
@@ -195,14 +195,11 @@ class ShallowWaterStep:
         self._graph.replay()
 
     # -- errors --------------------------------------------------------------------------------------------
-    def _bound_launches(self):
-        if self._fused is not None:
-            return self._fused if self._step is None else [self._step] + self._fused
-        return list(self._on_state + self._on_stage)
-
     def _raise_if_failed(self, what: str) -> None:
-        for launch in self._bound_launches():
-            launch.raise_if_failed(what)
+        launches = self._fused if self._fused is not None else self._on_state + self._on_stage
+        for launch in launches:             # (those of one plan share its status, the whole step's launch among them)
+            if launch.failed():
+                launch.raise_if_failed(what)
 
     def check(self) -> None:
         """Waits for the steps enqueued so far and raises FlexSpmvError if one of them gave up on the device (a bounded wait

@@ -205,8 +205,7 @@ def test_the_descriptor_caps_the_ctas(max_ctas):
     for step in (capped, usual):
         step.launch()
     ext.check()
-    arrivals = int(capped._keep[-1][:256].cpu().numpy().view(np.uint64)[24])          # step_barrier of struct WorkspaceHeader
-    assert arrivals == 3 * min(max_ctas, -(-2 * 30 * 30 // 32), sms())
+    assert capped.rows_a_cta == -(-(-(-1800 // min(max_ctas, 57, sms()))) // 32) * 32
     for k in STATE:
         assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k
 
@@ -268,3 +267,16 @@ def test_two_models_on_two_streams(n, captured):
         torch.cuda.synchronize()
         for k in STATE:
             assert torch.isfinite(m[k]).all() and torch.equal(m[k], meshes[2][k]), k
+
+
+def test_launches_of_different_grids_on_one_workspace():
+    """A descriptor's max_ctas may change from launch to launch: the barrier's counter, which stays in the workspace, does not know grids."""
+    a, b = mesh_of(30, np.float64, True), mesh_of(30, np.float64, True)
+    (ext, changing), (_, usual) = bind(a, 32), bind(b, 32)
+    for max_ctas in (5, 0, 33, 1, 100, 0, 7, 7, 0):
+        changing._desc.max_ctas = max_ctas
+        changing.launch()
+        usual.launch()
+        ext.check()
+    for k in STATE:
+        assert torch.isfinite(a[k]).all() and torch.equal(a[k], b[k]), k

@@ -44,7 +44,7 @@ def test_replay_raises_where_an_earlier_step_failed(form):
     else:
         step._fused = [bare_launch(plan) for _ in range(4)]
         if form == "one":
-            step._step = bare_launch(plan)
+            step._step = bare_launch(plan)          # a launch on the four ones' plan
     step.replay()
     assert step._graph.replays == 1
     plan._flag_view[0] = -6
