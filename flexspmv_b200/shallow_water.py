@@ -107,12 +107,14 @@ class ShallowWaterStep:
             dst = other if k % 2 else self.stage          # the last stage writes the state itself
             values = [m["alpha"], m["sx"], m["sy"]] + src + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [self._coef[k]]
             launches.append(ext.prepare(values, [m["src"], m["dst"]], self.ro, dst, self.nc, self.ne, self.nc))
-            if k == 0 and not ext.planned_whole_rows():
-                return None
+            if k == 0:
+                longest = ext.longest_row_of(launches[0])
+                if longest == 0 and not ext.planned_whole_rows():       # (a mesh without edges has whole rows, too)
+                    return None
         # meshes that fit the chip in even shares: the four stages in one launch (csrc/flex_swe_step.cuh)
         values = [m["alpha"], m["sx"], m["sy"]] + state + [m["area"], m["bsx"], m["bsy"], self._wall_start, cells] + state + self.acc + [self._coef]
         step = ext.prepare_step(values, [m["src"], m["dst"]], self.ro, self.stage + other, self.nc, self.ne, self.nc)
-        if step is not None and self._shares_are_even(step.rows_a_cta, ext.longest_row_of(step)):
+        if step is not None and self._shares_are_even(step.rows_a_cta, longest):
             self._step = step
         return launches
 
