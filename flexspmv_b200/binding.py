@@ -30,6 +30,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import time
 from collections import OrderedDict
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -97,7 +98,7 @@ class _Plan:
     def __init__(self, ws, nbytes, keep, desc):
         self.ws, self.nbytes, self.keep = ws, nbytes, keep
         self.desc, self.ws_ptr = desc, ws.data_ptr()
-        self.flag = torch.zeros(2, dtype=torch.int32).pin_memory()          # the status, and what _longest_row reads back
+        self.flag = torch.zeros(2, dtype=torch.int32).pin_memory()          # the status, and the longest row once the plan is complete
         self._flag_view = self.flag.numpy()
 
     def status(self) -> int:
@@ -304,14 +305,15 @@ class GraphExtension:
         return plan
 
     def _longest_row(self, plan: "_Plan") -> int:
-        """Part of the first call on a matrix: one copy to page-locked memory and a wait for the stream, 25 us (through a device tensor and
-        its ``item`` 40; with the first launch enqueued in front of the wait, and again where the tiles turn out to be others, 23)."""
-        stream = torch.cuda.current_stream(plan.ws.device)
-        self.lib.flexspmv_workspace_longest_row.restype = ctypes.c_int
-        check(self.lib, self.lib.flexspmv_workspace_longest_row(ctypes.c_void_p(plan.ws_ptr), ctypes.c_void_p(plan.flag.data_ptr() + 4),
-                                                                ctypes.c_void_p(stream.cuda_stream)), "workspace_longest_row")
-        stream.synchronize()
-        return int(plan._flag_view[1])
+        """Part of the first call on a matrix: the plan's last kernel leaves the word in page-locked memory, and the host looks at it until it
+        has changed (15 us of a first call; with a copy and a wait for the stream 25, with a device tensor and its ``item`` 40); behind much other work on the
+        stream it waits for that instead."""
+        view, until = plan._flag_view, time.perf_counter() + 100e-6
+        while view[1] < 0 and time.perf_counter() < until:
+            pass
+        if view[1] < 0:
+            torch.cuda.current_stream(plan.ws.device).synchronize()
+        return int(view[1])
 
     def _plan_once(self, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device, indices: Sequence[torch.Tensor]) -> "_Plan":
         nbytes = ctypes.c_size_t()
@@ -327,9 +329,9 @@ class GraphExtension:
                                               ctypes.c_size_t(nbytes.value), _stream_ptr()), "plan_windows")
         # keep the row-offset tensor alive so its address cannot be recycled under a cached plan
         plan = _Plan(ws, nbytes.value, (ro, tuple(indices) if (desc.reserved & 1) else None), desc)
-        check(self.lib, self.lib.flexspmv_workspace_status_mirror(ctypes.c_void_p(ws.data_ptr()),
-                                                                  ctypes.c_void_p(plan.flag.data_ptr()), _stream_ptr()),
-              "workspace_status_mirror")
+        plan._flag_view[1] = -1
+        check(self.lib, self.lib.flexspmv_workspace_mirrors(ctypes.c_void_p(ws.data_ptr()), ctypes.c_void_p(plan.flag.data_ptr()),
+                                                            ctypes.c_void_p(plan.flag.data_ptr() + 4), _stream_ptr()), "workspace_mirrors")
         self.launches += self.lib.flexspmv_plan_launches() - before
         return plan
 

@@ -340,10 +340,12 @@ __global__ void debug_withhold_kernel(WorkspaceHeader* h, uint32_t first_tile_pl
 __global__ void window_ready_kernel(WorkspaceHeader* h) {
   if (threadIdx.x == 0 && blockIdx.x == 0) h->win_ready = 1;
 }
-__global__ void status_mirror_kernel(WorkspaceHeader* h, int32_t* mirror) {
+__global__ void status_mirror_kernel(WorkspaceHeader* h, int32_t* mirror, int32_t* longest_row) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     h->status_mirror = reinterpret_cast<uint64_t>(mirror);
-    if (mirror) { *reinterpret_cast<volatile int32_t*>(mirror) = h->status; __threadfence_system(); }
+    if (mirror) *reinterpret_cast<volatile int32_t*>(mirror) = h->status;
+    if (longest_row) *reinterpret_cast<volatile int32_t*>(longest_row) = h->longest_row;
+    __threadfence_system();
   }
 }
 int window_ready_launch(void* ws, cudaStream_t st) {
@@ -711,18 +713,23 @@ int flexspmv_debug_last_kernel(void) { return flex::last_kernel; }
 
 int flexspmv_debug_last_row_batch(void) { return flex::last_row_batch; }
 
-int flexspmv_workspace_status_mirror(void* d_workspace, int32_t* pinned_host_status, void* stream) {
+int flexspmv_workspace_mirrors(void* d_workspace, int32_t* pinned_status, int32_t* pinned_longest_row, void* stream) {
   if (!d_workspace) return FLEXSPMV_ERR_WORKSPACE;
-  int32_t* alias = nullptr;
-  if (pinned_host_status) {
-    void* dptr = nullptr;
-    cudaError_t e = cudaHostGetDevicePointer(&dptr, pinned_host_status, 0);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
-    alias = static_cast<int32_t*>(dptr);
-  }
+  void* alias[2] = {nullptr, nullptr};
+  int32_t* const host[2] = {pinned_status, pinned_longest_row};
+  for (int i = 0; i < 2; ++i)
+    if (host[i]) {
+      cudaError_t e = cudaHostGetDevicePointer(&alias[i], host[i], 0);
+      if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+    }
   ++flex::plan_launches;
-  flex::status_mirror_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<flex::WorkspaceHeader*>(d_workspace), alias);
+  flex::status_mirror_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<flex::WorkspaceHeader*>(d_workspace),
+                                                                             static_cast<int32_t*>(alias[0]), static_cast<int32_t*>(alias[1]));
   return (int)cudaGetLastError();
+}
+
+int flexspmv_workspace_status_mirror(void* d_workspace, int32_t* pinned_host_status, void* stream) {
+  return flexspmv_workspace_mirrors(d_workspace, pinned_host_status, nullptr, stream);
 }
 
 int64_t flexspmv_plan_launches(void) { return flex::plan_launches; }

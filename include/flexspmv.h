@@ -175,6 +175,12 @@ int flexspmv_probe_gather(const int32_t *d_idx, const float *d_vals, const float
 int flexspmv_workspace_status_mirror(void *d_workspace, int32_t *pinned_host_status, void *stream);
 
 /*
+ * The same, and once the plan is complete the number of flexspmv_workspace_longest_row in a second page-locked int (NULL: not wanted): a
+ * host that has put a negative number there waits for it to change, without a copy or a call.
+ */
+int flexspmv_workspace_mirrors(void *d_workspace, int32_t *pinned_status, int32_t *pinned_longest_row, void *stream);
+
+/*
  * Halo plan of a 1-D row-block partition (host only, pure integers): given the world + 1 block
  * boundaries and, per block, the smallest and largest global column its rows reference (for an empty
  * block: row_begin and row_begin - 1), computes for every rank how many vector entries it needs from
@@ -245,7 +251,7 @@ int flexspmv_swe_rk_stage(int32_t value_bytes, const void *const *d_r, const voi
                           void *const *d_stage, double c, double w, int64_t n, int32_t first,
                           int32_t last, void *stream);
 
-/* Kernels that plan, plan_indexed, plan_windows and flexspmv_workspace_status_mirror have enqueued from the calling thread
+/* Kernels that plan, plan_indexed, plan_windows and flexspmv_workspace_mirrors have enqueued from the calling thread
  * since it started; the difference over a call is that call's. */
 int64_t flexspmv_plan_launches(void);
 

@@ -1,12 +1,14 @@
 """The large configuration of the row-mode graphs (GraphApi::use_big): the sizes on both sides of its rule, tiles of equal number
 and of the largest size, both orders of the tiles, plans with and without whole rows -- each against the configuration that a caller
 who names a number of CTAs gets, bit for bit where sums run left to right in both, and against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from flexspmv_b200 import graphs
-from flexspmv_b200.binding import GraphExtension
+from flexspmv_b200.binding import GraphExtension, load_library
 from oracle import ir_eval
 from parity import assert_outputs_match
 from test_gpu_launch_sizes import ROUNDS, default_tile, header_word, launch, run_gpu, with_lengths
@@ -24,7 +26,11 @@ def sms():
 
 def longest_row_of(ext):
     plan = next(reversed(ext._plans.values()))
-    return ext._longest_row(plan)
+    out = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    assert load_library().flexspmv_workspace_longest_row(ctypes.c_void_p(plan.ws_ptr), ctypes.c_void_p(out.data_ptr()), None) == 0
+    torch.cuda.synchronize()
+    assert int(out) == ext._longest_row(plan)
+    return int(out)
 
 
 def small_limit(ir, dtype):
