@@ -313,7 +313,7 @@ class GraphExtension:
             pass
         if view[1] < 0:
             torch.cuda.current_stream(plan.ws.device).synchronize()
-        return int(view[1])
+        return max(int(view[1]), 0)
 
     def _plan_once(self, syms: _Symbols, desc: Desc, ro: Optional[torch.Tensor], device, indices: Sequence[torch.Tensor]) -> "_Plan":
         nbytes = ctypes.c_size_t()
